@@ -127,38 +127,135 @@ __global__ void __launch_bounds__(256) k_adam_quant(const AdamParams p) {
 
 // ---------------------------------------------------------------------------------------------------------------
 // Fast variant of the production configuration (bf16 chain, bf16 qparams and gradient, 3-fold codec, hash dither, group a
-// power of two >= 8): packed bf16x2 reconstruction of the latent weights with the residual decode from a 256-entry table,
-// bf16 roundings as packed conversions (two values per instruction), and everything after Z = w/scale + zero from the
-// 64 KB table of the requantize fast path.  Same results as k_adam_a16w4, bit for bit; a word whose Z leaves the table's
-// range (|Z| >= 64, non-finite) is encoded by the generic chain.
+// power of two >= 8).  Same results as k_adam_quant, bit for bit.  The kernel is bound by instruction issue, not by its
+// 8 bytes per weight, so every step is the cheapest form that provably rounds the same way:
+//   states    decoded from two 256-entry tables per 2048-element block (one entry of each per thread): code -> bf16(m) * beta1
+//             and bf16(s2^2) * beta2, both already rounded.  128-element blocks have too few elements per table and decode
+//             in registers (LUT = false).
+//   sqrt      sqrt.approx (relative error <= 2^-23): the root of an 8-bit significand is at least 2^-19 (relative) away from
+//             every bf16 rounding boundary (the boundary's square has odd quarters, the operand is an integer on that scale),
+//             so the bf16 result is that of the exactly rounded root.
+//   m / d     rcp.approx and one residual correction: the quotient of two 8-bit significands is at least 2^-33 away from
+//             every midpoint of two fp32 numbers, the corrected quotient is 2^-44 off before its rounding.
+//   states    encoded with a quotient q0 from a two-term reciprocal, then one residual correction with RN(1/s): q0 is
+//             within one ulp, which makes the corrected quotient the correctly rounded one (Markstein).
+//   requantize  everything after Z = w/scale + zero from the table of the requantize fast path (int4: a byte per bf16 pattern,
+//             |Z| < 64; int8: two bytes, |Z| < 256); the kernel keeps the two runs of it that can be looked up and puts its other
+//             tables into the gap between them.
+// int4 codes: 50 KB and 256 threads per CTA, four CTAs per SM; int8 codes: 100 KB, so two teams of 256 threads share the tables
+// of a CTA and two CTAs fit.
+// A word whose Z leaves the table's range or is not finite, and every word of a block whose moments are not all finite, is
+// recomputed by the generic chain (adam_word_generic).
 // ---------------------------------------------------------------------------------------------------------------
 constexpr int ADAM_TRES_REPL = 8;
-constexpr int ADAM_FAST_SMEM = ENCZ_TABLE_ENTRIES + 256 * ADAM_TRES_REPL * 4;
+template <int WBITS> struct AdamFast {
+    static constexpr int TEAMS = WBITS == 8 ? 2 : 1;
+    static constexpr int THREADS = TEAMS * 256;
+    static constexpr int MIN_CTAS = 4 / TEAMS;
+    static constexpr int ENTRY = WBITS == 8 ? 2 : 1;                     // bytes per table entry
+    static constexpr int RUN = (WBITS == 8 ? 0x4380 : 0x4280) * ENTRY;   // bf16 patterns of [0, 256) / [0, 64)
+    static constexpr int NEG = 0x8000 * ENTRY;                           // the run of the negative patterns
+    static constexpr int TRES = (RUN + 1023) / 1024 * 1024;              // residual decode table
+    static constexpr int LUT = TRES + 256 * ADAM_TRES_REPL * 4;          // per team: [256] first state, [256] second state
+    static constexpr int RED = LUT + TEAMS * 2 * 256 * 4;                // per team: block extrema of the 8 warps
+    static constexpr int SMEM = NEG + RUN;
+    static constexpr uint32_t Z_LIMIT = WBITS == 8 ? 0x3c803c80u : 0x3d803d80u;    // carries into bit 15 from |Z| = 256 / 64 on
+    static_assert(RED + TEAMS * 64 <= NEG && RUN % 16 == 0, "tables in the gap of the encode table");
+};
 
-__device__ __forceinline__ void rb2(float a, float b, float& ra, float& rbv) {       // bf16 roundings of two values, one conversion
+__device__ __forceinline__ uint32_t pack2(float a, float b) {       // bf16 roundings of two values, one conversion
     const __nv_bfloat162 q = __floats2bfloat162_rn(a, b);
-    const uint32_t u = *reinterpret_cast<const uint32_t*>(&q);
-    ra = __uint_as_float(u << 16); rbv = __uint_as_float(u & 0xffff0000u);
+    return *reinterpret_cast<const uint32_t*>(&q);
+}
+__device__ __forceinline__ float lo2f(uint32_t u) { return __uint_as_float(u << 16); }
+__device__ __forceinline__ float hi2f(uint32_t u) { return __uint_as_float(u & 0xffff0000u); }
+__device__ __forceinline__ __nv_bfloat162 asbf2(uint32_t u) { return *reinterpret_cast<const __nv_bfloat162*>(&u); }
+__device__ __forceinline__ uint32_t asu32(__nv_bfloat162 v) { return *reinterpret_cast<const uint32_t*>(&v); }
+__device__ __forceinline__ uint32_t min2(uint32_t a, uint32_t b) { return asu32(__hmin2(asbf2(a), asbf2(b))); }
+__device__ __forceinline__ uint32_t max2(uint32_t a, uint32_t b) { return asu32(__hmax2(asbf2(a), asbf2(b))); }
+__device__ __forceinline__ float sqrt_approx(float x) { float r; asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+__device__ __forceinline__ float rcp_approx(float x) { float r; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+// a / b for bf16-valued a and b, 2^-64 <= b <= 2^64: see above (a residual of the opposite sign keeps -0 / b = -0)
+__device__ __forceinline__ float div_bf16(float a, float b) {
+    const float y = rcp_approx(b), q = __fmul_rn(a, y);
+    return __fmaf_rn(-__fmaf_rn(q, b, -a), y, q);
+}
+// (scale, its reciprocal as RN(1/s) + remainder) of one 8-bit state block: s = (mx - mn) / 255 + 1e-10
+struct OptScale { float s, r, rl; };
+__device__ __forceinline__ OptScale opt8_scale(float mx, float mn) {
+    const float a = __fsub_rn(mx, mn), r255 = 1.0f / 255.0f;
+    float q = __fmul_rn(a, r255);                                    // a / 255, correctly rounded (below 2^-100 the 1e-10 hides it)
+    q = __fmaf_rn(__fmaf_rn(-q, 255.0f, a), r255, q);
+    q = __fmaf_rn(__fmaf_rn(-q, 255.0f, a), r255, q);
+    OptScale o;
+    o.s = __fadd_rn(q, 1e-10f);
+    o.r = __frcp_rn(o.s);
+    o.rl = __fmul_rn(__fmaf_rn(-o.s, o.r, 1.0f), o.r);
+    return o;
+}
+__device__ __forceinline__ uint32_t opt8_code_bits(float x, float mx, const OptScale& o) {   // code in the low byte
+    const float a = __fsub_rn(mx, x);
+    float q = __fmaf_rn(a, o.r, __fmul_rn(a, o.rl));
+    q = __fmaf_rn(__fmaf_rn(-q, o.s, a), o.r, q);
+    return __float_as_uint(__fadd_rn(q, MAGIC_RNE));                 // 0 <= q <= 255 (1 + 2^-22)
+}
+__device__ __forceinline__ uint32_t opt8_codes4(uint32_t p01, uint32_t p23, float mx, const OptScale& o) {
+    return __byte_perm(__byte_perm(opt8_code_bits(lo2f(p01), mx, o), opt8_code_bits(hi2f(p01), mx, o), 0x0040),
+                       __byte_perm(opt8_code_bits(lo2f(p23), mx, o), opt8_code_bits(hi2f(p23), mx, o), 0x0040), 0x5410);
 }
 
-template <bool USE_RES>
-__global__ void __launch_bounds__(256, 3) k_adam_a16w4_fast(const AdamParams p, const int enc_slot) {
+// One word through the generic chain, from its inputs in memory (nothing of it has been written yet) and the block parameters
+// of its states before (s, t) and after (ns, mx) the step: what k_adam_quant does for it.
+template <int WBITS>
+__device__ __noinline__ void adam_word_generic(const AdamParams& p, const int64_t w, const float s1, const float t1, const float s2, const float t2,
+                                               const float mx1, const float ns1, const float mx2, const float ns2) {
+    const int64_t e0 = w * 8;
+    const int64_t g = p.rq.group_shift >= 0 ? (e0 >> p.rq.group_shift) : (e0 / p.rq.group);
+    const float s = load1(p.rq.scales, p.rq.qp_dtype, g), z = (WBITS == 4) ? load1(p.rq.zeros, p.rq.qp_dtype, g) : 0.0f;
+    float lat[8], m[8], d[8], gr[8];
+    load8(p.grad, p.grad_dtype, e0, gr);
+    latent_load<WBITS, LQ_CODEC_THREEFOLD, true>(p.rq, w, s, z, lat);
+#pragma unroll 1
+    for (int k = 0; k < 8; ++k) {
+        m[k] = rb<true>(__fsub_rn(t1, __fmul_rn((float)p.st1[e0 + k], s1)));
+        const float r2 = __fsub_rn(t2, __fmul_rn((float)p.st2[e0 + k], s2));
+        d[k] = rb<true>(__fmul_rn(r2, r2));
+        adam_moments<true>(p.h, gr[k], m[k], d[k]);
+        lat[k] = adam_apply<true>(p.h, lat[k], m[k], d[k]);
+    }
+    *reinterpret_cast<uint2*>(p.st1 + e0) = opt8_encode8(m, mx1, ns1);
+    *reinterpret_cast<uint2*>(p.st2 + e0) = opt8_encode8(d, mx2, ns2);
+    latent_store<WBITS, LQ_CODEC_THREEFOLD, LQ_DITHER_HASH, true>(p.rq, w, s, z, lat);
+}
+
+// row_magic (int8 codes): ceil(2^64 / words per weight row)
+template <int WBITS, bool USE_RES, bool LUT>
+__global__ void __launch_bounds__(AdamFast<WBITS>::THREADS, AdamFast<WBITS>::MIN_CTAS)
+k_adam_fast(const __grid_constant__ AdamParams p, const int enc_slot, const uint64_t row_magic) {
+    using AF = AdamFast<WBITS>;
+    constexpr bool W8 = WBITS == 8;
     extern __shared__ __align__(16) uint8_t asm_[];
-    uint8_t* encz = asm_;
-    uint32_t* tres = reinterpret_cast<uint32_t*>(asm_ + ENCZ_TABLE_ENTRIES);
-    __shared__ float s_red[4][8];
+    const uint8_t* encz = asm_;
+    const uint16_t* enc8 = reinterpret_cast<const uint16_t*>(asm_);
+    uint32_t* tres = reinterpret_cast<uint32_t*>(asm_ + AF::TRES);
     {
-        const uint4* src = reinterpret_cast<const uint4*>(g_encz_table[enc_slot]);
-        uint4* dst = reinterpret_cast<uint4*>(encz);
-        for (int i = threadIdx.x; i < ENCZ_TABLE_ENTRIES / 16; i += 256) dst[i] = __ldg(src + i);
-        for (int b = threadIdx.x; b < 256; b += 256) {
+        const uint4* src = W8 ? reinterpret_cast<const uint4*>(g_enc8_table[enc_slot]) : reinterpret_cast<const uint4*>(g_encz_table[enc_slot]);
+        uint4* dst = reinterpret_cast<uint4*>(asm_);
+        for (int i = threadIdx.x; i < AF::RUN / 16; i += AF::THREADS) { dst[i] = __ldg(src + i); dst[AF::NEG / 16 + i] = __ldg(src + AF::NEG / 16 + i); }
+        for (int b = threadIdx.x; b < 256; b += AF::THREADS) {
             const uint32_t lo = f32_to_bf16_bits(bf16r(res3_decode((uint32_t)b >> 4, p.rq.dec)));
             const uint32_t hi = f32_to_bf16_bits(bf16r(res3_decode((uint32_t)b & 15u, p.rq.dec)));
             for (int r = 0; r < ADAM_TRES_REPL; ++r) tres[b * ADAM_TRES_REPL + r] = lo | (hi << 16);
         }
     }
     __syncthreads();
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int team = AF::TEAMS == 1 ? 0 : (int)(threadIdx.x >> 8), tid = threadIdx.x & 255, lane = tid & 31, warp = tid >> 5;
+    float* lut = reinterpret_cast<float*>(asm_ + AF::LUT) + team * 512;
+    uint2* red = reinterpret_cast<uint2*>(asm_ + AF::RED) + team * 8;
+    auto team_sync = [&] {
+        if (AF::TEAMS == 1) __syncthreads();
+        else asm volatile("bar.sync %0, 256;" ::"r"(team + 1) : "memory");
+    };
     const uint32_t tres_lane = tid & (ADAM_TRES_REPL - 1);
     const unsigned short* scales = reinterpret_cast<const unsigned short*>(p.rq.scales);
     const unsigned short* zeros = reinterpret_cast<const unsigned short*>(p.rq.zeros);
@@ -166,117 +263,184 @@ __global__ void __launch_bounds__(256, 3) k_adam_a16w4_fast(const AdamParams p, 
     const int gsh = p.rq.group_shift - 3;                     // word index -> group index
     const int osh = p.opt_shift - 3;                          // word index -> optimizer-state block
     const uint32_t c128u = 0x43004300u;
-    for (uint32_t tile = blockIdx.x; tile < (uint32_t)p.n_tiles; tile += gridDim.x) {
+    // the loads of the next tile are in flight while the current one is computed
+    struct In { uint2 q1, q2, pk; uint4 gv; uint32_t rw, sb, zb; float s1, t1, s2, t2; };
+    auto load_in = [&](uint32_t w) -> In {
+        In in;
+        const uint32_t g = W8 ? (uint32_t)__umul64hi((uint64_t)w, row_magic) : w >> gsh, ob = w >> osh;
+        in.q1 = *reinterpret_cast<const uint2*>(p.st1 + (size_t)w * 8);
+        in.q2 = *reinterpret_cast<const uint2*>(p.st2 + (size_t)w * 8);
+        in.gv = __ldg(reinterpret_cast<const uint4*>(p.grad) + w);
+        if (W8) in.pk = __ldg(reinterpret_cast<const uint2*>(p.rq.codes_in) + w);
+        else in.pk = make_uint2(__ldg(reinterpret_cast<const uint32_t*>(p.rq.codes_in) + w), 0u);
+        in.rw = USE_RES ? (uint32_t)__ldg(p.rq.words_in + w) : 0u;
+        in.sb = __ldg(scales + g); in.zb = W8 ? 0u : __ldg(zeros + g);
+        in.s1 = p.sc1[ob]; in.t1 = p.tm1[ob]; in.s2 = p.sc2[ob]; in.t2 = p.tm2[ob];
+        return in;
+    };
+    In nxt;
+    nxt.q1 = nxt.q2 = nxt.pk = make_uint2(0u, 0u); nxt.gv = make_uint4(0u, 0u, 0u, 0u); nxt.rw = nxt.zb = 0u; nxt.sb = 0x3f80u;
+    nxt.s1 = nxt.t1 = nxt.s2 = nxt.t2 = 0.0f;
+    const uint32_t tile0 = blockIdx.x * AF::TEAMS + team, tile_step = gridDim.x * AF::TEAMS;
+    if (tile0 < (uint32_t)p.n_tiles && tile0 * 256u + (uint32_t)tid < n_words) nxt = load_in(tile0 * 256u + (uint32_t)tid);
+    for (uint32_t tile = tile0; tile < (uint32_t)p.n_tiles; tile += tile_step) {
         const uint32_t w = tile * 256u + (uint32_t)tid;
-        const bool active = w < n_words;
-        float lat[8], m[8], d[8];
-        float sf = 1.0f;
-        uint32_t zb = 0u, ob = 0u;
-        float mn1 = INFINITY, mx1 = -INFINITY, mn2 = INFINITY, mx2 = -INFINITY;
+        const bool active = LUT || w < n_words;               // LUT: whole 2048-element blocks only
+        const In in = nxt;
+        {
+            const uint32_t wn = w + tile_step * 256u;
+            if (tile + tile_step < (uint32_t)p.n_tiles && wn < n_words) nxt = load_in(wn);
+        }
+        auto dec1 = [&](float c) { return bf16r(__fmul_rn(bf16r(__fsub_rn(in.t1, __fmul_rn(c, in.s1))), p.h.beta1)); };     // m * beta1
+        auto dec2 = [&](float c) { const float r = __fsub_rn(in.t2, __fmul_rn(c, in.s2)); return bf16r(__fmul_rn(bf16r(__fmul_rn(r, r)), p.h.beta2)); };
+        if (LUT) {
+            const float c = u2f((uint32_t)tid);
+            lut[tid] = dec1(c); lut[256 + tid] = dec2(c);
+            team_sync();
+        }
+        uint32_t lat[4], m[4], d[4];
+        uint32_t mn1 = 0x7f807f80u, mx1 = 0xff80ff80u, mn2 = 0x7f807f80u, mx2 = 0xff80ff80u;
         if (active) {
-            const uint32_t g = w >> gsh;
-            const uint32_t sb = __ldg(scales + g);
-            zb = __ldg(zeros + g);
-            ob = w >> osh;
-            const float s1 = p.sc1[ob], t1 = p.tm1[ob], s2f = p.sc2[ob], t2 = p.tm2[ob];
-            const uint2 q1 = *reinterpret_cast<const uint2*>(p.st1 + (size_t)w * 8);
-            const uint2 q2 = *reinterpret_cast<const uint2*>(p.st2 + (size_t)w * 8);
-            const uint4 gv = __ldg(reinterpret_cast<const uint4*>(p.grad) + w);
-            const uint32_t pk = __ldg(reinterpret_cast<const uint32_t*>(p.rq.codes_in) + w);
-            uint32_t rw = 0u;
-            if (USE_RES) rw = (uint32_t)__ldg(p.rq.words_in + w);
-            sf = __uint_as_float(sb << 16);
             // latent weights: bf16((q - z) * s) (+ bf16(bf16(res * s) + that)), packed
-            const uint32_t s2u = sb * 0x00010001u, z2u = zb * 0x00010001u;
-            const __nv_bfloat162 s2 = *reinterpret_cast<const __nv_bfloat162*>(&s2u);
-            const __nv_bfloat162 z128 = __hadd2_rn(*reinterpret_cast<const __nv_bfloat162*>(&z2u), *reinterpret_cast<const __nv_bfloat162*>(&c128u));
-            const uint32_t lo_n = pk & 0x0F0F0F0Fu, hi_n = (pk >> 4) & 0x0F0F0F0Fu;
+            const __nv_bfloat162 s2 = asbf2(in.sb * 0x00010001u);
+            const __nv_bfloat162 z128 = __hadd2_rn(asbf2(in.zb * 0x00010001u), asbf2(c128u));
+            const uint32_t lo_n = in.pk.x & 0x0F0F0F0Fu, hi_n = (in.pk.x >> 4) & 0x0F0F0F0Fu;
             const uint32_t c03 = __byte_perm(hi_n, lo_n, 0x5140), c47 = __byte_perm(hi_n, lo_n, 0x7362);
-            const uint32_t gw[4] = {gv.x, gv.y, gv.z, gv.w};
+            const uint32_t gw[4] = {in.gv.x, in.gv.y, in.gv.z, in.gv.w};
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const uint32_t pair = __byte_perm((j < 2) ? c03 : c47, 0x43434343u, (j & 1) ? 0x4342 : 0x4140);
-                __nv_bfloat162 v = __hmul2_rn(__hsub2_rn(*reinterpret_cast<const __nv_bfloat162*>(&pair), z128), s2);
-                if (USE_RES) {
-                    const uint32_t b = (rw >> (24 - 8 * j)) & 0xffu;
-                    const uint32_t tr = tres[b * ADAM_TRES_REPL + tres_lane];
-                    v = __hadd2_rn(__hmul2_rn(*reinterpret_cast<const __nv_bfloat162*>(&tr), s2), v);
+                __nv_bfloat162 v;
+                if (W8) {
+                    // byte ^ 0x80 = code + 128 in the mantissa of fp16 1024.0, minus 1152: exact, as is the integer in bf16
+                    const uint32_t h2 = __byte_perm(((j < 2) ? in.pk.x : in.pk.y) ^ 0x80808080u, 0x64646464u, (j & 1) ? 0x4342 : 0x4140);
+                    const float2 cf = __half22float2(__hsub2(*reinterpret_cast<const __half2*>(&h2), __floats2half2_rn(1152.0f, 1152.0f)));
+                    v = __hmul2_rn(__floats2bfloat162_rn(cf.x, cf.y), s2);
+                } else {
+                    const uint32_t pair = __byte_perm((j < 2) ? c03 : c47, 0x43434343u, (j & 1) ? 0x4342 : 0x4140);
+                    v = __hmul2_rn(__hsub2_rn(asbf2(pair), z128), s2);
                 }
-                const uint32_t vu = *reinterpret_cast<const uint32_t*>(&v);
-                lat[2 * j] = __uint_as_float(vu << 16); lat[2 * j + 1] = __uint_as_float(vu & 0xffff0000u);
+                if (USE_RES) {
+                    const uint32_t b = (in.rw >> (24 - 8 * j)) & 0xffu;
+                    v = __hadd2_rn(__hmul2_rn(asbf2(tres[b * ADAM_TRES_REPL + tres_lane]), s2), v);
+                }
+                const uint32_t vu = asu32(v);
                 // the two elements of the pair through the optimizer chain (every intermediate rounded to bf16)
-                const int k0 = 2 * j, k1 = 2 * j + 1;
-                const float g0 = __uint_as_float(gw[j] << 16), g1 = __uint_as_float(gw[j] & 0xffff0000u);
-                const float c10 = u2f(((k0 < 4 ? q1.x : q1.y) >> (8 * (k0 & 3))) & 0xffu), c11 = u2f(((k1 < 4 ? q1.x : q1.y) >> (8 * (k1 & 3))) & 0xffu);
-                const float c20 = u2f(((k0 < 4 ? q2.x : q2.y) >> (8 * (k0 & 3))) & 0xffu), c21 = u2f(((k1 < 4 ? q2.x : q2.y) >> (8 * (k1 & 3))) & 0xffu);
-                float m0, m1, v0, v1, t0, t1v;
-                rb2(__fsub_rn(t1, __fmul_rn(c10, s1)), __fsub_rn(t1, __fmul_rn(c11, s1)), m0, m1);       // DeQfunc_8bit_opt(...).to(bf16)
-                const float r20 = __fsub_rn(t2, __fmul_rn(c20, s2f)), r21 = __fsub_rn(t2, __fmul_rn(c21, s2f));
-                rb2(__fmul_rn(r20, r20), __fmul_rn(r21, r21), v0, v1);                                   // (s2 * s2).to(bf16)
-                rb2(__fmul_rn(m0, p.h.beta1), __fmul_rn(m1, p.h.beta1), m0, m1);
-                rb2(__fmaf_rn(p.h.one_minus_beta1, g0, m0), __fmaf_rn(p.h.one_minus_beta1, g1, m1), m0, m1);
-                rb2(__fmul_rn(v0, p.h.beta2), __fmul_rn(v1, p.h.beta2), v0, v1);
-                rb2(__fmaf_rn(p.h.one_minus_beta2, __fmul_rn(g0, g0), v0), __fmaf_rn(p.h.one_minus_beta2, __fmul_rn(g1, g1), v1), v0, v1);
-                rb2(__fsqrt_rn(v0), __fsqrt_rn(v1), t0, t1v);
-                rb2(__fadd_rn(t0, p.h.eps), __fadd_rn(t1v, p.h.eps), v0, v1);                            // sqrt(v) + eps
-                rb2(__fmaf_rn(p.h.neg_step_size, __fdiv_rn(m0, v0), lat[k0]), __fmaf_rn(p.h.neg_step_size, __fdiv_rn(m1, v1), lat[k1]), lat[k0], lat[k1]);
-                m[k0] = m0; m[k1] = m1; d[k0] = v0; d[k1] = v1;
-                mn1 = fminf(mn1, fminf(m0, m1)); mx1 = fmaxf(mx1, fmaxf(m0, m1));
-                mn2 = fminf(mn2, fminf(v0, v1)); mx2 = fmaxf(mx2, fmaxf(v0, v1));
+                const float g0 = lo2f(gw[j]), g1 = hi2f(gw[j]);
+                const uint32_t w1 = (j < 2) ? in.q1.x : in.q1.y, w2 = (j < 2) ? in.q2.x : in.q2.y;
+                const uint32_t a0 = (w1 >> (16 * (j & 1))) & 0xffu, a1 = (w1 >> (16 * (j & 1) + 8)) & 0xffu;
+                const uint32_t b0 = (w2 >> (16 * (j & 1))) & 0xffu, b1 = (w2 >> (16 * (j & 1) + 8)) & 0xffu;
+                const float m0 = LUT ? lut[a0] : dec1(u2f(a0)), m1 = LUT ? lut[a1] : dec1(u2f(a1));
+                const float v0 = LUT ? lut[256 + b0] : dec2(u2f(b0)), v1 = LUT ? lut[256 + b1] : dec2(u2f(b1));
+                m[j] = pack2(__fmaf_rn(p.h.one_minus_beta1, g0, m0), __fmaf_rn(p.h.one_minus_beta1, g1, m1));
+                const uint32_t vv = pack2(__fmaf_rn(p.h.one_minus_beta2, __fmul_rn(g0, g0), v0), __fmaf_rn(p.h.one_minus_beta2, __fmul_rn(g1, g1), v1));
+                const uint32_t t = pack2(sqrt_approx(lo2f(vv)), sqrt_approx(hi2f(vv)));
+                d[j] = pack2(__fadd_rn(lo2f(t), p.h.eps), __fadd_rn(hi2f(t), p.h.eps));              // sqrt(v) + eps
+                lat[j] = pack2(__fmaf_rn(p.h.neg_step_size, div_bf16(lo2f(m[j]), lo2f(d[j])), lo2f(vu)),
+                               __fmaf_rn(p.h.neg_step_size, div_bf16(hi2f(m[j]), hi2f(d[j])), hi2f(vu)));
+                mn1 = min2(mn1, m[j]); mx1 = max2(mx1, m[j]);
+                mn2 = min2(mn2, d[j]); mx2 = max2(mx2, d[j]);
             }
         }
+        // block extrema of both states in two registers: (min m, min d) and (-max m, -max d)
+        uint32_t lo, hi;
+        {
+            mn1 = min2(mn1, __byte_perm(mn1, 0u, 0x1032)); mx1 = max2(mx1, __byte_perm(mx1, 0u, 0x1032));
+            mn2 = min2(mn2, __byte_perm(mn2, 0u, 0x1032)); mx2 = max2(mx2, __byte_perm(mx2, 0u, 0x1032));
+            lo = __byte_perm(mn1, mn2, 0x5410); hi = __byte_perm(mx1, mx2, 0x5410) ^ 0x80008000u;
 #pragma unroll
-        for (int o = 8; o > 0; o >>= 1) {
-            mn1 = fminf(mn1, __shfl_xor_sync(0xffffffffu, mn1, o)); mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, o));
-            mn2 = fminf(mn2, __shfl_xor_sync(0xffffffffu, mn2, o)); mx2 = fmaxf(mx2, __shfl_xor_sync(0xffffffffu, mx2, o));
-        }
-        if (p.opt_shift == 11) {
-            mn1 = fminf(mn1, __shfl_xor_sync(0xffffffffu, mn1, 16)); mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 16));
-            mn2 = fminf(mn2, __shfl_xor_sync(0xffffffffu, mn2, 16)); mx2 = fmaxf(mx2, __shfl_xor_sync(0xffffffffu, mx2, 16));
-            __syncthreads();
-            if (lane == 0) { s_red[0][warp] = mn1; s_red[1][warp] = mx1; s_red[2][warp] = mn2; s_red[3][warp] = mx2; }
-            __syncthreads();
+            for (int o = LUT ? 16 : 8; o > 0; o >>= 1) {
+                lo = min2(lo, __shfl_xor_sync(0xffffffffu, lo, o)); hi = min2(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+            }
+            if (LUT) {
+                if (lane == 0) red[warp] = make_uint2(lo, hi);
+                team_sync();                                  // also: every read of this tile's state tables is done
+                const uint4* r4 = reinterpret_cast<const uint4*>(red);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                mn1 = fminf(mn1, s_red[0][i]); mx1 = fmaxf(mx1, s_red[1][i]);
-                mn2 = fminf(mn2, s_red[2][i]); mx2 = fmaxf(mx2, s_red[3][i]);
+                for (int i = 0; i < 4; ++i) {
+                    const uint4 r = r4[i];
+                    lo = min2(min2(lo, r.x), r.z); hi = min2(min2(hi, r.y), r.w);
+                }
             }
         }
         if (active) {
-            const float ns1 = __fadd_rn(__fdiv_rn(__fsub_rn(mx1, mn1), 255.0f), 1e-10f);
-            const float ns2 = __fadd_rn(__fdiv_rn(__fsub_rn(mx2, mn2), 255.0f), 1e-10f);
-            *reinterpret_cast<uint2*>(p.st1 + (size_t)w * 8) = opt8_encode8(m, mx1, ns1);
-            *reinterpret_cast<uint2*>(p.st2 + (size_t)w * 8) = opt8_encode8(d, mx2, ns2);
-            const bool leader = p.opt_shift == 11 ? (tid == 0) : ((tid & 15) == 0);
-            if (leader) { p.sc1[ob] = ns1; p.tm1[ob] = mx1; p.sc2[ob] = ns2; p.tm2[ob] = mx2; }
+            const float fmn1 = lo2f(lo), fmn2 = hi2f(lo), fmx1 = -lo2f(hi), fmx2 = -hi2f(hi);
+            OptScale o1 = opt8_scale(fmx1, fmn1), o2 = opt8_scale(fmx2, fmn2);
             // requantize: Z = bf16(bf16(lat / s) + z), then one table byte per element
+            const float sf = __uint_as_float(in.sb << 16);
             const float rs = __frcp_rn(sf);
-            const uint32_t z2u = zb * 0x00010001u;
-            const __nv_bfloat162 z2 = *reinterpret_cast<const __nv_bfloat162*>(&z2u);
+            const __nv_bfloat162 z2 = asbf2(in.zb * 0x00010001u);
             uint32_t zbits[4], zmax = 0u;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const __nv_bfloat162 Zp = __hadd2_rn(__floats2bfloat162_rn(__fmul_rn(lat[2 * j], rs), __fmul_rn(lat[2 * j + 1], rs)), z2);
-                zbits[j] = *reinterpret_cast<const uint32_t*>(&Zp);
+                __nv_bfloat162 Zp = asbf2(pack2(__fmul_rn(lo2f(lat[j]), rs), __fmul_rn(hi2f(lat[j]), rs)));
+                if (!W8) Zp = __hadd2_rn(Zp, z2);
+                zbits[j] = asu32(Zp);
                 __nv_bfloat162 az = __habs2(Zp);
-                if (j) az = __hmax2_nan(*reinterpret_cast<const __nv_bfloat162*>(&zmax), az);        // NaN-propagating max of the magnitudes
-                zmax = *reinterpret_cast<const uint32_t*>(&az);
+                if (j) az = __hmax2_nan(asbf2(zmax), az);                                            // NaN-propagating max of the magnitudes
+                zmax = asu32(az);
             }
-            const bool bad = (((zmax & 0x7fff7fffu) + 0x3d803d80u) & 0x80008000u) != 0u || !fastdiv_ok_scale(sf);
+            // |Z| beyond the table or not finite, an extreme scale, or extrema that are not finite (exponent field all ones)
+            const uint32_t inf_lo = (lo & 0x7fff7fffu) + 0x00800080u, inf_hi = (hi & 0x7fff7fffu) + 0x00800080u;
+            const bool bad = ((((zmax & 0x7fff7fffu) + AF::Z_LIMIT) | inf_lo | inf_hi) & 0x80008000u) != 0u || !fastdiv_ok_scale(sf);
             if (__builtin_expect(bad, 0)) {
-                const float z = __uint_as_float(zb << 16);
-                latent_store<4, LQ_CODEC_THREEFOLD, LQ_DITHER_HASH, true>(p.rq, (int64_t)w, sf, z, lat);
+                o1.s = __fadd_rn(__fdiv_rn(__fsub_rn(fmx1, fmn1), 255.0f), 1e-10f);      // (the fast division is for finite extrema)
+                o2.s = __fadd_rn(__fdiv_rn(__fsub_rn(fmx2, fmn2), 255.0f), 1e-10f);
+                adam_word_generic<WBITS>(p, (int64_t)w, in.s1, in.t1, in.s2, in.t2, fmx1, o1.s, fmx2, o2.s);
             } else {
+                *reinterpret_cast<uint2*>(p.st1 + (size_t)w * 8) = make_uint2(opt8_codes4(m[0], m[1], fmx1, o1), opt8_codes4(m[2], m[3], fmx1, o1));
+                *reinterpret_cast<uint2*>(p.st2 + (size_t)w * 8) = make_uint2(opt8_codes4(d[0], d[1], fmx2, o2), opt8_codes4(d[2], d[3], fmx2, o2));
                 uint32_t ev[4], od[4];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) { ev[j] = encz[zbits[j] & 0xffffu]; od[j] = encz[zbits[j] >> 16]; }
-                const uint32_t e_even = __byte_perm(__byte_perm(ev[0], ev[1], 0x4040), __byte_perm(ev[2], ev[3], 0x4040), 0x5410);
-                const uint32_t e_odd = __byte_perm(__byte_perm(od[0], od[1], 0x4040), __byte_perm(od[2], od[3], 0x4040), 0x5410);
-                reinterpret_cast<uint32_t*>(p.rq.codes_out)[w] = (e_even & 0xF0F0F0F0u) | ((e_odd >> 4) & 0x0F0F0F0Fu);
-                p.rq.words_out[w] = (int32_t)__byte_perm(((e_even << 4) & 0xF0F0F0F0u) | (e_odd & 0x0F0F0F0Fu), 0u, 0x0123);
+                for (int j = 0; j < 4; ++j) {
+                    ev[j] = W8 ? (uint32_t)enc8[zbits[j] & 0xffffu] : (uint32_t)encz[zbits[j] & 0xffffu];
+                    od[j] = W8 ? (uint32_t)enc8[zbits[j] >> 16] : (uint32_t)encz[zbits[j] >> 16];
+                }
+                if (W8) {
+                    // code in byte 0, nibble in byte 1; residual element k at bits 28 - 4k
+                    const uint32_t p01 = __byte_perm(ev[0], od[0], 0x5140), p23 = __byte_perm(ev[1], od[1], 0x5140);   // (c0 c1 n0 n1)
+                    const uint32_t p45 = __byte_perm(ev[2], od[2], 0x5140), p67 = __byte_perm(ev[3], od[3], 0x5140);
+                    reinterpret_cast<uint2*>(p.rq.codes_out)[w] = make_uint2(__byte_perm(p01, p23, 0x5410), __byte_perm(p45, p67, 0x5410));
+                    const uint32_t hi = __byte_perm(__byte_perm(ev[3], ev[2], 0x0051), __byte_perm(ev[1], ev[0], 0x0051), 0x5410);   // n6 n4 n2 n0
+                    const uint32_t lo4 = __byte_perm(__byte_perm(od[3], od[2], 0x0051), __byte_perm(od[1], od[0], 0x0051), 0x5410);  // n7 n5 n3 n1
+                    p.rq.words_out[w] = (int32_t)((hi << 4) | lo4);
+                } else {
+                    const uint32_t e_even = __byte_perm(__byte_perm(ev[0], ev[1], 0x4040), __byte_perm(ev[2], ev[3], 0x4040), 0x5410);
+                    const uint32_t e_odd = __byte_perm(__byte_perm(od[0], od[1], 0x4040), __byte_perm(od[2], od[3], 0x4040), 0x5410);
+                    reinterpret_cast<uint32_t*>(p.rq.codes_out)[w] = (e_even & 0xF0F0F0F0u) | ((e_odd >> 4) & 0x0F0F0F0Fu);
+                    p.rq.words_out[w] = (int32_t)__byte_perm(((e_even << 4) & 0xF0F0F0F0u) | (e_odd & 0x0F0F0F0Fu), 0u, 0x0123);
+                }
             }
+            const uint32_t ob = w >> osh;
+            const bool leader = LUT ? (tid == 0) : ((tid & 15) == 0);
+            if (leader) { p.sc1[ob] = o1.s; p.tm1[ob] = fmx1; p.sc2[ob] = o2.s; p.tm2[ob] = fmx2; }
         }
     }
+}
+
+// What the fast variant's arithmetic relies on beside finite moments: eps hides a root that sqrt.approx flushes to zero (below
+// 2^-63) and keeps denominators normal; a sane step size keeps updates from moments below 2^-117, whose division residual is not
+// exact any more, far below the resolution of the codes.
+static inline bool adam_fast_hyper_ok(const lq_adam_hyper& h) {
+    return h.eps >= 4e-12f && h.eps <= 1.0f && h.neg_step_size >= -1e3f && h.neg_step_size <= 1e3f;
+}
+
+template <int WBITS>
+static int launch_adam_fast(const AdamParams& p, int enc_slot, int opt_block, uint64_t row_magic, cudaStream_t st) {
+    using AF = AdamFast<WBITS>;
+    const int v = (p.rq.has_residual ? 2 : 0) + (opt_block == 2048 ? 1 : 0);
+    auto* const kernel = v == 3 ? k_adam_fast<WBITS, true, true> : v == 2 ? k_adam_fast<WBITS, true, false>
+                         : v == 1 ? k_adam_fast<WBITS, false, true> : k_adam_fast<WBITS, false, false>;
+    static bool attr_done[64][4] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev >= 0 && dev < 64 && !attr_done[dev][v]) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AF::SMEM);
+        if (e != cudaSuccess) { set_cuda_error(e, "cudaFuncSetAttribute(k_adam_fast)"); return LQ_ECUDA; }
+        attr_done[dev][v] = true;
+    }
+    const int64_t cap = (int64_t)sm_count() * AF::MIN_CTAS, want = (p.n_tiles + AF::TEAMS - 1) / AF::TEAMS;
+    kernel<<<(int)(want < cap ? want : cap), AF::THREADS, AF::SMEM, st>>>(p, enc_slot, row_magic);
+    return check_launch("k_adam_fast");
 }
 
 template <int WBITS, int CODEC, int DITHER>
@@ -451,24 +615,10 @@ int lq_adam_a16w4_step(int8_t* codes, int32_t* words, const void* grad, int grad
     cudaStream_t st = LQ_ST(stream);
     if (opts->codec == LQ_CODEC_THREEFOLD && opts->dither == LQ_DITHER_HASH) {
         if (bf && p.rq.group_shift >= 3 && p.rq.n_words < ((int64_t)1 << 31) && opts->mu_enc >= 0 && opts->mu_enc <= 3 &&
-            opts->mu_dec >= 0 && opts->mu_dec <= 3 && !getenv("LQ_REQUANT_GENERIC")) {
+            opts->mu_dec >= 0 && opts->mu_dec <= 3 && adam_fast_hyper_ok(*hyper) && !getenv("LQ_REQUANT_GENERIC")) {
             rc = ensure_encz_table(opts->mu_enc, opts->v0, st);
             if (rc) return rc;
-            static bool attr_done[64][2] = {};
-            int dev = 0;
-            cudaGetDevice(&dev);
-            const int ur = p.rq.has_residual ? 1 : 0;
-            if (dev >= 0 && dev < 64 && !attr_done[dev][ur]) {
-                cudaError_t e = ur ? cudaFuncSetAttribute(k_adam_a16w4_fast<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, ADAM_FAST_SMEM)
-                                   : cudaFuncSetAttribute(k_adam_a16w4_fast<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, ADAM_FAST_SMEM);
-                if (e != cudaSuccess) { set_cuda_error(e, "cudaFuncSetAttribute(k_adam_a16w4_fast)"); return LQ_ECUDA; }
-                attr_done[dev][ur] = true;
-            }
-            const int64_t cap = (int64_t)sm_count() * 3;
-            const int grid = (int)(p.n_tiles < cap ? p.n_tiles : cap);
-            if (ur) k_adam_a16w4_fast<true><<<grid, 256, ADAM_FAST_SMEM, st>>>(p, opts->mu_enc);
-            else k_adam_a16w4_fast<false><<<grid, 256, ADAM_FAST_SMEM, st>>>(p, opts->mu_enc);
-            return check_launch("k_adam_a16w4_fast");
+            return launch_adam_fast<4>(p, opts->mu_enc, opt_block, 0, st);
         }
         return launch_adam<4, LQ_CODEC_THREEFOLD, LQ_DITHER_HASH>(p, bf, st);
     }
@@ -502,7 +652,15 @@ int lq_adam_a8w8_step(int8_t* codes, int32_t* words, const void* grad, int grad_
     p.h = *hyper;
     const bool bf = grad_dtype == LQ_BF16;
     cudaStream_t st = LQ_ST(stream);
-    if (opts->codec == LQ_CODEC_THREEFOLD && opts->dither == LQ_DITHER_HASH) return launch_adam<8, LQ_CODEC_THREEFOLD, LQ_DITHER_HASH>(p, bf, st);
+    if (opts->codec == LQ_CODEC_THREEFOLD && opts->dither == LQ_DITHER_HASH) {
+        const uint64_t wpr = (uint64_t)(cols / 8);               // words per weight row; the row of a word by multiply-high, exact below 2^24 words
+        if (bf && wpr > 1 && wpr < (1u << 24) && p.rq.n_words < ((int64_t)1 << 31) && opts->mu_enc >= 0 && opts->mu_enc <= 3 &&
+            opts->mu_dec >= 0 && opts->mu_dec <= 3 && adam_fast_hyper_ok(*hyper) && !getenv("LQ_REQUANT_GENERIC")) {
+            if ((rc = ensure_enc8_table(opts->mu_enc, opts->v0, st)) != LQ_OK) return rc;
+            return launch_adam_fast<8>(p, opts->mu_enc, opt_block, ~(uint64_t)0 / wpr + 1, st);
+        }
+        return launch_adam<8, LQ_CODEC_THREEFOLD, LQ_DITHER_HASH>(p, bf, st);
+    }
     if (opts->codec == LQ_CODEC_THREEFOLD && opts->dither == LQ_DITHER_PHILOX) return launch_adam<8, LQ_CODEC_THREEFOLD, LQ_DITHER_PHILOX>(p, bf, st);
     return LQ_EUNSUPPORTED;
 }

@@ -320,6 +320,29 @@ static inline int ensure_encz_table(int mu, float v0, cudaStream_t st) {
     built[dev][slot] = true; built_v0[dev][slot] = v0;
     return LQ_OK;
 }
-
+// The same for int8 codes: every bf16 pattern of Z = w/scale -> code & 0xff | nibble << 8 (|Z| < 256)
+static __device__ uint16_t g_enc8_table[4][65536];
+static __global__ void __launch_bounds__(256) k_build_enc8_table(int slot, Curve c, float v0) {
+    for (int h = blockIdx.x * blockDim.x + threadIdx.x; h < 65536; h += gridDim.x * blockDim.x) {
+        const float Z = __uint_as_float((uint32_t)h << 16);
+        g_enc8_table[slot][h] = (fabsf(Z) < 256.0f) ? (uint16_t)encode_from_z_w8_hash_bf16(Z, c, v0) : (uint16_t)0;
+    }
+}
+static inline int ensure_enc8_table(int mu, float v0, cudaStream_t st) {
+    static bool built[64][4] = {};
+    static float built_v0[64][4] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return LQ_EUNSUPPORTED;
+    const int slot = (mu < 0 || mu > 3) ? 0 : mu;
+    std::lock_guard<std::mutex> lock(g_encz_mutex);
+    if (built[dev][slot] && built_v0[dev][slot] == v0) return LQ_OK;
+    k_build_enc8_table<<<128, 256, 0, st>>>(slot, curve_for_level(slot), v0);
+    int rc = check_launch("k_build_enc8_table");
+    if (rc) return rc;
+    cudaError_t e = cudaStreamSynchronize(st);       // first use only: visible to every stream before anyone reads it
+    if (e != cudaSuccess) { set_cuda_error(e, "cudaStreamSynchronize"); return LQ_ECUDA; }
+    built[dev][slot] = true; built_v0[dev][slot] = v0;
+    return LQ_OK;
+}
 
 }  // namespace lq

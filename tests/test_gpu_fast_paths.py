@@ -1,0 +1,73 @@
+"""The specialised kernels against the general ones (bit for bit) and against 64-bit results, at the sizes and values where a
+specialised path can go wrong: tile edges, remainders, degenerate blocks, non-finite words."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(autouse=True)
+def _no_device_timeout():
+    yield
+    from latentq_llm_b200 import _lib
+    assert _lib.lib.lq_gemm_device_status(1) == 0, "a bounded device-side wait expired"
+
+
+def _gen(seed):
+    return torch.Generator(device="cuda").manual_seed(seed)
+
+
+# ---- fused optimizer step -------------------------------------------------------------------------------------------
+def _adam_case(wbit, N, K, seed, grad_kind):
+    from latentq_llm_b200 import ops
+    g = _gen(seed)
+    n = N * K
+    blocks = n // (2048 if n % 2048 == 0 else 128)
+    per = n // blocks
+    grad = (torch.randn(N, K, device="cuda", generator=g) * torch.exp(3 * torch.randn(N, 1, device="cuda", generator=g)) * 1e-4).to(torch.bfloat16)
+    if grad_kind == "zero":
+        grad.zero_()
+    elif grad_kind == "tiny":
+        grad = (grad.float() * 1e-33).to(torch.bfloat16)
+    elif grad_kind == "nonfinite":
+        flat = grad.view(-1)
+        flat[5], flat[(per + 3) % n], flat[n - 1] = float("inf"), float("nan"), -float("inf")
+        flat[2 * per:3 * per] = float("nan")
+    st = [torch.randint(0, 256, (N, K), device="cuda", generator=g, dtype=torch.uint8) for _ in range(2)]
+    sc = [torch.rand(blocks, 1, device="cuda", generator=g) * 1e-5 + 1e-10 for _ in range(2)]
+    tm = [torch.rand(blocks, 1, device="cuda", generator=g) * 1e-3 for _ in range(2)]
+    words = torch.randint(-2 ** 31, 2 ** 31, (n // 8,), device="cuda", generator=g, dtype=torch.int64).to(torch.int32)
+    hyper = ops.make_adam_hyper(0.9, 0.95, 1e-8, 1e-3)
+
+    def run(has_residual):
+        o = ops.make_opts(codec=ops.CODEC_THREEFOLD, dither=ops.DITHER_HASH, has_residual=has_residual, mu_enc=1, mu_dec=0)
+        a = [t.clone() for t in (st[0], sc[0], tm[0], st[1], sc[1], tm[1])]
+        w = words.clone()
+        gg = _gen(seed + 1)
+        if wbit == 4:
+            codes = torch.randint(-128, 128, (n // 2,), device="cuda", generator=gg, dtype=torch.int8)
+            s = (torch.rand(n // 128, device="cuda", generator=gg) * 0.01 + 1e-3).to(torch.bfloat16)
+            z = torch.randint(0, 16, (n // 128,), device="cuda", generator=gg).to(torch.bfloat16)
+            ops.adam_a16w4_step(codes, w, grad, s, z, *a, hyper, o)
+        else:
+            codes = torch.randint(-128, 128, (N, K), device="cuda", generator=gg, dtype=torch.int8)
+            s = (torch.rand(N, device="cuda", generator=gg) * 0.01 + 1e-4).to(torch.bfloat16)
+            ops.adam_a8w8_step(codes, w, grad, s, *a, hyper, o)
+        return [codes, w] + a
+
+    return run
+
+
+@pytest.mark.parametrize("wbit", [4, 8])
+@pytest.mark.parametrize("N,K", [(16, 128), (64, 32 * 128), (3, 1152), (1088, 1152), (520, 128)])
+@pytest.mark.parametrize("grad_kind", ["normal", "zero", "tiny", "nonfinite"])
+def test_fast_optimizer_step_equals_generic_kernel(monkeypatch, wbit, N, K, grad_kind):
+    run = _adam_case(wbit, N, K, 7 * N + K, grad_kind)
+    for has_residual in (True, False):
+        monkeypatch.delenv("LQ_REQUANT_GENERIC", raising=False)
+        fast = run(has_residual)
+        monkeypatch.setenv("LQ_REQUANT_GENERIC", "1")
+        slow = run(has_residual)
+        for a, b in zip(fast, slow):
+            assert torch.equal(torch.nan_to_num(a, nan=-1.0) if a.is_floating_point() else a,
+                               torch.nan_to_num(b, nan=-1.0) if b.is_floating_point() else b)
