@@ -119,6 +119,34 @@ __device__ __forceinline__ void philox4x32_10(uint32_t (&c)[4], uint32_t k0, uin
         k0 += 0x9E3779B9u; k1 += 0xBB67AE85u;
     }
 }
+// The same generator for counters (word, 0, stream) with word < 2^32: what does not depend on the word - the round keys, one of
+// the two products of the first two rounds and the words they leave - is computed once on the host and read as kernel constants.
+// 18 instead of 20 wide multiplies, 19 logic instructions, no key additions.
+struct PhiloxConsts { uint32_t x1, y0, y2, l0; uint32_t k0[8], k1[8]; };
+inline PhiloxConsts philox_consts(uint64_t seed, uint64_t stream_id) {
+    const uint32_t M0 = 0xD2511F53u, M1 = 0xCD9E8D57u, W0 = 0x9E3779B9u, W1 = 0xBB67AE85u;
+    const uint32_t s0 = (uint32_t)seed, s1 = (uint32_t)(seed >> 32), c2 = (uint32_t)stream_id, c3 = (uint32_t)(stream_id >> 32);
+    const uint64_t p1 = (uint64_t)M1 * c2;                                        // round 1: the product of the stream word
+    const uint64_t p0 = (uint64_t)M0 * ((uint32_t)(p1 >> 32) ^ s0);               // round 2: the product of what it leaves in c[0]
+    PhiloxConsts c;
+    c.x1 = c3 ^ s1;
+    c.y0 = (uint32_t)p1 ^ (s0 + W0);
+    c.y2 = (uint32_t)(p0 >> 32) ^ (s1 + W1);
+    c.l0 = (uint32_t)p0;
+    for (uint32_t r = 0; r < 8; ++r) { c.k0[r] = s0 + (r + 2) * W0; c.k1[r] = s1 + (r + 2) * W1; }
+    return c;
+}
+__device__ __forceinline__ void philox4x32_10_word(uint32_t word, const PhiloxConsts& k, uint32_t (&c)[4]) {
+    const uint64_t p = (uint64_t)0xD2511F53u * word;
+    const uint64_t q = (uint64_t)0xCD9E8D57u * ((uint32_t)(p >> 32) ^ k.x1);
+    c[0] = (uint32_t)(q >> 32) ^ k.y0; c[1] = (uint32_t)q; c[2] = (uint32_t)p ^ k.y2; c[3] = k.l0;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+        const uint64_t p0 = (uint64_t)0xD2511F53u * c[0], p1 = (uint64_t)0xCD9E8D57u * c[2];
+        const uint32_t n0 = (uint32_t)(p1 >> 32) ^ c[1] ^ k.k0[r], n2 = (uint32_t)(p0 >> 32) ^ c[3] ^ k.k1[r];
+        c[0] = n0; c[1] = (uint32_t)p1; c[2] = n2; c[3] = (uint32_t)p0;
+    }
+}
 // Dither of the 8 elements of residual word `word`: 16 random bits each, u = h/65536 - 0.5 (exact).
 __device__ __forceinline__ void philox_dither8(uint64_t seed, uint64_t stream_id, uint64_t word, float (&u)[8]) {
     uint32_t c[4] = {(uint32_t)word, (uint32_t)(word >> 32), (uint32_t)stream_id, (uint32_t)(stream_id >> 32)};

@@ -54,6 +54,7 @@ struct RequantParams {
     Curve enc, dec;
     float v0; uint64_t seed, stream_id; const float* dither_buf;
     int has_residual, res_round_bf16;
+    PhiloxConsts px;                       // of (seed, stream_id)
 };
 
 // ---- conversion-free arithmetic helpers -------------------------------------------------------
@@ -281,6 +282,7 @@ static inline int fill_requant(RequantParams& p, const lq_requant_opts* o, int64
     p.n_words = numel / 8; p.group = group; p.group_shift = -1;
     if ((group & (group - 1)) == 0) { int sh = 0; while (((int64_t)1 << sh) < group) ++sh; p.group_shift = sh; }
     p.enc = curve_for_level(o->mu_enc); p.dec = curve_for_level(o->mu_dec);
+    p.px = philox_consts(o->seed, o->stream_id);
     p.v0 = o->v0; p.seed = o->seed; p.stream_id = o->stream_id; p.dither_buf = o->dither_buf;
     p.has_residual = o->has_residual; p.res_round_bf16 = o->res_round_bf16;
     return LQ_OK;

@@ -509,24 +509,20 @@ __global__ void __launch_bounds__(FastCfg<DITHER>::THREADS, FastCfg<DITHER>::MIN
             uint32_t e_even, e_odd;
             if (FC::PX) {
                 // 16 dither bits per element from one Philox4x32-10 block per word: element 2j = low half of c[j], 2j+1 = high half
-                const uint64_t w64 = 2 * (uint64_t)wp + (uint64_t)h;
-                uint32_t c[4] = {(uint32_t)w64, (uint32_t)(w64 >> 32), (uint32_t)p.stream_id, (uint32_t)(p.stream_id >> 32)};
-                philox4x32_10(c, (uint32_t)p.seed, (uint32_t)(p.seed >> 32));
-                uint32_t ee[4], eo[4], se[4], so[4];
+                uint32_t c[4];
+                philox4x32_10_word(2u * wp + (uint32_t)h, p.px, c);       // fewer than 2^31 words here
+                uint32_t ee[4], eo[4];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const uint32_t zb2 = h2u(Z[h][j]);
                     ee[j] = encp[zb2 & 0xffffu]; eo[j] = encp[zb2 >> 16];
                     // dither bits in the high half, ones below: >= entry exactly when dither >= threshold.
-                    // The outcome is byte 0 or byte 1 of the entry: se / so are that byte's index.
-                    se[j] = (__byte_perm(c[j], 0xffffffffu, 0x1044) >= ee[j]) ? 1u : 0u;
-                    so[j] = ((c[j] | 0xffffu) >= eo[j]) ? 1u : 0u;
+                    // The outcome is byte 0 or byte 1 of the entry: a conditional shift brings it to byte 0.
+                    if (__byte_perm(c[j], 0xffffffffu, 0x1044) >= ee[j]) ee[j] >>= 8;
+                    if ((c[j] | 0xffffu) >= eo[j]) eo[j] >>= 8;
                 }
-                // gather the chosen bytes two entries at a time: selector nibbles (byte of the first entry, 4 + byte of the second)
-                e_even = __byte_perm(__byte_perm(ee[0], ee[1], 0x40u + se[0] + (se[1] << 4)),
-                                     __byte_perm(ee[2], ee[3], 0x40u + se[2] + (se[3] << 4)), 0x5410);
-                e_odd = __byte_perm(__byte_perm(eo[0], eo[1], 0x40u + so[0] + (so[1] << 4)),
-                                    __byte_perm(eo[2], eo[3], 0x40u + so[2] + (so[3] << 4)), 0x5410);
+                e_even = __byte_perm(__byte_perm(ee[0], ee[1], 0x4040), __byte_perm(ee[2], ee[3], 0x4040), 0x5410);
+                e_odd = __byte_perm(__byte_perm(eo[0], eo[1], 0x4040), __byte_perm(eo[2], eo[3], 0x4040), 0x5410);
             } else {
                 uint32_t ev[4], od[4];
 #pragma unroll

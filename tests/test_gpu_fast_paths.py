@@ -71,3 +71,24 @@ def test_fast_optimizer_step_equals_generic_kernel(monkeypatch, wbit, N, K, grad
         for a, b in zip(fast, slow):
             assert torch.equal(torch.nan_to_num(a, nan=-1.0) if a.is_floating_point() else a,
                                torch.nan_to_num(b, nan=-1.0) if b.is_floating_point() else b)
+
+
+# ---- requantize with Philox dither ----------------------------------------------------------------------------------
+@pytest.mark.parametrize("seed,step,param", [(0, 0, 0), (1234, 7, 3), (2 ** 64 - 1, 2 ** 32 - 1, 2 ** 32 - 1)])
+def test_philox_fold_equals_generic_kernel(monkeypatch, seed, step, param):
+    from latentq_llm_b200 import ops
+    g = _gen(3)
+    n = 1024 * 128
+    codes = torch.randint(-128, 128, (n // 2,), device="cuda", generator=g, dtype=torch.int8)
+    words = torch.randint(-2 ** 31, 2 ** 31, (n // 8,), device="cuda", generator=g, dtype=torch.int64).to(torch.int32)
+    s = (torch.rand(n // 128, device="cuda", generator=g) * 0.01 + 1e-3).to(torch.bfloat16)
+    z = torch.randint(0, 16, (n // 128,), device="cuda", generator=g).to(torch.bfloat16)
+    delta = (torch.randn(n, device="cuda", generator=g) * 1e-3).to(torch.bfloat16)
+    out = []
+    for generic in (False, True):
+        monkeypatch.setenv("LQ_REQUANT_GENERIC", "1") if generic else monkeypatch.delenv("LQ_REQUANT_GENERIC", raising=False)
+        c, w = codes.clone(), words.clone()
+        ops.a16w4_fold_delta(c, w, delta, s, z, ops.make_opts(codec=ops.CODEC_THREEFOLD, dither=ops.DITHER_PHILOX, seed=seed, step=step,
+                                                              param_id=param))
+        out.append((c, w))
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
