@@ -240,6 +240,18 @@ LQ_API int lq_gemm_a8w8(const int8_t* x8, const int8_t* w8, const float* row_sca
                         float alpha, const void* bias, void* y, int32_t* acc_out,
                         int64_t M, int64_t N, int64_t K, void* workspace, size_t workspace_bytes,
                         lq_stream_t stream);
+/* The forward of the A8W8 linear behind its input quantizer (utils/quant.py:268-271) in one launch:
+ *   y = bf16( bf16( acc * a + bf16(bias / qscales) ) * qscales ),  a = bf16(clampv / 127)
+ * clampv: device fp32[1] as lq_act_quant_per_tensor leaves it, or NULL (a = alpha as given); bias bf16[N] or NULL;
+ * qscales bf16[N].  Same bits as lq_gemm_a8w8 with the scale, bias and product as separate bf16 tensor operations.
+ * Workspace as lq_gemm_a8w8. */
+LQ_API int lq_gemm_a8w8_module(const int8_t* x8, const int8_t* w8, const float* clampv, float alpha, const void* bias,
+                               const void* qscales, void* y, int64_t M, int64_t N, int64_t K, void* workspace,
+                               size_t workspace_bytes, lq_stream_t stream);
+/* int8 codes [rows, cols] -> bf16(code * s): s = row_scales[row] (bf16[rows]: a weight, utils/quant.py:283-284) or, when
+ * row_scales is NULL, bf16(clampv / 127) of a device fp32[1] (quantized activations, utils/quant.py:240-243). */
+LQ_API int lq_i8_dequant(const int8_t* codes, const void* row_scales, const float* clampv, int64_t rows, int64_t cols,
+                         void* out, lq_stream_t stream);
 
 /* Decode-sized forward (M <= 2, K = 4096, group 128) with the residual add and the RMSNorm in front of it folded into the
  * kernel's token staging (PTQ/quant/triton_norm.py:7-39 followed by the int4 matmul of PTQ/quant/fused_attn.py:164-204 /

@@ -99,6 +99,8 @@ SIGNATURES = {
     "lq_gemm_a16w4_fwd_static": [_p, _p, _p, _p, _p, _p, _i64, _i64, _i64, _i, _p],
     "lq_gemm_a16w4_fwd_static_peek": [_p, _sz, _sz],
     "lq_gemm_a8w8": [_p, _p, _p, _p, _f, _p, _p, _p, _i64, _i64, _i64, _p, _sz, _p],
+    "lq_gemm_a8w8_module": [_p, _p, _p, _f, _p, _p, _p, _i64, _i64, _i64, _p, _sz, _p],
+    "lq_i8_dequant": [_p, _p, _p, _i64, _i64, _p, _p],
     "lq_mma_issue_rate": [_i, _i, _i, _i, _i, _i, _p, _p],
     "lq_gemm_a16w4_fwd_rmsnorm": [_p, _p, _p, _f, _i, _p, _p, _p, _p, _p, _i64, _i64, _i64, _i, _i, _p],
     "lq_gemm_a16w4_fwd_qkv_rope": [_p, _p, _p, _p, _f, _p, _p, _p, _p, _p, _p, _p, _p, _p, _i64, _i, _i, _i, _i64, _i, _i64, _i, _i, _p],

@@ -68,6 +68,8 @@ struct GemmParams {
     float alpha;
     __nv_bfloat16* out;            // [M, R]
     int32_t* acc_out;              // int8: raw accumulators [M, R] or null
+    const __nv_bfloat16* post_scale;   // int8: per output channel, multiplied onto the bf16 result (the bias is divided by it first), or null
+    const float* clampv;           // int8: device scalar, alpha = bf16(clampv / 127), or null (alpha as given)
     void* partial;                 // split-K partial sums [splits][M][R] (fp32 / int32); balanced mode: slots + flags
     // balanced mode (SK), see SegWalk
     int sk_full;                   // tiles computed whole (a multiple of the grid size), the first ones
@@ -316,6 +318,24 @@ __global__ void __launch_bounds__(256) k_w4_qp_transpose(const __nv_bfloat16* __
     dst[0] = make_uint4(sv[0] | sv[4] << 16, sv[1] | sv[5] << 16, sv[2] | sv[6] << 16, sv[3] | sv[7] << 16);
     dst[1] = make_uint4(zv[0] | zv[4] << 16, zv[1] | zv[5] << 16, zv[2] | zv[6] << 16, zv[3] | zv[7] << 16);
 }
+
+// Epilogue constants of one output channel of the int8 kernels.  With post_scale the result is what the module's op chain
+// bf16(bf16(acc * alpha + bf16(bias / q)) * q), alpha = bf16(clampv / 127), leaves (utils/quant.py:268-271; a tensor divided by
+// a number is multiplied by its fp32 reciprocal there).
+struct I8Epi { float cs, bias, alpha, post; };
+__device__ __forceinline__ I8Epi i8_epilogue(const GemmParams& p, int r, bool r_ok) {
+    I8Epi e;
+    e.cs = (p.col_scale && r_ok) ? __ldg(p.col_scale + r) : 1.0f;
+    e.bias = (p.bias && r_ok) ? __bfloat162float(p.bias[r]) : 0.0f;
+    e.alpha = p.clampv ? bf16r(__fmul_rn(bf16r(__ldg(p.clampv)), 1.0f / 127.0f)) : p.alpha;
+    e.post = 1.0f;
+    if (p.post_scale) {
+        e.post = r_ok ? __bfloat162float(p.post_scale[r]) : 1.0f;
+        e.bias = p.bias ? bf16r(__fdiv_rn(e.bias, e.post)) : bf16r(__fmul_rn(0.0f, e.post));
+    }
+    return e;
+}
+__device__ __forceinline__ float i8_scaled(const I8Epi& e, float f) { return __fadd_rn(__fmul_rn(__fmul_rn(f, e.cs), e.alpha), e.bias); }
 
 // ---------------------------------------------------------------------------------------------
 // The kernel
@@ -569,8 +589,9 @@ k_gemm(const __grid_constant__ CUtensorMap map_tok, const __grid_constant__ CUte
             for (int rr = 0; rr < RT; ++rr) {
                 const int r = (r_tile * RT + rr) * TILE_R + quad * 32 + lane;
                 const bool r_ok = r < p.R;
-                const float cs = (C::I8 && p.col_scale && r_ok) ? __ldg(p.col_scale + r) : 1.0f;
-                const float bias = (p.bias && r_ok) ? __bfloat162float(p.bias[r]) : 0.0f;
+                I8Epi e8 = {};
+                if (C::I8) e8 = i8_epilogue(p, r, r_ok);
+                const float bias = (!C::I8 && p.bias && r_ok) ? __bfloat162float(p.bias[r]) : 0.0f;
                 // tokens per TMEM read-out: the int8 kernel has registers to spare (6 warps) and halves the number of
                 // load-wait round trips; the A16W4 kernels run at the register cap of a 22-warp CTA
                 constexpr int SLAB = (C::I8 && TN >= 32) ? 32 : 16;
@@ -666,9 +687,10 @@ k_gemm(const __grid_constant__ CUtensorMap map_tok, const __grid_constant__ CUte
                             for (int i = 0; i < SLAB / 2; ++i) {
                                 float f0 = (float)(int32_t)v[2 * i], f1 = (float)(int32_t)v[2 * i + 1];
                                 if (p.row_scale) { f0 = __fmul_rn(f0, rs[2 * i]); f1 = __fmul_rn(f1, rs[2 * i + 1]); }
-                                f0 = __fadd_rn(__fmul_rn(__fmul_rn(f0, cs), p.alpha), bias);
-                                f1 = __fadd_rn(__fmul_rn(__fmul_rn(f1, cs), p.alpha), bias);
-                                pk[i] = bf2_as_u32(__floats2bfloat162_rn(f0, f1));
+                                pk[i] = bf2_as_u32(__floats2bfloat162_rn(i8_scaled(e8, f0), i8_scaled(e8, f1)));
+                                if (p.post_scale)
+                                    pk[i] = bf2_as_u32(__floats2bfloat162_rn(__fmul_rn(__uint_as_float(pk[i] << 16), e8.post),
+                                                                             __fmul_rn(__uint_as_float(pk[i] & 0xffff0000u), e8.post)));
                             }
                         }
                         // (a transpose through shared memory into 16-byte stores was tried: slower than these 2-byte stores)
@@ -695,8 +717,8 @@ k_gemm(const __grid_constant__ CUtensorMap map_tok, const __grid_constant__ CUte
                             if (p.acc_out) p.acc_out[o] = a;
                             float f = (float)a;
                             if (p.row_scale) f = __fmul_rn(f, __ldg(p.row_scale + t));
-                            f = __fmul_rn(__fmul_rn(f, cs), p.alpha);
-                            p.out[o] = __float2bfloat16_rn(__fadd_rn(f, bias));
+                            f = i8_scaled(e8, f);
+                            p.out[o] = __float2bfloat16_rn(p.post_scale ? __fmul_rn(bf16r(f), e8.post) : f);
                         } else {
                             float f = bf16r(__uint_as_float(v[j]));          // mm output is bf16, bias added after
                             p.out[o] = __float2bfloat16_rn(p.bias ? __fadd_rn(f, bias) : f);
@@ -921,8 +943,9 @@ __global__ void __launch_bounds__(256) k_splitk_reduce(const GemmParams p) {
             if (p.acc_out) p.acc_out[i] = a;
             float f = (float)a;
             if (p.row_scale) f = __fmul_rn(f, __ldg(p.row_scale + t));
-            f = __fmul_rn(__fmul_rn(f, p.col_scale ? __ldg(p.col_scale + r) : 1.0f), p.alpha);
-            p.out[i] = __float2bfloat16_rn(__fadd_rn(f, p.bias ? __bfloat162float(p.bias[r]) : 0.0f));
+            const I8Epi e8 = i8_epilogue(p, r, true);
+            f = i8_scaled(e8, f);
+            p.out[i] = __float2bfloat16_rn(p.post_scale ? __fmul_rn(bf16r(f), e8.post) : f);
         } else {
             float a = 0.0f;
             for (int s = 0; s < p.splits; ++s) a = __fadd_rn(a, reinterpret_cast<const float*>(p.partial)[(size_t)s * total + i]);
@@ -1288,6 +1311,16 @@ int lq_gemm_a8w8(const int8_t* x8, const int8_t* w8, const float* row_scale, con
     GemmParams p{};
     p.row_scale = row_scale; p.col_scale = col_scale; p.alpha = alpha; p.bias = (const __nv_bfloat16*)bias;
     p.out = (__nv_bfloat16*)y; p.acc_out = acc_out;
+    return run_gemm(KIND_I8, x8, w8, p, M, N, K, workspace, workspace_bytes, (cudaStream_t)stream);
+}
+
+int lq_gemm_a8w8_module(const int8_t* x8, const int8_t* w8, const float* clampv, float alpha, const void* bias, const void* qscales,
+                        void* y, int64_t M, int64_t N, int64_t K, void* workspace, size_t workspace_bytes, lq_stream_t stream) {
+    if (!x8 || !w8 || !qscales || !y || !al16(x8) || !al16(w8)) return LQ_EINVAL;
+    if (M < 0 || N <= 0 || K <= 0 || M >= (1 << 30) || N >= (1 << 30) || K >= (1 << 30) || (K % 128) != 0) return LQ_EUNSUPPORTED;
+    GemmParams p{};
+    p.alpha = alpha; p.clampv = clampv; p.bias = (const __nv_bfloat16*)bias; p.post_scale = (const __nv_bfloat16*)qscales;
+    p.out = (__nv_bfloat16*)y;
     return run_gemm(KIND_I8, x8, w8, p, M, N, K, workspace, workspace_bytes, (cudaStream_t)stream);
 }
 

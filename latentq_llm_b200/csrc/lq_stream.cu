@@ -1049,15 +1049,19 @@ __global__ void __launch_bounds__(256) k_tensor_max(const __nv_bfloat16* __restr
 __global__ void __launch_bounds__(256) k_act_quant_per_tensor(const __nv_bfloat16* __restrict__ x, int64_t n_words,
                                                               const float* __restrict__ clampv, int8_t* __restrict__ x8) {
     const float c = *clampv;
+    // t and c have 8-bit significands: t / c is at least 2^-17 (relative) away from every bf16 rounding boundary and never on
+    // one, so t * RN(1/c) rounds to the same bf16 value
+    const float rc = __frcp_rn(c);
+    const bool c_ok = fastdiv_ok_scale(c);
     for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < n_words; w += (int64_t)gridDim.x * blockDim.x) {
         float v[8];
         load8(x, LQ_BF16, w * 8, v);
         uint32_t b[8];
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
-            float t = bf16r(__fmul_rn(v[k], 127.0f));       // input*127. rounds to bf16 first (utils/quant.py:264)
-            t = rintf(bf16r(__fdiv_rn(t, c)));
-            b[k] = (uint32_t)(int)fminf(fmaxf(t, -128.0f), 127.0f) & 0xffu;
+            const float t = bf16r(__fmul_rn(v[k], 127.0f));       // input*127. rounds to bf16 first (utils/quant.py:264)
+            const float q = bf16r(c_ok ? __fmul_rn(t, rc) : __fdiv_rn(t, c));
+            b[k] = f2bits(rne(fminf(fmaxf(q, -128.0f), 127.0f))) & 0xffu;
         }
         uint2 o2;
         o2.x = b[0] | (b[1] << 8) | (b[2] << 16) | (b[3] << 24);
@@ -1066,6 +1070,32 @@ __global__ void __launch_bounds__(256) k_act_quant_per_tensor(const __nv_bfloat1
     }
 }
 
+
+// bf16(code * s) for int8 codes [rows, cols]: one scale per row, or bf16(clampv / 127) for all (a bf16 tensor divided by a number is
+// multiplied by its fp32 reciprocal).  A thread converts 16 codes; 3 bytes of traffic per code.
+__device__ __forceinline__ uint32_t i8x2_scaled(uint32_t wx, uint32_t sel, float s) {       // wx: codes ^ 0x80
+    const uint32_t h2 = __byte_perm(wx, 0x64646464u, sel);                                  // fp16 1024 + code + 128, exact
+    const float2 f = __half22float2(__hsub2(*reinterpret_cast<const __half2*>(&h2), __floats2half2_rn(1152.0f, 1152.0f)));
+    const __nv_bfloat162 v = __floats2bfloat162_rn(__fmul_rn(f.x, s), __fmul_rn(f.y, s));
+    return *reinterpret_cast<const uint32_t*>(&v);
+}
+__global__ void __launch_bounds__(256) k_i8_dequant(const uint4* __restrict__ codes, const __nv_bfloat16* __restrict__ row_scales,
+                                                    const float* __restrict__ clampv, int64_t n_vec, int vec_per_row, uint4* __restrict__ out) {
+    const float all = row_scales ? 0.0f : bf16r(__fmul_rn(bf16r(*clampv), 1.0f / 127.0f));
+    for (int64_t v = (int64_t)blockIdx.x * 256 + threadIdx.x; v < n_vec; v += (int64_t)gridDim.x * 256) {
+        const uint4 c = __ldg(codes + v);
+        const float s = row_scales ? __bfloat162float(row_scales[v / vec_per_row]) : all;
+        const uint32_t w[4] = {c.x ^ 0x80808080u, c.y ^ 0x80808080u, c.z ^ 0x80808080u, c.w ^ 0x80808080u};
+        out[2 * v] = make_uint4(i8x2_scaled(w[0], 0x4140, s), i8x2_scaled(w[0], 0x4342, s), i8x2_scaled(w[1], 0x4140, s), i8x2_scaled(w[1], 0x4342, s));
+        out[2 * v + 1] = make_uint4(i8x2_scaled(w[2], 0x4140, s), i8x2_scaled(w[2], 0x4342, s), i8x2_scaled(w[3], 0x4140, s), i8x2_scaled(w[3], 0x4342, s));
+    }
+}
+__global__ void __launch_bounds__(256) k_i8_dequant_any(const int8_t* __restrict__ codes, const __nv_bfloat16* __restrict__ row_scales,
+                                                        const float* __restrict__ clampv, int64_t n, int64_t cols, __nv_bfloat16* __restrict__ out) {
+    const float all = row_scales ? 0.0f : bf16r(__fmul_rn(bf16r(*clampv), 1.0f / 127.0f));
+    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256)
+        out[i] = __float2bfloat16_rn(__fmul_rn((float)codes[i], row_scales ? __bfloat162float(row_scales[i / cols]) : all));
+}
 
 // =================================================================================================
 // Layout conversion: nibble-pair int8 [N, K/2] (utils/quant.py:4-9)  <->  GPTQ int32 [K/8, N]
@@ -1406,6 +1436,19 @@ int lq_act_quant_per_token(const void* x, int64_t M, int64_t K, int8_t* x8, floa
     else if (K <= 16384) k_act_quant_per_token<16><<<grid, 128, 0, LQ_ST(stream)>>>(xb, K, x8, a_scale);
     else k_act_quant_per_token<0><<<grid, 256, 0, LQ_ST(stream)>>>(xb, K, x8, a_scale);
     return check_launch("lq_act_quant_per_token");
+}
+int lq_i8_dequant(const int8_t* codes, const void* row_scales, const float* clampv, int64_t rows, int64_t cols, void* out, lq_stream_t stream) {
+    if (rows == 0 || cols == 0) return LQ_OK;
+    if (!codes || !out || rows < 0 || cols < 0 || (!row_scales && !clampv)) return LQ_EINVAL;
+    { int rc_dev = ensure_device_for(codes); if (rc_dev) return rc_dev; }
+    const int64_t n = rows * cols;
+    const __nv_bfloat16* rs = reinterpret_cast<const __nv_bfloat16*>(row_scales);
+    if ((cols % 16) == 0 && cols < ((int64_t)1 << 34) && aligned(codes, 16) && aligned(out, 16))
+        k_i8_dequant<<<grid_for(n / 16, 256, 8), 256, 0, LQ_ST(stream)>>>(reinterpret_cast<const uint4*>(codes), rs, clampv, n / 16, (int)(cols / 16),
+                                                                         reinterpret_cast<uint4*>(out));
+    else
+        k_i8_dequant_any<<<grid_for(n, 256, 8), 256, 0, LQ_ST(stream)>>>(codes, rs, clampv, n, cols, reinterpret_cast<__nv_bfloat16*>(out));
+    return check_launch("lq_i8_dequant");
 }
 int lq_act_quant_per_tensor(const void* x, int64_t n, float* clampv_out, int8_t* x8, lq_stream_t stream) {
     if (n == 0) return LQ_OK;

@@ -398,6 +398,38 @@ def gemm_a8w8(x8, w8, row_scale=None, col_scale=None, alpha=1.0, bias=None, want
     return (y, acc) if want_acc else y
 
 
+def gemm_a8w8_module(x8, w8, clampv, alpha, bias, qscales):
+    """Forward of an A8W8 linear behind its input quantizer (utils/quant.py:268-271): one launch for
+    `(acc * a + bias / qscales) * qscales` with a = clampv / 127 from the device (`clampv` fp32[1]) or `alpha`."""
+    _chk(x8, "x8", torch.int8); _chk(w8, "w8", torch.int8); _chk(qscales, "qscales", torch.bfloat16)
+    M, K = x8.shape
+    N = w8.shape[0]
+    assert w8.shape[1] == K and qscales.numel() == N
+    if clampv is not None:
+        _chk(clampv, "clampv", torch.float32)
+    if bias is not None:
+        _chk(bias, "bias", torch.bfloat16)
+    y = torch.empty((M, N), dtype=torch.bfloat16, device=x8.device)
+    ws, nb = _workspace(L.GEMM_A8W8, M, N, K, x8.device)
+    L.call("lq_gemm_a8w8_module", _ptr(x8), _ptr(w8), _ptr(clampv), float(alpha), _ptr(bias), _ptr(qscales), _ptr(y), M, N, K, _ptr(ws), nb,
+           _stream())
+    return y
+
+
+def i8_dequant(codes, row_scales=None, clampv=None):
+    """bf16(code * s): s per row (`row_scales` bf16) or bf16(clampv / 127) of the whole tensor (`clampv` fp32[1])."""
+    _chk(codes, "codes", torch.int8)
+    rows, cols = codes.shape
+    if row_scales is not None:
+        _chk(row_scales, "row_scales", torch.bfloat16)
+        assert row_scales.numel() == rows
+    else:
+        _chk(clampv, "clampv", torch.float32)
+    y = torch.empty((rows, cols), dtype=torch.bfloat16, device=codes.device)
+    L.call("lq_i8_dequant", _ptr(codes), _ptr(row_scales), _ptr(clampv), rows, cols, _ptr(y), _stream())
+    return y
+
+
 class decode_chain:
     """Context manager: launches inside it form a decode chain (every kernel consumes its predecessor's output, the
     weights are constant), so the decode kernels may be started while their predecessor is still running; they read what

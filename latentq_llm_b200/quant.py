@@ -226,6 +226,12 @@ def _a8w8_forward(input8, clampv, weight_d, qscales, bias):
     (utils/quant.py:268-271).  `clampv` is a Python float (static) or a device tensor (dynamic: input.max());
     the tensor case avoids the host synchronisation of converting it to a float."""
     M = input8.shape[0]
+    qs = qscales.detach()
+    if qs.dtype == torch.bfloat16 and qs.is_contiguous() and (bias is None or bias.dtype == torch.bfloat16) and (
+            not torch.is_tensor(clampv) or clampv.dtype == torch.float32):
+        on_device = torch.is_tensor(clampv)
+        return ops.gemm_a8w8_module(input8, weight_d, clampv if on_device else None, 1.0 if on_device else float(clampv) / 127.,
+                                    None if bias is None else bias.detach().contiguous(), qs)
     if torch.is_tensor(clampv):
         # clampv/127. on the reference's 0-dim bf16 tensor rounds to bf16
         alpha = (clampv.to(torch.bfloat16) / 127.).float().reshape(1).expand(M).contiguous()
@@ -246,9 +252,13 @@ def _quant_input_static(input, clampv):
 
 
 def _a8w8_backward(ctx, grad_output, input_f, weight_d, qscales, bias, detach=False):
-    weight_forward = weight_d.to(grad_output.dtype) * qscales
     grad_input = grad_bias = None
     if ctx.needs_input_grad[0]:
+        if (grad_output.dtype == torch.bfloat16 and qscales.dtype == torch.bfloat16 and qscales.is_contiguous()
+                and qscales.numel() == weight_d.shape[0] == qscales.shape[0]):
+            weight_forward = ops.i8_dequant(weight_d, row_scales=qscales)
+        else:
+            weight_forward = weight_d.to(grad_output.dtype) * qscales
         grad_input = grad_output.mm(weight_forward)
     grad_weight = grad_output.t().mm(input_f)
     dict_temp.append(grad_weight.data if detach else grad_weight)
@@ -297,8 +307,10 @@ class QLinearFunctionA8W8_dynamic(torch.autograd.Function):
     def backward(ctx, grad_output):
         input8, weight_d, bias = ctx.saved_tensors
         clampv, qscales = ctx.save_qparamaw
-        int_s = (clampv.to(grad_output.dtype) / 127.)
-        input_f = input8.to(grad_output.dtype) * int_s
+        if grad_output.dtype == torch.bfloat16:
+            input_f = ops.i8_dequant(input8, clampv=clampv)
+        else:
+            input_f = input8.to(grad_output.dtype) * (clampv.to(grad_output.dtype) / 127.)
         return _a8w8_backward(ctx, grad_output, input_f, weight_d, qscales, bias, detach=True)
 
 

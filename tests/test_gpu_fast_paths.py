@@ -92,3 +92,42 @@ def test_philox_fold_equals_generic_kernel(monkeypatch, seed, step, param):
                                                               param_id=param))
         out.append((c, w))
     assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+
+
+# ---- A8W8 linear ------------------------------------------------------------------------------------------------------
+@pytest.mark.parametrize("M,N,K", [(5, 64, 128), (130, 200, 256), (2048, 512, 1024), (64, 4096, 2048)])
+@pytest.mark.parametrize("with_bias", [True, False])
+def test_a8w8_module_launch_equals_the_op_chain(M, N, K, with_bias):
+    from latentq_llm_b200 import ops
+    g = _gen(M + N)
+    x = torch.randn(M, K, device="cuda", generator=g).to(torch.bfloat16)
+    w8 = torch.randint(-128, 128, (N, K), device="cuda", generator=g, dtype=torch.int8)
+    qs = (torch.rand(N, 1, device="cuda", generator=g) * 0.01 + 1e-4).to(torch.bfloat16)
+    bias = (torch.randn(N, device="cuda", generator=g) * 0.1).to(torch.bfloat16) if with_bias else None
+    x8, clampv = ops.act_quant_per_tensor(x)
+    b = ((bias if with_bias else 0 * qs.view(-1)) / (qs.view(-1) if with_bias else 1)).to(torch.bfloat16).contiguous()
+    alpha = (clampv.to(torch.bfloat16) / 127.).float().reshape(1).expand(M).contiguous()
+    ref = ops.gemm_a8w8(x8, w8, alpha, None, 1.0, b) * qs.view(1, -1)
+    assert torch.equal(ops.gemm_a8w8_module(x8, w8, clampv, 1.0, bias, qs), ref)
+    static = ops.gemm_a8w8(x8, w8, torch.full((M,), 2.5 / 127., device="cuda"), None, 1.0, b) * qs.view(1, -1)
+    assert torch.equal(ops.gemm_a8w8_module(x8, w8, None, 2.5 / 127., bias, qs), static)
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 16), (7, 48), (33, 1000), (512, 2048)])
+def test_i8_dequant_equals_the_op_chain(rows, cols):
+    from latentq_llm_b200 import ops
+    g = _gen(rows)
+    c = torch.randint(-128, 128, (rows, cols), device="cuda", generator=g, dtype=torch.int8)
+    qs = (torch.rand(rows, 1, device="cuda", generator=g) * 0.01).to(torch.bfloat16)
+    clampv = torch.tensor([3.140625], device="cuda")
+    assert torch.equal(ops.i8_dequant(c, row_scales=qs), c.to(torch.bfloat16) * qs)
+    assert torch.equal(ops.i8_dequant(c, clampv=clampv), c.to(torch.bfloat16) * (clampv.to(torch.bfloat16) / 127.))
+
+
+@pytest.mark.parametrize("scale", [1.0, 1e-30, 3e4])
+def test_per_tensor_activation_quantizer_equals_the_op_chain(scale):
+    from latentq_llm_b200 import ops
+    x = (torch.randn(64, 4096, device="cuda", generator=_gen(9)) * scale).to(torch.bfloat16)
+    x8, clampv = ops.act_quant_per_tensor(x)
+    ref = (x * 127. / x.max()).round_().clamp_(-128, 127).to(torch.int8)
+    assert float(clampv) == float(x.max()) and torch.equal(x8, ref)
