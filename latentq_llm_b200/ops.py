@@ -12,8 +12,12 @@ from ._lib import (CODEC_NONE, CODEC_THREEFOLD, CODEC_UNIFORM16, DITHER_EXPLICIT
                    DITHER_PHILOX, LQ_BF16, LQ_F32, RequantOpts)
 
 
+_raw_stream, _current_device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
+
+
 def _stream():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    """Handle of torch's current stream (an int; the ctypes signatures make it a pointer)."""
+    return _raw_stream(_current_device())
 
 
 def _dt(t: torch.Tensor) -> int:
@@ -35,7 +39,7 @@ def _chk(t: torch.Tensor, name: str, dtype=None):
 
 
 def _ptr(t):
-    return C.c_void_p(0 if t is None else t.data_ptr())
+    return None if t is None else t.data_ptr()
 
 
 def make_opts(codec=CODEC_THREEFOLD, dither=DITHER_HASH, math_dtype=torch.bfloat16, res_round_bf16=True,
@@ -329,7 +333,7 @@ def _workspace(kind, M, N, K, device):
         need = _ws_need[(kind, M, N, K)] = int(L.lib.lq_gemm_workspace_bytes(kind, M, N, K))
     if need == 0:
         return None, 0
-    key = (device.index, torch.cuda.current_stream().cuda_stream)
+    key = (device.index, _stream())
     ws = _workspaces.get(key)
     if ws is None or ws.numel() < need:
         ws = torch.empty(max(need, 1 << 20), dtype=torch.uint8, device=device)
@@ -556,7 +560,7 @@ def decode_attention(qkv, positions, k_cache, v_cache, Hq, Hkv, hd, scale=None, 
     need = int(L.lib.lq_decode_attention_workspace_bytes(B, Hq, hd, max_len))
     # one workspace per shape and stream: the ticket counters sit behind the partial results, at an offset that depends on
     # the shape, and must be zero when a call starts (every call leaves them zero)
-    key = (qkv.device.index, torch.cuda.current_stream().cuda_stream, B, Hq, hd, max_len)
+    key = (qkv.device.index, _stream(), B, Hq, hd, max_len)
     ws = _attn_ws.get(key)
     if ws is None:
         ws = _attn_ws[key] = torch.zeros(max(need, 1), dtype=torch.uint8, device=qkv.device)

@@ -129,6 +129,16 @@ def _w4_args(qparamw4):
     return scales.contiguous().reshape(-1), zeros.contiguous().reshape(-1), int(shape[0]), int(shape[1])
 
 
+def _apply(fn, *args):
+    """`fn.apply(*args)`; with gradients off and no transform looking on, the function's forward itself (an autograd node costs
+    more host time than a decode-sized launch takes on the GPU).  Forward-mode duals and functorch transforms go through
+    `apply`, which refuses or handles them as before."""
+    if (torch.is_grad_enabled() or torch._C._are_functorch_transforms_active() or torch.autograd.forward_ad._current_level >= 0
+            or torch.compiler.is_compiling()):
+        return fn.apply(*args)
+    return fn.forward(*args)
+
+
 class QLinearFunctionW4(torch.autograd.Function):
     """utils/quant.py:112-146.  forward: x·deq(W)^T (+bias); backward: dY·deq(W), dY^T·x (dense, to `dict_temp`)."""
 
@@ -450,12 +460,12 @@ class QLinearA16W4(nn.Module):
                                                 self.output_features, self.input_features)
             return out.reshape(out_shape)
         fn = QLinearFunctionW4_eval if self.hook_handle is None else QLinearFunctionW4
-        out = fn.apply(x.reshape(-1, x.shape[-1]), self.weight.data, self.weight.qparam, self.bias)
+        out = _apply(fn, x.reshape(-1, x.shape[-1]), self.weight.data, self.weight.qparam, self.bias)
         return out.reshape(out_shape)
 
     def forward_eval(self, x):
         out_shape = x.shape[:-1] + (self.output_features,)
-        out = QLinearFunctionW4_eval.apply(x.reshape(-1, x.shape[-1]), self.weight.data, self.weight.qparam, self.bias)
+        out = _apply(QLinearFunctionW4_eval, x.reshape(-1, x.shape[-1]), self.weight.data, self.weight.qparam, self.bias)
         return out.reshape(out_shape)
 
     def to(self, device: Optional[Union[int, torch.device]]):
