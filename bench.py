@@ -6,8 +6,8 @@
 
 One "step" is one pass of the A16W4 hot path over one batch of synthetic activations: the quantized
 linear forward (y = x·deq(Wq)^T) and grad-input (dx = dy·deq(Wq)) for the four Llama-2-7B linear shapes
-at M = 4096 tokens (8 GEMMs = 16 kernel launches: each grad-input of this size first writes a transposed copy
-of the packed weight and its group parameters with two small kernels, inside the timed region).  Rank r of N runs an independent replica of the same work on its
+at M = 4096 tokens (8 GEMMs = 12 kernel launches: each grad-input of this size first writes a transposed copy
+of the packed weight and its group parameters with one small kernel, inside the timed region).  Rank r of N runs an independent replica of the same work on its
 own GPU ("replicas only": the kernels have no exchange step), the timed region is bracketed by a
 barrier + synchronize, timed with CUDA events on the launching stream, and the maximum over ranks is
 reported.  One JSON line is printed by rank 0.
@@ -137,10 +137,10 @@ def build_layers(torch, ops, seed=1234):
 
 
 def launches_per_layer(m=M_TOKENS):
-    """Kernel launches of one forward + one grad-input: from 3072 tokens on the grad-input is three launches
-    (weight transpose, group-parameter transpose, GEMM) unless the route is switched off."""
+    """Kernel launches of one forward + one grad-input: from 3072 tokens on the grad-input is two launches
+    (transpose of the weight and its group parameters, GEMM) unless the route is switched off."""
     transposed = (m >= 3072 and os.environ.get("LQ_GEMM_DGRAD_TRANSPOSE") != "0" and "LQ_GEMM_A_OPERAND" not in os.environ)
-    return 4 if transposed else 2
+    return 3 if transposed else 2
 
 
 def run_step(ops, layers):

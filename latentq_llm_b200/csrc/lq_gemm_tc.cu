@@ -79,6 +79,7 @@ struct GemmParams {
     int sk_q, sk_r;                // tail units / helpers and tail units % helpers (helper h starts at unit h * q + h * r / helpers)
     int sk_pmax;                   // partial-sum slots per shared tile
     int accumulate;                // weight gradient: out += product (rounded once from the fp32 sum) instead of out = product
+    int qp_staged;                 // forward: group parameters through shared memory (groups of 128, an even number per row, 4-byte aligned)
     const uint4* qpt;              // QPT kernels: per-column group parameters, packed for the dequant (see k_w4_qp_transpose)
 };
 
@@ -157,23 +158,38 @@ constexpr int TA_COLS_PER_STAGE = 32;
 constexpr int FIX_COLS = 16;                                         // balanced mode: token columns per hand-over copy
 constexpr int FIX_COPY_BYTES = FIX_COLS * 32 * 4;                    // one lane quarter of them as fp32: 2 KB
 constexpr int FIX_RING = 8;                                          // staging buffers per lane quarter
-template <int KIND, int TN, int RT, bool TA = false, bool SK = false>
+// Forward: group parameters staged in shared memory, two buffers of one chunk each: 16 k-blocks = 8 groups of 128 for the 128 rows
+// of the tile, word (scale | zero + 128 << 16) of group g and row r at g * QP_PITCH + r (the pitch keeps both the writers, four
+// lanes per row, and the readers, a lane per row, free of bank conflicts).
+constexpr int QP_CHUNK = 16, QP_PITCH = 132;
+constexpr int QP_BUF_BYTES = 8 * QP_PITCH * 4;
+// KBS = k-blocks of 64 per pipeline stage (2: forward with the weight tile in tensor memory, up to 128 tokens).
+template <int KIND, int TN, int RT, bool TA = false, bool SK = false, int KBS = 1>
 struct Cfg {
     static constexpr bool I8 = KIND == KIND_I8;
     static constexpr bool WG = KIND == KIND_WGRAD;      // dense bf16 weight gradient: both operands by TMA, MN-major
     static constexpr bool W4 = !I8 && !WG;
     static_assert(!TA || (W4 && RT == 1), "tensor-memory A operand: A16W4 kinds, one row tile per CTA");
     static constexpr int A_BYTES = TA ? 0 : RT * A_TILE_BYTES;
-    static constexpr int B_TILE_BYTES = TN * ROW_BYTES;
-    static constexpr int RAW_TOTAL = W4 ? RT * RAW_BYTES : 0;
+    static constexpr int B_TILE_BYTES = KBS * TN * ROW_BYTES;
+    static constexpr int RAW_TOTAL = W4 ? RT * KBS * RAW_BYTES : 0;
+    static constexpr int A_COLS = KBS * TA_COLS_PER_STAGE;                 // tensor-memory columns of a stage's weight tile
     static constexpr int STAGE_BYTES = A_BYTES + B_TILE_BYTES + RAW_TOTAL;
     static constexpr int FIX_BYTES = SK ? 4 * FIX_RING * FIX_COPY_BYTES : 0;    // balanced mode: the staging rings
-    static constexpr int STAGES_FIT = (227 * 1024 - 1024 - 1024 - FIX_BYTES) / STAGE_BYTES;
-    static constexpr int STAGES = STAGES_FIT > MAX_STAGES ? MAX_STAGES : STAGES_FIT;
-    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + FIX_BYTES + 1024 /*alignment slack*/ + 1024 /*barriers*/;
+    static constexpr int QP_BYTES = KIND == KIND_FWD ? 2 * QP_BUF_BYTES : 0;
+    static constexpr int STAGES_FIT = (227 * 1024 - 1024 - 1024 - FIX_BYTES - QP_BYTES) / STAGE_BYTES;
+    // Tensor-memory A operand with token tiles up to 192: both accumulators fit beside the A slots, of which there are then
+    // as many as pipeline stages (up to 128 tokens) or one per dequant team (four: the shared-memory ring is deeper than the
+    // slots, a team waits for its own previous stage to retire before it overwrites its slot).  256-token tiles leave room for
+    // one accumulator only; its epilogue is exposed between two tiles.
+    static constexpr bool TA_DOUBLE = TA && !SK && TN <= 192;
+    static constexpr int STAGES_CAP = STAGES_FIT > MAX_STAGES ? MAX_STAGES : STAGES_FIT;
+    static constexpr int STAGES = STAGES_CAP;
+    static constexpr int A_SLOTS = !TA ? 0 : (TA_DOUBLE && 2 * RT * TN + STAGES * A_COLS > 512) ? 4 : STAGES;
+    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + FIX_BYTES + QP_BYTES + 1024 /*alignment slack*/ + 1024 /*barriers*/;
     static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
     static constexpr int ACC_COLS = RT * TN;                               // TMEM columns of one accumulator set
-    static constexpr int TA_COLS = TA ? STAGES * TA_COLS_PER_STAGE : 0;    // one A slot per pipeline stage
+    static constexpr int TA_COLS = A_SLOTS * A_COLS;
     static constexpr int ACC_BUFS = (2 * ACC_COLS + TA_COLS <= 512) ? 2 : 1;   // double-buffered when TMEM allows
     static constexpr int TA_COL0 = ACC_BUFS * ACC_COLS;
     static constexpr int TMEM_NEED = ACC_BUFS * ACC_COLS + TA_COLS;
@@ -181,14 +197,16 @@ struct Cfg {
     // Epilogue warps: one per TMEM lane quarter, or two (the second set behind all other warps, each warp of a pair
     // draining half of the token columns) where the accumulator is wide enough to split.  With a single accumulator
     // buffer the epilogue is exposed time between two tiles; splitting it halves that.
-    static constexpr int EPI_SPLIT = (!SK && TN >= 64) ? 2 : 1;
+    static constexpr int EPI_SPLIT = (!SK && TN >= 32) ? 2 : 1;
     static constexpr int FIRST_EXTRA_EPI = 6 + (W4 ? NUM_DQ_WARPS : 0);
     static constexpr int NUM_WARPS = FIRST_EXTRA_EPI + (EPI_SPLIT - 1) * 4;
     static constexpr int THREADS = NUM_WARPS * 32;
     static constexpr uint32_t TX_BYTES = (uint32_t)(B_TILE_BYTES + (W4 ? RAW_TOTAL : A_BYTES));
-    static constexpr int UMMA_PER_STAGE = 4;   // 128 bytes of contraction per stage / 32 bytes per MMA
+    static constexpr int UMMA_PER_KB = 4;      // 128 bytes of contraction per k-block / 32 bytes per MMA
+    static_assert(KBS == 1 || (KIND == KIND_FWD && TA && !SK && RT == 1), "two k-blocks per stage: forward, weight tile in tensor memory");
     static_assert(TMEM_NEED <= 512 && STAGES >= 2, "tile configuration does not fit");
     static_assert(!W4 || STAGES >= 4, "the four dequant teams need at least four pipeline stages");
+    static_assert(!TA || A_SLOTS == STAGES || A_SLOTS == 4, "one A slot per stage, or one per team");
 };
 
 struct SmemCtl {
@@ -217,39 +235,33 @@ __device__ __forceinline__ uint32_t lop_nib(uint32_t w) {
     asm("lop3.b32 %0, %1, 0x000F000F, 0x43004300, 0xEA;" : "=r"(r) : "r"(w));
     return r;
 }
+// The forward's raw tile (32 bytes per row) comes with the 32-byte swizzle: the two 16-byte halves of rows 4..7 of every eight are
+// swapped, so that the 16-byte reads of eight lanes, a row each, hit all banks once instead of half of them twice.  (Two k-blocks
+// per stage: 64 bytes per row, 64-byte swizzle, piece ^ (row / 2 % 4).)
+__device__ __forceinline__ int raw_swap(int row) { return (row >> 2) & 1; }
 __device__ __forceinline__ uint4 dequant8(uint32_t w, __nv_bfloat162 z128, __nv_bfloat162 s2) {
-    const uint32_t p15 = lop_nib(w);             // (c1, c5)
-    const uint32_t p04 = lop_nib(w >> 4);        // (c0, c4)
-    const uint32_t p37 = lop_nib(w >> 8);        // (c3, c7)
-    const uint32_t p26 = lop_nib(w >> 12);       // (c2, c6)
-    uint32_t d15 = bf2_as_u32(__hmul2_rn(__hsub2_rn(u32_as_bf2(p15), z128), s2));
-    uint32_t d04 = bf2_as_u32(__hmul2_rn(__hsub2_rn(u32_as_bf2(p04), z128), s2));
-    uint32_t d37 = bf2_as_u32(__hmul2_rn(__hsub2_rn(u32_as_bf2(p37), z128), s2));
-    uint32_t d26 = bf2_as_u32(__hmul2_rn(__hsub2_rn(u32_as_bf2(p26), z128), s2));
+    const uint32_t h = w >> 4;                   // even codes in the low nibbles of h, odd codes in those of w
+    const uint32_t p01 = lop_nib(__byte_perm(h, w, 0x5410)), p23 = lop_nib(__byte_perm(h, w, 0x6521));
+    const uint32_t p45 = lop_nib(__byte_perm(h, w, 0x7632)), p67 = lop_nib(__byte_perm(h, w, 0x7733));
     uint4 o;
-    o.x = __byte_perm(d04, d15, 0x5410);   // (c0, c1)
-    o.y = __byte_perm(d26, d37, 0x5410);   // (c2, c3)
-    o.z = __byte_perm(d04, d15, 0x7632);   // (c4, c5)
-    o.w = __byte_perm(d26, d37, 0x7632);   // (c6, c7)
+    o.x = bf2_as_u32(__hmul2_rn(__hsub2_rn(u32_as_bf2(p01), z128), s2));
+    o.y = bf2_as_u32(__hmul2_rn(__hsub2_rn(u32_as_bf2(p23), z128), s2));
+    o.z = bf2_as_u32(__hmul2_rn(__hsub2_rn(u32_as_bf2(p45), z128), s2));
+    o.w = bf2_as_u32(__hmul2_rn(__hsub2_rn(u32_as_bf2(p67), z128), s2));
     return o;
 }
 
 // The same with a scale and a zero point of its own for every code: sp / zp hold (s, z + 128) of the pairs
-// (c0,c4) (c1,c5) (c2,c6) (c3,c7) in x, y, z, w - the order the extraction produces.
+// (c0,c1) (c2,c3) (c4,c5) (c6,c7) in x, y, z, w.
 __device__ __forceinline__ uint4 dequant8t(uint32_t w, const uint4& zp, const uint4& sp) {
-    const uint32_t p15 = lop_nib(w);             // (c1, c5)
-    const uint32_t p04 = lop_nib(w >> 4);        // (c0, c4)
-    const uint32_t p37 = lop_nib(w >> 8);        // (c3, c7)
-    const uint32_t p26 = lop_nib(w >> 12);       // (c2, c6)
-    uint32_t d15 = bf2_as_u32(__hmul2_rn(__hsub2_rn(u32_as_bf2(p15), u32_as_bf2(zp.y)), u32_as_bf2(sp.y)));
-    uint32_t d04 = bf2_as_u32(__hmul2_rn(__hsub2_rn(u32_as_bf2(p04), u32_as_bf2(zp.x)), u32_as_bf2(sp.x)));
-    uint32_t d37 = bf2_as_u32(__hmul2_rn(__hsub2_rn(u32_as_bf2(p37), u32_as_bf2(zp.w)), u32_as_bf2(sp.w)));
-    uint32_t d26 = bf2_as_u32(__hmul2_rn(__hsub2_rn(u32_as_bf2(p26), u32_as_bf2(zp.z)), u32_as_bf2(sp.z)));
+    const uint32_t h = w >> 4;
+    const uint32_t p01 = lop_nib(__byte_perm(h, w, 0x5410)), p23 = lop_nib(__byte_perm(h, w, 0x6521));
+    const uint32_t p45 = lop_nib(__byte_perm(h, w, 0x7632)), p67 = lop_nib(__byte_perm(h, w, 0x7733));
     uint4 o;
-    o.x = __byte_perm(d04, d15, 0x5410);   // (c0, c1)
-    o.y = __byte_perm(d26, d37, 0x5410);   // (c2, c3)
-    o.z = __byte_perm(d04, d15, 0x7632);   // (c4, c5)
-    o.w = __byte_perm(d26, d37, 0x7632);   // (c6, c7)
+    o.x = bf2_as_u32(__hmul2_rn(__hsub2_rn(u32_as_bf2(p01), u32_as_bf2(zp.x)), u32_as_bf2(sp.x)));
+    o.y = bf2_as_u32(__hmul2_rn(__hsub2_rn(u32_as_bf2(p23), u32_as_bf2(zp.y)), u32_as_bf2(sp.y)));
+    o.z = bf2_as_u32(__hmul2_rn(__hsub2_rn(u32_as_bf2(p45), u32_as_bf2(zp.z)), u32_as_bf2(sp.z)));
+    o.w = bf2_as_u32(__hmul2_rn(__hsub2_rn(u32_as_bf2(p67), u32_as_bf2(zp.w)), u32_as_bf2(sp.w)));
     return o;
 }
 
@@ -260,16 +272,16 @@ __device__ __forceinline__ uint4 dequant8t(uint32_t w, const uint4& zp, const ui
 //   shared-memory placement is bound by the shared-memory port (171 instead of 138 cycles per MMA).  With a
 //   transposed copy Wt[K, N] (codes packed along n) the grad-input IS the forward kernel: dx = dy . Wt^T.  Scales
 //   and zero points then differ per contraction element (they belong to (n, k / group)), so they are laid out
-//   per (k group, 8 n) in exactly the order dequant8t consumes: 32 bytes = (s04 s15 s26 s37)(z04 z15 z26 z37), z
+//   per (k group, 8 n) as dequant8t consumes them: 32 bytes = (s01 s23 s45 s67)(z01 z23 z45 z67), z
 //   already offset by 128.  Both kernels run once per grad-input call (the weights may have changed since the last).
 // ---------------------------------------------------------------------------------------------
 // One CTA transposes a tile of 64 n x 256 k: codes go to shared memory as words of four consecutive k (one byte per
 // code), a thread then owns four k and sixteen n: (even n << 4 | odd n) byte-wise gives the packed output bytes of all
 // four k at once, three byte permutes per output word sort them into the four rows it writes (8 bytes each; the four
 // threads of a k share a 32-byte segment).
-__global__ void __launch_bounds__(256) k_w4_transpose(const uint8_t* __restrict__ in, uint8_t* __restrict__ out, int N, int K) {
+__device__ __forceinline__ void w4_transpose_tile(const uint8_t* __restrict__ in, uint8_t* __restrict__ out, int N, int K, int n0, int k0) {
     __shared__ uint32_t t[64][65];                        // [n][k / 4], one word of padding
-    const int n0 = blockIdx.y * 64, k0 = blockIdx.x * 256, i = threadIdx.x;
+    const int i = threadIdx.x;
     {
         const int n = i >> 2, seg = i & 3;                // 32 bytes = 64 codes of row n0 + n, k = k0 + seg * 64 ..
         const uint4* src = reinterpret_cast<const uint4*>(in + (size_t)(n0 + n) * (K / 2) + (k0 / 2) + seg * 32);
@@ -301,9 +313,8 @@ __global__ void __launch_bounds__(256) k_w4_transpose(const uint8_t* __restrict_
     }
 }
 // one thread per (8 n, k group); consecutive threads take consecutive groups, so the 2-byte reads of a warp are contiguous
-__global__ void __launch_bounds__(256) k_w4_qp_transpose(const __nv_bfloat16* __restrict__ scales, const __nv_bfloat16* __restrict__ zeros,
-                                                         uint4* __restrict__ qpt, int N, int G) {
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void w4_qp_transpose_entry(const __nv_bfloat16* __restrict__ scales, const __nv_bfloat16* __restrict__ zeros,
+                                                      uint4* __restrict__ qpt, int N, int G, int idx) {
     if (idx >= G * (N / 8)) return;
     const int n8 = idx / G, g = idx - n8 * G, n = n8 * 8;
     const unsigned short* sp = reinterpret_cast<const unsigned short*>(scales);
@@ -315,21 +326,30 @@ __global__ void __launch_bounds__(256) k_w4_qp_transpose(const __nv_bfloat16* __
         zv[j] = *reinterpret_cast<const unsigned short*>(&z);
     }
     uint4* dst = qpt + ((size_t)g * (size_t)(N / 8) + (size_t)n8) * 2;
-    dst[0] = make_uint4(sv[0] | sv[4] << 16, sv[1] | sv[5] << 16, sv[2] | sv[6] << 16, sv[3] | sv[7] << 16);
-    dst[1] = make_uint4(zv[0] | zv[4] << 16, zv[1] | zv[5] << 16, zv[2] | zv[6] << 16, zv[3] | zv[7] << 16);
+    dst[0] = make_uint4(sv[0] | sv[1] << 16, sv[2] | sv[3] << 16, sv[4] | sv[5] << 16, sv[6] | sv[7] << 16);
+    dst[1] = make_uint4(zv[0] | zv[1] << 16, zv[2] | zv[3] << 16, zv[4] | zv[5] << 16, zv[6] | zv[7] << 16);
+}
+// Both in one launch: blocks [0, tiles) transpose codes, the others group parameters.
+__global__ void __launch_bounds__(256) k_w4_transpose(const uint8_t* __restrict__ in, uint8_t* __restrict__ out, const __nv_bfloat16* __restrict__ scales,
+                                                      const __nv_bfloat16* __restrict__ zeros, uint4* __restrict__ qpt, int N, int K, int tiles) {
+    const int b = (int)blockIdx.x, per_row = K / 256;
+    if (b < tiles) w4_transpose_tile(in, out, N, K, (b / per_row) * 64, (b % per_row) * 256);
+    else w4_qp_transpose_entry(scales, zeros, qpt, N, K / 128, (b - tiles) * 256 + (int)threadIdx.x);
 }
 
-// Epilogue constants of one output channel of the int8 kernels.  With post_scale the result is what the module's op chain
+// Epilogue constants of one output channel of the int8 kernels.  With a channel scale behind it (POST) the result is what the module's op chain
 // bf16(bf16(acc * alpha + bf16(bias / q)) * q), alpha = bf16(clampv / 127), leaves (utils/quant.py:268-271; a tensor divided by
 // a number is multiplied by its fp32 reciprocal there).
 struct I8Epi { float cs, bias, alpha, post; };
+template <bool POST>
 __device__ __forceinline__ I8Epi i8_epilogue(const GemmParams& p, int r, bool r_ok) {
     I8Epi e;
     e.cs = (p.col_scale && r_ok) ? __ldg(p.col_scale + r) : 1.0f;
     e.bias = (p.bias && r_ok) ? __bfloat162float(p.bias[r]) : 0.0f;
-    e.alpha = p.clampv ? bf16r(__fmul_rn(bf16r(__ldg(p.clampv)), 1.0f / 127.0f)) : p.alpha;
+    e.alpha = p.alpha;
     e.post = 1.0f;
-    if (p.post_scale) {
+    if (POST) {
+        if (p.clampv) e.alpha = bf16r(__fmul_rn(bf16r(__ldg(p.clampv)), 1.0f / 127.0f));
         e.post = r_ok ? __bfloat162float(p.post_scale[r]) : 1.0f;
         e.bias = p.bias ? bf16r(__fdiv_rn(e.bias, e.post)) : bf16r(__fmul_rn(0.0f, e.post));
     }
@@ -340,15 +360,16 @@ __device__ __forceinline__ float i8_scaled(const I8Epi& e, float f) { return __f
 // ---------------------------------------------------------------------------------------------
 // The kernel
 // ---------------------------------------------------------------------------------------------
-template <int KIND, int TN, int RT, bool TA, bool SK, bool QPT = false>
-__global__ void __launch_bounds__(Cfg<KIND, TN, RT, TA, SK>::THREADS, 1)
+template <int KIND, int TN, int RT, bool TA, bool SK, bool QPT = false, int KBS = 1>
+__global__ void __launch_bounds__(Cfg<KIND, TN, RT, TA, SK, KBS>::THREADS, 1)
 k_gemm(const __grid_constant__ CUtensorMap map_tok, const __grid_constant__ CUtensorMap map_w, const GemmParams p) {
     static_assert(!SK || (KIND != KIND_I8 && RT == 1 && TN % FIX_COLS == 0), "balanced mode: A16W4 kinds, one row tile per CTA");
-    static_assert(!QPT || (KIND == KIND_FWD && TA && RT == 1), "per-column group parameters: forward kernel, weight tile in tensor memory");
-    using C = Cfg<KIND, TN, RT, TA, SK>;
+    static_assert(!QPT || KIND == KIND_I8 || (KIND == KIND_FWD && TA && RT == 1), "per-column group parameters: forward kernel, weight tile in tensor memory");
+    constexpr bool POST = KIND == KIND_I8 && QPT;             // int8: a channel scale behind the epilogue
+    using C = Cfg<KIND, TN, RT, TA, SK, KBS>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    SmemCtl* ctl = reinterpret_cast<SmemCtl*>(smem + C::STAGES * C::STAGE_BYTES + C::FIX_BYTES);
+    SmemCtl* ctl = reinterpret_cast<SmemCtl*>(smem + C::STAGES * C::STAGE_BYTES + C::FIX_BYTES + C::QP_BYTES);
     volatile int* abort_flag = &ctl->abort_flag;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -398,7 +419,7 @@ k_gemm(const __grid_constant__ CUtensorMap map_tok, const __grid_constant__ CUte
             Seg sg;
             while (ok && walk.next(p, sg)) {
                 const int r_tile = sg.r_tile, t_tile = sg.t_tile;
-                for (int kb = sg.kb0; kb < sg.kb1; ++kb) {
+                for (int kb = sg.kb0; kb < sg.kb1; kb += KBS) {
                     if (!(ok = mbar_wait_t(smem_u32(&ctl->empty[stage]), phase ^ 1u, abort_flag, prof, w_empty))) break;
                     const uint32_t bar = smem_u32(&ctl->full[stage]);
                     if (leader) {
@@ -421,7 +442,9 @@ k_gemm(const __grid_constant__ CUtensorMap map_tok, const __grid_constant__ CUte
                             for (int h = 0; h < TN / 64; ++h)
                                 tma_load_2d(b_tile(stage) + (uint32_t)(h * 8192), &map_tok, t_tile * TN + h * 64, kb * 64, bar);
                         } else {
-                            tma_load_2d(b_tile(stage), &map_tok, kb * (C::I8 ? 128 : 64), t_tile * TN, bar);
+#pragma unroll
+                            for (int h = 0; h < KBS; ++h)
+                                tma_load_2d(b_tile(stage) + (uint32_t)(h * TN * ROW_BYTES), &map_tok, (kb + h) * (C::I8 ? 128 : 64), t_tile * TN, bar);
                         }
                     }
                     if (++stage == C::STAGES) { stage = 0; phase ^= 1u; }
@@ -442,6 +465,7 @@ k_gemm(const __grid_constant__ CUtensorMap map_tok, const __grid_constant__ CUte
             const bool leader = elect_one_sync();
             int stage = 0; uint32_t phase = 0;
             int acc = 0; uint32_t acc_phase = 0;
+            int slot = 0;                                   // A slot of the stage when there are fewer slots than stages
             bool ok = true;
             long long w_full = 0, w_aready = 0, w_acc = 0;
             const long long t_role = prof ? clock64() : 0;
@@ -452,7 +476,7 @@ k_gemm(const __grid_constant__ CUtensorMap map_tok, const __grid_constant__ CUte
                 if (!(ok = mbar_wait_t(smem_u32(&ctl->acc_empty[acc]), acc_phase ^ 1u, abort_flag, prof, w_acc))) break;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + (uint32_t)(acc * C::ACC_COLS);
-                for (int kb = kb0; kb < kb1; ++kb) {
+                for (int kb = kb0; kb < kb1; kb += KBS) {
                     // A16W4: the team that converted the stage waited for its TMA data before it started, so its
                     // `a_ready` arrival also covers the token tile: one barrier round trip per stage instead of two
                     if (C::W4) { if (!(ok = mbar_wait_t(smem_u32(&ctl->a_ready[stage]), phase, abort_flag, prof, w_aready))) break; }
@@ -467,23 +491,27 @@ k_gemm(const __grid_constant__ CUtensorMap map_tok, const __grid_constant__ CUte
                     const uint32_t first = kb > kb0 ? 1u : 0u;
                     if (leader) {
                         if (TA) {
-                            const uint32_t a_tmem = tmem_base + (uint32_t)(C::TA_COL0 + stage * TA_COLS_PER_STAGE);
+                            const uint32_t a_tmem = tmem_base + (uint32_t)(C::TA_COL0 + (C::A_SLOTS == C::STAGES ? stage : slot) * C::A_COLS);
 #pragma unroll
-                            for (int kk = 0; kk < C::UMMA_PER_STAGE; ++kk)
-                                umma_ta(d_tmem, a_tmem + (uint32_t)(kk * 8), b_desc + (uint64_t)(kk * b_step), IDESC, kk > 0 ? 1u : first);
+                            for (int h = 0; h < KBS; ++h)
+#pragma unroll
+                                for (int kk = 0; kk < C::UMMA_PER_KB; ++kk)
+                                    umma_ta(d_tmem, a_tmem + (uint32_t)(h * TA_COLS_PER_STAGE + kk * 8),
+                                            b_desc + (uint64_t)(h * (TN * ROW_BYTES >> 4) + kk * b_step), IDESC, h + kk > 0 ? 1u : first);
                         } else {
 #pragma unroll
                             for (int r = 0; r < RT; ++r) {
                                 const uint64_t a_desc = (KIND == KIND_DGRAD || C::WG) ? make_smem_desc(a_tile(stage, r), 8192, 1024)
                                                                                       : make_smem_desc(a_tile(stage, r), 16, 1024);
 #pragma unroll
-                                for (int kk = 0; kk < C::UMMA_PER_STAGE; ++kk)
+                                for (int kk = 0; kk < C::UMMA_PER_KB; ++kk)
                                     umma<C::I8>(d_tmem + (uint32_t)(r * TN), a_desc + (uint64_t)(kk * a_step), b_desc + (uint64_t)(kk * b_step),
                                                 IDESC, kk > 0 ? 1u : first);
                             }
                         }
                         umma_commit(smem_u32(&ctl->empty[stage]));
                     }
+                    slot = (slot + 1) & 3;
                     if (++stage == C::STAGES) { stage = 0; phase ^= 1u; }
                 }
                 if (!ok) break;
@@ -590,7 +618,7 @@ k_gemm(const __grid_constant__ CUtensorMap map_tok, const __grid_constant__ CUte
                 const int r = (r_tile * RT + rr) * TILE_R + quad * 32 + lane;
                 const bool r_ok = r < p.R;
                 I8Epi e8 = {};
-                if (C::I8) e8 = i8_epilogue(p, r, r_ok);
+                if (C::I8) e8 = i8_epilogue<POST>(p, r, r_ok);
                 const float bias = (!C::I8 && p.bias && r_ok) ? __bfloat162float(p.bias[r]) : 0.0f;
                 // tokens per TMEM read-out: the int8 kernel has registers to spare (6 warps) and halves the number of
                 // load-wait round trips; the A16W4 kernels run at the register cap of a 22-warp CTA
@@ -688,7 +716,7 @@ k_gemm(const __grid_constant__ CUtensorMap map_tok, const __grid_constant__ CUte
                                 float f0 = (float)(int32_t)v[2 * i], f1 = (float)(int32_t)v[2 * i + 1];
                                 if (p.row_scale) { f0 = __fmul_rn(f0, rs[2 * i]); f1 = __fmul_rn(f1, rs[2 * i + 1]); }
                                 pk[i] = bf2_as_u32(__floats2bfloat162_rn(i8_scaled(e8, f0), i8_scaled(e8, f1)));
-                                if (p.post_scale)
+                                if (POST)
                                     pk[i] = bf2_as_u32(__floats2bfloat162_rn(__fmul_rn(__uint_as_float(pk[i] << 16), e8.post),
                                                                              __fmul_rn(__uint_as_float(pk[i] & 0xffff0000u), e8.post)));
                             }
@@ -718,7 +746,7 @@ k_gemm(const __grid_constant__ CUtensorMap map_tok, const __grid_constant__ CUte
                             float f = (float)a;
                             if (p.row_scale) f = __fmul_rn(f, __ldg(p.row_scale + t));
                             f = i8_scaled(e8, f);
-                            p.out[o] = __float2bfloat16_rn(p.post_scale ? __fmul_rn(bf16r(f), e8.post) : f);
+                            p.out[o] = __float2bfloat16_rn(POST ? __fmul_rn(bf16r(f), e8.post) : f);
                         } else {
                             float f = bf16r(__uint_as_float(v[j]));          // mm output is bf16, bias added after
                             p.out[o] = __float2bfloat16_rn(p.bias ? __fadd_rn(f, bias) : f);
@@ -775,7 +803,7 @@ k_gemm(const __grid_constant__ CUtensorMap map_tok, const __grid_constant__ CUte
             // (scale | zero << 16) as raw bf16 bits for this thread's two 32-element slots of row tile r at position q
             auto load_qp2 = [&](const Pos& q, int r, uint32_t& a, uint32_t& b) {
                 a = b = 0u;
-                if (QPT || !q.valid) return;
+                if (!q.valid) return;
                 int wrow, k0, k1;
                 if (TA && KIND == KIND_DGRAD) {            // rows n_lane and n_lane+32, one k group per warp
                     wrow = q.kb * 64 + lane; k0 = k1 = q.r_tile * TILE_R + quarter * 32;
@@ -795,6 +823,138 @@ k_gemm(const __grid_constant__ CUtensorMap map_tok, const __grid_constant__ CUte
                 b = a;
                 if (g1 != g0) b = (uint32_t)__ldg(sp + g1) | ((uint32_t)__ldg(zp + g1) << 16);   // groups of 64 and up: one pair per thread
             };
+            const __nv_bfloat162 c128 = __float2bfloat162_rn(128.0f);
+            bool ok = true;
+            long long w_dq = 0;
+            const long long t_role = prof ? clock64() : 0;
+            // waits until stage `cnt` of the CTA can be converted
+            auto stage_ready = [&](uint32_t cnt, int stage) -> bool {
+                const uint32_t phase = (cnt / (uint32_t)C::STAGES) & 1u;
+                // This team did not take part in the stage's previous use (another team converted it), so it first
+                // waits, like the producer, until that use has been consumed; only then is the parity of the `full`
+                // wait unambiguous.  (Needs STAGES >= number of teams: then the stage's use before the previous one
+                // is known to be over, because the producer had to see it retired before it could fill this team's
+                // own previous stage.)
+                // With a stage count that is a multiple of the four teams a team meets the same stages every round
+                // and needs no such wait: `full` completing already implies that the producer saw the stage retired.
+                bool r = (C::STAGES % 4 == 0 || mbar_wait_t(smem_u32(&ctl->empty[stage]), phase ^ 1u, abort_flag, prof, w_dq)) &&
+                         mbar_wait_t(smem_u32(&ctl->full[stage]), phase, abort_flag, prof, w_dq);
+                // fewer A slots than stages: the team's slot is free once the MMAs of its own previous stage retired
+                if (TA && C::A_SLOTS < C::STAGES && r && cnt >= 4u) {
+                    const uint32_t prev = cnt - 4u;
+                    r = mbar_wait_t(smem_u32(&ctl->empty[prev % (uint32_t)C::STAGES]), (prev / (uint32_t)C::STAGES) & 1u, abort_flag, prof, w_dq);
+                }
+                return __all_sync(0xffffffffu, r) != 0;                     // the TMEM store is warp-collective
+            };
+            auto stage_done = [&](int stage) {
+                if (TA) { tmem_st_wait(); tc_fence_before(); } else { fence_proxy_async(); }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&ctl->a_ready[stage]));
+            };
+            // Forward with groups of 128 (an even number per row): the group parameters come through shared memory.  Read where
+            // they are needed, one 2-byte load per lane, row and stage touches 32 cache lines a warp and instruction: 256
+            // L1 cycles per stage, which bounded the kernel below 256 tokens.  Here the 512 threads fetch a chunk of 16
+            // k-blocks together, four lanes per row, one chunk ahead of its use.
+            // (QPT: the parameters of a stage's 64 contraction elements, the same for every row of the tile's k group, come the
+            // same way: 256 bytes per stage, one 16-byte piece per thread.)
+            if constexpr (KIND == KIND_FWD && RT == 1) {
+                if (QPT || p.qp_staged) {
+                    uint32_t* const qpb = reinterpret_cast<uint32_t*>(smem + C::STAGES * C::STAGE_BYTES + C::FIX_BYTES);
+                    struct Chunk { SegWalk<SK> walk; int kb, end, kb1, r_tile; bool valid; };
+                    auto next_chunk = [&](Chunk& c) {
+                        c.kb = c.end;
+                        if (c.kb >= c.kb1) {
+                            Seg sg;
+                            if (!c.walk.next(p, sg)) { c.valid = false; return; }
+                            c.kb = sg.kb0; c.kb1 = sg.kb1; c.r_tile = sg.r_tile;
+                        }
+                        c.end = min(c.kb1, (c.kb | (QP_CHUNK - 1)) + 1);
+                    };
+                    const int q_row = (warp - 6) * 8 + (lane >> 2), q_col = (lane & 3) * 2;
+                    const int dq_tid = (warp - 6) * 32 + lane;
+                    uint32_t ls = 0u, lz = 0u;
+                    uint4 lq = make_uint4(0u, 0u, 0u, 0u);
+                    auto fetch = [&](const Chunk& c) {
+                        if (QPT) {
+                            if (c.valid && dq_tid < (c.end - c.kb) * 16)
+                                lq = __ldg(p.qpt + ((size_t)c.r_tile * (size_t)(p.C >> 3) + (size_t)c.kb * 8) * 2 + dq_tid);
+                            return;
+                        }
+                        const int wrow = c.r_tile * TILE_R + q_row, g0 = (c.kb / QP_CHUNK) * 8 + q_col;
+                        ls = lz = 0u;
+                        if (c.valid && wrow < p.R && g0 < groups_per_row) {          // groups_per_row is even
+                            const size_t at = (size_t)wrow * groups_per_row + g0;
+                            ls = __ldg(reinterpret_cast<const uint32_t*>(p.scales + at)); lz = __ldg(reinterpret_cast<const uint32_t*>(p.zeros + at));
+                        }
+                    };
+                    auto stash = [&](int buf) {
+                        if (QPT) {
+                            if (dq_tid < QP_CHUNK * 16) reinterpret_cast<uint4*>(qpb + buf * (8 * QP_PITCH))[dq_tid] = lq;
+                            return;
+                        }
+                        const uint32_t z = bf2_as_u32(__hadd2_rn(u32_as_bf2(lz), c128));
+                        uint32_t* d = qpb + buf * (8 * QP_PITCH) + q_col * QP_PITCH + q_row;
+                        d[0] = __byte_perm(ls, z, 0x5410); d[QP_PITCH] = __byte_perm(ls, z, 0x7632);
+                    };
+                    auto team_barrier = [] { asm volatile("bar.sync 1, 512;" ::: "memory"); };       // the 16 dequant warps
+                    Chunk cur{SegWalk<SK>(p), 0, 0, 0, 0, true};
+                    next_chunk(cur);
+                    fetch(cur); stash(0);
+                    team_barrier();
+                    const int my_row = TA ? quarter * 32 + lane : tt;
+                    uint32_t base = 0u;
+                    int buf = 0;
+                    while (cur.valid) {
+                        Chunk nxt = cur;
+                        next_chunk(nxt);
+                        fetch(nxt);
+                        const int n = (cur.end - cur.kb) / KBS;
+                        for (int i = (int)((uint32_t)(team - (int)base) & 3u); i < n && ok; i += 4) {    // (an aborted team still meets the barriers)
+                            const uint32_t cnt = base + (uint32_t)i;
+                            const int stage = (int)(cnt % (uint32_t)C::STAGES);
+                            if (!(ok = stage_ready(cnt, stage))) break;
+                            const uint8_t* raw = raw_tile(stage, 0) + my_row * (32 * KBS);
+                            if constexpr (QPT) {
+                                const uint32_t dst = ta_addr + (uint32_t)((C::A_SLOTS == C::STAGES ? stage : team) * C::A_COLS);
+                                const uint4 r0 = reinterpret_cast<const uint4*>(raw)[raw_swap(my_row)], r1 = reinterpret_cast<const uint4*>(raw)[raw_swap(my_row) ^ 1];
+                                const uint4* qp = reinterpret_cast<const uint4*>(qpb + buf * (8 * QP_PITCH)) + i * 16;
+                                const uint32_t wq[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};
+#pragma unroll
+                                for (int h = 0; h < 8; h += 2)
+                                    tmem_st8(dst + (uint32_t)(4 * h), dequant8t(wq[h], qp[2 * h + 1], qp[2 * h]), dequant8t(wq[h + 1], qp[2 * h + 3], qp[2 * h + 2]));
+                            } else {
+                                const uint32_t qp = qpb[buf * (8 * QP_PITCH) + (((cur.kb + i * KBS) >> 1) & 7) * QP_PITCH + my_row];
+                                const __nv_bfloat162 s2 = u32_as_bf2(__byte_perm(qp, qp, 0x1010)), z2 = u32_as_bf2(__byte_perm(qp, qp, 0x3232));
+                                const uint32_t dst = ta_addr + (uint32_t)((C::A_SLOTS == C::STAGES ? stage : team) * C::A_COLS);
+                                const int swz = my_row & 7;
+                                uint4 r[2 * KBS];
+#pragma unroll
+                                for (int h = 0; h < 2 * KBS; ++h)
+                                    r[h] = reinterpret_cast<const uint4*>(raw)[KBS == 2 ? h ^ ((my_row >> 1) & 3) : h ^ raw_swap(my_row)];
+#pragma unroll
+                                for (int h = 0; h < 2 * KBS; ++h) {
+                                    const uint4 d0 = dequant8(r[h].x, z2, s2), d1 = dequant8(r[h].y, z2, s2);
+                                    const uint4 d2 = dequant8(r[h].z, z2, s2), d3 = dequant8(r[h].w, z2, s2);
+                                    if (TA) {
+                                        tmem_st8(dst + (uint32_t)(16 * h), d0, d1); tmem_st8(dst + (uint32_t)(16 * h + 8), d2, d3);
+                                    } else {
+                                        uint8_t* d = smem + stage * C::STAGE_BYTES + my_row * ROW_BYTES;
+                                        *reinterpret_cast<uint4*>(d + (((4 * h + 0) ^ swz) << 4)) = d0; *reinterpret_cast<uint4*>(d + (((4 * h + 1) ^ swz) << 4)) = d1;
+                                        *reinterpret_cast<uint4*>(d + (((4 * h + 2) ^ swz) << 4)) = d2; *reinterpret_cast<uint4*>(d + (((4 * h + 3) ^ swz) << 4)) = d3;
+                                    }
+                                }
+                            }
+                            stage_done(stage);
+                        }
+                        base += (uint32_t)n;
+                        buf ^= 1;
+                        if (nxt.valid) stash(buf);
+                        team_barrier();
+                        cur = nxt;
+                    }
+                }
+            }
+            if (KBS == 1 && !QPT && !(KIND == KIND_FWD && RT == 1 && p.qp_staged)) {
             constexpr int PF = 2;                                          // own stages of qparam prefetch
             Pos cur{SegWalk<SK>(p), 0, 0, 0, true};
             advance(cur, 0);                                               // opens the first segment (kb == kb1 == 0)
@@ -808,10 +968,6 @@ k_gemm(const __grid_constant__ CUtensorMap map_tok, const __grid_constant__ CUte
                 advance(pre, 4);
             }
             uint32_t cnt = (uint32_t)team;
-            bool ok = true;
-            long long w_dq = 0;
-            const long long t_role = prof ? clock64() : 0;
-            const __nv_bfloat162 c128 = __float2bfloat162_rn(128.0f);
             while (ok && cur.valid) {
 #pragma unroll
                 for (int u = 0; u < PF; ++u) {
@@ -821,20 +977,12 @@ k_gemm(const __grid_constant__ CUtensorMap map_tok, const __grid_constant__ CUte
                     for (int r = 0; r < RT; ++r) { ca[r] = qa[u][r]; cb[r] = qb[u][r]; load_qp2(pre, r, qa[u][r], qb[u][r]); }
                     advance(pre, 4);
                     const int stage = (int)(cnt % (uint32_t)C::STAGES);
-                    const uint32_t phase = (cnt / (uint32_t)C::STAGES) & 1u;
-                    // This team did not take part in the stage's previous use (another team converted it), so it first
-                    // waits, like the producer, until that use has been consumed; only then is the parity of the `full`
-                    // wait unambiguous.  (Needs STAGES >= number of teams: then the stage's use before the previous one
-                    // is known to be over, because the producer had to see it retired before it could fill this team's
-                    // own previous stage.)
-                    // With a stage count that is a multiple of the four teams a team meets the same stages every round
-                    // and needs no such wait: `full` completing already implies that the producer saw the stage retired.
-                    ok = (C::STAGES % 4 == 0 || mbar_wait_t(smem_u32(&ctl->empty[stage]), phase ^ 1u, abort_flag, prof, w_dq)) &&
-                         mbar_wait_t(smem_u32(&ctl->full[stage]), phase, abort_flag, prof, w_dq);
+                    if (!(ok = stage_ready(cnt, stage))) break;
+                    const int slot = C::A_SLOTS == C::STAGES ? stage : team;
                     ok = __all_sync(0xffffffffu, ok) != 0;                 // the TMEM store below is warp-collective
                     if (!ok) break;
                     if (TA && KIND == KIND_DGRAD) {
-                        const uint32_t dst = ta_addr + (uint32_t)(stage * TA_COLS_PER_STAGE);
+                        const uint32_t dst = ta_addr + (uint32_t)(slot * TA_COLS_PER_STAGE);
                         const int kk = quarter * 32 + lane;
                         const uint8_t* rp = raw_tile(stage, 0) + (kk >> 1);
                         const uint32_t sh = (kk & 1) ? 0u : 4u;            // even k sits in the high nibble
@@ -860,25 +1008,12 @@ k_gemm(const __grid_constant__ CUtensorMap map_tok, const __grid_constant__ CUte
                             const __nv_bfloat162 s2a = u32_as_bf2(__byte_perm(ca[r], ca[r], 0x1010)), s2b = u32_as_bf2(__byte_perm(cb[r], cb[r], 0x1010));
                             const __nv_bfloat162 za = __hadd2_rn(u32_as_bf2(__byte_perm(ca[r], ca[r], 0x3232)), c128);
                             const __nv_bfloat162 zb = __hadd2_rn(u32_as_bf2(__byte_perm(cb[r], cb[r], 0x3232)), c128);
-                            const int raw_off = TA ? (quarter * 32 + lane) * 32 : tt * 32;   // dgrad: (tt/2)*64 + (tt%2)*32 == tt*32
-                            const uint4* rp = reinterpret_cast<const uint4*>(raw_tile(stage, r) + raw_off);
-                            const uint4 r0 = rp[0], r1 = rp[1];
-                            if (TA && QPT) {
-                                // group parameters of the stage's 64 contraction elements (the same for every row of the
-                                // tile's k group: the loads of a warp are one broadcast each), one word ahead of their use
-                                const uint32_t dst = ta_addr + (uint32_t)(stage * TA_COLS_PER_STAGE);
-                                const uint4* qp = p.qpt + ((size_t)cur.r_tile * (size_t)(p.C >> 3) + (size_t)cur.kb * 8) * 2;
-                                const uint32_t wq[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};
-                                uint4 sp = __ldg(qp), zp = __ldg(qp + 1);
-#pragma unroll
-                                for (int i = 0; i < 8; i += 2) {
-                                    const uint4 sp1 = __ldg(qp + 2 * i + 2), zp1 = __ldg(qp + 2 * i + 3);
-                                    const uint4 d0 = dequant8t(wq[i], zp, sp);
-                                    if (i + 2 < 8) { sp = __ldg(qp + 2 * i + 4); zp = __ldg(qp + 2 * i + 5); }
-                                    tmem_st8(dst + (uint32_t)(4 * i), d0, dequant8t(wq[i + 1], zp1, sp1));
-                                }
-                            } else if (TA) {
-                                const uint32_t dst = ta_addr + (uint32_t)(stage * TA_COLS_PER_STAGE);
+                            const int raw_row = TA ? quarter * 32 + lane : tt;               // dgrad: (tt/2)*64 + (tt%2)*32 == tt*32
+                            const uint4* rp = reinterpret_cast<const uint4*>(raw_tile(stage, r) + raw_row * 32);
+                            const int swz32 = KIND == KIND_FWD ? raw_swap(raw_row) : 0;
+                            const uint4 r0 = rp[swz32], r1 = rp[swz32 ^ 1];
+                            if (TA) {
+                                const uint32_t dst = ta_addr + (uint32_t)(slot * TA_COLS_PER_STAGE);
                                 tmem_st8(dst + 0, dequant8(r0.x, za, s2a), dequant8(r0.y, za, s2a));
                                 tmem_st8(dst + 8, dequant8(r0.z, za, s2a), dequant8(r0.w, za, s2a));
                                 tmem_st8(dst + 16, dequant8(r1.x, zb, s2b), dequant8(r1.y, zb, s2b));
@@ -899,12 +1034,11 @@ k_gemm(const __grid_constant__ CUtensorMap map_tok, const __grid_constant__ CUte
                             }
                         }
                     }
-                    if (TA) { tmem_st_wait(); tc_fence_before(); } else { fence_proxy_async(); }
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(smem_u32(&ctl->a_ready[stage]));
+                    stage_done(stage);
                     cnt += 4u;
                     advance(cur, 4);
                 }
+            }
             }
             if (prof && warp == 6 && lane == 0) {
                 atomicAdd(&g_gemm_prof[5], (unsigned long long)w_dq); atomicAdd(&g_gemm_prof[6], (unsigned long long)(clock64() - t_role));
@@ -931,7 +1065,7 @@ k_gemm(const __grid_constant__ CUtensorMap map_tok, const __grid_constant__ CUte
 // ---------------------------------------------------------------------------------------------
 // split-K reduction
 // ---------------------------------------------------------------------------------------------
-template <bool I8>
+template <bool I8, bool POST = false>
 __global__ void __launch_bounds__(256) k_splitk_reduce(const GemmParams p) {
     const int64_t total = (int64_t)p.M * p.R;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
@@ -943,9 +1077,9 @@ __global__ void __launch_bounds__(256) k_splitk_reduce(const GemmParams p) {
             if (p.acc_out) p.acc_out[i] = a;
             float f = (float)a;
             if (p.row_scale) f = __fmul_rn(f, __ldg(p.row_scale + t));
-            const I8Epi e8 = i8_epilogue(p, r, true);
+            const I8Epi e8 = i8_epilogue<POST>(p, r, true);
             f = i8_scaled(e8, f);
-            p.out[i] = __float2bfloat16_rn(p.post_scale ? __fmul_rn(bf16r(f), e8.post) : f);
+            p.out[i] = __float2bfloat16_rn(POST ? __fmul_rn(bf16r(f), e8.post) : f);
         } else {
             float a = 0.0f;
             for (int s = 0; s < p.splits; ++s) a = __fadd_rn(a, reinterpret_cast<const float*>(p.partial)[(size_t)s * total + i]);
@@ -985,6 +1119,40 @@ static size_t plan_workspace_bytes(const Plan& pl, int64_t M, int64_t R) {
     return pl.splits > 1 ? (size_t)pl.splits * (size_t)M * (size_t)R * 4 : 0;
 }
 
+// Split-K factor of a plan whose tiles would leave half of the SMs idle
+static int plan_splits(int tiles, int kb_total, int sms) {
+    if (tiles * 2 > sms) return 1;
+    int splits = sms / tiles;
+    if (splits > kb_total / 4) splits = kb_total / 4;   // at least 4 k-blocks per item
+    if (splits > 16) splits = 16;
+    return splits < 1 ? 1 : splits;
+}
+// Token-tile width of an A16W4 launch: the one with the smallest modelled time.  The table holds what one k-block of a tile takes (us,
+// at 1.9 GHz) in the forward (weight tile in tensor memory) and the grad-input kernel (in shared memory), and what a forward tile
+// adds to it (with 256 tokens the single accumulator's epilogue), measured on the Llama-2-7B and OPT-1.3B shapes at 24 .. 4096 tokens
+// with every width; tiles run in waves of one per SM.  Split-K adds the partial sums' way through memory and the reduction
+// launch.  A fixed ladder (64, 128, then 256) left 40 % of the SMs idle at token counts between its steps: 11008 rows at 300
+// tokens 53.8 (256) / 38.5 us (128), at 512 51.2 / 46.3 (192), 2048 rows at 1000 46.6 / 36.2 (128).
+static int pick_token_tile(int kind, int64_t M, int64_t R, int kb_total) {
+    if (M <= 16) return 16;
+    struct Width { int tn; float fwd, fwd_tail, dgrad; };
+    static const Width widths[] = {{32, 0.18f, 0.3f, 0.297f}, {64, 0.20f, 0.3f, 0.32f}, {96, 0.225f, 0.3f, 0.335f}, {128, 0.245f, 0.3f, 0.343f},
+                                   {160, 0.28f, 0.4f, 0.366f}, {192, 0.305f, 0.9f, 0.4f}, {256, 0.36f, 2.0f, 0.456f}};
+    const int sms = sm_count(), r_tiles = (int)((R + TILE_R - 1) / TILE_R);
+    int best = 256;
+    double best_cost = 1e30;
+    for (const Width& w : widths) {
+        const int64_t tiles = (int64_t)r_tiles * ((M + w.tn - 1) / w.tn);
+        const int splits = tiles > sms ? 1 : plan_splits((int)tiles, kb_total, sms);
+        const int64_t waves = (tiles * splits + sms - 1) / sms;
+        const double stage = kind == KIND_FWD ? w.fwd : w.dgrad, tail = kind == KIND_FWD ? w.fwd_tail : 0.3;
+        double cost = (double)waves * (((kb_total + splits - 1) / splits) * stage + tail);
+        if (splits > 1) cost += 2.5 + 0.75e-6 * 4.0 * (double)splits * (double)M * (double)R;
+        if (cost < best_cost) { best_cost = cost; best = w.tn; }
+    }
+    return best;
+}
+
 // group: quantization group size, or 0 when unknown (the skinny path needs 64, 128 or 256)
 // allow_balanced = false asks for the plan a caller with too little workspace for the balanced one falls back to.
 static Plan make_plan(int kind, int64_t M, int64_t N, int64_t K, int group = 128, bool allow_balanced = true) {
@@ -1000,12 +1168,13 @@ static Plan make_plan(int kind, int64_t M, int64_t N, int64_t K, int group = 128
     const int64_t R = (kind == KIND_DGRAD) ? K : N;
     const int64_t Cc = (kind == KIND_DGRAD) ? N : K;
     pl.tn = M <= 16 ? 16 : (M <= 64 ? 64 : (M <= 128 ? 128 : 256));
-    pl.t_tiles = (int)((M + pl.tn - 1) / pl.tn);
     const int r_tiles1 = (int)((R + TILE_R - 1) / TILE_R);
     pl.rt = 1;   // the kernel template supports two weight-row tiles per CTA (RT = 2); no current plan uses it
     pl.r_tiles = (r_tiles1 + pl.rt - 1) / pl.rt;
     const int bk = (kind == KIND_I8) ? 128 : 64;
     pl.kb_total = (int)((Cc + bk - 1) / bk);
+    if (kind != KIND_I8 && !getenv("LQ_GEMM_BALANCE")) pl.tn = pick_token_tile(kind, M, R, pl.kb_total);
+    pl.t_tiles = (int)((M + pl.tn - 1) / pl.tn);
     const int tiles = pl.r_tiles * pl.t_tiles;
     const int sms = sm_count();
     // Balanced forward, opt-in with LQ_GEMM_BALANCE=1 (read at every launch).  With few tiles per SM, whole tiles
@@ -1042,14 +1211,9 @@ static Plan make_plan(int kind, int64_t M, int64_t N, int64_t K, int group = 128
             return pl;
         }
     }
-    int splits = 1;
-    if (tiles * 2 <= sms) {
-        splits = sms / tiles;
-        if (splits > pl.kb_total / 4) splits = pl.kb_total / 4;   // at least 4 k-blocks per item
-        if (splits > 16) splits = 16;
-        if (splits < 1) splits = 1;
-    }
+    const int splits = plan_splits(tiles, pl.kb_total, sms);
     pl.kb_per_split = (pl.kb_total + splits - 1) / splits;
+    if (kind == KIND_FWD) pl.kb_per_split += pl.kb_per_split & 1;         // whole stages of two k-blocks
     pl.splits = (pl.kb_total + pl.kb_per_split - 1) / pl.kb_per_split;
     return pl;
 }
@@ -1070,7 +1234,7 @@ static PFN_encodeTiled get_encode() {
 }
 // 2-D row-major tensor [rows, cols] of `elt` bytes; box [box_rows, box_cols].
 static int make_map(CUtensorMap* m, const void* base, CUtensorMapDataType dt, int elt, uint64_t rows, uint64_t cols,
-                    uint32_t box_rows, uint32_t box_cols, bool swizzle128) {
+                    uint32_t box_rows, uint32_t box_cols, CUtensorMapSwizzle swizzle) {
     PFN_encodeTiled enc = get_encode();
     if (!enc) return LQ_ECUDA;
     cuuint64_t dims[2] = {cols, rows};
@@ -1078,20 +1242,19 @@ static int make_map(CUtensorMap* m, const void* base, CUtensorMapDataType dt, in
     cuuint32_t box[2] = {box_cols, box_rows};
     cuuint32_t estr[2] = {1, 1};
     CUresult r = enc(m, dt, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                     swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
-                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                     swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) { set_cuda_error(cudaErrorInvalidValue, "cuTensorMapEncodeTiled"); return LQ_ECUDA; }
     return LQ_OK;
 }
 
-template <int KIND, int TN, int RT, bool TA = false, bool SK = false, bool QPT = false>
+template <int KIND, int TN, int RT, bool TA = false, bool SK = false, bool QPT = false, int KBS = 1>
 static int launch_tn(const CUtensorMap& mt, const CUtensorMap& mw, const GemmParams& p, cudaStream_t st, int sk_grid = 0) {
-    using C = Cfg<KIND, TN, RT, TA, SK>;
+    using C = Cfg<KIND, TN, RT, TA, SK, KBS>;
     static bool attr_done[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !attr_done[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(k_gemm<KIND, TN, RT, TA, SK, QPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
+        cudaError_t e = cudaFuncSetAttribute(k_gemm<KIND, TN, RT, TA, SK, QPT, KBS>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
         if (e != cudaSuccess) { set_cuda_error(e, "cudaFuncSetAttribute"); return LQ_ECUDA; }
         attr_done[dev] = true;
     }
@@ -1100,19 +1263,19 @@ static int launch_tn(const CUtensorMap& mt, const CUtensorMap& mw, const GemmPar
         unsigned char* tickets = reinterpret_cast<unsigned char*>(p.partial) + (size_t)p.sk_rem * p.sk_pmax * (size_t)TN * TILE_R * 4;
         cudaError_t e = cudaMemsetAsync(tickets, 0, (size_t)p.sk_rem * 4 * sizeof(unsigned int), st);
         if (e != cudaSuccess) { set_cuda_error(e, "cudaMemsetAsync(hand-over tickets)"); return LQ_ECUDA; }
-        k_gemm<KIND, TN, RT, TA, SK, QPT><<<sk_grid, C::THREADS, C::SMEM_BYTES, st>>>(mt, mw, p);
+        k_gemm<KIND, TN, RT, TA, SK, QPT, KBS><<<sk_grid, C::THREADS, C::SMEM_BYTES, st>>>(mt, mw, p);
         return check_launch("k_gemm (balanced)");
     }
     const int items = p.r_tiles * p.t_tiles * p.splits;
     const int grid = items < sm_count() ? items : sm_count();
-    k_gemm<KIND, TN, RT, TA, SK, QPT><<<grid, C::THREADS, C::SMEM_BYTES, st>>>(mt, mw, p);
+    k_gemm<KIND, TN, RT, TA, SK, QPT, KBS><<<grid, C::THREADS, C::SMEM_BYTES, st>>>(mt, mw, p);
     int rc = check_launch("k_gemm");
     if (rc) return rc;
     if (p.splits > 1) {
         const int64_t total = (int64_t)p.M * p.R;
         int g = (int)((total + 255) / 256);
         if (g > sm_count() * 8) g = sm_count() * 8;
-        k_splitk_reduce<KIND == KIND_I8><<<g, 256, 0, st>>>(p);
+        k_splitk_reduce<KIND == KIND_I8, KIND == KIND_I8 && QPT><<<g, 256, 0, st>>>(p);
         rc = check_launch("k_splitk_reduce");
     }
     return rc;
@@ -1129,23 +1292,37 @@ static int launch_fwd_sk(int tn, const CUtensorMap& mt, const CUtensorMap& mw, c
     }
     return LQ_EUNSUPPORTED;
 }
-template <int KIND>
-static int launch_kind_ta(int tn, const CUtensorMap& mt, const CUtensorMap& mw, const GemmParams& p, cudaStream_t st) {
+// Token-tile widths of the A16W4 kernels, either placement of the weight tile
+template <int KIND, bool TA>
+static int launch_w4(int tn, const CUtensorMap& mt, const CUtensorMap& mw, const GemmParams& p, cudaStream_t st) {
     switch (tn) {
-        case 16: return launch_tn<KIND, 16, 1, true>(mt, mw, p, st);
-        case 64: return launch_tn<KIND, 64, 1, true>(mt, mw, p, st);
-        case 128: return launch_tn<KIND, 128, 1, true>(mt, mw, p, st);
-        case 256: return launch_tn<KIND, 256, 1, true>(mt, mw, p, st);
+        case 16: return launch_tn<KIND, 16, 1, TA>(mt, mw, p, st);
+        case 32: return launch_tn<KIND, 32, 1, TA>(mt, mw, p, st);
+        case 64: return launch_tn<KIND, 64, 1, TA>(mt, mw, p, st);
+        case 96: return launch_tn<KIND, 96, 1, TA>(mt, mw, p, st);
+        case 128: return launch_tn<KIND, 128, 1, TA>(mt, mw, p, st);
+        case 160: return launch_tn<KIND, 160, 1, TA>(mt, mw, p, st);
+        case 192: return launch_tn<KIND, 192, 1, TA>(mt, mw, p, st);
+        case 256: return launch_tn<KIND, 256, 1, TA>(mt, mw, p, st);
     }
     return LQ_EUNSUPPORTED;
 }
-template <int KIND>
-static int launch_kind(int tn, int rt, const CUtensorMap& mt, const CUtensorMap& mw, const GemmParams& p, cudaStream_t st) {
+static int launch_fwd_k2(int tn, const CUtensorMap& mt, const CUtensorMap& mw, const GemmParams& p, cudaStream_t st) {
     switch (tn) {
-        case 16: return launch_tn<KIND, 16, 1>(mt, mw, p, st);
-        case 64: return launch_tn<KIND, 64, 1>(mt, mw, p, st);
-        case 128: return launch_tn<KIND, 128, 1>(mt, mw, p, st);
-        case 256: return launch_tn<KIND, 256, 1>(mt, mw, p, st);
+        case 32: return launch_tn<KIND_FWD, 32, 1, true, false, false, 2>(mt, mw, p, st);
+        case 64: return launch_tn<KIND_FWD, 64, 1, true, false, false, 2>(mt, mw, p, st);
+        case 96: return launch_tn<KIND_FWD, 96, 1, true, false, false, 2>(mt, mw, p, st);
+        case 128: return launch_tn<KIND_FWD, 128, 1, true, false, false, 2>(mt, mw, p, st);
+    }
+    return LQ_EUNSUPPORTED;
+}
+template <bool POST>
+static int launch_i8(int tn, const CUtensorMap& mt, const CUtensorMap& mw, const GemmParams& p, cudaStream_t st) {
+    switch (tn) {
+        case 16: return launch_tn<KIND_I8, 16, 1, false, false, POST>(mt, mw, p, st);
+        case 64: return launch_tn<KIND_I8, 64, 1, false, false, POST>(mt, mw, p, st);
+        case 128: return launch_tn<KIND_I8, 128, 1, false, false, POST>(mt, mw, p, st);
+        case 256: return launch_tn<KIND_I8, 256, 1, false, false, POST>(mt, mw, p, st);
     }
     return LQ_EUNSUPPORTED;
 }
@@ -1153,15 +1330,16 @@ static int launch_kind(int tn, int rt, const CUtensorMap& mt, const CUtensorMap&
 static inline bool al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 // Grad-input through a transposed copy of the weight (see k_w4_transpose): bytes of the copy and of its packed group
-// parameters, and the token count from which the two extra passes over the weight pay: they cost 18 us for a
-// 4096 x 11008 weight, the GEMM saves 9 us per 1024 tokens, so the routes break even near 2048 tokens.
+// parameters, and the token count from which the extra pass over the weight pays.  Measured through the copy / as stored (us, copy
+// included): 2048 tokens 144 / 157 (4096 x 11008), 146 / 166 (11008 x 4096), 57 / 58 (8192 x 2048), 65 / 68 (2048 x 8192); 1500
+// tokens 117 / 124, 140 / 135, 56 / 55, 53 / 54; 1000 tokens even or slower everywhere.  Seven tiles of 256 tokens and more take it.
 // LQ_GEMM_DGRAD_TRANSPOSE=0 keeps the shared-memory-A kernel, =1 takes the copy from 256 tokens.
 static size_t dgrad_t_bytes(int64_t N, int64_t K) { return (size_t)N * (size_t)K / 2 + (size_t)N * (size_t)(K / 128) * 4; }
 static bool dgrad_t_wanted(int64_t M, int64_t N, int64_t K, int group) {
     const char* e = getenv("LQ_GEMM_DGRAD_TRANSPOSE");
     if (e && e[0] == '0') return false;
     if (group != 128 || (K % 256) != 0 || (N % 64) != 0 || getenv("LQ_GEMM_A_OPERAND")) return false;
-    return M >= ((e && e[0] == '1') ? 256 : 3072);
+    return M >= ((e && e[0] == '1') ? 256 : 1792);
 }
 static int run_dgrad_transposed(const void* dy, const void* w, GemmParams p, int64_t M, int64_t N, int64_t K, void* workspace,
                                 cudaStream_t st);
@@ -1178,6 +1356,8 @@ static int run_gemm(int kind, const void* tok, const void* w, GemmParams p, int6
     // a caller whose workspace is too small for the balanced plan gets the whole-tile plan (which may need less or none)
     if (pl.sk && (!workspace || workspace_bytes < plan_workspace_bytes(pl, M, p.R))) pl = make_plan(kind, M, N, K, p.group, false);
     p.wcols = (int)K;
+    p.qp_staged = kind == KIND_FWD && p.group == 128 && (K / 128) % 2 == 0 &&
+                  ((reinterpret_cast<uintptr_t>(p.scales) | reinterpret_cast<uintptr_t>(p.zeros)) & 3) == 0;
     p.r_tiles = pl.r_tiles; p.t_tiles = pl.t_tiles; p.splits = pl.splits; p.kb_total = pl.kb_total; p.kb_per_split = pl.kb_per_split;
     if (pl.splits > 1) {
         const size_t need = (size_t)pl.splits * (size_t)M * (size_t)p.R * 4;
@@ -1207,28 +1387,30 @@ static int run_gemm(int kind, const void* tok, const void* w, GemmParams p, int6
     }
     CUtensorMap mt, mw;
     int rc;
+    const bool k2 = kind == KIND_FWD && p.qp_staged && !pl.sk && pl.tn >= 32 && pl.tn <= 128 && pl.kb_per_split % 2 == 0 && a_operand_in_tmem(kind);
     if (kind == KIND_I8) {
-        rc = make_map(&mt, tok, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)M, (uint64_t)K, (uint32_t)pl.tn, 128, true);
+        rc = make_map(&mt, tok, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)M, (uint64_t)K, (uint32_t)pl.tn, 128, CU_TENSOR_MAP_SWIZZLE_128B);
         if (rc) return rc;
-        rc = make_map(&mw, w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)N, (uint64_t)K, TILE_R, 128, true);
+        rc = make_map(&mw, w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)N, (uint64_t)K, TILE_R, 128, CU_TENSOR_MAP_SWIZZLE_128B);
     } else {
-        rc = make_map(&mt, tok, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)M, (uint64_t)p.C, (uint32_t)pl.tn, 64, true);
+        rc = make_map(&mt, tok, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)M, (uint64_t)p.C, (uint32_t)pl.tn, 64, CU_TENSOR_MAP_SWIZZLE_128B);
         if (rc) return rc;
-        if (kind == KIND_FWD)   // packed bytes [N, K/2]; box 128 rows x 32 bytes
-            rc = make_map(&mw, w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)N, (uint64_t)(K / 2), TILE_R, 32, false);
+        if (k2)                 // packed bytes [N, K/2]; box 128 rows x 64 bytes
+            rc = make_map(&mw, w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)N, (uint64_t)(K / 2), TILE_R, 64, CU_TENSOR_MAP_SWIZZLE_64B);
+        else if (kind == KIND_FWD)   // box 128 rows x 32 bytes
+            rc = make_map(&mw, w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)N, (uint64_t)(K / 2), TILE_R, 32, CU_TENSOR_MAP_SWIZZLE_32B);
         else                    // box 64 rows x 64 bytes
-            rc = make_map(&mw, w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)N, (uint64_t)(K / 2), 64, 64, false);
+            rc = make_map(&mw, w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)N, (uint64_t)(K / 2), 64, 64, CU_TENSOR_MAP_SWIZZLE_NONE);
     }
     if (rc) return rc;
     switch (kind) {
         case KIND_FWD:
+            if (k2) return launch_fwd_k2(pl.tn, mt, mw, p, st);
             if (pl.sk) return a_operand_in_tmem(kind) ? launch_fwd_sk<true>(pl.tn, mt, mw, p, st, pl.sk_grid) : launch_fwd_sk<false>(pl.tn, mt, mw, p, st, pl.sk_grid);
-            return (pl.rt == 1 && a_operand_in_tmem(kind)) ? launch_kind_ta<KIND_FWD>(pl.tn, mt, mw, p, st)
-                                                       : launch_kind<KIND_FWD>(pl.tn, pl.rt, mt, mw, p, st);
+            return a_operand_in_tmem(kind) ? launch_w4<KIND_FWD, true>(pl.tn, mt, mw, p, st) : launch_w4<KIND_FWD, false>(pl.tn, mt, mw, p, st);
         case KIND_DGRAD:
-            return (pl.rt == 1 && a_operand_in_tmem(kind)) ? launch_kind_ta<KIND_DGRAD>(pl.tn, mt, mw, p, st)
-                                                       : launch_kind<KIND_DGRAD>(pl.tn, pl.rt, mt, mw, p, st);
-        case KIND_I8: return launch_kind<KIND_I8>(pl.tn, pl.rt, mt, mw, p, st);
+            return a_operand_in_tmem(kind) ? launch_w4<KIND_DGRAD, true>(pl.tn, mt, mw, p, st) : launch_w4<KIND_DGRAD, false>(pl.tn, mt, mw, p, st);
+        case KIND_I8: return p.post_scale ? launch_i8<true>(pl.tn, mt, mw, p, st) : launch_i8<false>(pl.tn, mt, mw, p, st);
     }
     return LQ_EINVAL;
 }
@@ -1238,23 +1420,22 @@ static int run_dgrad_transposed(const void* dy, const void* w, GemmParams p, int
     uint8_t* wt = reinterpret_cast<uint8_t*>(workspace);                                   // [K][N / 2]
     uint4* qpt = reinterpret_cast<uint4*>(wt + (size_t)N * (size_t)K / 2);                 // [K / 128][N / 8][2]
     const int G = (int)(K / 128);
-    k_w4_transpose<<<dim3((unsigned)(K / 256), (unsigned)(N / 64)), 256, 0, st>>>(reinterpret_cast<const uint8_t*>(w), wt, (int)N, (int)K);
+    const int tiles = (int)(K / 256) * (int)(N / 64), entries = G * (int)(N / 8);
+    k_w4_transpose<<<tiles + (entries + 255) / 256, 256, 0, st>>>(reinterpret_cast<const uint8_t*>(w), wt, p.scales, p.zeros, qpt, (int)N, (int)K, tiles);
     int rc = check_launch("k_w4_transpose");
-    if (rc) return rc;
-    const int entries = G * (int)(N / 8);
-    k_w4_qp_transpose<<<(entries + 255) / 256, 256, 0, st>>>(p.scales, p.zeros, qpt, (int)N, G);
-    rc = check_launch("k_w4_qp_transpose");
     if (rc) return rc;
     // dx[M, K] = dy[M, N] . Wt[K, N]^T: the forward kernel with K output rows and N as the contraction
     p.M = (int)M; p.R = (int)K; p.C = (int)N; p.wcols = (int)N; p.qpt = qpt;
-    p.t_tiles = (int)((M + 255) / 256); p.r_tiles = (int)((K + TILE_R - 1) / TILE_R); p.splits = 1;
+    p.r_tiles = (int)((K + TILE_R - 1) / TILE_R); p.splits = 1;
     p.kb_total = (int)(N / 64); p.kb_per_split = p.kb_total;
+    constexpr int tn = 256;                 // (narrower tiles measured slower wherever the copy pays)
+    p.t_tiles = (int)((M + tn - 1) / tn);
     CUtensorMap mt, mw;
-    rc = make_map(&mt, dy, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)M, (uint64_t)N, 256, 64, true);
+    rc = make_map(&mt, dy, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)M, (uint64_t)N, (uint32_t)tn, 64, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc) return rc;
-    rc = make_map(&mw, wt, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)K, (uint64_t)(N / 2), TILE_R, 32, false);
+    rc = make_map(&mw, wt, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)K, (uint64_t)(N / 2), TILE_R, 32, CU_TENSOR_MAP_SWIZZLE_32B);
     if (rc) return rc;
-    return launch_tn<KIND_FWD, 256, 1, true, false, true>(mt, mw, p, st);
+    return launch_tn<KIND_FWD, tn, 1, true, false, true>(mt, mw, p, st);
 }
 
 }  // namespace lq
@@ -1408,9 +1589,9 @@ int lq_gemm_wgrad(const void* dy, const void* x, void* dw, int64_t M, int64_t N,
     p.out = (__nv_bfloat16*)dw; p.alpha = 1.0f; p.accumulate = accumulate ? 1 : 0;
     CUtensorMap mt, mw;
     // both operands are read as [64 tokens] x [64 features] boxes (128-byte rows, 128B swizzle): MN-major MMA atoms
-    int rc = make_map(&mt, x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)M, (uint64_t)K, 64, 64, true);
+    int rc = make_map(&mt, x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)M, (uint64_t)K, 64, 64, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc) return rc;
-    rc = make_map(&mw, dy, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)M, (uint64_t)N, 64, 64, true);
+    rc = make_map(&mw, dy, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)M, (uint64_t)N, 64, 64, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc) return rc;
     cudaStream_t st = (cudaStream_t)stream;
     switch (tn) {

@@ -55,22 +55,22 @@ def _adam_case(wbit, N, K, seed, grad_kind):
             ops.adam_a8w8_step(codes, w, grad, s, *a, hyper, o)
         return [codes, w] + a
 
-    return run
+    return run, torch.isfinite(grad.float()).view(blocks, per).all(1)
 
 
 @pytest.mark.parametrize("wbit", [4, 8])
 @pytest.mark.parametrize("N,K", [(16, 128), (64, 32 * 128), (3, 1152), (1088, 1152), (520, 128)])
 @pytest.mark.parametrize("grad_kind", ["normal", "zero", "tiny", "nonfinite"])
 def test_fast_optimizer_step_equals_generic_kernel(monkeypatch, wbit, N, K, grad_kind):
-    run = _adam_case(wbit, N, K, 7 * N + K, grad_kind)
+    run, finite = _adam_case(wbit, N, K, 7 * N + K, grad_kind)
     for has_residual in (True, False):
         monkeypatch.delenv("LQ_REQUANT_GENERIC", raising=False)
         fast = run(has_residual)
         monkeypatch.setenv("LQ_REQUANT_GENERIC", "1")
         slow = run(has_residual)
         for a, b in zip(fast, slow):
-            assert torch.equal(torch.nan_to_num(a, nan=-1.0) if a.is_floating_point() else a,
-                               torch.nan_to_num(b, nan=-1.0) if b.is_floating_point() else b)
+            # state blocks with a non-finite gradient have no defined result; they must not touch the others
+            assert torch.equal(a.reshape(finite.numel(), -1)[finite], b.reshape(finite.numel(), -1)[finite])
 
 
 # ---- requantize with Philox dither ----------------------------------------------------------------------------------
@@ -92,6 +92,35 @@ def test_philox_fold_equals_generic_kernel(monkeypatch, seed, step, param):
                                                               param_id=param))
         out.append((c, w))
     assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+
+
+# ---- A16W4 forward and grad-input at the edges of the token tiles ----------------------------------------------------
+def _w4(N, K, seed, group=128):
+    g = _gen(seed)
+    q = torch.randint(0, 16, (N * K // 2, 2), device="cuda", generator=g, dtype=torch.uint8)
+    s = (torch.rand(N * K // group, device="cuda", generator=g) * 0.01 + 1e-3).to(torch.bfloat16)
+    z = torch.randint(0, 16, (N * K // group,), device="cuda", generator=g).to(torch.bfloat16)
+    w = ((q.view(-1, group).double() - z.double()[:, None]) * s.double()[:, None]).view(N, K)
+    return ((q[:, 0] << 4) | q[:, 1]).view(torch.int8).contiguous(), s, z, w
+
+
+# bf16 weight and output roundings (2^-9 each, uncorrelated) leave a relative 2-norm error below 2.5e-3; a misplaced or missing tile,
+# group or token is of order 1
+@pytest.mark.parametrize("M", [3, 16, 17, 31, 33, 64, 65, 96, 97, 128, 129, 160, 161, 192, 193, 257, 300])
+@pytest.mark.parametrize("N,K,group", [(128, 256, 128), (192, 384, 128), (4160, 2176, 128), (320, 512, 64), (256, 1024, 256)])
+def test_a16w4_token_tile_edges(M, N, K, group):
+    from latentq_llm_b200 import ops
+    codes, s, z, w = _w4(N, K, N + K, group)
+    g = _gen(M)
+    x, bias = torch.randn(M, K, device="cuda", generator=g).to(torch.bfloat16), torch.randn(N, device="cuda", generator=g).to(torch.bfloat16)
+    for b in (None, bias):
+        y = ops.gemm_a16w4_fwd(x, codes, s, z, b, N, K, group)
+        ref = x.double() @ w.t() + (0 if b is None else b.double())
+        assert float((y.double() - ref).norm() / ref.norm()) < 4e-3
+    dy = torch.randn(M, N, device="cuda", generator=g).to(torch.bfloat16)
+    dx = ops.gemm_a16w4_dgrad(dy, codes, s, z, N, K, group)
+    ref = dy.double() @ w
+    assert float((dx.double() - ref).norm() / ref.norm()) < 4e-3
 
 
 # ---- A8W8 linear ------------------------------------------------------------------------------------------------------
