@@ -261,7 +261,11 @@ constexpr int RB_CHUNK = 128;         // k per chunk
 // NCH = 11: K = 11008 (86 groups: eleven chunks per warp, nine in the last warp): the same loop written out for up
 // to eleven chunks, each guarded by the warp's own count; group parameters stay 2-byte loads (rows of 86 groups are
 // not 8-byte aligned) but at constant offsets.
-template <int MT, int GC, int NCH = 0>
+// W64: a thread's four packed words of a row and chunk are words 2t, 2t+1, 8+2t, 9+2t (two 8-byte loads) instead of 4t .. 4t+3 (one
+// 16-byte load).  Its 16-byte token loads are then 32 bytes apart from its neighbour's instead of 64: a warp's token load touches one
+// cache line per token instead of two (8 tokens: 8 instead of 16 L1 cycles, four of them per chunk and token group), a weight load
+// still takes whole sectors.  Pays from five tokens on, where the token loads are what bounds the L1 pipe.
+template <int MT, int GC, int NCH = 0, bool W64 = false>
 __global__ void __launch_bounds__(RB_WARPS * 32, 2) k_skinny_rows(const SkinnyParams p) {
     constexpr int RB_PF = MT == 1 ? 4 : 2;
     constexpr bool XPF = MT == 1;
@@ -280,8 +284,14 @@ __global__ void __launch_bounds__(RB_WARPS * 32, 2) k_skinny_rows(const SkinnyPa
     const int g_begin = NC4 ? warp * 4 : min(gpr, warp * gper), n_groups = NC4 ? 4 : min(gpr, g_begin + gper) - g_begin;
     const int n_chunks = n_groups * GC;
     const int row_bytes = NC4 ? 2048 : p.K / 2, row_elems = NC4 ? 4096 : p.K;
-    const uint4* wa = reinterpret_cast<const uint4*>(p.qweight + (size_t)ra * row_bytes + (size_t)g_begin * GC * (RB_CHUNK / 2)) + t;
-    const uint4* wb = reinterpret_cast<const uint4*>(p.qweight + (size_t)rb * row_bytes + (size_t)g_begin * GC * (RB_CHUNK / 2)) + t;
+    const uint8_t* wa = p.qweight + (size_t)ra * row_bytes + (size_t)g_begin * GC * (RB_CHUNK / 2) + t * (W64 ? 8 : 16);
+    const uint8_t* wb = p.qweight + (size_t)rb * row_bytes + (size_t)g_begin * GC * (RB_CHUNK / 2) + t * (W64 ? 8 : 16);
+    auto load_words = [](const uint8_t* w, int c) -> uint4 {                        // chunk c (64 bytes per row): this thread's four words
+        if (!W64) return __ldg(reinterpret_cast<const uint4*>(w + c * 64));
+        const uint2 lo = __ldg(reinterpret_cast<const uint2*>(w + c * 64)), hi = __ldg(reinterpret_cast<const uint2*>(w + c * 64 + 32));
+        return make_uint4(lo.x, lo.y, hi.x, hi.y);
+    };
+    constexpr auto x_at = [](int j) { return W64 ? (j >> 1) * 8 + (j & 1) : j; };   // token vector of word j, from the thread's first
     const unsigned short* sca = reinterpret_cast<const unsigned short*>(p.scales) + (size_t)ra * gpr + g_begin;
     const unsigned short* scb = reinterpret_cast<const unsigned short*>(p.scales) + (size_t)rb * gpr + g_begin;
     const unsigned short* zpa = reinterpret_cast<const unsigned short*>(p.zeros) + (size_t)ra * gpr + g_begin;
@@ -290,14 +300,14 @@ __global__ void __launch_bounds__(RB_WARPS * 32, 2) k_skinny_rows(const SkinnyPa
     const uint4* xp[MT];
 #pragma unroll
     for (int m = 0; m < MT; ++m)
-        xp[m] = (m * 8 + g < p.M) ? reinterpret_cast<const uint4*>(p.x + (size_t)(m * 8 + g) * row_elems + (size_t)g_begin * GC * RB_CHUNK + t * 32)
+        xp[m] = (m * 8 + g < p.M) ? reinterpret_cast<const uint4*>(p.x + (size_t)(m * 8 + g) * row_elems + (size_t)g_begin * GC * RB_CHUNK + t * (W64 ? 16 : 32))
                                   : nullptr;
 
     uint4 qa[RB_PF], qb[RB_PF];
 #pragma unroll
     for (int u = 0; u < RB_PF; ++u) {
         qa[u] = qb[u] = make_uint4(0, 0, 0, 0);
-        if (u < n_chunks) { qa[u] = __ldg(wa + u * 4); qb[u] = __ldg(wb + u * 4); }       // a chunk is 64 bytes = 4 uint4 per row
+        if (u < n_chunks) { qa[u] = load_words(wa, u); qb[u] = load_words(wb, u); }
     }
     // (scale | zero << 16) of the group that starts with the chunk in ring slot u: fetched as far ahead as the chunk
     // itself (they come from DRAM too; one group ahead was a stall per group)
@@ -321,7 +331,7 @@ __global__ void __launch_bounds__(RB_WARPS * 32, 2) k_skinny_rows(const SkinnyPa
 #pragma unroll
     for (int m = 0; m < MT; ++m)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) xn[m][j] = (XPF && xp[m] && n_chunks > 0) ? xp[m][j] : make_uint4(0, 0, 0, 0);
+        for (int j = 0; j < 4; ++j) xn[m][j] = (XPF && xp[m] && n_chunks > 0) ? xp[m][x_at(j)] : make_uint4(0, 0, 0, 0);
 
     float tot[MT][4], acc[MT][2][4];     // two accumulator chains per token group
 #pragma unroll
@@ -352,7 +362,7 @@ __global__ void __launch_bounds__(RB_WARPS * 32, 2) k_skinny_rows(const SkinnyPa
         const uint4 ca = qa[u], cq = qb[u];
         if (u % GC == 0) sz_of_chunk(c, u);
         if (c + RB_PF < n_chunks) {
-            qa[u] = __ldg(wa + (c + RB_PF) * 4); qb[u] = __ldg(wb + (c + RB_PF) * 4);
+            qa[u] = load_words(wa, c + RB_PF); qb[u] = load_words(wb, c + RB_PF);
             if (!NC4 && u % GC == 0) {
                 const int gn = (c + RB_PF) / GC;
                 sza[u] = (uint32_t)__ldg(sca + gn) | ((uint32_t)__ldg(zpa + gn) << 16);
@@ -366,9 +376,9 @@ __global__ void __launch_bounds__(RB_WARPS * 32, 2) k_skinny_rows(const SkinnyPa
             for (int j = 0; j < 4; ++j) {
                 if (XPF) {
                     xc[m][j] = xn[m][j];
-                    if (xp[m] && c + 1 < n_chunks) xn[m][j] = xp[m][(c + 1) * (RB_CHUNK * 2 / 16) + j];
+                    if (xp[m] && c + 1 < n_chunks) xn[m][j] = xp[m][(c + 1) * (RB_CHUNK * 2 / 16) + x_at(j)];
                 } else {
-                    xc[m][j] = xp[m] ? xp[m][c * (RB_CHUNK * 2 / 16) + j] : make_uint4(0, 0, 0, 0);
+                    xc[m][j] = xp[m] ? xp[m][c * (RB_CHUNK * 2 / 16) + x_at(j)] : make_uint4(0, 0, 0, 0);
                 }
             }
         const uint32_t wsa[4] = {ca.x, ca.y, ca.z, ca.w}, wsb[4] = {cq.x, cq.y, cq.z, cq.w};
@@ -936,18 +946,24 @@ int launch_skinny_rows(const SkinnyParams& p, cudaStream_t st) {
     // K = 4096 with groups of 128: the written-out loop (scales / zeros are read as 8-byte words there)
     const bool nc4 = g128 && p.K == 4096 && !getenv("LQ_SKINNY_NO_NC4") &&
                      (reinterpret_cast<uintptr_t>(p.scales) & 7) == 0 && (reinterpret_cast<uintptr_t>(p.zeros) & 7) == 0;
+    const dim3 g(grid);
+    const unsigned th = RB_WARPS * 32;
+    const bool w64 = p.M > 4;
     if (nc4) {
-        if (p.M <= 8) launch_pdl(k_skinny_rows<1, 1, 4>, dim3(grid), RB_WARPS * 32, 0, st, p);
-        else launch_pdl(k_skinny_rows<2, 1, 4>, dim3(grid), RB_WARPS * 32, 0, st, p);
-        return check_launch("k_skinny_rows");
+        if (p.M > 8) launch_pdl(k_skinny_rows<2, 1, 4, true>, g, th, 0, st, p);
+        else if (w64) launch_pdl(k_skinny_rows<1, 1, 4, true>, g, th, 0, st, p);
+        else launch_pdl(k_skinny_rows<1, 1, 4>, g, th, 0, st, p);
+    } else if (g128 && p.K == 11008 && !getenv("LQ_SKINNY_NO_NC4")) {          // eleven chunks per warp, written out
+        if (p.M > 8) launch_pdl(k_skinny_rows<2, 1, 11, true>, g, th, 0, st, p);
+        else if (w64) launch_pdl(k_skinny_rows<1, 1, 11, true>, g, th, 0, st, p);
+        else launch_pdl(k_skinny_rows<1, 1, 11>, g, th, 0, st, p);
+    } else if (p.M > 8) {
+        if (g128) launch_pdl(k_skinny_rows<2, 1, 0, true>, g, th, 0, st, p); else launch_pdl(k_skinny_rows<2, 2, 0, true>, g, th, 0, st, p);
+    } else if (w64) {
+        if (g128) launch_pdl(k_skinny_rows<1, 1, 0, true>, g, th, 0, st, p); else launch_pdl(k_skinny_rows<1, 2, 0, true>, g, th, 0, st, p);
+    } else {
+        if (g128) launch_pdl(k_skinny_rows<1, 1>, g, th, 0, st, p); else launch_pdl(k_skinny_rows<1, 2>, g, th, 0, st, p);
     }
-    if (g128 && p.K == 11008 && !getenv("LQ_SKINNY_NO_NC4")) {          // eleven chunks per warp, written out
-        if (p.M <= 8) launch_pdl(k_skinny_rows<1, 1, 11>, dim3(grid), RB_WARPS * 32, 0, st, p);
-        else launch_pdl(k_skinny_rows<2, 1, 11>, dim3(grid), RB_WARPS * 32, 0, st, p);
-        return check_launch("k_skinny_rows");
-    }
-    if (p.M <= 8) { if (g128) launch_pdl(k_skinny_rows<1, 1>, dim3(grid), RB_WARPS * 32, 0, st, p); else launch_pdl(k_skinny_rows<1, 2>, dim3(grid), RB_WARPS * 32, 0, st, p); }
-    else { if (g128) launch_pdl(k_skinny_rows<2, 1>, dim3(grid), RB_WARPS * 32, 0, st, p); else launch_pdl(k_skinny_rows<2, 2>, dim3(grid), RB_WARPS * 32, 0, st, p); }
     return check_launch("k_skinny_rows");
 }
 
