@@ -311,16 +311,31 @@ __global__ void __launch_bounds__(ATT_THREADS) k_decode_attn(const __nv_bfloat16
     __syncthreads();
     if (!is_last) return;
     __threadfence();
+    // The splits' (max, sum) come in one load per lane and their weights go through shared memory; the weighted values of eight
+    // splits are requested together.  (Read split by split the combination was a chain of L2 round trips: two per split.)
+    __shared__ float sp_w[32], sp_l[32];                        // splits <= 32
+    const float* base = part + (size_t)bh * splits * (HD + 2);
+    if (threadIdx.x < 32) {
+        const int s2 = threadIdx.x;
+        const bool have = s2 < splits;
+        const float ms = have ? __ldcg(base + (size_t)s2 * (HD + 2) + HD) : -INFINITY;
+        const float ls = have ? __ldcg(base + (size_t)s2 * (HD + 2) + HD + 1) : 0.0f;
+        float M = ms;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+        sp_w[s2] = (ms == -INFINITY) ? 0.0f : __expf(ms - M);
+        sp_l[s2] = ls;
+    }
+    __syncthreads();
     if (threadIdx.x < HD) {
-        const float* base = part + (size_t)bh * splits * (HD + 2);
-        float M = -INFINITY;
-        for (int s2 = 0; s2 < splits; ++s2) M = fmaxf(M, __ldcg(base + (size_t)s2 * (HD + 2) + HD));
         float L = 0.0f, a = 0.0f;
-        for (int s2 = 0; s2 < splits; ++s2) {
-            const float ms = __ldcg(base + (size_t)s2 * (HD + 2) + HD);
-            const float w = (ms == -INFINITY) ? 0.0f : __expf(ms - M);
-            L = fmaf(__ldcg(base + (size_t)s2 * (HD + 2) + HD + 1), w, L);
-            a = fmaf(__ldcg(base + (size_t)s2 * (HD + 2) + threadIdx.x), w, a);
+        for (int s0 = 0; s0 < splits; s0 += 8) {
+            float v[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] = (s0 + i < splits) ? __ldcg(base + (size_t)(s0 + i) * (HD + 2) + threadIdx.x) : 0.0f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                if (s0 + i < splits) { L = fmaf(sp_l[s0 + i], sp_w[s0 + i], L); a = fmaf(v[i], sp_w[s0 + i], a); }
         }
         out[(size_t)b * Hq * HD + (size_t)h * HD + threadIdx.x] = __float2bfloat16_rn(L > 0.0f ? a / L : 0.0f);
     }
