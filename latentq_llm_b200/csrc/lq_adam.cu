@@ -41,6 +41,10 @@ __device__ __forceinline__ float adam_apply(const lq_adam_hyper& h, float p, flo
     return rb<BF>(__fmaf_rn(h.neg_step_size, __fdiv_rn(m, d), p));
 }
 
+__device__ __forceinline__ uint8_t opt8_encode1(float x, float mx, float s) {
+    const float t = rne(div_rn(__fsub_rn(mx, x), s, __frcp_rn(s), fastdiv_ok_scale(s)));
+    return (uint8_t)(f2bits(fminf(fmaxf(t, 0.0f), 255.0f)) & 0xffu);
+}
 __device__ __forceinline__ uint2 opt8_encode8(const float (&x)[8], float mx, float s) {
     const float rs = __frcp_rn(s);
     const bool ok = fastdiv_ok_scale(s);
@@ -142,25 +146,27 @@ __global__ void __launch_bounds__(256) k_adam_quant(const AdamParams p) {
 //   requantize  everything after Z = w/scale + zero from the table of the requantize fast path (int4: a byte per bf16 pattern,
 //             |Z| < 64; int8: two bytes, |Z| < 256); the kernel keeps the two runs of it that can be looked up and puts its other
 //             tables into the gap between them.
-// int4 codes: 50 KB and 256 threads per CTA, four CTAs per SM; int8 codes: 100 KB, so two teams of 256 threads share the tables
-// of a CTA and two CTAs fit.
+// int4 codes: 50 KB and 256 threads per CTA, three CTAs per SM (four would fit, but at 64 registers the loop spills: 176 instead of
+// 157 us for 4096 x 11008); int8 codes: 100 KB, so two teams of 256 threads share the tables of a CTA and two CTAs fit.
+// Measured, a whole optimizer step of one 4096 x 11008 weight: int4 268 -> 157 us (2.3 TB/s), int8 586 -> 183 us.
 // A word whose Z leaves the table's range or is not finite, and every word of a block whose moments are not all finite, is
-// recomputed by the generic chain (adam_word_generic).
+// recomputed with IEEE operations (adam_word_generic).
 // ---------------------------------------------------------------------------------------------------------------
 constexpr int ADAM_TRES_REPL = 8;
 template <int WBITS> struct AdamFast {
     static constexpr int TEAMS = WBITS == 8 ? 2 : 1;
     static constexpr int THREADS = TEAMS * 256;
-    static constexpr int MIN_CTAS = 4 / TEAMS;
+    static constexpr int MIN_CTAS = WBITS == 8 ? 2 : 3;
     static constexpr int ENTRY = WBITS == 8 ? 2 : 1;                     // bytes per table entry
     static constexpr int RUN = (WBITS == 8 ? 0x4380 : 0x4280) * ENTRY;   // bf16 patterns of [0, 256) / [0, 64)
     static constexpr int NEG = 0x8000 * ENTRY;                           // the run of the negative patterns
     static constexpr int TRES = (RUN + 1023) / 1024 * 1024;              // residual decode table
     static constexpr int LUT = TRES + 256 * ADAM_TRES_REPL * 4;          // per team: [256] first state, [256] second state
     static constexpr int RED = LUT + TEAMS * 2 * 256 * 4;                // per team: block extrema of the 8 warps
+    static constexpr int PRM = RED + TEAMS * 64;                         // per team: (s1, t1, s2, t2) of this tile and the next
     static constexpr int SMEM = NEG + RUN;
     static constexpr uint32_t Z_LIMIT = WBITS == 8 ? 0x3c803c80u : 0x3d803d80u;    // carries into bit 15 from |Z| = 256 / 64 on
-    static_assert(RED + TEAMS * 64 <= NEG && RUN % 16 == 0, "tables in the gap of the encode table");
+    static_assert(PRM + TEAMS * 32 <= NEG && RUN % 16 == 0, "tables in the gap of the encode table");
 };
 
 __device__ __forceinline__ uint32_t pack2(float a, float b) {       // bf16 roundings of two values, one conversion
@@ -204,27 +210,31 @@ __device__ __forceinline__ uint32_t opt8_codes4(uint32_t p01, uint32_t p23, floa
                        __byte_perm(opt8_code_bits(lo2f(p23), mx, o), opt8_code_bits(hi2f(p23), mx, o), 0x0040), 0x5410);
 }
 
-// One word through the generic chain, from its inputs in memory (nothing of it has been written yet) and the block parameters
-// of its states before (s, t) and after (ns, mx) the step: what k_adam_quant does for it.
+// One word from its inputs in memory (nothing of it has been written yet) and the block parameters of its states before (s, t) and
+// after (ns, mx) the step, with IEEE divisions and roots and the generic requantize.  Elements come one at a time through memory:
+// the cold path must not cost the hot one registers.
 template <int WBITS>
-__device__ __noinline__ void adam_word_generic(const AdamParams& p, const int64_t w, const float s1, const float t1, const float s2, const float t2,
-                                               const float mx1, const float ns1, const float mx2, const float ns2) {
+__device__ __forceinline__ void adam_word_generic(const AdamParams& p, const int64_t w, const float s1, const float t1, const float s2, const float t2,
+                                                  const float mx1, const float ns1, const float mx2, const float ns2) {
     const int64_t e0 = w * 8;
     const int64_t g = p.rq.group_shift >= 0 ? (e0 >> p.rq.group_shift) : (e0 / p.rq.group);
     const float s = load1(p.rq.scales, p.rq.qp_dtype, g), z = (WBITS == 4) ? load1(p.rq.zeros, p.rq.qp_dtype, g) : 0.0f;
-    float lat[8], m[8], d[8], gr[8];
-    load8(p.grad, p.grad_dtype, e0, gr);
+    float lat[8];
     latent_load<WBITS, LQ_CODEC_THREEFOLD, true>(p.rq, w, s, z, lat);
-#pragma unroll 1
+    const __nv_bfloat16* grad = reinterpret_cast<const __nv_bfloat16*>(p.grad) + e0;
+#pragma unroll
     for (int k = 0; k < 8; ++k) {
-        m[k] = rb<true>(__fsub_rn(t1, __fmul_rn((float)p.st1[e0 + k], s1)));
+        const float gr = __bfloat162float(grad[k]);
+        float m = bf16r(__fsub_rn(t1, __fmul_rn((float)p.st1[e0 + k], s1)));
+        m = bf16r(__fmaf_rn(p.h.one_minus_beta1, gr, bf16r(__fmul_rn(m, p.h.beta1))));
         const float r2 = __fsub_rn(t2, __fmul_rn((float)p.st2[e0 + k], s2));
-        d[k] = rb<true>(__fmul_rn(r2, r2));
-        adam_moments<true>(p.h, gr[k], m[k], d[k]);
-        lat[k] = adam_apply<true>(p.h, lat[k], m[k], d[k]);
+        float d = bf16r(__fmul_rn(bf16r(__fmul_rn(r2, r2)), p.h.beta2));
+        d = bf16r(__fmaf_rn(p.h.one_minus_beta2, __fmul_rn(gr, gr), d));
+        d = bf16r(__fadd_rn(bf16r(__fsqrt_rn(d)), p.h.eps));
+        lat[k] = bf16r(__fmaf_rn(p.h.neg_step_size, __fdiv_rn(m, d), lat[k]));
+        p.st1[e0 + k] = opt8_encode1(m, mx1, ns1);
+        p.st2[e0 + k] = opt8_encode1(d, mx2, ns2);
     }
-    *reinterpret_cast<uint2*>(p.st1 + e0) = opt8_encode8(m, mx1, ns1);
-    *reinterpret_cast<uint2*>(p.st2 + e0) = opt8_encode8(d, mx2, ns2);
     latent_store<WBITS, LQ_CODEC_THREEFOLD, LQ_DITHER_HASH, true>(p.rq, w, s, z, lat);
 }
 
@@ -252,6 +262,8 @@ k_adam_fast(const __grid_constant__ AdamParams p, const int enc_slot, const uint
     const int team = AF::TEAMS == 1 ? 0 : (int)(threadIdx.x >> 8), tid = threadIdx.x & 255, lane = tid & 31, warp = tid >> 5;
     float* lut = reinterpret_cast<float*>(asm_ + AF::LUT) + team * 512;
     uint2* red = reinterpret_cast<uint2*>(asm_ + AF::RED) + team * 8;
+    float4* prm = reinterpret_cast<float4*>(asm_ + AF::PRM) + team * 2;       // for the cold path: keeps four registers free
+    int parity = 0;
     auto team_sync = [&] {
         if (AF::TEAMS == 1) __syncthreads();
         else asm volatile("bar.sync %0, 256;" ::"r"(team + 1) : "memory");
@@ -296,6 +308,7 @@ k_adam_fast(const __grid_constant__ AdamParams p, const int enc_slot, const uint
         if (LUT) {
             const float c = u2f((uint32_t)tid);
             lut[tid] = dec1(c); lut[256 + tid] = dec2(c);
+            if (tid == 0) prm[parity] = make_float4(in.s1, in.t1, in.s2, in.t2);
             team_sync();
         }
         uint32_t lat[4], m[4], d[4];
@@ -385,7 +398,8 @@ k_adam_fast(const __grid_constant__ AdamParams p, const int enc_slot, const uint
             if (__builtin_expect(bad, 0)) {
                 o1.s = __fadd_rn(__fdiv_rn(__fsub_rn(fmx1, fmn1), 255.0f), 1e-10f);      // (the fast division is for finite extrema)
                 o2.s = __fadd_rn(__fdiv_rn(__fsub_rn(fmx2, fmn2), 255.0f), 1e-10f);
-                adam_word_generic<WBITS>(p, (int64_t)w, in.s1, in.t1, in.s2, in.t2, fmx1, o1.s, fmx2, o2.s);
+                const float4 q = LUT ? prm[parity] : make_float4(in.s1, in.t1, in.s2, in.t2);
+                adam_word_generic<WBITS>(p, (int64_t)w, q.x, q.y, q.z, q.w, fmx1, o1.s, fmx2, o2.s);
             } else {
                 *reinterpret_cast<uint2*>(p.st1 + (size_t)w * 8) = make_uint2(opt8_codes4(m[0], m[1], fmx1, o1), opt8_codes4(m[2], m[3], fmx1, o1));
                 *reinterpret_cast<uint2*>(p.st2 + (size_t)w * 8) = make_uint2(opt8_codes4(d[0], d[1], fmx2, o2), opt8_codes4(d[2], d[3], fmx2, o2));
@@ -414,6 +428,7 @@ k_adam_fast(const __grid_constant__ AdamParams p, const int enc_slot, const uint
             const bool leader = LUT ? (tid == 0) : ((tid & 15) == 0);
             if (leader) { p.sc1[ob] = o1.s; p.tm1[ob] = fmx1; p.sc2[ob] = o2.s; p.tm2[ob] = fmx2; }
         }
+        parity ^= 1;
     }
 }
 
