@@ -338,6 +338,9 @@ static inline int ensure_enc8_table(int mu, float v0, cudaStream_t st) {
     const int slot = (mu < 0 || mu > 3) ? 0 : mu;
     std::lock_guard<std::mutex> lock(g_encz_mutex);
     if (built[dev][slot] && built_v0[dev][slot] == v0) return LQ_OK;
+    // building ends with a synchronisation, which a stream that is being captured does not allow: the caller takes its generic kernel
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) return LQ_EUNSUPPORTED;
     k_build_enc8_table<<<128, 256, 0, st>>>(slot, curve_for_level(slot), v0);
     int rc = check_launch("k_build_enc8_table");
     if (rc) return rc;

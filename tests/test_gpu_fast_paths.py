@@ -73,6 +73,32 @@ def test_fast_optimizer_step_equals_generic_kernel(monkeypatch, wbit, N, K, grad
             assert torch.equal(a.reshape(finite.numel(), -1)[finite], b.reshape(finite.numel(), -1)[finite])
 
 
+def test_int8_optimizer_step_captured_before_its_table_exists():
+    """The first step at a curve level builds a table, which ends with a synchronisation; under capture the generic kernel steps in."""
+    from latentq_llm_b200 import ops
+    g = _gen(5)
+    N, K = 8, 256
+    grad = (torch.randn(N, K, device="cuda", generator=g) * 1e-3).to(torch.bfloat16)
+    qs = torch.full((N,), 0.01, device="cuda").to(torch.bfloat16)
+    codes0 = torch.randint(-100, 100, (N, K), device="cuda", generator=g, dtype=torch.int8)
+    hyper = ops.make_adam_hyper(0.9, 0.95, 1e-8, 1e-3)
+    o = ops.make_opts(codec=ops.CODEC_THREEFOLD, dither=ops.DITHER_HASH, has_residual=False, mu_enc=3, v0=0.03125)   # a table of its own
+
+    def state():
+        z = torch.zeros(1, 1, device="cuda")
+        return [codes0.clone(), torch.zeros(N * K // 8, dtype=torch.int32, device="cuda")] + [
+            t for _ in range(2) for t in (torch.zeros(N, K, dtype=torch.uint8, device="cuda"), z + 1e-10, z.clone())]
+
+    a, b = state(), state()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        ops.adam_a8w8_step(a[0], a[1], grad, qs, *a[2:], hyper, o)
+    graph.replay()
+    ops.adam_a8w8_step(b[0], b[1], grad, qs, *b[2:], hyper, o)
+    for x, y in zip(a, b):
+        assert torch.equal(x, y)
+
+
 # ---- requantize with Philox dither ----------------------------------------------------------------------------------
 @pytest.mark.parametrize("seed,step,param", [(0, 0, 0), (1234, 7, 3), (2 ** 64 - 1, 2 ** 32 - 1, 2 ** 32 - 1)])
 def test_philox_fold_equals_generic_kernel(monkeypatch, seed, step, param):
