@@ -480,7 +480,10 @@ int lq_rope_kv_store(void* qkv, const int64_t* positions, const float* inv_freq,
 
 static int attn_splits(int64_t B, int Hq, int64_t max_len) {
     const int64_t ctas = B * Hq;
-    int64_t s = (4 * (int64_t)sm_count() + ctas - 1) / ctas;      // about four CTAs per SM in flight
+    // As many splits as fit beside one another (four CTAs per SM by registers): rounded up, a few CTAs more than that made a second
+    // wave of the whole kernel.  Measured (us, up / down): 4 sequences of 512 keys 16.7 / 13.1, 8: 22.1 / 17.9, 16: 30.7 / 25.7, one of
+    // 1500 keys 15.8 / 11.9, four 28.7 / 22.6; 32 and more take one split either way.
+    int64_t s = 4 * (int64_t)sm_count() / ctas;
     const int64_t cap = (max_len + 63) / 64;                        // at least 64 keys (two rounds of the 16 slots x 2) per split
     if (s > cap) s = cap;
     if (s > 32) s = 32;
