@@ -158,7 +158,7 @@ constexpr int TA_COLS_PER_STAGE = 32;
 constexpr int FIX_COLS = 16;                                         // balanced mode: token columns per hand-over copy
 constexpr int FIX_COPY_BYTES = FIX_COLS * 32 * 4;                    // one lane quarter of them as fp32: 2 KB
 constexpr int FIX_RING = 8;                                          // staging buffers per lane quarter
-// Forward: group parameters staged in shared memory, two buffers of one chunk each: 16 k-blocks = 8 groups of 128 for the 128 rows
+// Forward: group parameters staged in shared memory, three buffers (256-token tiles leave room for two) of one chunk each: 16 k-blocks = 8 groups of 128 for the 128 rows
 // of the tile, word (scale | zero + 128 << 16) of group g and row r at g * QP_PITCH + r (the pitch keeps both the writers, four
 // lanes per row, and the readers, a lane per row, free of bank conflicts).
 constexpr int QP_CHUNK = 16, QP_PITCH = 132;
@@ -176,7 +176,8 @@ struct Cfg {
     static constexpr int A_COLS = KBS * TA_COLS_PER_STAGE;                 // tensor-memory columns of a stage's weight tile
     static constexpr int STAGE_BYTES = A_BYTES + B_TILE_BYTES + RAW_TOTAL;
     static constexpr int FIX_BYTES = SK ? 4 * FIX_RING * FIX_COPY_BYTES : 0;    // balanced mode: the staging rings
-    static constexpr int QP_BYTES = KIND == KIND_FWD ? 2 * QP_BUF_BYTES : 0;
+    static constexpr int QP_BUFS = TN == 256 || SK ? 2 : 3;
+    static constexpr int QP_BYTES = KIND == KIND_FWD ? QP_BUFS * QP_BUF_BYTES : 0;
     static constexpr int STAGES_FIT = (227 * 1024 - 1024 - 1024 - FIX_BYTES - QP_BYTES) / STAGE_BYTES;
     // Tensor-memory A operand with token tiles up to 192: both accumulators fit beside the A slots, of which there are then
     // as many as pipeline stages (up to 128 tokens) or one per dequant team (four: the shared-memory ring is deeper than the
@@ -215,6 +216,7 @@ struct SmemCtl {
     uint64_t empty[MAX_STAGES];    // MMAs that read the stage retired
     uint64_t acc_full[2];
     uint64_t acc_empty[2];
+    uint64_t qp_ready[3];          // staged group parameters written (one arrival per dequant warp)
     uint64_t fix_full[4][FIX_RING];   // balanced mode: hand-over copy landed (per lane quarter, per staging buffer)
     uint32_t tmem_base;
     int abort_flag;
@@ -389,6 +391,7 @@ k_gemm(const __grid_constant__ CUtensorMap map_tok, const __grid_constant__ CUte
             mbar_init(smem_u32(&ctl->acc_full[a]), 1);
             mbar_init(smem_u32(&ctl->acc_empty[a]), 4 * C::EPI_SPLIT);
         }
+        for (int b = 0; b < 3; ++b) mbar_init(smem_u32(&ctl->qp_ready[b]), NUM_DQ_WARPS);
         for (int q = 0; q < 4; ++q)
             for (int b = 0; b < FIX_RING; ++b) mbar_init(smem_u32(&ctl->fix_full[q][b]), 1);
         ctl->abort_flag = 0;
@@ -897,17 +900,42 @@ k_gemm(const __grid_constant__ CUtensorMap map_tok, const __grid_constant__ CUte
                         d[0] = __byte_perm(ls, z, 0x5410); d[QP_PITCH] = __byte_perm(ls, z, 0x7632);
                     };
                     auto team_barrier = [] { asm volatile("bar.sync 1, 512;" ::: "memory"); };       // the 16 dequant warps
+                    // Two buffers: every warp has read chunk c and written chunk c + 1 when the barrier at the end of chunk c lets it go on.
+                    // Three buffers: a warp writes chunk c + 1 when it begins chunk c and waits, one chunk later, for the others
+                    // to have done so - they have, unless they lag by a whole chunk.  (Beginning chunk c means that all warps
+                    // began chunk c - 1, i.e. are done with chunk c - 2, whose buffer chunk c + 1 takes.)  The barrier at the end of every chunk
+                    // held the dequant warps for a quarter of their time.
+                    constexpr bool QP3 = C::QP_BUFS == 3;
+                    auto announce = [&](int buf) {
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(smem_u32(&ctl->qp_ready[buf]));
+                    };
                     Chunk cur{SegWalk<SK>(p), 0, 0, 0, 0, true};
                     next_chunk(cur);
                     fetch(cur); stash(0);
-                    team_barrier();
+                    Chunk ahead = cur;                                       // three buffers: the chunk whose parameters are in registers
+                    uint32_t qp_phase = 0u;
+                    if (QP3) { announce(0); if (ahead.valid) next_chunk(ahead); fetch(ahead); }
+                    else team_barrier();
                     const int my_row = TA ? quarter * 32 + lane : tt;
                     uint32_t base = 0u;
                     int buf = 0;
                     while (cur.valid) {
-                        Chunk nxt = cur;
-                        next_chunk(nxt);
-                        fetch(nxt);
+                        Chunk nxt = ahead;
+                        if (QP3) {
+                            ok = mbar_wait(smem_u32(&ctl->qp_ready[buf]), qp_phase, abort_flag) && ok;
+                            if (nxt.valid) {
+                                const int to = buf == 2 ? 0 : buf + 1;
+                                stash(to);
+                                announce(to);
+                                next_chunk(ahead);
+                                fetch(ahead);
+                            }
+                        } else {
+                            nxt = cur;
+                            next_chunk(nxt);
+                            fetch(nxt);
+                        }
                         const int n = (cur.end - cur.kb) / KBS;
                         for (int i = (int)((uint32_t)(team - (int)base) & 3u); i < n && ok; i += 4) {    // (an aborted team still meets the barriers)
                             const uint32_t cnt = base + (uint32_t)i;
@@ -947,9 +975,13 @@ k_gemm(const __grid_constant__ CUtensorMap map_tok, const __grid_constant__ CUte
                             stage_done(stage);
                         }
                         base += (uint32_t)n;
-                        buf ^= 1;
-                        if (nxt.valid) stash(buf);
-                        team_barrier();
+                        if (QP3) {
+                            if (++buf == 3) { buf = 0; qp_phase ^= 1u; }
+                        } else {
+                            buf ^= 1;
+                            if (nxt.valid) stash(buf);
+                            team_barrier();
+                        }
                         cur = nxt;
                     }
                 }
