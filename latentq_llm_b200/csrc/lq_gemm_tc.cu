@@ -158,11 +158,11 @@ constexpr int TA_COLS_PER_STAGE = 32;
 constexpr int FIX_COLS = 16;                                         // balanced mode: token columns per hand-over copy
 constexpr int FIX_COPY_BYTES = FIX_COLS * 32 * 4;                    // one lane quarter of them as fp32: 2 KB
 constexpr int FIX_RING = 8;                                          // staging buffers per lane quarter
-// Forward: group parameters staged in shared memory, three buffers (256-token tiles leave room for two) of one chunk each: 16 k-blocks = 8 groups of 128 for the 128 rows
-// of the tile, word (scale | zero + 128 << 16) of group g and row r at g * QP_PITCH + r (the pitch keeps both the writers, four
-// lanes per row, and the readers, a lane per row, free of bank conflicts).
-constexpr int QP_CHUNK = 16, QP_PITCH = 132;
-constexpr int QP_BUF_BYTES = 8 * QP_PITCH * 4;
+// Forward: group parameters staged in shared memory, three buffers of one chunk each: 16 k-blocks = 8 groups of 128 for the 128 rows
+// of the tile (256-token tiles: 8 k-blocks, their pipeline leaves no more room), word (scale | zero + 128 << 16) of group g and row
+// r at g * QP_PITCH + r (the pitch keeps both the writers, neighbouring lanes on neighbouring groups, and the readers, a lane per
+// row, off each other's banks).
+constexpr int QP_PITCH = 132;
 // KBS = k-blocks of 64 per pipeline stage (2: forward with the weight tile in tensor memory, up to 128 tokens).
 template <int KIND, int TN, int RT, bool TA = false, bool SK = false, int KBS = 1>
 struct Cfg {
@@ -176,8 +176,10 @@ struct Cfg {
     static constexpr int A_COLS = KBS * TA_COLS_PER_STAGE;                 // tensor-memory columns of a stage's weight tile
     static constexpr int STAGE_BYTES = A_BYTES + B_TILE_BYTES + RAW_TOTAL;
     static constexpr int FIX_BYTES = SK ? 4 * FIX_RING * FIX_COPY_BYTES : 0;    // balanced mode: the staging rings
-    static constexpr int QP_BUFS = TN == 256 || SK ? 2 : 3;
-    static constexpr int QP_BYTES = KIND == KIND_FWD ? QP_BUFS * QP_BUF_BYTES : 0;
+    static constexpr int QP_CHUNK = TN == 256 ? 8 : 16;                    // k-blocks per chunk of staged group parameters
+    static constexpr int QP_WORDS = QP_CHUNK / 2 * QP_PITCH;               // words per buffer
+    static constexpr int QP_BYTES = KIND == KIND_FWD ? 3 * QP_WORDS * 4 : 0;
+    static_assert(QP_WORDS * 4 >= QP_CHUNK * 256, "a chunk of per-column parameters fits a buffer");
     static constexpr int STAGES_FIT = (227 * 1024 - 1024 - 1024 - FIX_BYTES - QP_BYTES) / STAGE_BYTES;
     // Tensor-memory A operand with token tiles up to 192: both accumulators fit beside the A slots, of which there are then
     // as many as pipeline stages (up to 128 tokens) or one per dequant team (four: the shared-memory ring is deeper than the
@@ -857,7 +859,7 @@ k_gemm(const __grid_constant__ CUtensorMap map_tok, const __grid_constant__ CUte
             // Forward with groups of 128 (an even number per row): the group parameters come through shared memory.  Read where
             // they are needed, one 2-byte load per lane, row and stage touches 32 cache lines a warp and instruction: 256
             // L1 cycles per stage, which bounded the kernel below 256 tokens.  Here the 512 threads fetch a chunk of 16
-            // k-blocks together, four lanes per row, one chunk ahead of its use.
+            // k-blocks together, four lanes per row, ahead of its use.
             // (QPT: the parameters of a stage's 64 contraction elements, the same for every row of the tile's k group, come the
             // same way: 256 bytes per stage, one 16-byte piece per thread.)
             if constexpr (KIND == KIND_FWD && RT == 1) {
@@ -871,10 +873,11 @@ k_gemm(const __grid_constant__ CUtensorMap map_tok, const __grid_constant__ CUte
                             if (!c.walk.next(p, sg)) { c.valid = false; return; }
                             c.kb = sg.kb0; c.kb1 = sg.kb1; c.r_tile = sg.r_tile;
                         }
-                        c.end = min(c.kb1, (c.kb | (QP_CHUNK - 1)) + 1);
+                        c.end = min(c.kb1, (c.kb | (C::QP_CHUNK - 1)) + 1);
                     };
-                    const int q_row = (warp - 6) * 8 + (lane >> 2), q_col = (lane & 3) * 2;
+                    constexpr int LPR = C::QP_CHUNK / 4;                              // lanes per row, two groups each
                     const int dq_tid = (warp - 6) * 32 + lane;
+                    const int q_row = dq_tid / LPR, q_col = (dq_tid % LPR) * 2;
                     uint32_t ls = 0u, lz = 0u;
                     uint4 lq = make_uint4(0u, 0u, 0u, 0u);
                     auto fetch = [&](const Chunk& c) {
@@ -883,29 +886,27 @@ k_gemm(const __grid_constant__ CUtensorMap map_tok, const __grid_constant__ CUte
                                 lq = __ldg(p.qpt + ((size_t)c.r_tile * (size_t)(p.C >> 3) + (size_t)c.kb * 8) * 2 + dq_tid);
                             return;
                         }
-                        const int wrow = c.r_tile * TILE_R + q_row, g0 = (c.kb / QP_CHUNK) * 8 + q_col;
+                        const int wrow = c.r_tile * TILE_R + q_row, g0 = (c.kb / C::QP_CHUNK) * (C::QP_CHUNK / 2) + q_col;
                         ls = lz = 0u;
-                        if (c.valid && wrow < p.R && g0 < groups_per_row) {          // groups_per_row is even
+                        if (c.valid && q_row < TILE_R && wrow < p.R && g0 < groups_per_row) {          // groups_per_row is even
                             const size_t at = (size_t)wrow * groups_per_row + g0;
                             ls = __ldg(reinterpret_cast<const uint32_t*>(p.scales + at)); lz = __ldg(reinterpret_cast<const uint32_t*>(p.zeros + at));
                         }
                     };
                     auto stash = [&](int buf) {
                         if (QPT) {
-                            if (dq_tid < QP_CHUNK * 16) reinterpret_cast<uint4*>(qpb + buf * (8 * QP_PITCH))[dq_tid] = lq;
+                            if (dq_tid < C::QP_CHUNK * 16) reinterpret_cast<uint4*>(qpb + buf * C::QP_WORDS)[dq_tid] = lq;
                             return;
                         }
+                        if (q_row >= TILE_R) return;
                         const uint32_t z = bf2_as_u32(__hadd2_rn(u32_as_bf2(lz), c128));
-                        uint32_t* d = qpb + buf * (8 * QP_PITCH) + q_col * QP_PITCH + q_row;
+                        uint32_t* d = qpb + buf * C::QP_WORDS + q_col * QP_PITCH + q_row;
                         d[0] = __byte_perm(ls, z, 0x5410); d[QP_PITCH] = __byte_perm(ls, z, 0x7632);
                     };
-                    auto team_barrier = [] { asm volatile("bar.sync 1, 512;" ::: "memory"); };       // the 16 dequant warps
-                    // Two buffers: every warp has read chunk c and written chunk c + 1 when the barrier at the end of chunk c lets it go on.
-                    // Three buffers: a warp writes chunk c + 1 when it begins chunk c and waits, one chunk later, for the others
-                    // to have done so - they have, unless they lag by a whole chunk.  (Beginning chunk c means that all warps
-                    // began chunk c - 1, i.e. are done with chunk c - 2, whose buffer chunk c + 1 takes.)  The barrier at the end of every chunk
-                    // held the dequant warps for a quarter of their time.
-                    constexpr bool QP3 = C::QP_BUFS == 3;
+                    // A warp writes chunk c + 1 when it begins chunk c and waits, one chunk later, for the others to have done so - they
+                    // have, unless they lag by a whole chunk.  (Beginning chunk c means that all warps began chunk c - 1, i.e. are
+                    // done with chunk c - 2, whose buffer chunk c + 1 takes.)  Two buffers and a barrier at the end of every chunk held
+                    // the dequant warps for a quarter of their time.
                     auto announce = [&](int buf) {
                         __syncwarp();
                         if (lane == 0) mbar_arrive(smem_u32(&ctl->qp_ready[buf]));
@@ -913,31 +914,26 @@ k_gemm(const __grid_constant__ CUtensorMap map_tok, const __grid_constant__ CUte
                     Chunk cur{SegWalk<SK>(p), 0, 0, 0, 0, true};
                     next_chunk(cur);
                     fetch(cur); stash(0);
-                    Chunk ahead = cur;                                       // three buffers: the chunk whose parameters are in registers
+                    Chunk ahead = cur;                                       // the chunk whose parameters are in registers
                     uint32_t qp_phase = 0u;
-                    if (QP3) { announce(0); if (ahead.valid) next_chunk(ahead); fetch(ahead); }
-                    else team_barrier();
+                    announce(0);
+                    if (ahead.valid) next_chunk(ahead);
+                    fetch(ahead);
                     const int my_row = TA ? quarter * 32 + lane : tt;
                     uint32_t base = 0u;
                     int buf = 0;
                     while (cur.valid) {
-                        Chunk nxt = ahead;
-                        if (QP3) {
-                            ok = mbar_wait(smem_u32(&ctl->qp_ready[buf]), qp_phase, abort_flag) && ok;
-                            if (nxt.valid) {
-                                const int to = buf == 2 ? 0 : buf + 1;
-                                stash(to);
-                                announce(to);
-                                next_chunk(ahead);
-                                fetch(ahead);
-                            }
-                        } else {
-                            nxt = cur;
-                            next_chunk(nxt);
-                            fetch(nxt);
+                        const Chunk nxt = ahead;
+                        ok = mbar_wait(smem_u32(&ctl->qp_ready[buf]), qp_phase, abort_flag) && ok;
+                        if (nxt.valid) {
+                            const int to = buf == 2 ? 0 : buf + 1;
+                            stash(to);
+                            announce(to);
+                            next_chunk(ahead);
+                            fetch(ahead);
                         }
                         const int n = (cur.end - cur.kb) / KBS;
-                        for (int i = (int)((uint32_t)(team - (int)base) & 3u); i < n && ok; i += 4) {    // (an aborted team still meets the barriers)
+                        for (int i = (int)((uint32_t)(team - (int)base) & 3u); i < n && ok; i += 4) {
                             const uint32_t cnt = base + (uint32_t)i;
                             const int stage = (int)(cnt % (uint32_t)C::STAGES);
                             if (!(ok = stage_ready(cnt, stage))) break;
@@ -945,13 +941,13 @@ k_gemm(const __grid_constant__ CUtensorMap map_tok, const __grid_constant__ CUte
                             if constexpr (QPT) {
                                 const uint32_t dst = ta_addr + (uint32_t)((C::A_SLOTS == C::STAGES ? stage : team) * C::A_COLS);
                                 const uint4 r0 = reinterpret_cast<const uint4*>(raw)[raw_swap(my_row)], r1 = reinterpret_cast<const uint4*>(raw)[raw_swap(my_row) ^ 1];
-                                const uint4* qp = reinterpret_cast<const uint4*>(qpb + buf * (8 * QP_PITCH)) + i * 16;
+                                const uint4* qp = reinterpret_cast<const uint4*>(qpb + buf * C::QP_WORDS) + i * 16;
                                 const uint32_t wq[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};
 #pragma unroll
                                 for (int h = 0; h < 8; h += 2)
                                     tmem_st8(dst + (uint32_t)(4 * h), dequant8t(wq[h], qp[2 * h + 1], qp[2 * h]), dequant8t(wq[h + 1], qp[2 * h + 3], qp[2 * h + 2]));
                             } else {
-                                const uint32_t qp = qpb[buf * (8 * QP_PITCH) + (((cur.kb + i * KBS) >> 1) & 7) * QP_PITCH + my_row];
+                                const uint32_t qp = qpb[buf * C::QP_WORDS + (((cur.kb + i * KBS) >> 1) & (C::QP_CHUNK / 2 - 1)) * QP_PITCH + my_row];
                                 const __nv_bfloat162 s2 = u32_as_bf2(__byte_perm(qp, qp, 0x1010)), z2 = u32_as_bf2(__byte_perm(qp, qp, 0x3232));
                                 const uint32_t dst = ta_addr + (uint32_t)((C::A_SLOTS == C::STAGES ? stage : team) * C::A_COLS);
                                 const int swz = my_row & 7;
@@ -975,13 +971,7 @@ k_gemm(const __grid_constant__ CUtensorMap map_tok, const __grid_constant__ CUte
                             stage_done(stage);
                         }
                         base += (uint32_t)n;
-                        if (QP3) {
-                            if (++buf == 3) { buf = 0; qp_phase ^= 1u; }
-                        } else {
-                            buf ^= 1;
-                            if (nxt.valid) stash(buf);
-                            team_barrier();
-                        }
+                        if (++buf == 3) { buf = 0; qp_phase ^= 1u; }
                         cur = nxt;
                     }
                 }
