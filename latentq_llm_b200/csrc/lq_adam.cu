@@ -42,16 +42,15 @@ __device__ __forceinline__ float adam_apply(const lq_adam_hyper& h, float p, flo
 }
 
 __device__ __forceinline__ uint8_t opt8_encode1(float x, float mx, float s) {
-    const float t = rne(div_rn(__fsub_rn(mx, x), s, __frcp_rn(s), fastdiv_ok_scale(s)));
+    const float t = rne(div_rn(__fsub_rn(mx, x), div_by(s)));
     return (uint8_t)(f2bits(fminf(fmaxf(t, 0.0f), 255.0f)) & 0xffu);
 }
 __device__ __forceinline__ uint2 opt8_encode8(const float (&x)[8], float mx, float s) {
-    const float rs = __frcp_rn(s);
-    const bool ok = fastdiv_ok_scale(s);
+    const DivBy by_s = div_by(s);
     uint32_t b[8];
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-        float t = rne(div_rn(__fsub_rn(mx, x[k]), s, rs, ok));
+        float t = rne(div_rn(__fsub_rn(mx, x[k]), by_s));
         t = fminf(fmaxf(t, 0.0f), 255.0f);
         b[k] = f2bits(t) & 0xffu;
     }
@@ -141,8 +140,8 @@ __global__ void __launch_bounds__(256) k_adam_quant(const AdamParams p) {
 //             so the bf16 result is that of the exactly rounded root.
 //   m / d     rcp.approx and one residual correction: the quotient of two 8-bit significands is at least 2^-33 away from
 //             every midpoint of two fp32 numbers, the corrected quotient is 2^-44 off before its rounding.
-//   states    encoded with a quotient q0 from a two-term reciprocal, then one residual correction with RN(1/s): q0 is
-//             within one ulp, which makes the corrected quotient the correctly rounded one (Markstein).
+//   states    encoded with a quotient from a two-term reciprocal and one residual correction (Markstein's theorem, see div_by), as is
+//             the division of the block's range by 255.
 //   requantize  everything after Z = w/scale + zero from the table of the requantize fast path (int4: a byte per bf16 pattern,
 //             |Z| < 64; int8: two bytes, |Z| < 256); the kernel keeps the two runs of it that can be looked up and puts its other
 //             tables into the gap between them.
@@ -189,9 +188,9 @@ __device__ __forceinline__ float div_bf16(float a, float b) {
 // (scale, its reciprocal as RN(1/s) + remainder) of one 8-bit state block: s = (mx - mn) / 255 + 1e-10
 struct OptScale { float s, r, rl; };
 __device__ __forceinline__ OptScale opt8_scale(float mx, float mn) {
-    const float a = __fsub_rn(mx, mn), r255 = 1.0f / 255.0f;
-    float q = __fmul_rn(a, r255);                                    // a / 255, correctly rounded (below 2^-100 the 1e-10 hides it)
-    q = __fmaf_rn(__fmaf_rn(-q, 255.0f, a), r255, q);
+    constexpr float r255 = 1.0f / 255.0f, r255l = (float)(1.0 / 255.0 - (double)r255);
+    const float a = __fsub_rn(mx, mn);
+    float q = __fmaf_rn(a, r255, __fmul_rn(a, r255l));               // a / 255, correctly rounded (below 2^-100 the 1e-10 hides it)
     q = __fmaf_rn(__fmaf_rn(-q, 255.0f, a), r255, q);
     OptScale o;
     o.s = __fadd_rn(q, 1e-10f);

@@ -160,23 +160,31 @@ __device__ __forceinline__ void philox_dither8(uint64_t seed, uint64_t stream_id
     }
 }
 
-// Correctly rounded a/s from r = RN(1/s): q0 = a*r followed by two FMA residual corrections (the
-// refinement CUDA's own division uses).  Valid for normal, mid-range operands; callers fall back to
-// __fdiv_rn otherwise.
+// Correctly rounded quotients by a divisor that several elements share.  Method: Markstein's theorem (P. Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34(1), 1990): with y = RN(1/s) and q within one unit
+// in the last place of a/s, the remainder a - q s is exact in one FMA and RN(q + y (a - q s)) = RN(a/s).  The first quotient q comes from a
+// reciprocal in two terms, y + yl = (1/s)(1 + e) with |e| < 2^-46: q = RN(a y + RN(a yl)) is off by half a unit (its rounding) and less than
+// 2^-20 units more.  Everything stays normal, and the remainder exact, for divisors and dividends in the ranges tested below;
+// outside them __fdiv_rn divides.
 __device__ __forceinline__ bool fastdiv_ok_scale(float s) {
     float a = fabsf(s);
     return a >= 9.094947e-13f && a <= 1.0995116e12f;  // 2^-40 .. 2^40
 }
-__device__ __forceinline__ float div_rn(float a, float s, float r, bool scale_ok) {
-    float m = fabsf(a);
-    if (scale_ok && (m == 0.0f || (m >= 8.6736174e-19f && m <= 1.1529215e18f))) {  // 2^-60 .. 2^60
-        float q = __fmul_rn(a, r);
-        float e = __fmaf_rn(-q, s, a);
-        q = __fmaf_rn(e, r, q);
-        e = __fmaf_rn(-q, s, a);
-        return __fmaf_rn(e, r, q);
-    }
-    return __fdiv_rn(a, s);
+struct DivBy { float s, y, yl; bool ok; };
+__device__ __forceinline__ DivBy div_by(float s) {
+    DivBy d;
+    d.s = s; d.y = __frcp_rn(s); d.ok = fastdiv_ok_scale(s);
+    d.yl = __fmul_rn(__fmaf_rn(-s, d.y, 1.0f), d.y);
+    return d;
+}
+__device__ __forceinline__ float markstein_div(float a, const DivBy& d) {
+    const float q = __fmaf_rn(a, d.y, __fmul_rn(a, d.yl));
+    return __fmaf_rn(__fmaf_rn(-q, d.s, a), d.y, q);
+}
+__device__ __forceinline__ float div_rn(float a, const DivBy& d) {
+    const float m = fabsf(a);
+    if (d.ok && (m == 0.0f || (m >= 8.6736174e-19f && m <= 1.1529215e18f))) return markstein_div(a, d);  // 2^-60 .. 2^60
+    return __fdiv_rn(a, d.s);
 }
 
 }  // namespace lq

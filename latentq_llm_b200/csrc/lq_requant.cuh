@@ -111,17 +111,11 @@ template <bool BF> __device__ __forceinline__ float rb(float x) {
     u += 0x7fffu + ((u >> 16) & 1u);
     return __uint_as_float(u & 0xffff0000u);
 }
-// correctly rounded a/s from r = RN(1/s); only large |a| needs the slow path (tiny |a| cannot change any
-// output of the chain: the quotient stays below 2^-19 either way)
-__device__ __forceinline__ float div_fast(float a, float s, float r, bool scale_ok) {
-    if (scale_ok && fabsf(a) <= 1.1529215e18f) {
-        float q = __fmul_rn(a, r);
-        float e = __fmaf_rn(-q, s, a);
-        q = __fmaf_rn(e, r, q);
-        e = __fmaf_rn(-q, s, a);
-        return __fmaf_rn(e, r, q);
-    }
-    return __fdiv_rn(a, s);
+// a/s; only large |a| needs the slow path (tiny |a| cannot change any output of the chain: the quotient stays below 2^-19
+// either way)
+__device__ __forceinline__ float div_fast(float a, const DivBy& d) {
+    if (d.ok && fabsf(a) <= 1.1529215e18f) return markstein_div(a, d);
+    return __fdiv_rn(a, d.s);
 }
 
 // WBITS 4: codes are nibble pairs (4 bytes per 8 elements), zero point per group, clamp [0,15].
@@ -206,8 +200,7 @@ template <int WBITS, int CODEC, int DITHER, bool BF>
 __device__ __forceinline__ void latent_store(const RequantParams& p, const int64_t w, const float s, const float z,
                                              const float (&lat)[8]) {
         const int64_t e0 = w * 8;
-        const float rs = __frcp_rn(s);
-        const bool s_ok = fastdiv_ok_scale(s);
+        const DivBy by_s = div_by(s);
         float u[8];
         if (CODEC != LQ_CODEC_NONE) {
             if (DITHER == LQ_DITHER_EXPLICIT) load8(p.dither_buf, LQ_F32, e0, u);
@@ -217,7 +210,7 @@ __device__ __forceinline__ void latent_store(const RequantParams& p, const int64
         uint32_t rword = 0, q[8];
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
-            float Z = rb<BF>(div_fast(lat[k], s, rs, s_ok));
+            float Z = rb<BF>(div_fast(lat[k], by_s));
             if (WBITS == 4) Z = rb<BF>(__fadd_rn(Z, z));
             float qf = rne(Z);
             float r = rb<BF>(__fsub_rn(Z, qf));

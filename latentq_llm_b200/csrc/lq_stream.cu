@@ -859,15 +859,14 @@ __global__ void __launch_bounds__(256) k_opt8_quant(const float* __restrict__ x,
     for (int i = 1; i < (int)(blockDim.x >> 5); ++i) { mn = fminf(mn, s_mn[i]); mx = fmaxf(mx, s_mx[i]); }
     const float s = __fadd_rn(__fdiv_rn(__fsub_rn(mx, mn), 255.0f), 1e-10f);
     if (threadIdx.x == 0) { scale[blockIdx.x] = s; tmax[blockIdx.x] = mx; }
-    const float rs = __frcp_rn(s);
-    const bool ok = fastdiv_ok_scale(s);
+    const DivBy by_s = div_by(s);
     uint32_t* qv = reinterpret_cast<uint32_t*>(q + base);
     auto quant4 = [&](const float4& v) {
         const float f[4] = {v.x, v.y, v.z, v.w};
         uint32_t o = 0;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            const float t = rintf(div_rn(__fsub_rn(mx, f[k]), s, rs, ok));
+            const float t = rintf(div_rn(__fsub_rn(mx, f[k]), by_s));
             o |= (uint32_t)(int)fminf(fmaxf(t, 0.0f), 255.0f) << (8 * k);
         }
         return o;
@@ -910,8 +909,7 @@ __global__ void __launch_bounds__(256) k_opt8_quant_warp(const float* __restrict
     }
     const float s = __fadd_rn(__fdiv_rn(__fsub_rn(mx, mn), 255.0f), 1e-10f);
     if (lane == 0) { scale[blk] = s; tmax[blk] = mx; }
-    const float rs = __frcp_rn(s);
-    const bool ok = fastdiv_ok_scale(s);
+    const DivBy by_s = div_by(s);
     uint32_t* qv = reinterpret_cast<uint32_t*>(q + blk * block);
 #pragma unroll
     for (int u = 0; u < VW; ++u) {
@@ -921,7 +919,7 @@ __global__ void __launch_bounds__(256) k_opt8_quant_warp(const float* __restrict
             uint32_t o = 0;
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                const float t = rintf(div_rn(__fsub_rn(mx, f[k]), s, rs, ok));
+                const float t = rintf(div_rn(__fsub_rn(mx, f[k]), by_s));
                 o |= (uint32_t)(int)fminf(fmaxf(t, 0.0f), 255.0f) << (8 * k);
             }
             qv[i] = o;
