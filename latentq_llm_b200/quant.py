@@ -132,9 +132,9 @@ def _w4_args(qparamw4):
 def _apply(fn, *args):
     """`fn.apply(*args)`; with gradients off and no transform looking on, the function's forward itself (an autograd node costs
     more host time than a decode-sized launch takes on the GPU).  Forward-mode duals and functorch transforms go through
-    `apply`, which refuses or handles them as before."""
+    `apply`, which refuses or handles them as before; a trace records the function there, and could not see a launch here."""
     if (torch.is_grad_enabled() or torch._C._are_functorch_transforms_active() or torch.autograd.forward_ad._current_level >= 0
-            or torch.compiler.is_compiling()):
+            or torch.jit.is_tracing() or torch.compiler.is_compiling()):
         return fn.apply(*args)
     return fn.forward(*args)
 

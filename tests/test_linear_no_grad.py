@@ -1,5 +1,7 @@
 """The linear's no-gradient route: calls the autograd function's forward directly, and leaves every case that autograd has a say in
-(gradients on, forward-mode duals, functorch transforms) to `apply`."""
+(gradients on, forward-mode duals, functorch transforms, traces) to `apply`."""
+import ctypes
+
 import torch
 import torch.autograd.forward_ad as fwd
 
@@ -48,3 +50,26 @@ def test_direct_call_only_where_autograd_has_no_say():
     assert _went_through_apply(x)
     with torch.inference_mode():
         assert torch.equal(quant._apply(_Double, x), 2 * x)
+
+
+class _Foreign(torch.autograd.Function):
+    """Writes its output behind torch's back, as the kernels do."""
+
+    @staticmethod
+    def forward(x):
+        y = torch.empty_like(x)
+        ctypes.memmove(y.data_ptr(), x.data_ptr(), x.numel() * x.element_size())
+        return y
+
+    @staticmethod
+    def setup_context(ctx, inputs, output):
+        pass
+
+
+def test_a_trace_records_the_function():
+    with torch.no_grad():
+        traced = torch.jit.trace(lambda v: quant._apply(_Foreign, v), torch.randn(64), check_trace=False)
+        assert "Foreign" in str(traced.graph)
+        for i in range(4):
+            x = torch.randn(64)
+            assert torch.equal(traced(x), x)
