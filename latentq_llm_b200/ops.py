@@ -411,8 +411,10 @@ def gemm_a8w8_module(x8, w8, clampv, alpha, bias, qscales):
     assert w8.shape[1] == K and qscales.numel() == N
     if clampv is not None:
         _chk(clampv, "clampv", torch.float32)
+        assert clampv.numel() == 1
     if bias is not None:
         _chk(bias, "bias", torch.bfloat16)
+        assert bias.numel() == N
     y = torch.empty((M, N), dtype=torch.bfloat16, device=x8.device)
     ws, nb = _workspace(L.GEMM_A8W8, M, N, K, x8.device)
     L.call("lq_gemm_a8w8_module", _ptr(x8), _ptr(w8), _ptr(clampv), float(alpha), _ptr(bias), _ptr(qscales), _ptr(y), M, N, K, _ptr(ws), nb,
@@ -429,6 +431,7 @@ def i8_dequant(codes, row_scales=None, clampv=None):
         assert row_scales.numel() == rows
     else:
         _chk(clampv, "clampv", torch.float32)
+        assert clampv.numel() == 1
     y = torch.empty((rows, cols), dtype=torch.bfloat16, device=codes.device)
     L.call("lq_i8_dequant", _ptr(codes), _ptr(row_scales), _ptr(clampv), rows, cols, _ptr(y), _stream())
     return y

@@ -235,23 +235,28 @@ def _a8w8_forward(input8, clampv, weight_d, qscales, bias):
     """The reference's call `linear_a8_w8_bbf16_obf16(x8, w8, bias/qscales, clampv/127.) * qscales`
     (utils/quant.py:268-271).  `clampv` is a Python float (static) or a device tensor (dynamic: input.max());
     the tensor case avoids the host synchronisation of converting it to a float."""
-    M = input8.shape[0]
+    M, N = input8.shape[0], weight_d.shape[0]
     qs = qscales.detach()
-    if qs.dtype == torch.bfloat16 and qs.is_contiguous() and (bias is None or bias.dtype == torch.bfloat16) and (
-            not torch.is_tensor(clampv) or clampv.dtype == torch.float32):
-        on_device = torch.is_tensor(clampv)
+    on_device = torch.is_tensor(clampv)
+    # one launch for a scale and a bias of one element per output channel; other forms broadcast, or are refused, below
+    if (qs.dtype == torch.bfloat16 and qs.is_contiguous() and qs.numel() == N
+            and (bias is None or (bias.dtype == torch.bfloat16 and bias.numel() == N and bias.shape[-1:] == (N,)))
+            and (not on_device or (clampv.dtype == torch.float32 and clampv.numel() == 1))):
         return ops.gemm_a8w8_module(input8, weight_d, clampv if on_device else None, 1.0 if on_device else float(clampv) / 127.,
                                     None if bias is None else bias.detach().contiguous(), qs)
-    if torch.is_tensor(clampv):
+    if on_device:
         # clampv/127. on the reference's 0-dim bf16 tensor rounds to bf16
         alpha = (clampv.to(torch.bfloat16) / 127.).float().reshape(1).expand(M).contiguous()
     else:
         alpha = torch.full((M,), float(clampv) / 127., dtype=torch.float32, device=input8.device)
     if bias is not None:
-        b = (bias / qscales.view(-1)).to(torch.bfloat16).contiguous()
+        b = (bias / qscales.view(-1)).to(torch.bfloat16)
     else:
-        b = (0 * qscales.view(-1)).to(torch.bfloat16).contiguous()
-    out = ops.gemm_a8w8(input8, weight_d, alpha, None, 1.0, b)
+        b = (0 * qscales.view(-1)).to(torch.bfloat16)
+    b = b.reshape(-1)
+    if b.numel() < N:                            # one element for all channels; the kernel reads N
+        b = b.expand(N)
+    out = ops.gemm_a8w8(input8, weight_d, alpha, None, 1.0, b.contiguous())
     return out * qscales.view(1, -1)
 
 
@@ -265,7 +270,7 @@ def _a8w8_backward(ctx, grad_output, input_f, weight_d, qscales, bias, detach=Fa
     grad_input = grad_bias = None
     if ctx.needs_input_grad[0]:
         if (grad_output.dtype == torch.bfloat16 and qscales.dtype == torch.bfloat16 and qscales.is_contiguous()
-                and qscales.numel() == weight_d.shape[0] == qscales.shape[0]):
+                and qscales.shape == (weight_d.shape[0], 1)):
             weight_forward = ops.i8_dequant(weight_d, row_scales=qscales)
         else:
             weight_forward = weight_d.to(grad_output.dtype) * qscales
