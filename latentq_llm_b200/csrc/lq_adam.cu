@@ -630,9 +630,10 @@ int lq_adam_a16w4_step(int8_t* codes, int32_t* words, const void* grad, int grad
     if (opts->codec == LQ_CODEC_THREEFOLD && opts->dither == LQ_DITHER_HASH) {
         if (bf && p.rq.group_shift >= 3 && p.rq.n_words < ((int64_t)1 << 31) && opts->mu_enc >= 0 && opts->mu_enc <= 3 &&
             opts->mu_dec >= 0 && opts->mu_dec <= 3 && adam_fast_hyper_ok(*hyper) && !getenv("LQ_REQUANT_GENERIC")) {
-            rc = ensure_encz_table(opts->mu_enc, opts->v0, st);
-            if (rc) return rc;
-            return launch_adam_fast<4>(p, opts->mu_enc, opt_block, 0, st);
+            int table = 0;
+            rc = ensure_encz_table(opts->mu_enc, opts->v0, st, table);
+            if (rc == LQ_OK) return launch_adam_fast<4>(p, table, opt_block, 0, st);
+            if (rc != LQ_EUNSUPPORTED) return rc;
         }
         return launch_adam<4, LQ_CODEC_THREEFOLD, LQ_DITHER_HASH>(p, bf, st);
     }
@@ -670,8 +671,9 @@ int lq_adam_a8w8_step(int8_t* codes, int32_t* words, const void* grad, int grad_
         const uint64_t wpr = (uint64_t)(cols / 8);               // words per weight row; the row of a word by multiply-high, exact below 2^24 words
         if (bf && wpr > 1 && wpr < (1u << 24) && p.rq.n_words < ((int64_t)1 << 31) && opts->mu_enc >= 0 && opts->mu_enc <= 3 &&
             opts->mu_dec >= 0 && opts->mu_dec <= 3 && adam_fast_hyper_ok(*hyper) && !getenv("LQ_REQUANT_GENERIC")) {
-            rc = ensure_enc8_table(opts->mu_enc, opts->v0, st);
-            if (rc == LQ_OK) return launch_adam_fast<8>(p, opts->mu_enc, opt_block, ~(uint64_t)0 / wpr + 1, st);
+            int table = 0;
+            rc = ensure_enc8_table(opts->mu_enc, opts->v0, st, table);
+            if (rc == LQ_OK) return launch_adam_fast<8>(p, table, opt_block, ~(uint64_t)0 / wpr + 1, st);
             if (rc != LQ_EUNSUPPORTED) return rc;
         }
         return launch_adam<8, LQ_CODEC_THREEFOLD, LQ_DITHER_HASH>(p, bf, st);

@@ -283,10 +283,24 @@ static inline int fill_requant(RequantParams& p, const lq_requant_opts* o, int64
 static inline bool dtype_ok(int d) { return d == LQ_F32 || d == LQ_BF16; }
 
 
-// ---- table of the bf16 fast paths: everything after Z as one byte (each translation unit that launches a kernel
-// reading it holds its own copy; built once per device, curve level and hash offset) ---------------------------
+// ---- tables of the bf16 fast paths: everything after Z as one byte or two (each translation unit that launches a kernel
+// reading one holds its own copy) -------------------------------------------------------------------------------
+// A table belongs to a device, a curve level and a hash offset v0, is built on first use and is never rewritten: a captured launch, or
+// one still running on another stream, goes on reading the table it was launched with.  Each level has two: of v0 = 0, which the
+// package passes everywhere, and of the first other offset; a further one gets LQ_EUNSUPPORTED, and its caller takes the
+// generic kernel, which has v0 by value.
+constexpr int ENC_TABLES = 8;
+struct EncTables { bool built[64][ENC_TABLES]; float v0[64][ENC_TABLES]; };
+static std::mutex g_encz_mutex;
+// Table index of (mu, v0) on the current device; `ready` if it has been built.
+static inline int enc_table_of(const EncTables& t, int mu, float v0, int& dev, int& slot, bool& ready) {
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return LQ_EUNSUPPORTED;
+    slot = 2 * ((mu < 0 || mu > 3) ? 0 : mu) + (v0 == 0.0f ? 0 : 1);
+    ready = t.built[dev][slot];
+    return ready && t.v0[dev][slot] != v0 ? LQ_EUNSUPPORTED : LQ_OK;
+}
 constexpr int ENCZ_TABLE_ENTRIES = 65536;               // every bf16 pattern of Z = w/scale + zero
-static __device__ uint8_t g_encz_table[4][ENCZ_TABLE_ENTRIES]; // one per curve level; entry = final code << 4 | residual nibble
+static __device__ __align__(16) uint8_t g_encz_table[ENC_TABLES][ENCZ_TABLE_ENTRIES];       // entry = final code << 4 | residual nibble
 static __global__ void __launch_bounds__(256) k_build_encz_table(int slot, Curve c, float v0) {
     for (int h = blockIdx.x * blockDim.x + threadIdx.x; h < ENCZ_TABLE_ENTRIES; h += gridDim.x * blockDim.x) {
         const float Z = __uint_as_float((uint32_t)h << 16);
@@ -295,51 +309,46 @@ static __global__ void __launch_bounds__(256) k_build_encz_table(int slot, Curve
         g_encz_table[slot][h] = e;
     }
 }
-
-static std::mutex g_encz_mutex;
-// Builds (once per device, curve level and v0) the encode table the fast path reads.
-static inline int ensure_encz_table(int mu, float v0, cudaStream_t st) {
-    static bool built[64][4] = {};
-    static float built_v0[64][4] = {};
+static inline int ensure_encz_table(int mu, float v0, cudaStream_t st, int& slot) {
+    static EncTables tables = {};
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return LQ_EUNSUPPORTED;
-    const int slot = (mu < 0 || mu > 3) ? 0 : mu;
+    bool ready = false;
     std::lock_guard<std::mutex> lock(g_encz_mutex);
-    if (built[dev][slot] && built_v0[dev][slot] == v0) return LQ_OK;
-    k_build_encz_table<<<128, 256, 0, st>>>(slot, curve_for_level(slot), v0);
-    int rc = check_launch("k_build_encz_table");
+    int rc = enc_table_of(tables, mu, v0, dev, slot, ready);
+    if (rc || ready) return rc;
+    k_build_encz_table<<<128, 256, 0, st>>>(slot, curve_for_level(slot / 2), v0);
+    rc = check_launch("k_build_encz_table");
     if (rc) return rc;
     // first use only: make the table visible to every stream before anyone else may read it
     cudaError_t e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) { set_cuda_error(e, "cudaStreamSynchronize"); return LQ_ECUDA; }
-    built[dev][slot] = true; built_v0[dev][slot] = v0;
+    tables.built[dev][slot] = true; tables.v0[dev][slot] = v0;
     return LQ_OK;
 }
 // The same for int8 codes: every bf16 pattern of Z = w/scale -> code & 0xff | nibble << 8 (|Z| < 256)
-static __device__ uint16_t g_enc8_table[4][65536];
+static __device__ __align__(16) uint16_t g_enc8_table[ENC_TABLES][65536];
 static __global__ void __launch_bounds__(256) k_build_enc8_table(int slot, Curve c, float v0) {
     for (int h = blockIdx.x * blockDim.x + threadIdx.x; h < 65536; h += gridDim.x * blockDim.x) {
         const float Z = __uint_as_float((uint32_t)h << 16);
         g_enc8_table[slot][h] = (fabsf(Z) < 256.0f) ? (uint16_t)encode_from_z_w8_hash_bf16(Z, c, v0) : (uint16_t)0;
     }
 }
-static inline int ensure_enc8_table(int mu, float v0, cudaStream_t st) {
-    static bool built[64][4] = {};
-    static float built_v0[64][4] = {};
+static inline int ensure_enc8_table(int mu, float v0, cudaStream_t st, int& slot) {
+    static EncTables tables = {};
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return LQ_EUNSUPPORTED;
-    const int slot = (mu < 0 || mu > 3) ? 0 : mu;
+    bool ready = false;
     std::lock_guard<std::mutex> lock(g_encz_mutex);
-    if (built[dev][slot] && built_v0[dev][slot] == v0) return LQ_OK;
+    int rc = enc_table_of(tables, mu, v0, dev, slot, ready);
+    if (rc || ready) return rc;
     // building ends with a synchronisation, which a stream that is being captured does not allow: the caller takes its generic kernel
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) return LQ_EUNSUPPORTED;
-    k_build_enc8_table<<<128, 256, 0, st>>>(slot, curve_for_level(slot), v0);
-    int rc = check_launch("k_build_enc8_table");
+    k_build_enc8_table<<<128, 256, 0, st>>>(slot, curve_for_level(slot / 2), v0);
+    rc = check_launch("k_build_enc8_table");
     if (rc) return rc;
     cudaError_t e = cudaStreamSynchronize(st);       // first use only: visible to every stream before anyone reads it
     if (e != cudaSuccess) { set_cuda_error(e, "cudaStreamSynchronize"); return LQ_ECUDA; }
-    built[dev][slot] = true; built_v0[dev][slot] = v0;
+    tables.built[dev][slot] = true; tables.v0[dev][slot] = v0;
     return LQ_OK;
 }
 

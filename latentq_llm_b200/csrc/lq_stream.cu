@@ -349,7 +349,7 @@ __global__ void __launch_bounds__(256) k_requant(const RequantParams p) {
 // Indexed by the bf16 pattern of Z itself for |Z| < 32: 0x0000..0x41ff and 0x8000..0xc1ff; the entries between the two
 // runs are never read (such a Z takes the generic path) and never written.
 constexpr int ENCP_HALF = 0x4200, ENCP_ENTRIES = 2 * ENCP_HALF, ENCP_SPAN = 0x8000 + ENCP_HALF;
-__device__ uint32_t g_encp_table[4][ENCP_SPAN];
+__device__ __align__(16) uint32_t g_encp_table[4][ENCP_SPAN];
 __device__ unsigned int g_encp_not_a_step[4];           // patterns whose outcome is not a single step in h (expected: 0)
 __global__ void __launch_bounds__(256) k_build_encp_table(int slot, Curve c) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ENCP_ENTRIES; i += gridDim.x * blockDim.x) {
@@ -712,9 +712,9 @@ static int launch_fold_fast8_v(const RequantParams& p, int slot, cudaStream_t st
     return check_launch("k_fold_fast8");
 }
 static int launch_fold_fast8(const RequantParams& p, const lq_requant_opts* o, cudaStream_t st) {
-    int rc = ensure_enc8_table(o->mu_enc, o->v0, st);
+    int slot = 0;
+    int rc = ensure_enc8_table(o->mu_enc, o->v0, st, slot);
     if (rc) return rc;
-    const int slot = o->mu_enc;
     if (p.w_in) return launch_fold_fast8_v<true, false, false>(p, slot, st);
     const bool res = p.has_residual != 0, dl = p.delta != nullptr;
     if (res && dl) return launch_fold_fast8_v<false, true, true>(p, slot, st);
@@ -768,9 +768,10 @@ static int launch_fold_fast(const RequantParams& p, const lq_requant_opts* o, cu
         if (rc) return rc;
         return launch_fold_fast_d<LQ_DITHER_PHILOX>(p, o->mu_enc, st);
     }
-    int rc = ensure_encz_table(o->mu_enc, o->v0, st);
+    int slot = 0;
+    int rc = ensure_encz_table(o->mu_enc, o->v0, st, slot);
     if (rc) return rc;
-    return launch_fold_fast_d<LQ_DITHER_HASH>(p, o->mu_enc, st);
+    return launch_fold_fast_d<LQ_DITHER_HASH>(p, slot, st);
 }
 
 template <int WBITS, int CODEC, int DITHER, bool BF>

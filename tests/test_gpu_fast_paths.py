@@ -99,6 +99,51 @@ def test_int8_optimizer_step_captured_before_its_table_exists():
         assert torch.equal(x, y)
 
 
+@pytest.mark.parametrize("kind", ["step4", "step8", "fold4", "fold8"])
+@pytest.mark.parametrize("v0", [0.0, 0.125])
+def test_captured_launch_keeps_its_hash_offset(monkeypatch, kind, v0):
+    """A launch captured with one hash offset replays with it after calls with other offsets have built what they need."""
+    from latentq_llm_b200 import ops
+    g = _gen(11)
+    N, K = 16, 2048
+    n, blocks = N * K, N * K // 2048
+    codes0 = torch.randint(-128, 128, (N, K) if kind.endswith("8") else (n // 2,), device="cuda", generator=g, dtype=torch.int8)
+    words0 = torch.randint(-2 ** 31, 2 ** 31, (n // 8,), device="cuda", generator=g, dtype=torch.int64).to(torch.int32)
+    upd = (torch.randn(N, K, device="cuda", generator=g) * 1e-3).to(torch.bfloat16)
+    rows = N if kind.endswith("8") else n // 128
+    s = (torch.rand(rows, device="cuda", generator=g) * 0.01 + 1e-3).to(torch.bfloat16)
+    z = torch.randint(0, 16, (rows,), device="cuda", generator=g).to(torch.bfloat16)
+    hyper = ops.make_adam_hyper(0.9, 0.95, 1e-8, 1e-3)
+
+    def launch(offset):
+        o = ops.make_opts(codec=ops.CODEC_THREEFOLD, dither=ops.DITHER_HASH, has_residual=True, mu_enc=2, mu_dec=2, v0=offset)
+        c, w = codes0.clone(), words0.clone()
+        st = [t for _ in range(2) for t in (torch.zeros(N, K, dtype=torch.uint8, device="cuda"), torch.full((blocks, 1), 1e-10, device="cuda"),
+                                            torch.zeros(blocks, 1, device="cuda"))]
+        if kind == "step4":
+            ops.adam_a16w4_step(c, w, upd, s, z, *st, hyper, o)
+        elif kind == "step8":
+            ops.adam_a8w8_step(c, w, upd, s, *st, hyper, o)
+        elif kind == "fold4":
+            ops.a16w4_fold_delta(c, w, upd.view(-1), s, z, o)
+        else:
+            ops.a8w8_fold_delta(c, w, upd, s, o)
+        return c, w
+
+    monkeypatch.setenv("LQ_REQUANT_GENERIC", "1")
+    want = launch(v0)
+    monkeypatch.delenv("LQ_REQUANT_GENERIC")
+    launch(v0)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = launch(v0)
+    for other in (0.0, 0.125, 0.25, 0.375):
+        if other != v0:
+            launch(other)
+    graph.replay()
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
 # ---- requantize with Philox dither ----------------------------------------------------------------------------------
 @pytest.mark.parametrize("seed,step,param", [(0, 0, 0), (1234, 7, 3), (2 ** 64 - 1, 2 ** 32 - 1, 2 ** 32 - 1)])
 def test_philox_fold_equals_generic_kernel(monkeypatch, seed, step, param):
