@@ -553,7 +553,7 @@ k_gemm(const __grid_constant__ CUtensorMap map_tok, const __grid_constant__ CUte
         uint32_t fix_phase = 0;                    // bit b: parity to wait for on staging buffer b of this quarter
         while (ok && walk.next(p, sg)) {
             const int r_tile = sg.r_tile, t_tile = sg.t_tile, split = sg.split;
-            if (!(ok = mbar_wait_t(smem_u32(&ctl->acc_full[acc]), acc_phase, abort_flag, prof, w_accf))) break;
+            if (!(ok = warp_vote(mbar_wait_t(smem_u32(&ctl->acc_full[acc]), acc_phase, abort_flag, prof, w_accf)))) break;
             tc_fence_after();
             bool emit = true, sk_sum = false;
             int sk_parts = 1, sk_part_lo = 0;      // parts of the tile; first part that comes through the ring (1: own sums from the accumulator)
@@ -641,7 +641,7 @@ k_gemm(const __grid_constant__ CUtensorMap map_tok, const __grid_constant__ CUte
 #pragma unroll 1
                         for (int part = sk_part_lo; part < sk_parts; ++part) {
                             const int b = sk_taken & (FIX_RING - 1);
-                            if (ok) ok = mbar_wait(smem_u32(&ctl->fix_full[quad][b]), (fix_phase >> b) & 1u, abort_flag);
+                            if (ok) ok = warp_vote(mbar_wait(smem_u32(&ctl->fix_full[quad][b]), (fix_phase >> b) & 1u, abort_flag));
                             fix_phase ^= 1u << b;
                             const float* src = reinterpret_cast<const float*>(fix_ring + b * FIX_COPY_BYTES) + lane;
                             if (part == 0) {
@@ -849,7 +849,7 @@ k_gemm(const __grid_constant__ CUtensorMap map_tok, const __grid_constant__ CUte
                     const uint32_t prev = cnt - 4u;
                     r = mbar_wait_t(smem_u32(&ctl->empty[prev % (uint32_t)C::STAGES]), (prev / (uint32_t)C::STAGES) & 1u, abort_flag, prof, w_dq);
                 }
-                return __all_sync(0xffffffffu, r) != 0;                     // the TMEM store is warp-collective
+                return warp_vote(r);
             };
             auto stage_done = [&](int stage) {
                 if (TA) { tmem_st_wait(); tc_fence_before(); } else { fence_proxy_async(); }
@@ -925,7 +925,7 @@ k_gemm(const __grid_constant__ CUtensorMap map_tok, const __grid_constant__ CUte
                     int buf = 0;
                     while (cur.valid) {
                         const Chunk nxt = ahead;
-                        ok = mbar_wait(smem_u32(&ctl->qp_ready[buf]), qp_phase, abort_flag) && ok;
+                        if (!(ok = warp_vote(mbar_wait(smem_u32(&ctl->qp_ready[buf]), qp_phase, abort_flag)))) break;
                         if (nxt.valid) {
                             const int to = buf == 2 ? 0 : buf + 1;
                             stash(to);
@@ -934,7 +934,7 @@ k_gemm(const __grid_constant__ CUtensorMap map_tok, const __grid_constant__ CUte
                             fetch(ahead);
                         }
                         const int n = (cur.end - cur.kb) / KBS;
-                        for (int i = (int)((uint32_t)(team - (int)base) & 3u); i < n && ok; i += 4) {
+                        for (int i = (int)((uint32_t)(team - (int)base) & 3u); i < n; i += 4) {
                             const uint32_t cnt = base + (uint32_t)i;
                             const int stage = (int)(cnt % (uint32_t)C::STAGES);
                             if (!(ok = stage_ready(cnt, stage))) break;
@@ -971,6 +971,7 @@ k_gemm(const __grid_constant__ CUtensorMap map_tok, const __grid_constant__ CUte
                             }
                             stage_done(stage);
                         }
+                        if (!ok) break;
                         base += (uint32_t)n;
                         if (++buf == 3) { buf = 0; qp_phase ^= 1u; }
                         cur = nxt;
@@ -1002,8 +1003,6 @@ k_gemm(const __grid_constant__ CUtensorMap map_tok, const __grid_constant__ CUte
                     const int stage = (int)(cnt % (uint32_t)C::STAGES);
                     if (!(ok = stage_ready(cnt, stage))) break;
                     const int slot = C::A_SLOTS == C::STAGES ? stage : team;
-                    ok = __all_sync(0xffffffffu, ok) != 0;                 // the TMEM store below is warp-collective
-                    if (!ok) break;
                     if (TA && KIND == KIND_DGRAD) {
                         const uint32_t dst = ta_addr + (uint32_t)(slot * TA_COLS_PER_STAGE);
                         const int kk = quarter * 32 + lane;

@@ -52,6 +52,9 @@ __device__ __forceinline__ bool mbar_wait_t(uint32_t bar, uint32_t parity, volat
     acc += clock64() - t0;
     return ok;
 }
+// A wait's outcome as the whole warp's: lanes can give up at different polls, and a warp whose next steps are collective (tensor-memory
+// loads and stores, votes, __syncwarp) has to go on, or leave, together.
+__device__ __forceinline__ bool warp_vote(bool ok) { return __all_sync(0xffffffffu, ok) != 0; }
 // One lane of a converged warp (the same lane every time it is asked).
 __device__ __forceinline__ bool elect_one_sync() {
     uint32_t pred;
