@@ -1195,7 +1195,9 @@ static Plan make_plan(int kind, int64_t M, int64_t N, int64_t K, int group = 128
     pl.r_tiles = (r_tiles1 + pl.rt - 1) / pl.rt;
     const int bk = (kind == KIND_I8) ? 128 : 64;
     pl.kb_total = (int)((Cc + bk - 1) / bk);
-    if (kind != KIND_I8 && !getenv("LQ_GEMM_BALANCE")) pl.tn = pick_token_tile(kind, M, R, pl.kb_total);
+    const char* balance = getenv("LQ_GEMM_BALANCE");
+    const bool want_balanced = kind == KIND_FWD && balance && balance[0] == '1';      // its kernels exist for the widths above
+    if (kind != KIND_I8 && !want_balanced) pl.tn = pick_token_tile(kind, M, R, pl.kb_total);
     pl.t_tiles = (int)((M + pl.tn - 1) / pl.tn);
     const int tiles = pl.r_tiles * pl.t_tiles;
     const int sms = sm_count();
@@ -1207,16 +1209,14 @@ static Plan make_plan(int kind, int64_t M, int64_t N, int64_t K, int group = 128
     // it does not pay: adding up a tile's parts and the epilogue behind it are ~14 k cycles of single-warp-per-lane-
     // quarter work at the very end (470 cycles per 16-column slab and part), as much as the ~13 k cycles the shorter
     // main loop saves (41 us against 25 us for the 11008-row layer at 128 tokens), so whole tiles stay the default.
-    if (kind == KIND_FWD && pl.tn >= 64 && allow_balanced && (pl.tn < 256 || a_operand_in_tmem(kind))) {
-        const char* e = getenv("LQ_GEMM_BALANCE");
-        const bool off = !e || e[0] == '0', force = e && e[0] == '1';
+    if (want_balanced && pl.tn >= 64 && allow_balanced && (pl.tn < 256 || a_operand_in_tmem(kind))) {
         const int kb = pl.kb_total;
         const int full = tiles / sms * sms, rem = tiles - full;
         const int margin = 4 + pl.tn / 64;
         int helpers = sms - rem, h = 0;
         if (helpers > 6 * rem) helpers = 6 * rem;                   // a tile's sums are added up by one CTA: bound its parts
         bool found = false;
-        for (int it = 0; it < 16 && rem > 0 && helpers > 0 && !off; ++it) {
+        for (int it = 0; it < 16 && rem > 0 && helpers > 0; ++it) {
             h = (rem * kb + margin * helpers + rem + helpers - 1) / (rem + helpers);
             if (h < 1) h = 1;
             const int tail_units = rem * (kb - h);
@@ -1224,7 +1224,7 @@ static Plan make_plan(int kind, int64_t M, int64_t N, int64_t K, int group = 128
             if (tail_units >= 4 * helpers) { found = true; break; }
             helpers = tail_units / 4;                               // at least four k-blocks per helper
         }
-        if (found && force) {
+        if (found) {
             pl.sk = true; pl.splits = 1; pl.kb_per_split = kb;
             pl.sk_full = full; pl.sk_rem = rem; pl.sk_h = h; pl.sk_helpers = helpers;
             pl.sk_grid = full > 0 ? sms : rem + helpers;
