@@ -1155,15 +1155,15 @@ static int plan_splits(int tiles, int kb_total, int sms) {
 // with every width; tiles run in waves of one per SM.  Split-K adds the partial sums' way through memory and the reduction
 // launch.  A fixed ladder (64, 128, then 256) left 40 % of the SMs idle at token counts between its steps: 11008 rows at 300
 // tokens 53.8 (256) / 38.5 us (128), at 512 51.2 / 46.3 (192), 2048 rows at 1000 46.6 / 36.2 (128).
-static int pick_token_tile(int kind, int64_t M, int64_t R, int kb_total) {
+struct TokenTile { int tn; float fwd, fwd_tail, dgrad; };
+static const TokenTile token_tiles[] = {{32, 0.18f, 0.3f, 0.297f}, {64, 0.20f, 0.3f, 0.32f}, {96, 0.225f, 0.3f, 0.335f}, {128, 0.245f, 0.3f, 0.343f},
+                                        {160, 0.28f, 0.4f, 0.366f}, {192, 0.305f, 0.9f, 0.4f}, {256, 0.36f, 2.0f, 0.456f}};
+static int pick_token_tile(int kind, int64_t M, int64_t R, int kb_total, double* us = nullptr) {
     if (M <= 16) return 16;
-    struct Width { int tn; float fwd, fwd_tail, dgrad; };
-    static const Width widths[] = {{32, 0.18f, 0.3f, 0.297f}, {64, 0.20f, 0.3f, 0.32f}, {96, 0.225f, 0.3f, 0.335f}, {128, 0.245f, 0.3f, 0.343f},
-                                   {160, 0.28f, 0.4f, 0.366f}, {192, 0.305f, 0.9f, 0.4f}, {256, 0.36f, 2.0f, 0.456f}};
     const int sms = sm_count(), r_tiles = (int)((R + TILE_R - 1) / TILE_R);
     int best = 256;
     double best_cost = 1e30;
-    for (const Width& w : widths) {
+    for (const TokenTile& w : token_tiles) {
         const int64_t tiles = (int64_t)r_tiles * ((M + w.tn - 1) / w.tn);
         const int splits = tiles > sms ? 1 : plan_splits((int)tiles, kb_total, sms);
         const int64_t waves = (tiles * splits + sms - 1) / sms;
@@ -1172,6 +1172,7 @@ static int pick_token_tile(int kind, int64_t M, int64_t R, int kb_total) {
         if (splits > 1) cost += 2.5 + 0.75e-6 * 4.0 * (double)splits * (double)M * (double)R;
         if (cost < best_cost) { best_cost = cost; best = w.tn; }
     }
+    if (us) *us = best_cost;
     return best;
 }
 
@@ -1352,16 +1353,27 @@ static int launch_i8(int tn, const CUtensorMap& mt, const CUtensorMap& mw, const
 static inline bool al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 // Grad-input through a transposed copy of the weight (see k_w4_transpose): bytes of the copy and of its packed group
-// parameters, and the token count from which the extra pass over the weight pays.  Measured through the copy / as stored (us, copy
-// included): 2048 tokens 144 / 157 (4096 x 11008), 146 / 166 (11008 x 4096), 57 / 58 (8192 x 2048), 65 / 68 (2048 x 8192); 1500
-// tokens 117 / 124, 140 / 135, 56 / 55, 53 / 54; 1000 tokens even or slower everywhere.  Seven tiles of 256 tokens and more take it.
-// LQ_GEMM_DGRAD_TRANSPOSE=0 keeps the shared-memory-A kernel, =1 takes the copy from 256 tokens.
+// parameters, and when the extra pass over the weight pays.  The route's forward kernel has 256-token tiles and no split-K, so it needs
+// enough of them: with few output columns (K) it leaves most SMs idle, and just above a whole wave of tiles it pays a second one.  From
+// 1792 tokens on the tile model decides: the forward at 256 tokens and 0.3 us per million weights for the copy, against the best width of
+// the kernel that reads the weight as stored and 2 us, which that kernel takes beyond what the table holds.  Measured over 34 shapes
+// at 1792 .. 4096 tokens the rule's choice is 0.3 % slower than the faster route on average, 9 % at worst.  Copy / stored (us): 4096 x 11008 at
+// 2048 tokens 144 / 158, 8192 x 2048 58 / 73, 2048 x 2048 22 / 24, but 33 / 31 at 2560; 8192 x 1024 at 2048 53 / 48, at 1792 52 / 57; 8192
+// x 512 51 / 36, 512 x 8192 29 / 26.  Below 1792 tokens the copy is not taken: at 1000 it was even or slower at every shape measured, at 1536
+// 2048 x 8192 50 / 53, 8192 x 2048 55 / 54, 2048 x 4096 35 / 32.
+// LQ_GEMM_DGRAD_TRANSPOSE=0 keeps the kernel on the stored weight, =1 takes the copy from 256 tokens.
 static size_t dgrad_t_bytes(int64_t N, int64_t K) { return (size_t)N * (size_t)K / 2 + (size_t)N * (size_t)(K / 128) * 4; }
 static bool dgrad_t_wanted(int64_t M, int64_t N, int64_t K, int group) {
     const char* e = getenv("LQ_GEMM_DGRAD_TRANSPOSE");
     if (e && e[0] == '0') return false;
     if (group != 128 || (K % 256) != 0 || (N % 64) != 0 || getenv("LQ_GEMM_A_OPERAND")) return false;
-    return M >= ((e && e[0] == '1') ? 256 : 1792);
+    if (e && e[0] == '1') return M >= 256;
+    if (M < 1792) return false;
+    const TokenTile& w = token_tiles[sizeof(token_tiles) / sizeof(token_tiles[0]) - 1];
+    const int64_t tiles = ((K + TILE_R - 1) / TILE_R) * ((M + w.tn - 1) / w.tn), waves = (tiles + sm_count() - 1) / sm_count();
+    double stored = 0.0;
+    pick_token_tile(KIND_DGRAD, M, K, (int)(N / 64), &stored);
+    return (double)waves * ((double)(N / 64) * w.fwd + w.fwd_tail) + 0.3e-6 * (double)N * (double)K < stored + 2.0;
 }
 static int run_dgrad_transposed(const void* dy, const void* w, GemmParams p, int64_t M, int64_t N, int64_t K, void* workspace,
                                 cudaStream_t st);

@@ -29,3 +29,21 @@ def test_balanced_forward_leaves_the_grad_input_plan_alone(monkeypatch):
     default = _scratch(DGRAD)
     monkeypatch.setenv("LQ_GEMM_BALANCE", "1")
     assert _scratch(DGRAD) == default
+
+
+# (tokens, out, in) and whether the grad-input goes through the transposed copy: measured 7 % and more apart (us, copy / stored), and the
+# kernel on the stored weight needs no scratch of its own there
+@pytest.mark.parametrize("M,N,K,copy", [
+    (2048, 4096, 11008, True),       # 144 / 158
+    (2048, 8192, 2048, True),        # 58 / 73
+    (1792, 4096, 4096, True),        # 58 / 68
+    (4096, 2048, 2048, True),        # 35 / 40
+    (1791, 4096, 4096, False),       # below the range
+    (2048, 8192, 1024, False),       # 53 / 48: 64 tiles of 256 tokens on 148 SMs
+    (1792, 512, 8192, False),        # 29 / 26
+    (1920, 2048, 5632, False),       # 51 / 44
+    (2560, 2048, 2048, False),       # 33 / 31: a second wave of 12 tiles
+])
+def test_route_of_the_grad_input(M, N, K, copy):
+    need = _lib.lib.lq_gemm_workspace_bytes(DGRAD, M, N, K)
+    assert need == (N * K // 2 + N * K // 128 * 4 if copy else 0)

@@ -194,6 +194,25 @@ def test_a16w4_token_tile_edges(M, N, K, group):
     assert float((dx.double() - ref).norm() / ref.norm()) < 4e-3
 
 
+# The grad-input at the token count from which the transposed copy is considered, on both sides of its rule, with the default dispatch.
+# Neither route splits the contraction at these shapes, so the bits agree.
+@pytest.mark.parametrize("M", [1791, 1792, 1793, 2047, 2560])
+@pytest.mark.parametrize("N,K", [(2112, 2048), (4160, 2304), (1088, 2560), (4096, 1536)])
+def test_grad_input_routes_agree_bitwise(monkeypatch, M, N, K):
+    from latentq_llm_b200 import ops
+    codes, s, z, w = _w4(N, K, N + K)
+    dy = torch.randn(M, N, device="cuda", generator=_gen(M)).to(torch.bfloat16)
+    out = []
+    for mode in (None, "0", "1"):
+        monkeypatch.delenv("LQ_GEMM_DGRAD_TRANSPOSE", raising=False) if mode is None else monkeypatch.setenv("LQ_GEMM_DGRAD_TRANSPOSE", mode)
+        ops._ws_need.clear()
+        out.append(ops.gemm_a16w4_dgrad(dy, codes, s, z, N, K))
+    ops._ws_need.clear()
+    ref = dy.double() @ w
+    assert float((out[0].double() - ref).norm() / ref.norm()) < 4e-3
+    assert torch.equal(out[0], out[1]) and torch.equal(out[0], out[2])
+
+
 # ---- A8W8 linear ------------------------------------------------------------------------------------------------------
 @pytest.mark.parametrize("M,N,K", [(5, 64, 128), (130, 200, 256), (2048, 512, 1024), (64, 4096, 2048)])
 @pytest.mark.parametrize("with_bias", [True, False])
