@@ -213,6 +213,25 @@ def test_grad_input_routes_agree_bitwise(monkeypatch, M, N, K):
     assert torch.equal(out[0], out[1]) and torch.equal(out[0], out[2])
 
 
+# Every token-tile width with the weight tile in tensor memory and in shared memory: the same bf16 weights in the same order, so the
+# same bits.  11008 rows, so that the widest tile without padding is the cheapest (24 tokens: 32 wide ... 250: 256); 1152 = nine groups, whose
+# parameters are not staged.
+@pytest.mark.parametrize("M", [24, 64, 90, 128, 150, 190, 250])
+@pytest.mark.parametrize("N,K", [(11008, 1024), (11008, 1152), (1024, 11008)])
+def test_operand_placements_agree_at_every_tile_width(monkeypatch, M, N, K):
+    from latentq_llm_b200 import ops
+    codes, s, z, w = _w4(N, K, N + K)
+    g = _gen(M)
+    x, dy = torch.randn(M, K, device="cuda", generator=g).to(torch.bfloat16), torch.randn(M, N, device="cuda", generator=g).to(torch.bfloat16)
+    out = {}
+    for where in ("tmem", "smem"):
+        monkeypatch.setenv("LQ_GEMM_A_OPERAND", where)
+        out[where] = (ops.gemm_a16w4_fwd(x, codes, s, z, None, N, K), ops.gemm_a16w4_dgrad(dy, codes, s, z, N, K))
+    for a, b, ref in zip(out["tmem"], out["smem"], (x.double() @ w.t(), dy.double() @ w)):
+        assert torch.equal(a, b)
+        assert float((a.double() - ref).norm() / ref.norm()) < 4e-3
+
+
 # ---- A8W8 linear ------------------------------------------------------------------------------------------------------
 @pytest.mark.parametrize("M,N,K", [(5, 64, 128), (130, 200, 256), (2048, 512, 1024), (64, 4096, 2048)])
 @pytest.mark.parametrize("with_bias", [True, False])
