@@ -13,6 +13,8 @@
 // needed.  Split-K partial sums go to the caller's workspace and are reduced by the GEMM's deterministic
 // reduction kernel.
 // Tensor-core rate is irrelevant here (the kernel is HBM-bound); tcgen05 serves the large-M path.
+#include <type_traits>
+
 #include "lq_common.cuh"
 #include "lq_gemv.h"
 
@@ -286,12 +288,16 @@ __global__ void __launch_bounds__(RB_WARPS * 32, 2) k_skinny_rows(const SkinnyPa
     const int g_begin = NC4 ? warp * 4 : min(gpr, warp * gper), n_groups = NC4 ? 4 : min(gpr, g_begin + gper) - g_begin;
     const int n_chunks = n_groups * GC;
     const int row_bytes = NC4 ? 2048 : p.K / 2, row_elems = NC4 ? 4096 : p.K;
-    const uint8_t* wa = p.qweight + (size_t)ra * row_bytes + (size_t)g_begin * GC * (RB_CHUNK / 2) + t * (W64 ? 8 : 16);
-    const uint8_t* wb = p.qweight + (size_t)rb * row_bytes + (size_t)g_begin * GC * (RB_CHUNK / 2) + t * (W64 ? 8 : 16);
-    auto load_words = [](const uint8_t* w, int c) -> uint4 {                        // chunk c (64 bytes per row): this thread's four words
-        if (!W64) return __ldg(reinterpret_cast<const uint4*>(w + c * 64));
-        const uint2 lo = __ldg(reinterpret_cast<const uint2*>(w + c * 64)), hi = __ldg(reinterpret_cast<const uint2*>(w + c * 64 + 32));
-        return make_uint4(lo.x, lo.y, hi.x, hi.y);
+    using WordVec = typename std::conditional<W64, uint2, uint4>::type;
+    const WordVec* wa = reinterpret_cast<const WordVec*>(p.qweight + (size_t)ra * row_bytes + (size_t)g_begin * GC * (RB_CHUNK / 2)) + t;
+    const WordVec* wb = reinterpret_cast<const WordVec*>(p.qweight + (size_t)rb * row_bytes + (size_t)g_begin * GC * (RB_CHUNK / 2)) + t;
+    auto load_words = [](const WordVec* w, int c) -> uint4 {                        // chunk c (64 bytes per row): this thread's four words
+        if constexpr (W64) {
+            const uint2 lo = __ldg(w + c * 8), hi = __ldg(w + c * 8 + 4);
+            return make_uint4(lo.x, lo.y, hi.x, hi.y);
+        } else {
+            return __ldg(w + c * 4);
+        }
     };
     constexpr auto x_at = [](int j) { return W64 ? (j >> 1) * 8 + (j & 1) : j; };   // token vector of word j, from the thread's first
     const unsigned short* sca = reinterpret_cast<const unsigned short*>(p.scales) + (size_t)ra * gpr + g_begin;
