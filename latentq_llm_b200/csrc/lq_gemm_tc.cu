@@ -1176,6 +1176,10 @@ static int pick_token_tile(int kind, int64_t M, int64_t R, int kb_total, double*
     return best;
 }
 
+// Forwards that may take the kernel of two k-blocks per stage: a split then covers whole stages.  (All others split evenly: rounded too, 1088
+// x 1152 had three splits of 6 k-blocks at up to 16 tokens instead of four of 5, 8.6 instead of 7.7 us.)
+static bool two_kb_stages(int group, int64_t K, int tn) { return group == 128 && (K / 128) % 2 == 0 && tn >= 32 && tn <= 128; }
+
 // group: quantization group size, or 0 when unknown (the skinny path needs 64, 128 or 256)
 // allow_balanced = false asks for the plan a caller with too little workspace for the balanced one falls back to.
 static Plan make_plan(int kind, int64_t M, int64_t N, int64_t K, int group = 128, bool allow_balanced = true) {
@@ -1236,7 +1240,7 @@ static Plan make_plan(int kind, int64_t M, int64_t N, int64_t K, int group = 128
     }
     const int splits = plan_splits(tiles, pl.kb_total, sms);
     pl.kb_per_split = (pl.kb_total + splits - 1) / splits;
-    if (kind == KIND_FWD) pl.kb_per_split += pl.kb_per_split & 1;         // whole stages of two k-blocks
+    if (kind == KIND_FWD && two_kb_stages(group, K, pl.tn)) pl.kb_per_split += pl.kb_per_split & 1;
     pl.splits = (pl.kb_total + pl.kb_per_split - 1) / pl.kb_per_split;
     return pl;
 }
@@ -1421,7 +1425,7 @@ static int run_gemm(int kind, const void* tok, const void* w, GemmParams p, int6
     }
     CUtensorMap mt, mw;
     int rc;
-    const bool k2 = kind == KIND_FWD && p.qp_staged && !pl.sk && pl.tn >= 32 && pl.tn <= 128 && pl.kb_per_split % 2 == 0 && a_operand_in_tmem(kind);
+    const bool k2 = kind == KIND_FWD && p.qp_staged && !pl.sk && two_kb_stages(p.group, K, pl.tn) && pl.kb_per_split % 2 == 0 && a_operand_in_tmem(kind);
     if (kind == KIND_I8) {
         rc = make_map(&mt, tok, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)M, (uint64_t)K, (uint32_t)pl.tn, 128, CU_TENSOR_MAP_SWIZZLE_128B);
         if (rc) return rc;

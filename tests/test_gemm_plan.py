@@ -47,3 +47,8 @@ def test_balanced_forward_leaves_the_grad_input_plan_alone(monkeypatch):
 def test_route_of_the_grad_input(M, N, K, copy):
     need = _lib.lib.lq_gemm_workspace_bytes(DGRAD, M, N, K)
     assert need == (N * K // 2 + N * K // 128 * 4 if copy else 0)
+
+
+def test_split_of_a_forward_without_two_block_stages():
+    """Nine groups per row: 18 k-blocks in four splits, not three of an even number."""
+    assert _lib.lib.lq_gemm_workspace_bytes(FWD, 8, 1088, 1152) == 4 * 8 * 1088 * 4
