@@ -1155,10 +1155,16 @@ static int plan_splits(int tiles, int kb_total, int sms) {
 // with every width; tiles run in waves of one per SM.  Split-K adds the partial sums' way through memory and the reduction
 // launch.  A fixed ladder (64, 128, then 256) left 40 % of the SMs idle at token counts between its steps: 11008 rows at 300
 // tokens 53.8 (256) / 38.5 us (128), at 512 51.2 / 46.3 (192), 2048 rows at 1000 46.6 / 36.2 (128).
-struct TokenTile { int tn; float fwd, fwd_tail, dgrad; };
-static const TokenTile token_tiles[] = {{32, 0.18f, 0.3f, 0.297f}, {64, 0.20f, 0.3f, 0.32f}, {96, 0.225f, 0.3f, 0.335f}, {128, 0.245f, 0.3f, 0.343f},
-                                        {160, 0.28f, 0.4f, 0.366f}, {192, 0.305f, 0.9f, 0.4f}, {256, 0.36f, 2.0f, 0.456f}};
-static int pick_token_tile(int kind, int64_t M, int64_t R, int kb_total, double* us = nullptr) {
+//   A forward whose group parameters are not staged has its own column: its loads of them bound the narrow tiles, so that
+// halving the width does not halve anything.  With the staged kernel's column 4096 -> 4096 with groups of 64 took 32-token tiles at 128
+// tokens, 21.6 instead of 19.2 us with 128, and 3968 -> 4096 at 128 tokens 19.9 instead of 18.6.
+struct TokenTile { int tn; float fwd, fwd_unstaged, fwd_tail, dgrad; };
+static const TokenTile token_tiles[] = {{32, 0.18f, 0.26f, 0.3f, 0.297f}, {64, 0.20f, 0.273f, 0.3f, 0.32f}, {96, 0.225f, 0.318f, 0.3f, 0.335f},
+                                        {128, 0.245f, 0.319f, 0.3f, 0.343f}, {160, 0.28f, 0.365f, 0.4f, 0.366f}, {192, 0.305f, 0.4f, 0.9f, 0.4f},
+                                        {256, 0.36f, 0.43f, 2.0f, 0.456f}};
+// Forwards whose group parameters come through shared memory, by their shape (their pointers decide too, see run_gemm)
+static bool qp_staging(int group, int64_t K) { return group == 128 && (K / 128) % 2 == 0; }
+static int pick_token_tile(int kind, bool staged, int64_t M, int64_t R, int kb_total, double* us = nullptr) {
     if (M <= 16) return 16;
     const int sms = sm_count(), r_tiles = (int)((R + TILE_R - 1) / TILE_R);
     int best = 256;
@@ -1167,7 +1173,7 @@ static int pick_token_tile(int kind, int64_t M, int64_t R, int kb_total, double*
         const int64_t tiles = (int64_t)r_tiles * ((M + w.tn - 1) / w.tn);
         const int splits = tiles > sms ? 1 : plan_splits((int)tiles, kb_total, sms);
         const int64_t waves = (tiles * splits + sms - 1) / sms;
-        const double stage = kind == KIND_FWD ? w.fwd : w.dgrad, tail = kind == KIND_FWD ? w.fwd_tail : 0.3;
+        const double stage = kind != KIND_FWD ? w.dgrad : staged ? w.fwd : w.fwd_unstaged, tail = kind == KIND_FWD ? w.fwd_tail : 0.3;
         double cost = (double)waves * (((kb_total + splits - 1) / splits) * stage + tail);
         if (splits > 1) cost += 2.5 + 0.75e-6 * 4.0 * (double)splits * (double)M * (double)R;
         if (cost < best_cost) { best_cost = cost; best = w.tn; }
@@ -1178,7 +1184,7 @@ static int pick_token_tile(int kind, int64_t M, int64_t R, int kb_total, double*
 
 // Forwards that may take the kernel of two k-blocks per stage: a split then covers whole stages.  (All others split evenly: rounded too, 1088
 // x 1152 had three splits of 6 k-blocks at up to 16 tokens instead of four of 5, 8.6 instead of 7.7 us.)
-static bool two_kb_stages(int group, int64_t K, int tn) { return group == 128 && (K / 128) % 2 == 0 && tn >= 32 && tn <= 128; }
+static bool two_kb_stages(int group, int64_t K, int tn) { return qp_staging(group, K) && tn >= 32 && tn <= 128; }
 
 // group: quantization group size, or 0 when unknown (the skinny path needs 64, 128 or 256)
 // allow_balanced = false asks for the plan a caller with too little workspace for the balanced one falls back to.
@@ -1202,7 +1208,7 @@ static Plan make_plan(int kind, int64_t M, int64_t N, int64_t K, int group = 128
     pl.kb_total = (int)((Cc + bk - 1) / bk);
     const char* balance = getenv("LQ_GEMM_BALANCE");
     const bool want_balanced = kind == KIND_FWD && balance && balance[0] == '1';      // its kernels exist for the widths above
-    if (kind != KIND_I8 && !want_balanced) pl.tn = pick_token_tile(kind, M, R, pl.kb_total);
+    if (kind != KIND_I8 && !want_balanced) pl.tn = pick_token_tile(kind, qp_staging(group, K), M, R, pl.kb_total);
     pl.t_tiles = (int)((M + pl.tn - 1) / pl.tn);
     const int tiles = pl.r_tiles * pl.t_tiles;
     const int sms = sm_count();
@@ -1376,7 +1382,7 @@ static bool dgrad_t_wanted(int64_t M, int64_t N, int64_t K, int group) {
     const TokenTile& w = token_tiles[sizeof(token_tiles) / sizeof(token_tiles[0]) - 1];
     const int64_t tiles = ((K + TILE_R - 1) / TILE_R) * ((M + w.tn - 1) / w.tn), waves = (tiles + sm_count() - 1) / sm_count();
     double stored = 0.0;
-    pick_token_tile(KIND_DGRAD, M, K, (int)(N / 64), &stored);
+    pick_token_tile(KIND_DGRAD, false, M, K, (int)(N / 64), &stored);
     return (double)waves * ((double)(N / 64) * w.fwd + w.fwd_tail) + 0.3e-6 * (double)N * (double)K < stored + 2.0;
 }
 static int run_dgrad_transposed(const void* dy, const void* w, GemmParams p, int64_t M, int64_t N, int64_t K, void* workspace,
@@ -1394,7 +1400,7 @@ static int run_gemm(int kind, const void* tok, const void* w, GemmParams p, int6
     // a caller whose workspace is too small for the balanced plan gets the whole-tile plan (which may need less or none)
     if (pl.sk && (!workspace || workspace_bytes < plan_workspace_bytes(pl, M, p.R))) pl = make_plan(kind, M, N, K, p.group, false);
     p.wcols = (int)K;
-    p.qp_staged = kind == KIND_FWD && p.group == 128 && (K / 128) % 2 == 0 &&
+    p.qp_staged = kind == KIND_FWD && qp_staging(p.group, K) &&
                   ((reinterpret_cast<uintptr_t>(p.scales) | reinterpret_cast<uintptr_t>(p.zeros)) & 3) == 0;
     p.r_tiles = pl.r_tiles; p.t_tiles = pl.t_tiles; p.splits = pl.splits; p.kb_total = pl.kb_total; p.kb_per_split = pl.kb_per_split;
     if (pl.splits > 1) {

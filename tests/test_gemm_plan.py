@@ -52,3 +52,8 @@ def test_route_of_the_grad_input(M, N, K, copy):
 def test_split_of_a_forward_without_two_block_stages():
     """Nine groups per row: 18 k-blocks in four splits, not three of an even number."""
     assert _lib.lib.lq_gemm_workspace_bytes(FWD, 8, 1088, 1152) == 4 * 8 * 1088 * 4
+
+
+def test_tiles_of_a_forward_without_staged_group_parameters():
+    """31 groups per row, 128 tokens: one 128-token tile in four splits, not four 32-token tiles."""
+    assert _lib.lib.lq_gemm_workspace_bytes(FWD, 128, 4096, 3968) == 4 * 128 * 4096 * 4
