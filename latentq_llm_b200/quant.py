@@ -134,7 +134,7 @@ def _apply(fn, *args):
     more host time than a decode-sized launch takes on the GPU).  Forward-mode duals and functorch transforms go through
     `apply`, which refuses or handles them as before; a trace records the function there, and could not see a launch here."""
     if (torch.is_grad_enabled() or torch._C._are_functorch_transforms_active() or torch.autograd.forward_ad._current_level >= 0
-            or torch.jit.is_tracing() or torch.compiler.is_compiling()):
+            or torch._C._is_tracing() or torch.compiler.is_compiling()):
         return fn.apply(*args)
     return fn.forward(*args)
 
@@ -240,7 +240,7 @@ def _a8w8_forward(input8, clampv, weight_d, qscales, bias):
     on_device = torch.is_tensor(clampv)
     # one launch for a scale and a bias of one element per output channel; other forms broadcast, or are refused, below
     if (qs.dtype == torch.bfloat16 and qs.is_contiguous() and qs.numel() == N
-            and (bias is None or (bias.dtype == torch.bfloat16 and bias.numel() == N and bias.shape[-1:] == (N,)))
+            and (bias is None or (bias.dtype == torch.bfloat16 and bias.dim() == 1 and bias.numel() == N))
             and (not on_device or (clampv.dtype == torch.float32 and clampv.numel() == 1))):
         return ops.gemm_a8w8_module(input8, weight_d, clampv if on_device else None, 1.0 if on_device else float(clampv) / 127.,
                                     None if bias is None else bias.detach().contiguous(), qs)
@@ -270,7 +270,7 @@ def _a8w8_backward(ctx, grad_output, input_f, weight_d, qscales, bias, detach=Fa
     grad_input = grad_bias = None
     if ctx.needs_input_grad[0]:
         if (grad_output.dtype == torch.bfloat16 and qscales.dtype == torch.bfloat16 and qscales.is_contiguous()
-                and qscales.shape == (weight_d.shape[0], 1)):
+                and qscales.dim() == 2 and qscales.numel() == weight_d.shape[0] == qscales.shape[0]):
             weight_forward = ops.i8_dequant(weight_d, row_scales=qscales)
         else:
             weight_forward = weight_d.to(grad_output.dtype) * qscales
