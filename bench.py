@@ -15,6 +15,7 @@ reported.  One JSON line is printed by rank 0.
 from __future__ import annotations
 
 import argparse
+import functools
 import json
 import os
 import statistics
@@ -37,8 +38,8 @@ WORKLOAD = "A16W4 dequant-GEMM fwd+grad-input, Llama-2-7B linear shapes (K,N) in
 
 # dram__bytes_read.sum + dram__bytes_write.sum per k_gemm launch from an ncu capture of the (K,N)=(4096,11008),
 # M=4096 launches (a tensor-bound kernel: the figure shows there are no re-reads)
-NCU_TRAFFIC_BYTES_PER_LAUNCH = 132.6e6
-NCU_TRAFFIC_NOTE = ("ncu capture of the (K,N)=(4096,11008), M=4096 launches: forward 116.0 MB, grad-input 149.3 MB, mean 132.6 MB "
+NCU_TRAFFIC_BYTES_PER_LAUNCH = 131.2e6
+NCU_TRAFFIC_NOTE = ("ncu capture of the (K,N)=(4096,11008), M=4096 launches: forward 116.3 MB, grad-input 146.2 MB, mean 131.2 MB "
                     "per launch against 146.8 MB algorithmic bytes of that shape")
 
 
@@ -136,18 +137,20 @@ def build_layers(torch, ops, seed=1234):
     return layers
 
 
-def launches_per_layer(m=M_TOKENS):
-    """Kernel launches of one forward + one grad-input: from 3072 tokens on the grad-input is two launches
-    (transpose of the weight and its group parameters, GEMM) unless the route is switched off."""
-    transposed = (m >= 3072 and os.environ.get("LQ_GEMM_DGRAD_TRANSPOSE") != "0" and "LQ_GEMM_A_OPERAND" not in os.environ)
-    return 3 if transposed else 2
+@functools.lru_cache(maxsize=None)
+def launches_of_layer(N, K, m=M_TOKENS):
+    """Kernel launches of one forward + one grad-input.  A grad-input that goes through the transposed copy of the weight is two
+    (transpose of the codes and group parameters, GEMM); it then asks for the copy as scratch, and at the token counts where that
+    route is taken neither kernel splits its contraction."""
+    from latentq_llm_b200 import _lib
+    return 3 if _lib.lib.lq_gemm_workspace_bytes(_lib.GEMM_A16W4_DGRAD, m, N, K) >= N * K // 2 + N * K // 128 * 4 else 2
 
 
 def run_step(ops, layers):
     for L in layers:
         ops.gemm_a16w4_fwd(L["x"], L["codes"], L["s"], L["z"], None, L["N"], L["K"], out=L["y"])
         ops.gemm_a16w4_dgrad(L["dy"], L["codes"], L["s"], L["z"], L["N"], L["K"], out=L["dx"])
-    return launches_per_layer() * len(layers)
+    return sum(launches_of_layer(L["N"], L["K"]) for L in layers)
 
 
 def timed(torch, fn, steps, barrier):
@@ -725,7 +728,7 @@ def run_ours(args):
                 with torch.cuda.stream(s_out):
                     host_out.copy_(dev_out, non_blocking=True)
         cur.wait_stream(s_out)                                   # results of this step are on the host before the next GEMM overwrites them
-        return launches_per_layer() * len(layers)
+        return sum(launches_of_layer(L["N"], L["K"]) for L in layers)
 
     e2e_step(); torch.cuda.synchronize()
     e2e_steps = max(2, min(args.steps, 10))
