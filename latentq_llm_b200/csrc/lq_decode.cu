@@ -481,8 +481,10 @@ int lq_rope_kv_store(void* qkv, const int64_t* positions, const float* inv_freq,
 static int attn_splits(int64_t B, int Hq, int64_t max_len) {
     const int64_t ctas = B * Hq;
     // As many splits as fit beside one another (four CTAs per SM by registers): rounded up, a few CTAs more than that made a second
-    // wave of the whole kernel.  Measured (us, up / down): 4 sequences of 512 keys 16.7 / 13.1, 8: 22.1 / 17.9, 16: 30.7 / 25.7, one of
-    // 1500 keys 15.8 / 11.9, four 28.7 / 22.6; 32 and more take one split either way.
+    // wave of the whole kernel.  Measured with 32 heads (us, up / down): 4 sequences of 512 keys 14.9 / 11.0, 8: 18.1 / 14.8, 16: 25.9 / 21.3,
+    // one of 1500 keys 11.7 / 10.3, four 23.9 / 19.2; also where half of the slots stay empty: 10 sequences (one split instead of two) of 128
+    // keys 10.9 / 6.9, of 512 19.5 / 15.0, of 1500 37.9 / 31.6; 12: 20.5 / 16.7 of 512, 47.9 / 41.2 of 1500; 18: 27.2 / 22.5 and 54.5 / 50.5.
+    // Nothing lost with 16 heads, or 32 on 8 key heads, at 1 .. 64 sequences of 128 to 1500 keys; from 19 sequences of 32 heads on one split either way.
     int64_t s = 4 * (int64_t)sm_count() / ctas;
     const int64_t cap = (max_len + 63) / 64;                        // at least 64 keys (two rounds of the 16 slots x 2) per split
     if (s > cap) s = cap;

@@ -80,7 +80,7 @@ struct GemmParams {
     int sk_pmax;                   // partial-sum slots per shared tile
     int accumulate;                // weight gradient: out += product (rounded once from the fp32 sum) instead of out = product
     int qp_staged;                 // forward: group parameters through shared memory (groups of 128, an even number per row, 4-byte aligned)
-    const uint4* qpt;              // QPT kernels: per-column group parameters, packed for the dequant (see k_w4_qp_transpose)
+    const uint4* qpt;              // QPT kernels: per-column group parameters, packed for the dequant (see w4_qp_transpose_entry)
 };
 
 // One CTA's share of the work as a sequence of segments (a tile and a range of its k-blocks).
@@ -859,8 +859,8 @@ k_gemm(const __grid_constant__ CUtensorMap map_tok, const __grid_constant__ CUte
             // Forward with groups of 128 (an even number per row): the group parameters come through shared memory.  Read where
             // they are needed, one 2-byte load per lane, row and stage touches 32 cache lines a warp and instruction: 256
             // L1 cycles per stage, which bounded the kernel below 256 tokens.  Here the 512 threads fetch a chunk of 16
-            // k-blocks together, four lanes per row, ahead of its use: 4096 -> 11008 at 128 tokens 23.4 -> 20.5 us (with two k-blocks per
-            // stage up to 128 tokens: 24 tokens 20.3 -> 17.5 us), 11008 -> 4096 at 4096 tokens 273 -> 253 us.
+            // k-blocks together, four lanes per row (256-token tiles: 8 k-blocks, two lanes), ahead of its use: 4096 -> 11008 at 128 tokens
+            // 23.4 -> 20.5 us (with two k-blocks per stage up to 128 tokens: 24 tokens 20.8 -> 17.5 us), 11008 -> 4096 at 4096 tokens 273 -> 253 us.
             // (QPT: the parameters of a stage's 64 contraction elements, the same for every row of the tile's k group, come the
             // same way: 256 bytes per stage, one 16-byte piece per thread.)
             if constexpr (KIND == KIND_FWD && RT == 1) {
