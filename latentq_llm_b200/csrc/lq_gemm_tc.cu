@@ -1155,6 +1155,8 @@ static int plan_splits(int tiles, int kb_total, int sms) {
 // with every width; tiles run in waves of one per SM.  Split-K adds the partial sums' way through memory and the reduction
 // launch.  A fixed ladder (64, 128, then 256) left 40 % of the SMs idle at token counts between its steps: 11008 rows at 300
 // tokens 53.8 (256) / 38.5 us (128), at 512 51.2 / 46.3 (192), 2048 rows at 1000 46.6 / 36.2 (128).
+//   Where it errs: some grad-inputs of 45 .. 63 tokens take two tiles of 32, up to 0.7 us (6 %) slower than one of 64 (4352 x 1152 at 50 tokens
+// 12.5 / 11.7); a smaller price for the partial sums mends them and loses 4 to 11 % at 280 to 700 tokens.
 //   A forward whose group parameters are not staged has its own column: its loads of them bound the narrow tiles, so that
 // halving the width does not halve anything.  With the staged kernel's column 4096 -> 4096 with groups of 64 took 32-token tiles at 128
 // tokens, 21.6 instead of 19.2 us with 128, and 3968 -> 4096 at 128 tokens 19.9 instead of 18.6.
