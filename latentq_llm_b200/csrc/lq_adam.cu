@@ -8,6 +8,7 @@
 // multiply-add into an FMA in torch's own build; the same contraction is spelled out here with __fmaf_rn
 // (checked on the GPU against torch's add_/addcmul_/addcdiv_ on 2^24-element bf16 tensors: the separately
 // rounded forms of add_(alpha) and addcdiv_ differ from torch in a few elements per million, the fused ones never).
+#include <type_traits>
 #include <cstdlib>
 
 #include "lq_requant.cuh"
@@ -142,12 +143,15 @@ __global__ void __launch_bounds__(256) k_adam_quant(const AdamParams p) {
 //             every midpoint of two fp32 numbers, the corrected quotient is 2^-44 off before its rounding.
 //   states    encoded with a quotient from a two-term reciprocal and one residual correction (Markstein's theorem, see div_by), as is
 //             the division of the block's range by 255.
+//   fp32      two elements per instruction (fma / mul / add .f32x2) for int4 codes: 157 -> 149 us for 4096 x
+//             11008.  The int8 kernel has no registers left for the pairs (64, two teams of 256 threads): 172 -> 178 us, so it keeps
+//             one element per instruction.
 //   requantize  everything after Z = w/scale + zero from the table of the requantize fast path (int4: a byte per bf16 pattern,
 //             |Z| < 64; int8: two bytes, |Z| < 256); the kernel keeps the two runs of it that can be looked up and puts its other
 //             tables into the gap between them.
 // int4 codes: 50 KB and 256 threads per CTA, three CTAs per SM (four would fit, but at 64 registers the loop spills: 176 instead of
 // 157 us for 4096 x 11008); int8 codes: 100 KB, so two teams of 256 threads share the tables of a CTA and two CTAs fit.
-// Measured, a whole optimizer step of one 4096 x 11008 weight: int4 268 -> 157 us (2.3 TB/s), int8 586 -> 183 us.
+// Measured, a whole optimizer step of one 4096 x 11008 weight: int4 268 -> 149 us (2.4 TB/s), int8 586 -> 172 us.
 // A word whose Z leaves the table's range or is not finite, and every word of a block whose moments are not all finite, is
 // recomputed with IEEE operations (adam_word_generic).
 // ---------------------------------------------------------------------------------------------------------------
@@ -180,10 +184,27 @@ __device__ __forceinline__ uint32_t min2(uint32_t a, uint32_t b) { return asu32(
 __device__ __forceinline__ uint32_t max2(uint32_t a, uint32_t b) { return asu32(__hmax2(asbf2(a), asbf2(b))); }
 __device__ __forceinline__ float sqrt_approx(float x) { float r; asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
 __device__ __forceinline__ float rcp_approx(float x) { float r; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
-// a / b for bf16-valued a and b, 2^-64 <= b <= 2^64: see above (a residual of the opposite sign keeps -0 / b = -0)
-__device__ __forceinline__ float div_bf16(float a, float b) {
-    const float y = rcp_approx(b), q = __fmul_rn(a, y);
-    return __fmaf_rn(-__fmaf_rn(q, b, -a), y, q);
+// Two fp32 values.  f32x2: in one 64-bit register pair, each operation one instruction for two IEEE results; float2: one by one.
+typedef unsigned long long f32x2;
+template <typename V> __device__ __forceinline__ V f2(float a, float b);
+template <> __device__ __forceinline__ f32x2 f2<f32x2>(float a, float b) { f32x2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
+template <> __device__ __forceinline__ float2 f2<float2>(float a, float b) { return make_float2(a, b); }
+template <typename V> __device__ __forceinline__ V f2(float a) { return f2<V>(a, a); }
+template <typename V> __device__ __forceinline__ V bf2f(uint32_t u) { return f2<V>(lo2f(u), hi2f(u)); }            // the two values of a bf16 pair
+__device__ __forceinline__ float2 of2(f32x2 v) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v)); return r; }
+__device__ __forceinline__ float2 of2(float2 v) { return v; }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) { f32x2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return make_float2(__fmaf_rn(a.x, b.x, c.x), __fmaf_rn(a.y, b.y, c.y)); }
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) { f32x2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return make_float2(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y)); }
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) { f32x2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return make_float2(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y)); }
+template <typename V> __device__ __forceinline__ uint32_t packv(V v) { const float2 f = of2(v); return pack2(f.x, f.y); }
+// -(a / b) for pairs of bf16-valued a and b, 2^-64 <= b <= 2^64: see above (the residual's sign keeps that of a zero quotient)
+template <typename V> __device__ __forceinline__ V neg_div_bf16(V a, V b) {
+    const float2 bb = of2(b);
+    const V ny = f2<V>(rcp_approx(-bb.x), rcp_approx(-bb.y)), nq = mul2(a, ny);
+    return fma2(fma2(nq, b, a), ny, nq);
 }
 // (scale, its reciprocal as RN(1/s) + remainder) of one 8-bit state block: s = (mx - mn) / 255 + 1e-10
 struct OptScale { float s, r, rl; };
@@ -198,15 +219,17 @@ __device__ __forceinline__ OptScale opt8_scale(float mx, float mn) {
     o.rl = __fmul_rn(__fmaf_rn(-o.s, o.r, 1.0f), o.r);
     return o;
 }
-__device__ __forceinline__ uint32_t opt8_code_bits(float x, float mx, const OptScale& o) {   // code in the low byte
-    const float a = __fsub_rn(mx, x);
-    float q = __fmaf_rn(a, o.r, __fmul_rn(a, o.rl));
-    q = __fmaf_rn(__fmaf_rn(-q, o.s, a), o.r, q);
-    return __float_as_uint(__fadd_rn(q, MAGIC_RNE));                 // 0 <= q <= 255 (1 + 2^-22)
+template <typename V>
+__device__ __forceinline__ uint32_t opt8_codes2(uint32_t x, float mx, const OptScale& o) {        // codes of a bf16 pair in bytes 0 and 1
+    const V r = f2<V>(o.r), a = fma2(bf2f<V>(x), f2<V>(-1.0f), f2<V>(mx));
+    V q = fma2(a, r, mul2(a, f2<V>(o.rl)));
+    q = fma2(fma2(q, f2<V>(-o.s), a), r, q);
+    const float2 c = of2(add2(q, f2<V>(MAGIC_RNE)));                 // 0 <= q <= 255 (1 + 2^-22)
+    return __byte_perm(__float_as_uint(c.x), __float_as_uint(c.y), 0x0040);
 }
+template <typename V>
 __device__ __forceinline__ uint32_t opt8_codes4(uint32_t p01, uint32_t p23, float mx, const OptScale& o) {
-    return __byte_perm(__byte_perm(opt8_code_bits(lo2f(p01), mx, o), opt8_code_bits(hi2f(p01), mx, o), 0x0040),
-                       __byte_perm(opt8_code_bits(lo2f(p23), mx, o), opt8_code_bits(hi2f(p23), mx, o), 0x0040), 0x5410);
+    return __byte_perm(opt8_codes2<V>(p01, mx, o), opt8_codes2<V>(p23, mx, o), 0x5410);
 }
 
 // One word from its inputs in memory (nothing of it has been written yet) and the block parameters of its states before (s, t) and
@@ -243,6 +266,7 @@ __global__ void __launch_bounds__(AdamFast<WBITS>::THREADS, AdamFast<WBITS>::MIN
 k_adam_fast(const __grid_constant__ AdamParams p, const int enc_slot, const uint64_t row_magic) {
     using AF = AdamFast<WBITS>;
     constexpr bool W8 = WBITS == 8;
+    using V = typename std::conditional<W8, float2, f32x2>::type;
     extern __shared__ __align__(16) uint8_t asm_[];
     const uint8_t* encz = asm_;
     const uint16_t* enc8 = reinterpret_cast<const uint16_t*>(asm_);
@@ -337,18 +361,17 @@ k_adam_fast(const __grid_constant__ AdamParams p, const int enc_slot, const uint
                 }
                 const uint32_t vu = asu32(v);
                 // the two elements of the pair through the optimizer chain (every intermediate rounded to bf16)
-                const float g0 = lo2f(gw[j]), g1 = hi2f(gw[j]);
                 const uint32_t w1 = (j < 2) ? in.q1.x : in.q1.y, w2 = (j < 2) ? in.q2.x : in.q2.y;
                 const uint32_t a0 = (w1 >> (16 * (j & 1))) & 0xffu, a1 = (w1 >> (16 * (j & 1) + 8)) & 0xffu;
                 const uint32_t b0 = (w2 >> (16 * (j & 1))) & 0xffu, b1 = (w2 >> (16 * (j & 1) + 8)) & 0xffu;
-                const float m0 = LUT ? lut[a0] : dec1(u2f(a0)), m1 = LUT ? lut[a1] : dec1(u2f(a1));
-                const float v0 = LUT ? lut[256 + b0] : dec2(u2f(b0)), v1 = LUT ? lut[256 + b1] : dec2(u2f(b1));
-                m[j] = pack2(__fmaf_rn(p.h.one_minus_beta1, g0, m0), __fmaf_rn(p.h.one_minus_beta1, g1, m1));
-                const uint32_t vv = pack2(__fmaf_rn(p.h.one_minus_beta2, __fmul_rn(g0, g0), v0), __fmaf_rn(p.h.one_minus_beta2, __fmul_rn(g1, g1), v1));
+                const V m01 = LUT ? f2<V>(lut[a0], lut[a1]) : f2<V>(dec1(u2f(a0)), dec1(u2f(a1)));
+                const V v01 = LUT ? f2<V>(lut[256 + b0], lut[256 + b1]) : f2<V>(dec2(u2f(b0)), dec2(u2f(b1)));
+                const V gr = bf2f<V>(gw[j]);
+                m[j] = packv(fma2(f2<V>(p.h.one_minus_beta1), gr, m01));
+                const uint32_t vv = packv(fma2(f2<V>(p.h.one_minus_beta2), mul2(gr, gr), v01));
                 const uint32_t t = pack2(sqrt_approx(lo2f(vv)), sqrt_approx(hi2f(vv)));
-                d[j] = pack2(__fadd_rn(lo2f(t), p.h.eps), __fadd_rn(hi2f(t), p.h.eps));              // sqrt(v) + eps
-                lat[j] = pack2(__fmaf_rn(p.h.neg_step_size, div_bf16(lo2f(m[j]), lo2f(d[j])), lo2f(vu)),
-                               __fmaf_rn(p.h.neg_step_size, div_bf16(hi2f(m[j]), hi2f(d[j])), hi2f(vu)));
+                d[j] = packv(add2(bf2f<V>(t), f2<V>(p.h.eps)));                                      // sqrt(v) + eps
+                lat[j] = packv(fma2(f2<V>(-p.h.neg_step_size), neg_div_bf16(bf2f<V>(m[j]), bf2f<V>(d[j])), bf2f<V>(vu)));
                 mn1 = min2(mn1, m[j]); mx1 = max2(mx1, m[j]);
                 mn2 = min2(mn2, d[j]); mx2 = max2(mx2, d[j]);
             }
@@ -384,7 +407,7 @@ k_adam_fast(const __grid_constant__ AdamParams p, const int enc_slot, const uint
             uint32_t zbits[4], zmax = 0u;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                __nv_bfloat162 Zp = asbf2(pack2(__fmul_rn(lo2f(lat[j]), rs), __fmul_rn(hi2f(lat[j]), rs)));
+                __nv_bfloat162 Zp = asbf2(packv(mul2(bf2f<V>(lat[j]), f2<V>(rs))));
                 if (!W8) Zp = __hadd2_rn(Zp, z2);
                 zbits[j] = asu32(Zp);
                 __nv_bfloat162 az = __habs2(Zp);
@@ -400,8 +423,8 @@ k_adam_fast(const __grid_constant__ AdamParams p, const int enc_slot, const uint
                 const float4 q = LUT ? prm[parity] : make_float4(in.s1, in.t1, in.s2, in.t2);
                 adam_word_generic<WBITS>(p, (int64_t)w, q.x, q.y, q.z, q.w, fmx1, o1.s, fmx2, o2.s);
             } else {
-                *reinterpret_cast<uint2*>(p.st1 + (size_t)w * 8) = make_uint2(opt8_codes4(m[0], m[1], fmx1, o1), opt8_codes4(m[2], m[3], fmx1, o1));
-                *reinterpret_cast<uint2*>(p.st2 + (size_t)w * 8) = make_uint2(opt8_codes4(d[0], d[1], fmx2, o2), opt8_codes4(d[2], d[3], fmx2, o2));
+                *reinterpret_cast<uint2*>(p.st1 + (size_t)w * 8) = make_uint2(opt8_codes4<V>(m[0], m[1], fmx1, o1), opt8_codes4<V>(m[2], m[3], fmx1, o1));
+                *reinterpret_cast<uint2*>(p.st2 + (size_t)w * 8) = make_uint2(opt8_codes4<V>(d[0], d[1], fmx2, o2), opt8_codes4<V>(d[2], d[3], fmx2, o2));
                 uint32_t ev[4], od[4];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
