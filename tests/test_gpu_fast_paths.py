@@ -269,3 +269,50 @@ def test_per_tensor_activation_quantizer_equals_the_op_chain(scale):
     x8, clampv = ops.act_quant_per_tensor(x)
     ref = (x * 127. / x.max()).round_().clamp_(-128, 127).to(torch.int8)
     assert float(clampv) == float(x.max()) and torch.equal(x8, ref)
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 8), (3, 2040), (5, 2056), (40, 8192)])
+def test_gradient_accumulator_with_philox_noise_equals_the_generic_kernel(rows, cols):
+    """bf16 gradients with the library's own noise take the packed kernel; the same noise from a buffer takes the generic one, which the
+    reference's vectors pin.  Bit for bit, first and later micro-batches, gradients that are not finite and scales whose reciprocal is
+    not used included."""
+    from latentq_llm_b200 import ops
+    g = _gen(cols)
+    q = [torch.zeros(rows, cols, dtype=torch.int8, device="cuda") for _ in range(2)]
+    sc = [torch.zeros(rows, dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+    for it in range(4):
+        f = (torch.randn(rows, cols, device="cuda", generator=g) * 10.0 ** (it - 3)).to(torch.bfloat16)
+        if it == 2:
+            f.view(-1)[:4] = torch.tensor([float("nan"), float("inf"), -float("inf"), 1e-40])
+        if it == 3:                                   # scales beyond 2^40 and below 2^-40
+            for s in sc:
+                s[0], s[rows - 1] = 2.0 ** 45, 2.0 ** -45 if rows > 1 else 2.0 ** 45
+        noise = ops.philox_dither(7, ((it + 1) << 32) | 11, rows * cols // 8, "cuda")
+        ops.gradq_accumulate(f, q[0], sc[0], it == 0, ops.make_opts(dither=ops.DITHER_PHILOX, seed=7, step=it + 1, param_id=11))
+        ops.gradq_accumulate(f, q[1], sc[1], it == 0, ops.make_opts(dither=ops.DITHER_EXPLICIT, dither_buf=noise))
+        assert torch.equal(q[0], q[1]) and torch.equal(sc[0], sc[1]), it
+
+
+@pytest.mark.parametrize("n", [8, 8 * 255, 8 * 257, 8 * 148 * 8 * 256 * 2 + 8])
+def test_per_tensor_activation_quantizer_sizes_and_special_values(n):
+    from latentq_llm_b200 import ops
+    x = (torch.randn(n, device="cuda", generator=_gen(n)) * 3).to(torch.bfloat16)
+    for case in ("plain", "negative", "nan", "max at the end"):
+        y = -x.abs() - 1 if case == "negative" else x.clone()
+        if case == "nan":
+            y[n // 2] = float("nan")
+        if case == "max at the end":
+            y[n - 1] = 100.0
+        x8, clampv = ops.act_quant_per_tensor(y)
+        top = torch.where(torch.isnan(y), torch.full_like(y, -float("inf")), y).max()          # NaN is passed over, and its code is -128
+        ref = (y * 127. / top).round_().clamp_(-128, 127)
+        ref = torch.where(torch.isnan(y), torch.full_like(y, -128.0), ref).to(torch.int8)
+        assert float(clampv) == float(top) and torch.equal(x8, ref), case
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 16), (3, 11008), (2047, 1040), (1200, 4112)])
+def test_i8_dequant_rows_by_multiplication(rows, cols):
+    from latentq_llm_b200 import ops
+    c = torch.randint(-128, 128, (rows, cols), device="cuda", generator=_gen(cols), dtype=torch.int8)
+    qs = (torch.rand(rows, 1, device="cuda", generator=_gen(rows)) * 0.01 + 1e-3).to(torch.bfloat16)
+    assert torch.equal(ops.i8_dequant(c, row_scales=qs), c.to(torch.bfloat16) * qs)
