@@ -1,8 +1,8 @@
-"""In-tree build of liblatentq.so (nvcc, sm_100a only).
+"""In-tree build of liblatentq.so (nvcc, sm_100a only) and of _lqhost.so, the native host path of the short calls (g++).
 
     python -m latentq_llm_b200.build [--force] [--verbose]
 
-The shared library lands next to this file so that it travels with the source
+The shared libraries land next to this file so that it travels with the source
 tree; nothing is installed into site-packages and nothing is JIT-cached.
 """
 from __future__ import annotations
@@ -10,11 +10,13 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+import sysconfig
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(PKG)
 CSRC = os.path.join(PKG, "csrc")
 LIB = os.path.join(PKG, "liblatentq.so")
+HOST = os.path.join(PKG, "_lqhost.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -27,16 +29,30 @@ def sources():
     return sorted(os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith(".cu"))
 
 
-def _stale() -> bool:
-    if not os.path.exists(LIB):
+def _stale(target, deps) -> bool:
+    if not os.path.exists(target):
         return True
-    t = os.path.getmtime(LIB)
-    deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)] + [os.path.join(ROOT, "include", "latentq.h"), __file__]
-    return any(os.path.getmtime(d) > t for d in deps)
+    t = os.path.getmtime(target)
+    return any(os.path.getmtime(d) > t for d in [*deps, os.path.join(ROOT, "include", "latentq.h"), __file__])
+
+
+def build_host(force: bool = False) -> str:
+    src = os.path.join(CSRC, "lq_host.cpp")
+    if not force and not _stale(HOST, [src]):
+        return HOST
+    import torch
+    t = os.path.dirname(torch.__file__)
+    inc = [os.path.join(ROOT, "include"), os.path.join(t, "include"), os.path.join(t, "include", "torch", "csrc", "api", "include"),
+           "/usr/local/cuda/include", sysconfig.get_paths()["include"]]
+    subprocess.check_call([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+                           *[f"-I{i}" for i in inc], src, "-o", HOST, f"-L{os.path.join(t, 'lib')}", "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda",
+                           f"-L{PKG}", "-l:liblatentq.so", "-Wl,-rpath,$ORIGIN"])
+    return HOST
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
-    if not force and not _stale():
+    if not force and not _stale(LIB, [os.path.join(CSRC, f) for f in os.listdir(CSRC) if not f.endswith(".cpp")]):
+        build_host()
         return LIB
     nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
     cmd = [nvcc, *NVCC_FLAGS, "--threads", "0"]
@@ -44,6 +60,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         cmd += ["-Xptxas", "-v"]
     cmd += ["-o", LIB, *sources()]
     subprocess.check_call(cmd)
+    build_host(force)
     return LIB
 
 

@@ -1,0 +1,154 @@
+// Host path of the calls whose launches take a few microseconds: argument checks, output allocation and launch in native code.
+// Every function serves the plain case (CUDA tensors with storage, contiguous, of the expected types and sizes) and returns None for
+// anything else and for a call that the library refuses, without having done anything: the caller's Python, which repeats the call,
+// then raises or handles it as it does without this module.
+#include <Python.h>
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include "latentq.h"
+
+namespace {
+
+using at::Tensor;
+
+bool plain(PyObject* o, at::ScalarType dtype) {
+    if (!THPVariable_Check(o)) return false;
+    const Tensor& t = THPVariable_Unpack(o);
+    if (!t.defined() || !t.is_cuda() || t.scalar_type() != dtype || !t.has_storage()) return false;
+    const c10::DispatchKeySet keys = t.key_set();                    // tensors that stand for others (functorch, __torch_dispatch__)
+    return !keys.has(c10::DispatchKey::Python) && !keys.has(c10::DispatchKey::FuncTorchBatched) && !keys.has(c10::DispatchKey::FuncTorchGradWrapper) &&
+           !keys.has(c10::DispatchKey::Functionalize) && t.is_contiguous();
+}
+bool plain_or_none(PyObject* o, at::ScalarType dtype) { return o == Py_None || plain(o, dtype); }
+const Tensor& tensor(PyObject* o) { return THPVariable_Unpack(o); }
+void* ptr(PyObject* o) { return o == Py_None ? nullptr : tensor(o).data_ptr(); }
+lq_stream_t stream() { return (lq_stream_t)c10::cuda::getCurrentCUDAStream().stream(); }
+bool count(Py_ssize_t n, Py_ssize_t want) {
+    if (n == want) return true;
+    PyErr_Format(PyExc_TypeError, "expected %zd arguments, got %zd", want, n);
+    return false;
+}
+PyObject* pair(Tensor a, Tensor b) {
+    PyObject* pa = THPVariable_Wrap(std::move(a));
+    PyObject* pb = pa ? THPVariable_Wrap(std::move(b)) : nullptr;
+    PyObject* r = pb ? PyTuple_Pack(2, pa, pb) : nullptr;
+    Py_XDECREF(pa); Py_XDECREF(pb);
+    return r;
+}
+
+// (grad_input, x, qweight, scales, zeros, bias, N, K, group, workspace, workspace_bytes)
+PyObject* w4_gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    if (!count(n, 11)) return nullptr;
+    const bool dgrad = a[0] == Py_True;
+    if (!plain(a[1], at::kBFloat16) || !plain(a[2], at::kChar) || !plain(a[3], at::kBFloat16) || !plain(a[4], at::kBFloat16) || !plain_or_none(a[5], at::kBFloat16) ||
+        !plain_or_none(a[9], at::kByte))
+        Py_RETURN_NONE;
+    const int64_t N = PyLong_AsLongLong(a[6]), K = PyLong_AsLongLong(a[7]), group = PyLong_AsLongLong(a[8]), nb = PyLong_AsLongLong(a[10]);
+    if (PyErr_Occurred()) return nullptr;
+    const Tensor& x = tensor(a[1]);
+    if (x.dim() != 2 || x.size(1) != (dgrad ? N : K) || tensor(a[2]).numel() * 2 != N * K) Py_RETURN_NONE;
+    const int64_t M = x.size(0);
+    Tensor y = at::empty({M, dgrad ? K : N}, x.options());
+    const int8_t* w = (const int8_t*)ptr(a[2]);
+    const int rc = dgrad ? lq_gemm_a16w4_dgrad(x.data_ptr(), w, ptr(a[3]), ptr(a[4]), y.data_ptr(), M, N, K, (int)group, ptr(a[9]), (size_t)nb, stream())
+                         : lq_gemm_a16w4_fwd(x.data_ptr(), w, ptr(a[3]), ptr(a[4]), ptr(a[5]), y.data_ptr(), M, N, K, (int)group, ptr(a[9]), (size_t)nb, stream());
+    if (rc != LQ_OK) Py_RETURN_NONE;
+    return THPVariable_Wrap(std::move(y));
+    END_HANDLE_TH_ERRORS
+}
+
+// (x8, w8, row_scale, col_scale, alpha, bias, workspace, workspace_bytes)
+PyObject* a8w8_gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    if (!count(n, 8)) return nullptr;
+    if (!plain(a[0], at::kChar) || !plain(a[1], at::kChar) || !plain_or_none(a[2], at::kFloat) || !plain_or_none(a[3], at::kFloat) || !plain_or_none(a[5], at::kBFloat16) ||
+        !plain_or_none(a[6], at::kByte))
+        Py_RETURN_NONE;
+    const double alpha = PyFloat_AsDouble(a[4]);
+    const int64_t nb = PyLong_AsLongLong(a[7]);
+    if (PyErr_Occurred()) return nullptr;
+    const Tensor &x = tensor(a[0]), &w = tensor(a[1]);
+    if (x.dim() != 2 || w.dim() != 2 || x.size(1) != w.size(1)) Py_RETURN_NONE;
+    const int64_t M = x.size(0), K = x.size(1), N = w.size(0);
+    Tensor y = at::empty({M, N}, x.options().dtype(at::kBFloat16));
+    if (lq_gemm_a8w8((const int8_t*)x.data_ptr(), (const int8_t*)w.data_ptr(), (const float*)ptr(a[2]), (const float*)ptr(a[3]), (float)alpha, ptr(a[5]), y.data_ptr(), nullptr,
+                     M, N, K, ptr(a[6]), (size_t)nb, stream()) != LQ_OK)
+        Py_RETURN_NONE;
+    return THPVariable_Wrap(std::move(y));
+    END_HANDLE_TH_ERRORS
+}
+
+// (x8, w8, clampv, alpha, bias, qscales, workspace, workspace_bytes)
+PyObject* a8w8_module(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    if (!count(n, 8)) return nullptr;
+    if (!plain(a[0], at::kChar) || !plain(a[1], at::kChar) || !plain_or_none(a[2], at::kFloat) || !plain_or_none(a[4], at::kBFloat16) || !plain(a[5], at::kBFloat16) ||
+        !plain_or_none(a[6], at::kByte))
+        Py_RETURN_NONE;
+    const double alpha = PyFloat_AsDouble(a[3]);
+    const int64_t nb = PyLong_AsLongLong(a[7]);
+    if (PyErr_Occurred()) return nullptr;
+    const Tensor &x = tensor(a[0]), &w = tensor(a[1]);
+    if (x.dim() != 2 || w.dim() != 2 || x.size(1) != w.size(1) || tensor(a[5]).numel() != w.size(0) || (a[2] != Py_None && tensor(a[2]).numel() != 1) ||
+        (a[4] != Py_None && tensor(a[4]).numel() != w.size(0)))
+        Py_RETURN_NONE;
+    const int64_t M = x.size(0), K = x.size(1), N = w.size(0);
+    Tensor y = at::empty({M, N}, x.options().dtype(at::kBFloat16));
+    if (lq_gemm_a8w8_module((const int8_t*)x.data_ptr(), (const int8_t*)w.data_ptr(), (const float*)ptr(a[2]), (float)alpha, ptr(a[4]), ptr(a[5]), y.data_ptr(), M, N, K,
+                            ptr(a[6]), (size_t)nb, stream()) != LQ_OK)
+        Py_RETURN_NONE;
+    return THPVariable_Wrap(std::move(y));
+    END_HANDLE_TH_ERRORS
+}
+
+// (x) -> (x8, scale per token)
+PyObject* act_quant_per_token(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    if (!count(n, 1)) return nullptr;
+    if (!plain(a[0], at::kBFloat16) || tensor(a[0]).dim() != 2) Py_RETURN_NONE;
+    const Tensor& x = tensor(a[0]);
+    Tensor x8 = at::empty(x.sizes(), x.options().dtype(at::kChar)), s = at::empty({x.size(0)}, x.options().dtype(at::kFloat));
+    if (lq_act_quant_per_token(x.data_ptr(), x.size(0), x.size(1), (int8_t*)x8.data_ptr(), (float*)s.data_ptr(), stream()) != LQ_OK) Py_RETURN_NONE;
+    return pair(std::move(x8), std::move(s));
+    END_HANDLE_TH_ERRORS
+}
+
+// (x) -> (x8, maximum)
+PyObject* act_quant_per_tensor(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    if (!count(n, 1)) return nullptr;
+    if (!plain(a[0], at::kBFloat16)) Py_RETURN_NONE;
+    const Tensor& x = tensor(a[0]);
+    Tensor x8 = at::empty(x.sizes(), x.options().dtype(at::kChar)), c = at::empty({1}, x.options().dtype(at::kFloat));
+    if (lq_act_quant_per_tensor(x.data_ptr(), x.numel(), (float*)c.data_ptr(), (int8_t*)x8.data_ptr(), stream()) != LQ_OK) Py_RETURN_NONE;
+    return pair(std::move(x8), std::move(c));
+    END_HANDLE_TH_ERRORS
+}
+
+// (codes, row_scales, clampv): one of the two scales
+PyObject* i8_dequant(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    if (!count(n, 3)) return nullptr;
+    const bool rows = a[1] != Py_None;
+    if (!plain(a[0], at::kChar) || tensor(a[0]).dim() != 2 || !(rows ? plain(a[1], at::kBFloat16) : plain(a[2], at::kFloat))) Py_RETURN_NONE;
+    const Tensor& c = tensor(a[0]);
+    if (rows ? tensor(a[1]).numel() != c.size(0) : tensor(a[2]).numel() != 1) Py_RETURN_NONE;
+    Tensor y = at::empty(c.sizes(), c.options().dtype(at::kBFloat16));
+    if (lq_i8_dequant((const int8_t*)c.data_ptr(), rows ? ptr(a[1]) : nullptr, rows ? nullptr : (const float*)ptr(a[2]), c.size(0), c.size(1), y.data_ptr(), stream()) != LQ_OK)
+        Py_RETURN_NONE;
+    return THPVariable_Wrap(std::move(y));
+    END_HANDLE_TH_ERRORS
+}
+
+#define LQ_METHOD(f) {#f, (PyCFunction)(void (*)(void))f, METH_FASTCALL, nullptr}
+PyMethodDef methods[] = {LQ_METHOD(w4_gemm), LQ_METHOD(a8w8_gemm), LQ_METHOD(a8w8_module), LQ_METHOD(act_quant_per_token), LQ_METHOD(act_quant_per_tensor),
+                         LQ_METHOD(i8_dequant), {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_lqhost", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__lqhost() { return PyModule_Create(&module); }

@@ -8,6 +8,7 @@ import ctypes as C
 import torch
 
 from . import _lib as L
+from . import _lqhost as _host
 from ._lib import (CODEC_NONE, CODEC_THREEFOLD, CODEC_UNIFORM16, DITHER_EXPLICIT, DITHER_HASH,  # noqa: F401
                    DITHER_PHILOX, LQ_BF16, LQ_F32, RequantOpts)
 
@@ -304,6 +305,9 @@ def adam_dense_multi(table: DenseAdamTable, hyper):
 
 
 def act_quant_per_token(x):
+    r = _host.act_quant_per_token(x)
+    if r is not None:
+        return r
     _chk(x, "x", torch.bfloat16)
     M, K = x.shape
     x8 = torch.empty((M, K), dtype=torch.int8, device=x.device)
@@ -313,6 +317,9 @@ def act_quant_per_token(x):
 
 
 def act_quant_per_tensor(x):
+    r = _host.act_quant_per_tensor(x)
+    if r is not None:
+        return r
     _chk(x, "x", torch.bfloat16)
     x8 = torch.empty(x.shape, dtype=torch.int8, device=x.device)
     clampv = torch.empty(1, dtype=torch.float32, device=x.device)
@@ -341,7 +348,16 @@ def _workspace(kind, M, N, K, device):
     return ws, ws.numel()
 
 
+def _matrix_on_gpu(x):
+    return isinstance(x, torch.Tensor) and x.is_cuda and x.dim() == 2
+
+
 def gemm_a16w4_fwd(x, qweight, scales, zeros, bias, N, K, group=128, out=None):
+    if out is None and _matrix_on_gpu(x):
+        ws, nb = _workspace(L.GEMM_A16W4_FWD, x.shape[0], N, K, x.device)
+        y = _host.w4_gemm(False, x, qweight, scales, zeros, bias, N, K, group, ws, nb)
+        if y is not None:
+            return y
     _chk(x, "x", torch.bfloat16); _chk(qweight, "qweight", torch.int8)
     _chk(scales, "scales", torch.bfloat16); _chk(zeros, "zeros", torch.bfloat16)
     M = x.shape[0]
@@ -356,6 +372,11 @@ def gemm_a16w4_fwd(x, qweight, scales, zeros, bias, N, K, group=128, out=None):
 
 
 def gemm_a16w4_dgrad(dy, qweight, scales, zeros, N, K, group=128, out=None):
+    if out is None and _matrix_on_gpu(dy):
+        ws, nb = _workspace(L.GEMM_A16W4_DGRAD, dy.shape[0], N, K, dy.device)
+        dx = _host.w4_gemm(True, dy, qweight, scales, zeros, None, N, K, group, ws, nb)
+        if dx is not None:
+            return dx
     _chk(dy, "dy", torch.bfloat16); _chk(qweight, "qweight", torch.int8)
     _chk(scales, "scales", torch.bfloat16); _chk(zeros, "zeros", torch.bfloat16)
     M = dy.shape[0]
@@ -385,6 +406,11 @@ def gemm_wgrad(dy, x, dw=None, accumulate=False):
 
 
 def gemm_a8w8(x8, w8, row_scale=None, col_scale=None, alpha=1.0, bias=None, want_acc=False):
+    if not want_acc and _matrix_on_gpu(x8) and _matrix_on_gpu(w8):
+        ws, nb = _workspace(L.GEMM_A8W8, x8.shape[0], w8.shape[0], x8.shape[1], x8.device)
+        y = _host.a8w8_gemm(x8, w8, row_scale, col_scale, float(alpha), bias, ws, nb)
+        if y is not None:
+            return y
     _chk(x8, "x8", torch.int8); _chk(w8, "w8", torch.int8)
     M, K = x8.shape
     N = w8.shape[0]
@@ -405,6 +431,11 @@ def gemm_a8w8(x8, w8, row_scale=None, col_scale=None, alpha=1.0, bias=None, want
 def gemm_a8w8_module(x8, w8, clampv, alpha, bias, qscales):
     """Forward of an A8W8 linear behind its input quantizer (utils/quant.py:268-271): one launch for
     `(acc * a + bias / qscales) * qscales` with a = clampv / 127 from the device (`clampv` fp32[1]) or `alpha`."""
+    if _matrix_on_gpu(x8) and _matrix_on_gpu(w8):
+        ws, nb = _workspace(L.GEMM_A8W8, x8.shape[0], w8.shape[0], x8.shape[1], x8.device)
+        y = _host.a8w8_module(x8, w8, clampv, float(alpha), bias, qscales, ws, nb)
+        if y is not None:
+            return y
     _chk(x8, "x8", torch.int8); _chk(w8, "w8", torch.int8); _chk(qscales, "qscales", torch.bfloat16)
     M, K = x8.shape
     N = w8.shape[0]
@@ -424,6 +455,9 @@ def gemm_a8w8_module(x8, w8, clampv, alpha, bias, qscales):
 
 def i8_dequant(codes, row_scales=None, clampv=None):
     """bf16(code * s): s per row (`row_scales` bf16) or bf16(clampv / 127) of the whole tensor (`clampv` fp32[1])."""
+    y = _host.i8_dequant(codes, row_scales, clampv)
+    if y is not None:
+        return y
     _chk(codes, "codes", torch.int8)
     rows, cols = codes.shape
     if row_scales is not None:

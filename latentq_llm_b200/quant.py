@@ -126,7 +126,7 @@ dict_temp = []  # utils/quant.py:109-110: weight gradients travel from backward(
 
 def _w4_args(qparamw4):
     scales, zeros, shape = qparamw4
-    return scales.contiguous().reshape(-1), zeros.contiguous().reshape(-1), int(shape[0]), int(shape[1])
+    return scales.contiguous(), zeros.contiguous(), int(shape[0]), int(shape[1])
 
 
 def _apply(fn, *args):
@@ -452,6 +452,9 @@ class QLinearA16W4(nn.Module):
         self.qweight.data = self.weight.data.cpu()
 
     def forward(self, x):
+        if self.hook_handle != "direct" and x.dim() == 2 and not torch.is_grad_enabled():       # no reshapes of what is a matrix already
+            w = self.weight
+            return _apply(QLinearFunctionW4_eval if self.hook_handle is None else QLinearFunctionW4, x, w.data, w.qparam, self.bias)
         out_shape = x.shape[:-1] + (self.output_features,)
         if self.hook_handle == "direct":
             fq = self._flat_qparams
