@@ -181,26 +181,52 @@ __global__ void k_rope_kv_store(__nv_bfloat16* __restrict__ qkv, const long long
 // ---------------------------------------------------------------------------------------------
 // Single-query attention over the cache: out[b, h, :] = softmax(q . K[0..pos] * scale) . V[0..pos].
 // grid (batch * q heads, splits); 128 threads = 16 key slots of 8 lanes, a lane holds hd/8 dims (hd = 64 or 128).
-// Each split covers a contiguous range of keys and leaves (max, sum, weighted V) in the workspace; the split
-// that finishes last for its (batch, head) combines them (a ticket counter; nobody waits for anybody).
+// Each split covers a contiguous range of keys.  CLUSTER: the splits of a (batch, head) are one cluster and leave (max, sum, weighted V)
+// in their own shared memory, where the first reads them.  Otherwise they go to the workspace and the split that finishes last
+// combines them (a ticket counter; nobody waits for anybody): store, fence, ticket and two dependent reads are five trips to L2 at
+// the end of a launch of a few microseconds.
+// Before the dependency wait every CTA asks for its first keys and values in L2 (`prefetch`): the position it goes by may still be the
+// previous step's (the rows then differ by one key), and it is read again behind the wait.
 // ---------------------------------------------------------------------------------------------
-constexpr int ATT_THREADS = 128, ATT_SLOTS = ATT_THREADS / 8;
-template <int HD>
+constexpr int ATT_THREADS = 128, ATT_SLOTS = ATT_THREADS / 8, ATT_CLUSTER_MAX = 8;
+__device__ __forceinline__ float ld_cluster(const float* local, int rank) {            // the same variable of the cluster's CTA `rank`
+    uint32_t a;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(local)), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ void att_cluster_sync() { asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+template <int HD, bool CLUSTER>
 __global__ void __launch_bounds__(ATT_THREADS) k_decode_attn(const __nv_bfloat16* __restrict__ q, int q_row_stride,
                                                               const __nv_bfloat16* __restrict__ k_cache,
                                                               const __nv_bfloat16* __restrict__ v_cache,
                                                               const long long* __restrict__ positions, __nv_bfloat16* __restrict__ out,
                                                               int Hq, int Hkv, int max_len, float scale, float* __restrict__ part,
-                                                              unsigned int* __restrict__ tickets) {
+                                                              unsigned int* __restrict__ tickets, int prefetch) {
     constexpr int D = HD / 8;                                 // dims per lane
     __shared__ float sm_m[ATT_SLOTS], sm_l[ATT_SLOTS], sm_acc[ATT_SLOTS][HD];
     __shared__ bool is_last;
+    __shared__ float cl_acc[HD], cl_ml[2];
     const int bh = blockIdx.x, b = bh / Hq, h = bh - b * Hq, hk = h / (Hq / Hkv);
     const int splits = gridDim.y, split = blockIdx.y;
     const int slot = threadIdx.x >> 3, sub = threadIdx.x & 7;
+    constexpr int KPI = 4;                                    // keys per slot in flight
+    const __nv_bfloat16* kb = k_cache + ((size_t)b * Hkv + hk) * (size_t)max_len * HD + sub * D;
+    const __nv_bfloat16* vb = v_cache + ((size_t)b * Hkv + hk) * (size_t)max_len * HD + sub * D;
     pdl_launch_dependents();
+    if (prefetch) {
+        const long long n = min(max(__ldcv(positions + b) + 1, 0ll), (long long)max_len);
+        const int per = (int)((n + splits - 1) / splits), j0 = split * per + slot, j1 = (int)min((long long)(split + 1) * per, n);
+#pragma unroll
+        for (int u = 0; u < KPI; ++u)
+            if (j0 + u * ATT_SLOTS < j1) {
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(kb + (size_t)(j0 + u * ATT_SLOTS) * HD));
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(vb + (size_t)(j0 + u * ATT_SLOTS) * HD));
+            }
+    }
     pdl_wait();                                       // q and the newest cache row are the predecessor's output
-    long long n_keys = positions[b] + 1;
+    long long n_keys = __ldcv(positions + b) + 1;
     if (n_keys > max_len) n_keys = max_len;
     if (n_keys < 0) n_keys = 0;
     const int per = (int)((n_keys + splits - 1) / splits);
@@ -215,8 +241,6 @@ __global__ void __launch_bounds__(ATT_THREADS) k_decode_attn(const __nv_bfloat16
             qf[d] = bf_lo(w) * scale; qf[d + 1] = bf_hi(w) * scale;
         }
     }
-    const __nv_bfloat16* kb = k_cache + ((size_t)b * Hkv + hk) * (size_t)max_len * HD + sub * D;
-    const __nv_bfloat16* vb = v_cache + ((size_t)b * Hkv + hk) * (size_t)max_len * HD + sub * D;
     const unsigned int slot_mask = 0xffu << (8 * (slot & 3));
     float mx = -INFINITY, l = 0.0f, acc[D];
 #pragma unroll
@@ -224,7 +248,6 @@ __global__ void __launch_bounds__(ATT_THREADS) k_decode_attn(const __nv_bfloat16
     // KPI keys per slot in flight: the K and V rows of all of them are requested before any arithmetic (the kernel is a
     // chain of memory latencies otherwise; a split covers about 64 keys, i.e. one such round per slot).  A key beyond the
     // range reads key j1-1 again and gets weight zero.
-    constexpr int KPI = 4;
     for (int j = j0 + slot; j < j1; j += KPI * ATT_SLOTS) {
         uint4 kq[KPI][D / 8], vq[KPI][D / 8];
         bool on[KPI];
@@ -293,12 +316,38 @@ __global__ void __launch_bounds__(ATT_THREADS) k_decode_attn(const __nv_bfloat16
             const float w = (sm_m[s2] == -INFINITY) ? 0.0f : __expf(sm_m[s2] - M);
             L = fmaf(sm_l[s2], w, L); a = fmaf(sm_acc[s2][threadIdx.x], w, a);
         }
-        if (splits == 1) {
+        if (CLUSTER) {
+            cl_acc[threadIdx.x] = a;
+            if (threadIdx.x == 0) { cl_ml[0] = M; cl_ml[1] = L; }
+        } else if (splits == 1) {
             out[(size_t)b * Hq * HD + (size_t)h * HD + threadIdx.x] = __float2bfloat16_rn(L > 0.0f ? a / L : 0.0f);
         } else {
             my[threadIdx.x] = a;
             if (threadIdx.x == 0) { my[HD] = M; my[HD + 1] = L; }
         }
+    }
+    if constexpr (CLUSTER) {
+        att_cluster_sync();
+        if (split == 0 && threadIdx.x < HD) {                   // the cluster's CTA ranks are its split numbers
+            float ms[ATT_CLUSTER_MAX], ls[ATT_CLUSTER_MAX], v[ATT_CLUSTER_MAX], M = -INFINITY;
+#pragma unroll
+            for (int i = 0; i < ATT_CLUSTER_MAX; ++i) {
+                ms[i] = -INFINITY;
+                if (i < splits) { ms[i] = ld_cluster(cl_ml, i); ls[i] = ld_cluster(cl_ml + 1, i); v[i] = ld_cluster(cl_acc + threadIdx.x, i); }
+            }
+#pragma unroll
+            for (int i = 0; i < ATT_CLUSTER_MAX; ++i) M = fmaxf(M, ms[i]);
+            float L = 0.0f, a = 0.0f;
+#pragma unroll
+            for (int i = 0; i < ATT_CLUSTER_MAX; ++i)
+                if (i < splits) {
+                    const float w = (ms[i] == -INFINITY) ? 0.0f : __expf(ms[i] - M);
+                    L = fmaf(ls[i], w, L); a = fmaf(v[i], w, a);
+                }
+            out[(size_t)b * Hq * HD + (size_t)h * HD + threadIdx.x] = __float2bfloat16_rn(L > 0.0f ? a / L : 0.0f);
+        }
+        att_cluster_sync();                                     // the others' shared memory has been read
+        return;
     }
     if (splits == 1) return;
     __threadfence();
@@ -444,6 +493,18 @@ static inline bool al16p(const void* p) { return (reinterpret_cast<uintptr_t>(p)
 
 using namespace lq;
 
+template <int HD>
+static cudaError_t launch_attn_cluster(cudaLaunchConfig_t cfg, const __nv_bfloat16* q, int q_row_stride, const __nv_bfloat16* k, const __nv_bfloat16* v, const long long* positions,
+                                       __nv_bfloat16* out, int Hq, int Hkv, int max_len, float scale, int prefetch) {
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = decode_chain_enabled() ? 1 : 0;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 1; attr[1].val.clusterDim.y = cfg.gridDim.y; attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr; cfg.numAttrs = 2;
+    return cudaLaunchKernelEx(&cfg, k_decode_attn<HD, true>, q, q_row_stride, k, v, positions, out, Hq, Hkv, max_len, scale, (float*)nullptr, (unsigned int*)nullptr, prefetch);
+}
+
 extern "C" {
 
 int lq_add_rmsnorm(void* h, const void* delta, const void* gamma, float eps, void* y, int64_t M, int64_t K, int hf_rounding,
@@ -492,6 +553,16 @@ static int attn_splits(int64_t B, int Hq, int64_t max_len) {
     if (s < 1) s = 1;
     return (int)s;
 }
+// Splits of a (batch, head) that run as one cluster, or 0: tickets.  Eight, four or two (clusters of three, six or sixteen leave room on the
+// chip's SM groups: a second wave, up to 40 % slower), from the context lengths at which so many pay, as long as all clusters are
+// resident together.  With 65 or more rows the tickets' finer splits win where they are half as many again: 96 rows of 1500 keys 15.0 / 14.1 us,
+// 160 rows of 1500 24.0 / 21.9.  Cluster / tickets (us; 32 heads): 1 sequence of 100 keys 4.1 / 5.2, 520 6.1 / 7.4, 1500 9.3 / 10.3; 2: 4.6 / 5.5, 7.5 / 8.5, 11.0 /
+// 12.1; 4: 5.8 / 6.7, 9.5 / 9.9, 14.9 / 15.3; 8: 7.2 / 7.5, 12.9 / 13.4, 27.9 / 28.8.
+static int attn_cluster(int64_t B, int Hq, int64_t max_len) {
+    const int64_t rows = B * Hq, sms = sm_count();
+    const int c = max_len >= 512 && rows * 16 <= 7 * sms ? 8 : max_len >= 192 && rows * 8 <= 7 * sms ? 4 : max_len > 64 && rows * 2 <= 4 * sms ? 2 : 0;
+    return c && (rows <= 64 || 10 * c >= 7 * attn_splits(B, Hq, max_len)) ? c : 0;
+}
 
 size_t lq_decode_attention_workspace_bytes(int64_t B, int Hq, int hd, int64_t max_len) {
     if (B <= 0 || Hq <= 0 || hd <= 0 || max_len <= 0) return 0;
@@ -508,21 +579,34 @@ int lq_decode_attention(const void* q, int64_t q_row_stride, const void* k_cache
         return LQ_EUNSUPPORTED;
     if (B == 0) return LQ_OK;
     { int rc = ensure_device_for(q); if (rc) return rc; }
-    const int splits = attn_splits(B, Hq, max_len);
+    const int cluster = attn_cluster(B, Hq, max_len), splits = cluster ? cluster : attn_splits(B, Hq, max_len);
     float* part = nullptr; unsigned int* tickets = nullptr;
-    if (splits > 1) {
+    if (attn_splits(B, Hq, max_len) > 1) {              // (clusters leave it untouched)
         if (!workspace || workspace_bytes < lq_decode_attention_workspace_bytes(B, Hq, hd, max_len) || !al16p(workspace)) return LQ_EWORKSPACE;
         part = (float*)workspace;
         tickets = (unsigned int*)(part + (size_t)B * Hq * splits * (hd + 2));
     }
     dim3 grid((unsigned)(B * Hq), (unsigned)splits);
     cudaStream_t st = (cudaStream_t)stream;
-    if (hd == 128)
-        launch_pdl(k_decode_attn<128>, grid, (unsigned)ATT_THREADS, 0, st, (const __nv_bfloat16*)q, (int)q_row_stride, (const __nv_bfloat16*)k_cache,
-                   (const __nv_bfloat16*)v_cache, (const long long*)positions, (__nv_bfloat16*)out, Hq, Hkv, (int)max_len, scale, part, tickets);
-    else
-        launch_pdl(k_decode_attn<64>, grid, (unsigned)ATT_THREADS, 0, st, (const __nv_bfloat16*)q, (int)q_row_stride, (const __nv_bfloat16*)k_cache,
-                   (const __nv_bfloat16*)v_cache, (const long long*)positions, (__nv_bfloat16*)out, Hq, Hkv, (int)max_len, scale, part, tickets);
+    // Worth its instructions where all CTAs start beside the predecessor's last ones and no two of them read the same keys (640 rows of 100 keys
+    // 9.4 / 9.9 us with it, 320 rows on 80 key heads 5.6 / 5.9; 1 to 16 sequences of 32 heads 2 to 7 % shorter with it).
+    const int prefetch = Hq == Hkv && B * Hq * splits <= 4 * (int64_t)sm_count() ? 1 : 0;
+    auto launch = [&](auto kern) {
+        launch_pdl(kern, grid, (unsigned)ATT_THREADS, 0, st, (const __nv_bfloat16*)q, (int)q_row_stride, (const __nv_bfloat16*)k_cache, (const __nv_bfloat16*)v_cache,
+                   (const long long*)positions, (__nv_bfloat16*)out, Hq, Hkv, (int)max_len, scale, part, tickets, prefetch);
+    };
+    if (cluster) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = grid; cfg.blockDim = dim3(ATT_THREADS); cfg.stream = st;
+        const cudaError_t e = (hd == 128 ? launch_attn_cluster<128> : launch_attn_cluster<64>)(
+            cfg, (const __nv_bfloat16*)q, (int)q_row_stride, (const __nv_bfloat16*)k_cache, (const __nv_bfloat16*)v_cache, (const long long*)positions,
+            (__nv_bfloat16*)out, Hq, Hkv, (int)max_len, scale, prefetch);
+        if (e != cudaSuccess) { set_cuda_error(e, "k_decode_attn (cluster)"); return LQ_ECUDA; }
+    } else if (hd == 128) {
+        launch(k_decode_attn<128, false>);
+    } else {
+        launch(k_decode_attn<64, false>);
+    }
     return check_launch("k_decode_attn");
 }
 

@@ -143,3 +143,25 @@ def test_argmax_embed(ops, B, V, D):
     tok2 = torch.full((B,), -1, dtype=torch.long, device="cuda")
     ops.argmax_embed(logits[:, : V - 1], tok2)
     assert torch.equal(tok2, logits[:, : V - 1].float().argmax(-1))
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,hd,max_len", [(1, 32, 32, 128, 64), (1, 32, 32, 128, 65), (2, 32, 8, 128, 192), (1, 16, 16, 64, 512), (2, 32, 32, 128, 1500),
+                                                 (4, 32, 32, 128, 511), (3, 32, 32, 64, 384), (9, 32, 32, 128, 100), (10, 32, 32, 128, 100), (1, 3, 1, 64, 700)])
+def test_decode_attention_split_plans(ops, B, Hq, Hkv, hd, max_len):
+    """Clusters of two, four and eight splits, tickets and a single split, next to the context lengths and row counts where the plan
+    changes, with sequences that leave splits without a key; inside a decode chain and outside of one the same bits."""
+    rng = np.random.default_rng(B * 5 + max_len)
+    qkv = orc.bf16_round(rng.standard_normal((B, (Hq + 2 * Hkv) * hd)).astype(np.float32))
+    kc = orc.bf16_round(rng.standard_normal((B, Hkv, max_len, hd)).astype(np.float32))
+    vc = orc.bf16_round(rng.standard_normal((B, Hkv, max_len, hd)).astype(np.float32))
+    for first in (max_len - 1, 0, 5):
+        pos = rng.integers(0, max_len, B).astype(np.int64)
+        pos[0] = first
+        args = (_bf(qkv), torch.from_numpy(pos).cuda(), _bf(kc), _bf(vc), Hq, Hkv, hd)
+        out = ops.decode_attention(*args)
+        with ops.decode_chain():
+            again = ops.decode_attention(*args)
+        want = orc.decode_attention(qkv[:, :Hq * hd].reshape(B, Hq, hd), kc, vc, pos, hd ** -0.5)
+        got = out.float().cpu().numpy().reshape(B, Hq, hd)
+        assert np.abs(got - want).max() <= 2.0 ** -7 * np.abs(want).max()
+        assert torch.equal(out, again)
