@@ -532,7 +532,8 @@ k_gemm(const __grid_constant__ CUtensorMap map_tok, const __grid_constant__ CUte
     } else if (warp < 6 || warp >= C::FIRST_EXTRA_EPI) {
         // ===================== epilogue =====================
         const int quad = warp & 3;                 // TMEM lane quadrant this warp may read
-        const int col_lo = (warp < 6 ? 0 : 1) * (TN / C::EPI_SPLIT), col_hi = col_lo + TN / C::EPI_SPLIT;   // its token columns
+        constexpr int COL_MID = C::EPI_SPLIT == 2 ? (TN / 2 + 15) / 16 * 16 : TN;
+        const int col_lo = warp < 6 ? 0 : COL_MID, col_hi = warp < 6 ? COL_MID : TN;                        // its token columns
         int acc = 0; uint32_t acc_phase = 0;
         bool ok = true;
         long long w_accf = 0;
@@ -1157,12 +1158,15 @@ static int plan_splits(int tiles, int kb_total, int sms) {
 // tokens 53.8 (256) / 38.5 us (128), at 512 51.2 / 46.3 (192), 2048 rows at 1000 46.6 / 36.2 (128).
 //   Where it errs: some grad-inputs of 45 .. 63 tokens take two tiles of 32, up to 0.7 us (6 %) slower than one of 64 (4352 x 1152 at 50 tokens
 // 12.5 / 11.7); a smaller price for the partial sums mends them and loses 4 to 11 % at 280 to 700 tokens.
+//   48, 80 and 112 tokens exist in the kernel of two k-blocks per stage, whose MMAs and token copies they shorten: 11008 rows at 40 / 72 / 100 tokens
+// 17.3 / 18.6 / 20.2 -> 16.4 / 17.9 / 19.3 us, 8192 x 2048 at 200 14.5 -> 13.5.  Taken where modelled at least 2 % shorter (below that the model's
+// choice between them and a split was up to 10 % wrong: 2048 x 2048 at 97 tokens 10.8 / 11.8).
 //   A forward whose group parameters are not staged has its own column: its loads of them bound the narrow tiles, so that
 // halving the width does not halve anything.  With the staged kernel's column 4096 -> 4096 with groups of 64 took 32-token tiles at 128
 // tokens, 21.6 instead of 19.2 us with 128, and 3968 -> 4096 at 128 tokens 19.9 instead of 18.6.
 struct TokenTile { int tn; float fwd, fwd_unstaged, fwd_tail, dgrad; };
-static const TokenTile token_tiles[] = {{32, 0.18f, 0.26f, 0.3f, 0.297f}, {64, 0.20f, 0.273f, 0.3f, 0.32f}, {96, 0.225f, 0.318f, 0.3f, 0.335f},
-                                        {128, 0.245f, 0.319f, 0.3f, 0.343f}, {160, 0.28f, 0.365f, 0.4f, 0.366f}, {192, 0.305f, 0.4f, 0.9f, 0.4f},
+static const TokenTile token_tiles[] = {{32, 0.18f, 0.26f, 0.3f, 0.297f}, {48, 0.19f, 0.0f, 0.3f, 0.0f}, {64, 0.20f, 0.273f, 0.3f, 0.32f}, {80, 0.2125f, 0.0f, 0.3f, 0.0f},
+                                        {96, 0.225f, 0.318f, 0.3f, 0.335f}, {112, 0.235f, 0.0f, 0.3f, 0.0f}, {128, 0.245f, 0.319f, 0.3f, 0.343f}, {160, 0.28f, 0.365f, 0.4f, 0.366f}, {192, 0.305f, 0.4f, 0.9f, 0.4f},
                                         {256, 0.36f, 0.43f, 2.0f, 0.456f}};
 // Forwards whose group parameters come through shared memory, by their shape (their pointers decide too, see run_gemm)
 static bool qp_staging(int group, int64_t K) { return group == 128 && (K / 128) % 2 == 0; }
@@ -1176,8 +1180,10 @@ static int pick_token_tile(int kind, bool staged, int64_t M, int64_t R, int kb_t
         const int splits = tiles > sms ? 1 : plan_splits((int)tiles, kb_total, sms);
         const int64_t waves = (tiles * splits + sms - 1) / sms;
         const double stage = kind != KIND_FWD ? w.dgrad : staged ? w.fwd : w.fwd_unstaged, tail = kind == KIND_FWD ? w.fwd_tail : 0.3;
+        if (stage == 0.0) continue;                     // a width that this kernel does not have
         double cost = (double)waves * (((kb_total + splits - 1) / splits) * stage + tail);
         if (splits > 1) cost += 2.5 + 0.75e-6 * 4.0 * (double)splits * (double)M * (double)R;
+        if (w.tn % 32) cost *= 1.02;
         if (cost < best_cost) { best_cost = cost; best = w.tn; }
     }
     if (us) *us = best_cost;
@@ -1345,7 +1351,10 @@ static int launch_w4(int tn, const CUtensorMap& mt, const CUtensorMap& mw, const
 static int launch_fwd_k2(int tn, const CUtensorMap& mt, const CUtensorMap& mw, const GemmParams& p, cudaStream_t st) {
     switch (tn) {
         case 32: return launch_tn<KIND_FWD, 32, 1, true, false, false, 2>(mt, mw, p, st);
+        case 48: return launch_tn<KIND_FWD, 48, 1, true, false, false, 2>(mt, mw, p, st);
         case 64: return launch_tn<KIND_FWD, 64, 1, true, false, false, 2>(mt, mw, p, st);
+        case 80: return launch_tn<KIND_FWD, 80, 1, true, false, false, 2>(mt, mw, p, st);
+        case 112: return launch_tn<KIND_FWD, 112, 1, true, false, false, 2>(mt, mw, p, st);
         case 96: return launch_tn<KIND_FWD, 96, 1, true, false, false, 2>(mt, mw, p, st);
         case 128: return launch_tn<KIND_FWD, 128, 1, true, false, false, 2>(mt, mw, p, st);
     }
@@ -1434,6 +1443,10 @@ static int run_gemm(int kind, const void* tok, const void* w, GemmParams p, int6
     CUtensorMap mt, mw;
     int rc;
     const bool k2 = kind == KIND_FWD && p.qp_staged && !pl.sk && two_kb_stages(p.group, K, pl.tn) && pl.kb_per_split % 2 == 0 && a_operand_in_tmem(kind);
+    if (kind == KIND_FWD && !k2 && pl.tn > 32 && pl.tn < 128 && pl.tn % 32 == 16) {       // widths of the two-block kernel only
+        pl.tn += 16;
+        p.t_tiles = pl.t_tiles = (int)((M + pl.tn - 1) / pl.tn);
+    }
     if (kind == KIND_I8) {
         rc = make_map(&mt, tok, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)M, (uint64_t)K, (uint32_t)pl.tn, 128, CU_TENSOR_MAP_SWIZZLE_128B);
         if (rc) return rc;

@@ -316,3 +316,21 @@ def test_i8_dequant_rows_by_multiplication(rows, cols):
     c = torch.randint(-128, 128, (rows, cols), device="cuda", generator=_gen(cols), dtype=torch.int8)
     qs = (torch.rand(rows, 1, device="cuda", generator=_gen(rows)) * 0.01 + 1e-3).to(torch.bfloat16)
     assert torch.equal(ops.i8_dequant(c, row_scales=qs), c.to(torch.bfloat16) * qs)
+
+
+# The widths of 48, 80 and 112 tokens, which only the two-block kernel has: one and two tiles, a token to spare and none, with and without
+# split-K; the same bits with the weight tile in shared memory, where those launches take the next width, and with group parameters
+# that cannot be staged (their address is odd).
+@pytest.mark.parametrize("M", [33, 48, 80, 81, 97, 112, 200, 224])
+@pytest.mark.parametrize("N,K", [(11008, 1024), (8192, 2048), (2048, 4096)])
+def test_token_tiles_between_the_multiples_of_32(monkeypatch, M, N, K):
+    from latentq_llm_b200 import ops
+    codes, s, z, w = _w4(N, K, N + K)
+    x = torch.randn(M, K, device="cuda", generator=_gen(M)).to(torch.bfloat16)
+    odd = [torch.cat([t.reshape(-1)[:1], t.reshape(-1)])[1:] for t in (s, z)]
+    out = [ops.gemm_a16w4_fwd(x, codes, s, z, None, N, K), ops.gemm_a16w4_fwd(x, codes, *odd, None, N, K)]
+    monkeypatch.setenv("LQ_GEMM_A_OPERAND", "smem")
+    out.append(ops.gemm_a16w4_fwd(x, codes, s, z, None, N, K))
+    ref = x.double() @ w.t()
+    assert float((out[0].double() - ref).norm() / ref.norm()) < 4e-3
+    assert torch.equal(out[0], out[1]) and torch.equal(out[0], out[2])
