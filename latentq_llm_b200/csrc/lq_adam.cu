@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(256) k_adam_quant(const AdamParams p) {
 //             every midpoint of two fp32 numbers, the corrected quotient is 2^-44 off before its rounding.
 //   states    encoded with a quotient from a two-term reciprocal and one residual correction (Markstein's theorem, see div_by), as is
 //             the division of the block's range by 255.
-//   fp32      two elements per instruction (fma / mul / add .f32x2) for int4 codes: 157 -> 149 us for 4096 x
+//   fp32      two elements per instruction (fma / mul / add .f32x2) for int4 codes: 83 -> 74 instructions per weight, 157 -> 149 us for 4096 x
 //             11008.  The int8 kernel has no registers left for the pairs (64, two teams of 256 threads): 172 -> 178 us, so it keeps
 //             one element per instruction.
 //   requantize  everything after Z = w/scale + zero from the table of the requantize fast path (int4: a byte per bf16 pattern,
