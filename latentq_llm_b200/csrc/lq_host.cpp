@@ -7,6 +7,7 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/utils/pybind.h>
 
 #include "latentq.h"
 
@@ -25,6 +26,12 @@ bool plain(PyObject* o, at::ScalarType dtype) {
 bool plain_or_none(PyObject* o, at::ScalarType dtype) { return o == Py_None || plain(o, dtype); }
 const Tensor& tensor(PyObject* o) { return THPVariable_Unpack(o); }
 void* ptr(PyObject* o) { return o == Py_None ? nullptr : tensor(o).data_ptr(); }
+// Allocation and launch with the GIL released, as torch.empty and a ctypes call do it: both may wait (cudaMalloc, a full launch queue), and
+// what they wait for may need another Python thread.  `f` uses nothing of the arguments' Python objects.
+template <typename F> int without_gil(F f) {
+    pybind11::gil_scoped_release nogil;
+    return f();
+}
 lq_stream_t stream() { return (lq_stream_t)c10::cuda::getCurrentCUDAStream().stream(); }
 bool count(Py_ssize_t n, Py_ssize_t want) {
     if (n == want) return true;
@@ -52,10 +59,16 @@ PyObject* w4_gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const Tensor& x = tensor(a[1]);
     if (x.dim() != 2 || x.size(1) != (dgrad ? N : K) || tensor(a[2]).numel() * 2 != N * K) Py_RETURN_NONE;
     const int64_t M = x.size(0);
-    Tensor y = at::empty({M, dgrad ? K : N}, x.options());
+    const at::TensorOptions opt = x.options();
     const int8_t* w = (const int8_t*)ptr(a[2]);
-    const int rc = dgrad ? lq_gemm_a16w4_dgrad(x.data_ptr(), w, ptr(a[3]), ptr(a[4]), y.data_ptr(), M, N, K, (int)group, ptr(a[9]), (size_t)nb, stream())
-                         : lq_gemm_a16w4_fwd(x.data_ptr(), w, ptr(a[3]), ptr(a[4]), ptr(a[5]), y.data_ptr(), M, N, K, (int)group, ptr(a[9]), (size_t)nb, stream());
+    const void *px = ptr(a[1]), *s = ptr(a[3]), *z = ptr(a[4]), *bias = ptr(a[5]);
+    void* ws = ptr(a[9]);
+    Tensor y;
+    const int rc = without_gil([&] {
+        y = at::empty({M, dgrad ? K : N}, opt);
+        return dgrad ? lq_gemm_a16w4_dgrad(px, w, s, z, y.data_ptr(), M, N, K, (int)group, ws, (size_t)nb, stream())
+                     : lq_gemm_a16w4_fwd(px, w, s, z, bias, y.data_ptr(), M, N, K, (int)group, ws, (size_t)nb, stream());
+    });
     if (rc != LQ_OK) Py_RETURN_NONE;
     return THPVariable_Wrap(std::move(y));
     END_HANDLE_TH_ERRORS
@@ -74,10 +87,17 @@ PyObject* a8w8_gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const Tensor &x = tensor(a[0]), &w = tensor(a[1]);
     if (x.dim() != 2 || w.dim() != 2 || x.size(1) != w.size(1)) Py_RETURN_NONE;
     const int64_t M = x.size(0), K = x.size(1), N = w.size(0);
-    Tensor y = at::empty({M, N}, x.options().dtype(at::kBFloat16));
-    if (lq_gemm_a8w8((const int8_t*)x.data_ptr(), (const int8_t*)w.data_ptr(), (const float*)ptr(a[2]), (const float*)ptr(a[3]), (float)alpha, ptr(a[5]), y.data_ptr(), nullptr,
-                     M, N, K, ptr(a[6]), (size_t)nb, stream()) != LQ_OK)
-        Py_RETURN_NONE;
+    const at::TensorOptions opt = x.options().dtype(at::kBFloat16);
+    const int8_t *px = (const int8_t*)ptr(a[0]), *pw = (const int8_t*)ptr(a[1]);
+    const float *row_scale = (const float*)ptr(a[2]), *col_scale = (const float*)ptr(a[3]);
+    const void* bias = ptr(a[5]);
+    void* ws = ptr(a[6]);
+    Tensor y;
+    const int rc = without_gil([&] {
+        y = at::empty({M, N}, opt);
+        return lq_gemm_a8w8(px, pw, row_scale, col_scale, (float)alpha, bias, y.data_ptr(), nullptr, M, N, K, ws, (size_t)nb, stream());
+    });
+    if (rc != LQ_OK) Py_RETURN_NONE;
     return THPVariable_Wrap(std::move(y));
     END_HANDLE_TH_ERRORS
 }
@@ -97,10 +117,17 @@ PyObject* a8w8_module(PyObject*, PyObject* const* a, Py_ssize_t n) {
         (a[4] != Py_None && tensor(a[4]).numel() != w.size(0)))
         Py_RETURN_NONE;
     const int64_t M = x.size(0), K = x.size(1), N = w.size(0);
-    Tensor y = at::empty({M, N}, x.options().dtype(at::kBFloat16));
-    if (lq_gemm_a8w8_module((const int8_t*)x.data_ptr(), (const int8_t*)w.data_ptr(), (const float*)ptr(a[2]), (float)alpha, ptr(a[4]), ptr(a[5]), y.data_ptr(), M, N, K,
-                            ptr(a[6]), (size_t)nb, stream()) != LQ_OK)
-        Py_RETURN_NONE;
+    const at::TensorOptions opt = x.options().dtype(at::kBFloat16);
+    const int8_t *px = (const int8_t*)ptr(a[0]), *pw = (const int8_t*)ptr(a[1]);
+    const float* clampv = (const float*)ptr(a[2]);
+    const void *bias = ptr(a[4]), *qscales = ptr(a[5]);
+    void* ws = ptr(a[6]);
+    Tensor y;
+    const int rc = without_gil([&] {
+        y = at::empty({M, N}, opt);
+        return lq_gemm_a8w8_module(px, pw, clampv, (float)alpha, bias, qscales, y.data_ptr(), M, N, K, ws, (size_t)nb, stream());
+    });
+    if (rc != LQ_OK) Py_RETURN_NONE;
     return THPVariable_Wrap(std::move(y));
     END_HANDLE_TH_ERRORS
 }
@@ -111,8 +138,16 @@ PyObject* act_quant_per_token(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (!count(n, 1)) return nullptr;
     if (!plain(a[0], at::kBFloat16) || tensor(a[0]).dim() != 2) Py_RETURN_NONE;
     const Tensor& x = tensor(a[0]);
-    Tensor x8 = at::empty(x.sizes(), x.options().dtype(at::kChar)), s = at::empty({x.size(0)}, x.options().dtype(at::kFloat));
-    if (lq_act_quant_per_token(x.data_ptr(), x.size(0), x.size(1), (int8_t*)x8.data_ptr(), (float*)s.data_ptr(), stream()) != LQ_OK) Py_RETURN_NONE;
+    const int64_t M = x.size(0), K = x.size(1);
+    const at::TensorOptions opt = x.options();
+    const void* px = ptr(a[0]);
+    Tensor x8, s;
+    const int rc = without_gil([&] {
+        x8 = at::empty({M, K}, opt.dtype(at::kChar));
+        s = at::empty({M}, opt.dtype(at::kFloat));
+        return lq_act_quant_per_token(px, M, K, (int8_t*)x8.data_ptr(), (float*)s.data_ptr(), stream());
+    });
+    if (rc != LQ_OK) Py_RETURN_NONE;
     return pair(std::move(x8), std::move(s));
     END_HANDLE_TH_ERRORS
 }
@@ -123,8 +158,17 @@ PyObject* act_quant_per_tensor(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (!count(n, 1)) return nullptr;
     if (!plain(a[0], at::kBFloat16)) Py_RETURN_NONE;
     const Tensor& x = tensor(a[0]);
-    Tensor x8 = at::empty(x.sizes(), x.options().dtype(at::kChar)), c = at::empty({1}, x.options().dtype(at::kFloat));
-    if (lq_act_quant_per_tensor(x.data_ptr(), x.numel(), (float*)c.data_ptr(), (int8_t*)x8.data_ptr(), stream()) != LQ_OK) Py_RETURN_NONE;
+    const std::vector<int64_t> shape = x.sizes().vec();
+    const int64_t numel = x.numel();
+    const at::TensorOptions opt = x.options();
+    const void* px = ptr(a[0]);
+    Tensor x8, c;
+    const int rc = without_gil([&] {
+        x8 = at::empty(shape, opt.dtype(at::kChar));
+        c = at::empty({1}, opt.dtype(at::kFloat));
+        return lq_act_quant_per_tensor(px, numel, (float*)c.data_ptr(), (int8_t*)x8.data_ptr(), stream());
+    });
+    if (rc != LQ_OK) Py_RETURN_NONE;
     return pair(std::move(x8), std::move(c));
     END_HANDLE_TH_ERRORS
 }
@@ -137,9 +181,17 @@ PyObject* i8_dequant(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (!plain(a[0], at::kChar) || tensor(a[0]).dim() != 2 || !(rows ? plain(a[1], at::kBFloat16) : plain(a[2], at::kFloat))) Py_RETURN_NONE;
     const Tensor& c = tensor(a[0]);
     if (rows ? tensor(a[1]).numel() != c.size(0) : tensor(a[2]).numel() != 1) Py_RETURN_NONE;
-    Tensor y = at::empty(c.sizes(), c.options().dtype(at::kBFloat16));
-    if (lq_i8_dequant((const int8_t*)c.data_ptr(), rows ? ptr(a[1]) : nullptr, rows ? nullptr : (const float*)ptr(a[2]), c.size(0), c.size(1), y.data_ptr(), stream()) != LQ_OK)
-        Py_RETURN_NONE;
+    const int64_t M = c.size(0), N = c.size(1);
+    const at::TensorOptions opt = c.options().dtype(at::kBFloat16);
+    const int8_t* codes = (const int8_t*)ptr(a[0]);
+    const void* row_scales = rows ? ptr(a[1]) : nullptr;
+    const float* clampv = rows ? nullptr : (const float*)ptr(a[2]);
+    Tensor y;
+    const int rc = without_gil([&] {
+        y = at::empty({M, N}, opt);
+        return lq_i8_dequant(codes, row_scales, clampv, M, N, y.data_ptr(), stream());
+    });
+    if (rc != LQ_OK) Py_RETURN_NONE;
     return THPVariable_Wrap(std::move(y));
     END_HANDLE_TH_ERRORS
 }

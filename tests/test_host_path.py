@@ -1,6 +1,12 @@
 """The native host path (`_lqhost`) serves plain calls and leaves every other to the Python that checks, raises or handles it."""
+import os
+import subprocess
+import sys
+
 import pytest
 import torch
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 def test_what_is_not_plain_is_left_to_python():
@@ -68,3 +74,59 @@ def test_native_and_python_paths_agree_and_refuse_alike(M, monkeypatch):
                 assert u.dtype == v.dtype and u.shape == v.shape and torch.equal(u, v), n
             else:
                 assert u == v, (n, a, b)
+
+
+# A process in which the functions that `_lqhost` calls are stand-ins that wait and return a given status (loaded first and globally, so that
+# the module binds to them; `_lib`, which looks its functions up in the library itself, does not).
+_STAND_IN = """
+#include <unistd.h>
+static int status, wait_us;
+void stand_in(int s, int us) { status = s; wait_us = us; }
+#define F(name) int name() { usleep(wait_us); return status; }
+F(lq_gemm_a16w4_fwd) F(lq_gemm_a16w4_dgrad) F(lq_gemm_a8w8) F(lq_gemm_a8w8_module) F(lq_act_quant_per_token) F(lq_act_quant_per_tensor) F(lq_i8_dequant)
+"""
+_CALLS = """
+import ctypes, sys, threading, time
+lib = ctypes.CDLL(sys.argv[1], mode=ctypes.RTLD_GLOBAL)
+import torch
+from latentq_llm_b200 import _lib, ops
+x = torch.zeros(20, 128, dtype=torch.bfloat16, device="cuda")
+w, s = torch.zeros(128 * 64, dtype=torch.int8, device="cuda"), torch.ones(128, dtype=torch.bfloat16, device="cuda")
+x8, w8, one = torch.zeros(20, 128, dtype=torch.int8, device="cuda"), torch.zeros(64, 128, dtype=torch.int8, device="cuda"), torch.ones(1, device="cuda")
+calls = dict(fwd=lambda: ops.gemm_a16w4_fwd(x, w, s, s, None, 128, 128), dgrad=lambda: ops.gemm_a16w4_dgrad(x, w, s, s, 128, 128), a8w8=lambda: ops.gemm_a8w8(x8, w8),
+             module=lambda: ops.gemm_a8w8_module(x8, w8, one, 1.0, None, s[:64]), per_token=lambda: ops.act_quant_per_token(x),
+             per_tensor=lambda: ops.act_quant_per_tensor(x), dequant=lambda: ops.i8_dequant(x8, clampv=one))
+for f in calls.values():
+    f()
+"""
+
+
+def _run_with_stand_in(tmp_path, body):
+    c, so = tmp_path / "stand_in.c", tmp_path / "stand_in.so"
+    c.write_text(_STAND_IN)
+    subprocess.check_call(["gcc", "-shared", "-fPIC", "-o", str(so), str(c)])
+    r = subprocess.run([sys.executable, "-c", _CALLS + body, str(so)], cwd=ROOT, capture_output=True, text=True, timeout=180)
+    assert r.returncode == 0, r.stderr[-2000:]
+
+
+@pytest.mark.gpu
+def test_other_threads_run_during_a_native_call(tmp_path):
+    """A launch may wait for a full queue, an allocation for the device: what ends the wait may be another Python thread's work."""
+    _run_with_stand_in(tmp_path, """
+ticks, stop = [], threading.Event()
+def tick():
+    while not stop.wait(0.002):
+        ticks.append(time.perf_counter())
+t = threading.Thread(target=tick, daemon=True)
+t.start()
+lib.stand_in(0, 200000)
+for name, f in calls.items():
+    a = time.perf_counter()
+    f()
+    b = time.perf_counter()
+    assert b - a > 0.19, (name, b - a)                               # the native function was the one that ran
+    n = sum(a < u < b for u in ticks)
+    assert n > 10, (name, n)
+stop.set()
+t.join()
+""")
