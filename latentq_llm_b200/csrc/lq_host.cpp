@@ -1,7 +1,7 @@
 // Host path of the calls whose launches take a few microseconds: argument checks, output allocation and launch in native code.
 // Every function serves the plain case (CUDA tensors with storage, contiguous, of the expected types and sizes) and returns None for
-// anything else and for a call that the library refuses, without having done anything: the caller's Python, which repeats the call,
-// then raises or handles it as it does without this module.
+// anything else and for a call that the library refuses, without having launched anything: the caller's Python, which repeats the call,
+// then raises or handles it as it does without this module.  Errors behind a launch are raised here: the call is not made twice.
 #include <Python.h>
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAStream.h>
@@ -33,6 +33,15 @@ template <typename F> int without_gil(F f) {
     return f();
 }
 lq_stream_t stream() { return (lq_stream_t)c10::cuda::getCurrentCUDAStream().stream(); }
+// A status other than LQ_OK.  These three are decided before anything is launched; any other is raised as `_lib.check` raises it.
+PyObject* refused(const char* name, int rc) {
+    if (rc == LQ_EINVAL || rc == LQ_EUNSUPPORTED || rc == LQ_EWORKSPACE) Py_RETURN_NONE;
+    PyObject* lib = PyImport_ImportModule("latentq_llm_b200._lib");
+    PyObject* r = lib ? PyObject_CallMethod(lib, "check", "si", name, rc) : nullptr;
+    if (r) PyErr_Format(PyExc_RuntimeError, "%s failed with status %d", name, rc);
+    Py_XDECREF(r); Py_XDECREF(lib);
+    return nullptr;
+}
 bool count(Py_ssize_t n, Py_ssize_t want) {
     if (n == want) return true;
     PyErr_Format(PyExc_TypeError, "expected %zd arguments, got %zd", want, n);
@@ -69,7 +78,7 @@ PyObject* w4_gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
         return dgrad ? lq_gemm_a16w4_dgrad(px, w, s, z, y.data_ptr(), M, N, K, (int)group, ws, (size_t)nb, stream())
                      : lq_gemm_a16w4_fwd(px, w, s, z, bias, y.data_ptr(), M, N, K, (int)group, ws, (size_t)nb, stream());
     });
-    if (rc != LQ_OK) Py_RETURN_NONE;
+    if (rc != LQ_OK) return refused(dgrad ? "lq_gemm_a16w4_dgrad" : "lq_gemm_a16w4_fwd", rc);
     return THPVariable_Wrap(std::move(y));
     END_HANDLE_TH_ERRORS
 }
@@ -97,7 +106,7 @@ PyObject* a8w8_gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
         y = at::empty({M, N}, opt);
         return lq_gemm_a8w8(px, pw, row_scale, col_scale, (float)alpha, bias, y.data_ptr(), nullptr, M, N, K, ws, (size_t)nb, stream());
     });
-    if (rc != LQ_OK) Py_RETURN_NONE;
+    if (rc != LQ_OK) return refused("lq_gemm_a8w8", rc);
     return THPVariable_Wrap(std::move(y));
     END_HANDLE_TH_ERRORS
 }
@@ -127,7 +136,7 @@ PyObject* a8w8_module(PyObject*, PyObject* const* a, Py_ssize_t n) {
         y = at::empty({M, N}, opt);
         return lq_gemm_a8w8_module(px, pw, clampv, (float)alpha, bias, qscales, y.data_ptr(), M, N, K, ws, (size_t)nb, stream());
     });
-    if (rc != LQ_OK) Py_RETURN_NONE;
+    if (rc != LQ_OK) return refused("lq_gemm_a8w8_module", rc);
     return THPVariable_Wrap(std::move(y));
     END_HANDLE_TH_ERRORS
 }
@@ -147,7 +156,7 @@ PyObject* act_quant_per_token(PyObject*, PyObject* const* a, Py_ssize_t n) {
         s = at::empty({M}, opt.dtype(at::kFloat));
         return lq_act_quant_per_token(px, M, K, (int8_t*)x8.data_ptr(), (float*)s.data_ptr(), stream());
     });
-    if (rc != LQ_OK) Py_RETURN_NONE;
+    if (rc != LQ_OK) return refused("lq_act_quant_per_token", rc);
     return pair(std::move(x8), std::move(s));
     END_HANDLE_TH_ERRORS
 }
@@ -168,7 +177,7 @@ PyObject* act_quant_per_tensor(PyObject*, PyObject* const* a, Py_ssize_t n) {
         c = at::empty({1}, opt.dtype(at::kFloat));
         return lq_act_quant_per_tensor(px, numel, (float*)c.data_ptr(), (int8_t*)x8.data_ptr(), stream());
     });
-    if (rc != LQ_OK) Py_RETURN_NONE;
+    if (rc != LQ_OK) return refused("lq_act_quant_per_tensor", rc);
     return pair(std::move(x8), std::move(c));
     END_HANDLE_TH_ERRORS
 }
@@ -191,7 +200,7 @@ PyObject* i8_dequant(PyObject*, PyObject* const* a, Py_ssize_t n) {
         y = at::empty({M, N}, opt);
         return lq_i8_dequant(codes, row_scales, clampv, M, N, y.data_ptr(), stream());
     });
-    if (rc != LQ_OK) Py_RETURN_NONE;
+    if (rc != LQ_OK) return refused("lq_i8_dequant", rc);
     return THPVariable_Wrap(std::move(y));
     END_HANDLE_TH_ERRORS
 }

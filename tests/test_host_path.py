@@ -130,3 +130,24 @@ for name, f in calls.items():
 stop.set()
 t.join()
 """)
+
+
+@pytest.mark.gpu
+def test_an_error_behind_a_launch_is_raised_and_the_call_not_repeated(tmp_path):
+    """What the library refuses before it launches goes to the Python, which repeats the call; any other status is an error at once."""
+    _run_with_stand_in(tmp_path, """
+for status in (_lib.LQ_ECUDA, _lib.LQ_ETIMEOUT, -77):
+    lib.stand_in(status, 0)
+    for name, f in calls.items():
+        try:
+            f()
+        except _lib.LatentQError as e:
+            assert e.status == status and str(e).startswith("lq_"), (name, e)
+        else:
+            raise AssertionError((name, status))
+for status in (_lib.LQ_EINVAL, _lib.LQ_EUNSUPPORTED, _lib.LQ_EWORKSPACE):
+    lib.stand_in(status, 0)
+    y = {name: f() for name, f in calls.items()}
+    torch.cuda.synchronize()
+    assert all(float(y[k].float().abs().max()) == 0.0 for k in ("fwd", "dgrad", "a8w8", "module", "dequant")), status
+""")
