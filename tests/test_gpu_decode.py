@@ -165,3 +165,24 @@ def test_decode_attention_split_plans(ops, B, Hq, Hkv, hd, max_len):
         got = out.float().cpu().numpy().reshape(B, Hq, hd)
         assert np.abs(got - want).max() <= 2.0 ** -7 * np.abs(want).max()
         assert torch.equal(out, again)
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,hd,max_len,cluster", [
+    (1, 8, 8, 128, 1500, True), (1, 8, 8, 128, 2048, True), (1, 8, 8, 128, 4096, False), (1, 4, 4, 128, 8192, False), (1, 16, 16, 64, 4096, False), (1, 32, 8, 128, 4096, False),
+    (1, 32, 32, 128, 4096, True), (1, 32, 32, 128, 16384, False), (2, 32, 32, 128, 4096, True), (7, 16, 4, 128, 3072, False)])
+def test_decode_attention_long_contexts(ops, B, Hq, Hkv, hd, max_len, cluster):
+    """Few rows and a long context keep the tickets, whose splits are finer (a cluster has eight at most).  The plan shows in the scratch:
+    clusters leave it untouched.  Full caches, against 64-bit arithmetic."""
+    from latentq_llm_b200 import _lib
+    g = torch.Generator(device="cuda").manual_seed(max_len + Hq)
+    qkv = torch.randn(B, (Hq + 2 * Hkv) * hd, device="cuda", generator=g).to(torch.bfloat16)
+    kc, vc = (torch.randn(B, Hkv, max_len, hd, device="cuda", generator=g).to(torch.bfloat16) for _ in range(2))
+    pos, out = torch.full((B,), max_len - 1, device="cuda"), torch.empty(B, Hq * hd, dtype=torch.bfloat16, device="cuda")
+    ws = torch.zeros(_lib.lib.lq_decode_attention_workspace_bytes(B, Hq, hd, max_len), dtype=torch.uint8, device="cuda")
+    _lib.call("lq_decode_attention", qkv.data_ptr(), qkv.stride(0), kc.data_ptr(), vc.data_ptr(), pos.data_ptr(), out.data_ptr(), B, Hq, Hkv, hd, max_len, hd ** -0.5,
+              ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream)
+    assert bool(ws.any()) != cluster
+    q = qkv[:, :Hq * hd].double().view(B, Hkv, Hq // Hkv, hd)
+    p = torch.softmax(q @ kc.double().transpose(-1, -2) * hd ** -0.5, -1)
+    want = (p @ vc.double()).view(B, Hq * hd)
+    assert float((out.double() - want).abs().max()) <= 2.0 ** -7 * float(want.abs().max())
