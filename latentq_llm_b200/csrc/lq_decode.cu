@@ -558,19 +558,19 @@ static int attn_splits(int64_t B, int Hq, int64_t max_len) {
 // resident together.  With 65 or more rows the tickets' finer splits win where they are half as many again: 96 rows of 1500 keys 15.0 / 14.1 us,
 // 160 rows of 1500 24.0 / 21.9.  Cluster / tickets (us; 32 heads): 1 sequence of 100 keys 4.1 / 5.2, 520 6.1 / 7.4, 1500 9.3 / 10.3; 2: 4.6 / 5.5, 7.5 / 8.5, 11.0 /
 // 12.1; 4: 5.8 / 6.7, 9.5 / 9.9, 14.9 / 15.3; 8: 7.2 / 7.5, 12.9 / 13.4, 27.9 / 28.8.
-// What a cluster saves at the end is fixed, what it loses by its coarser splits grows with the context: `extra` keys per CTA, 17 to 23 ns each as a
-// chain of latencies.  Up to 24 of them per split the saving is the larger; up to 64 where so many CTAs stream that memory bounds both (at
-// 6.3 TB/s the chip takes 17 ns for a key of each of 27648 / hd splits).  Cluster / tickets (us, caches not in L2), heads (key heads) x head size: 8 x 128 2048 keys
-// 9.2 / 9.5, 3072 11.3 / 10.7, 8192 22.0 / 14.1, 32768 73 / 32; 16 x 128 2048 10.2 / 11.8, 4096 15.1 / 13.7; 16 x 64 2048 9.6 / 9.6, 4096 15.1 / 11.4; 32 (8) x 128
-// 3072 11.9 / 12.2, 8192 22.5 / 18.7; 32 x 128 4096 17.1 / 17.8, 8192 28.5 / 28.3, 16384 49.6 / 46.8; 56 x 128 16384 73.3 / 73.8; 112 (28) x 128, clusters of
-// four, 1500 14.0 / 13.7, 4096 27.5 / 24.8.
-static int attn_cluster(int64_t B, int Hq, int Hkv, int hd, int64_t max_len) {
+// What a cluster saves at the end is fixed; what it loses by its coarser splits grows with the context (`extra` keys per CTA, 17 to 23 ns each as
+// a chain of latencies), and it starts only when a whole cluster finds room beside the predecessor's last CTAs.  So the lines lie where they cross behind a
+// projection with weights from memory, in a chain.  Projection and attention, tickets / cluster (us; heads (key heads) x head size): 8 x 128 1000 keys 12.1 / 11.5,
+// 2048 13.2 / 15.0; 32 x 128 1500 19.6 / 18.7, 2048 20.0 / 20.8, 4096 24.9 / 27.2; 32 (8) x 128 1500 16.8 / 15.4, 3072 18.2 / 19.5; 7 x 8 x 128 1500 16.8 /
+// 15.6; 8 x 8 x 128 1000 15.1 / 16.0, 2048 20.1 / 23.3; 4 x 16 x 64 1000 14.5 / 12.5; clusters of four: 64 x 128 760 25.8 / 24.7, 1000 26.3 / 26.7.  Launched by itself the attention
+// would still gain from clusters up to about twice as many extra keys (32 x 128 3072 keys 15.0 / 14.0 us, from 16384 on 46.8 / 49.6; 8 x 128 8192 14.1 / 22.0).
+static int attn_cluster(int64_t B, int Hq, int hd, int64_t max_len) {
     const int64_t rows = B * Hq, sms = sm_count();
-    const int c = max_len >= 512 && rows * 16 <= 7 * sms ? 8 : max_len >= 192 && rows * 8 <= 7 * sms ? 4 : max_len > 64 && rows * 2 <= 4 * sms ? 2 : 0;
+    const int c = max_len >= 512 && rows * 32 <= (hd == 64 ? 14 : 13) * sms ? 8 : max_len >= 192 && rows * 8 <= 7 * sms ? 4 : max_len > 64 && rows * 2 <= 4 * sms ? 2 : 0;
     const int tickets = attn_splits(B, Hq, max_len);
     if (!c || (rows > 64 && 10 * c < 7 * tickets)) return 0;
     const int64_t extra = (max_len + c - 1) / c - (max_len + tickets - 1) / tickets;
-    return extra <= (B * Hkv * hd * c >= 27648 ? 64 : 24) * c ? c : 0;
+    return extra <= (c == 8 ? 128 : 96) ? c : 0;
 }
 
 size_t lq_decode_attention_workspace_bytes(int64_t B, int Hq, int hd, int64_t max_len) {
@@ -588,7 +588,7 @@ int lq_decode_attention(const void* q, int64_t q_row_stride, const void* k_cache
         return LQ_EUNSUPPORTED;
     if (B == 0) return LQ_OK;
     { int rc = ensure_device_for(q); if (rc) return rc; }
-    const int cluster = attn_cluster(B, Hq, Hkv, hd, max_len), splits = cluster ? cluster : attn_splits(B, Hq, max_len);
+    const int cluster = attn_cluster(B, Hq, hd, max_len), splits = cluster ? cluster : attn_splits(B, Hq, max_len);
     float* part = nullptr; unsigned int* tickets = nullptr;
     if (attn_splits(B, Hq, max_len) > 1) {              // (clusters leave it untouched)
         if (!workspace || workspace_bytes < lq_decode_attention_workspace_bytes(B, Hq, hd, max_len) || !al16p(workspace)) return LQ_EWORKSPACE;
