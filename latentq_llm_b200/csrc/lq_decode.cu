@@ -494,7 +494,7 @@ static inline bool al16p(const void* p) { return (reinterpret_cast<uintptr_t>(p)
 using namespace lq;
 
 template <int HD, bool PREFETCH>
-static cudaError_t launch_attn_cluster(cudaLaunchConfig_t cfg, const __nv_bfloat16* q, int q_row_stride, const __nv_bfloat16* k, const __nv_bfloat16* v, const long long* positions,
+static void launch_attn_cluster(cudaLaunchConfig_t cfg, const __nv_bfloat16* q, int q_row_stride, const __nv_bfloat16* k, const __nv_bfloat16* v, const long long* positions,
                                        __nv_bfloat16* out, int Hq, int Hkv, int max_len, float scale) {
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -502,7 +502,7 @@ static cudaError_t launch_attn_cluster(cudaLaunchConfig_t cfg, const __nv_bfloat
     attr[1].id = cudaLaunchAttributeClusterDimension;
     attr[1].val.clusterDim.x = 1; attr[1].val.clusterDim.y = cfg.gridDim.y; attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr; cfg.numAttrs = 2;
-    return cudaLaunchKernelEx(&cfg, k_decode_attn<HD, true, PREFETCH>, q, q_row_stride, k, v, positions, out, Hq, Hkv, max_len, scale, (float*)nullptr, (unsigned int*)nullptr);
+    cudaLaunchKernelEx(&cfg, k_decode_attn<HD, true, PREFETCH>, q, q_row_stride, k, v, positions, out, Hq, Hkv, max_len, scale, (float*)nullptr, (unsigned int*)nullptr);
 }
 
 extern "C" {
@@ -610,12 +610,11 @@ int lq_decode_attention(const void* q, int64_t q_row_stride, const void* k_cache
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = grid; cfg.blockDim = dim3(ATT_THREADS); cfg.stream = st;
         auto launch_cl = [&](auto fn) {
-            return fn(cfg, (const __nv_bfloat16*)q, (int)q_row_stride, (const __nv_bfloat16*)k_cache, (const __nv_bfloat16*)v_cache, (const long long*)positions,
+            fn(cfg, (const __nv_bfloat16*)q, (int)q_row_stride, (const __nv_bfloat16*)k_cache, (const __nv_bfloat16*)v_cache, (const long long*)positions,
                       (__nv_bfloat16*)out, Hq, Hkv, (int)max_len, scale);
         };
-        const cudaError_t e = hd == 128 ? (prefetch ? launch_cl(launch_attn_cluster<128, true>) : launch_cl(launch_attn_cluster<128, false>))
-                                        : (prefetch ? launch_cl(launch_attn_cluster<64, true>) : launch_cl(launch_attn_cluster<64, false>));
-        if (e != cudaSuccess) { set_cuda_error(e, "k_decode_attn (cluster)"); return LQ_ECUDA; }
+        hd == 128 ? (prefetch ? launch_cl(launch_attn_cluster<128, true>) : launch_cl(launch_attn_cluster<128, false>))
+                  : (prefetch ? launch_cl(launch_attn_cluster<64, true>) : launch_cl(launch_attn_cluster<64, false>));
     } else if (hd == 128) {
         prefetch ? launch(k_decode_attn<128, false, true>) : launch(k_decode_attn<128, false, false>);
     } else {
