@@ -212,4 +212,8 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_lqhost", nullptr, -1, methods, nu
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__lqhost() { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__lqhost() {
+    PyObject* m = PyModule_Create(&module);
+    if (m && PyModule_AddStringConstant(m, "torch_build", LQ_TORCH_BUILD) != 0) { Py_DECREF(m); return nullptr; }   // what it was compiled against
+    return m;
+}

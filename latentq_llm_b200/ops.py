@@ -8,9 +8,18 @@ import ctypes as C
 import torch
 
 from . import _lib as L
-from . import _lqhost as _host
+from .build import torch_build
 from ._lib import (CODEC_NONE, CODEC_THREEFOLD, CODEC_UNIFORM16, DITHER_EXPLICIT, DITHER_HASH,  # noqa: F401
                    DITHER_PHILOX, LQ_BF16, LQ_F32, RequantOpts)
+
+try:
+    from . import _lqhost as _host
+except ImportError as e:
+    raise ImportError("the native host path latentq_llm_b200._lqhost is missing or does not load: build it with "
+                      "`python -m latentq_llm_b200.build` (g++, against this torch and this Python)") from e
+if getattr(_host, "torch_build", None) != torch_build():
+    raise ImportError(f"{_host.__file__} was built for torch {getattr(_host, 'torch_build', '(unknown)')}, this is {torch_build()}: "
+                      "rebuild it with `python -m latentq_llm_b200.build`")
 
 
 _raw_stream, _current_device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice

@@ -151,3 +151,19 @@ for status in (_lib.LQ_EINVAL, _lib.LQ_EUNSUPPORTED, _lib.LQ_EWORKSPACE):
     torch.cuda.synchronize()
     assert all(float(y[k].float().abs().max()) == 0.0 for k in ("fwd", "dgrad", "a8w8", "module", "dequant")), status
 """)
+
+
+@pytest.mark.parametrize("how,says", [("sys.modules['latentq_llm_b200._lqhost'] = None", "missing or does not load"),
+                                      ("import types; m = types.ModuleType('latentq_llm_b200._lqhost'); m.__file__ = 'x.so'; sys.modules[m.__name__] = p._lqhost = m", "built for torch"),
+                                      ("import torch; from latentq_llm_b200 import _lqhost; _lqhost.torch_build = '2.0.0 0'", "built for torch 2.0.0 0")])
+def test_a_missing_or_foreign_module_is_refused_with_the_command_to_build_it(how, says):
+    """The module holds torch's inline accessors: under another torch it does not load, or reads wrong fields."""
+    r = subprocess.run([sys.executable, "-c", f"import sys, latentq_llm_b200 as p; {how}\nfrom latentq_llm_b200 import ops"], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 1 and says in r.stderr and "python -m latentq_llm_b200.build" in r.stderr.splitlines()[-1], r.stderr[-1000:]
+
+
+def test_another_torch_makes_the_module_stale(monkeypatch):
+    from latentq_llm_b200 import _lqhost, build
+    assert _lqhost.__file__ == build.HOST and not build._host_stale()
+    monkeypatch.setattr(torch, "__version__", "2.0.0")
+    assert build._host_stale()
