@@ -1101,10 +1101,10 @@ __device__ __forceinline__ uint32_t i8x2_scaled(uint32_t wx, uint32_t sel, float
     const __nv_bfloat162 v = __floats2bfloat162_rn(__fmul_rn(f.x, s), __fmul_rn(f.y, s));
     return *reinterpret_cast<const uint32_t*>(&v);
 }
-// row_magic: ceil(2^64 / words per row), the row of a word (below 2^32) by one multiply-high.  Words of 8 codes, so that a warp's 16-byte
+// row_magic: ceil(2^64 / words per row), the row of a word by one multiply-high (exact as long as words x words per row fit 64 bits).  Words of 8 codes, so that a warp's 16-byte
 // stores are one contiguous run, two in flight per thread: 2048 x 8192 12.4 -> 8.7 us (5.8 TB/s).
 __global__ void __launch_bounds__(256) k_i8_dequant(const uint2* __restrict__ codes, const __nv_bfloat16* __restrict__ row_scales,
-                                                    const float* __restrict__ clampv, uint32_t n_words, uint64_t row_magic, uint4* __restrict__ out) {
+                                                    const float* __restrict__ clampv, uint64_t n_words, uint64_t row_magic, uint4* __restrict__ out) {
     const float all = row_scales ? 0.0f : bf16r(__fmul_rn(bf16r(*clampv), 1.0f / 127.0f));
     const uint64_t step = (uint64_t)gridDim.x * 256u;
     auto scale_of = [&](uint64_t w) { return row_scales ? __bfloat162float(row_scales[__umul64hi(w, row_magic)]) : all; };
@@ -1474,11 +1474,11 @@ int lq_i8_dequant(const int8_t* codes, const void* row_scales, const float* clam
     { int rc_dev = ensure_device_for(codes); if (rc_dev) return rc_dev; }
     const int64_t n = rows * cols;
     const __nv_bfloat16* rs = reinterpret_cast<const __nv_bfloat16*>(row_scales);
-    if ((cols % 16) == 0 && n / 8 < ((int64_t)1 << 32) && aligned(codes, 16) && aligned(out, 16)) {
-        const uint64_t words_per_row = (uint64_t)cols / 8;                          // at least two
-        k_i8_dequant<<<grid_for(n / 16, 256, 8), 256, 0, LQ_ST(stream)>>>(reinterpret_cast<const uint2*>(codes), rs, clampv, (uint32_t)(n / 8),
+    const uint64_t words_per_row = (uint64_t)cols / 8;                              // at least two where they are used
+    if ((cols % 16) == 0 && (uint64_t)(n / 8) <= ~(uint64_t)0 / words_per_row && aligned(codes, 16) && aligned(out, 16))
+        k_i8_dequant<<<grid_for(n / 16, 256, 8), 256, 0, LQ_ST(stream)>>>(reinterpret_cast<const uint2*>(codes), rs, clampv, (uint64_t)(n / 8),
                                                                          (~(uint64_t)0) / words_per_row + 1, reinterpret_cast<uint4*>(out));
-    } else
+    else
         k_i8_dequant_any<<<grid_for(n, 256, 8), 256, 0, LQ_ST(stream)>>>(codes, rs, clampv, n, cols, reinterpret_cast<__nv_bfloat16*>(out));
     return check_launch("lq_i8_dequant");
 }

@@ -334,3 +334,29 @@ def test_token_tiles_between_the_multiples_of_32(monkeypatch, M, N, K):
     ref = x.double() @ w.t()
     assert float((out[0].double() - ref).norm() / ref.norm()) < 4e-3
     assert torch.equal(out[0], out[1]) and torch.equal(out[0], out[2])
+
+
+def test_i8_dequant_beyond_2_to_the_35_codes():
+    """There is no size from which the codes are converted one by one (8.6 times slower per code); the last rows take their own scales."""
+    from latentq_llm_b200 import ops
+    if torch.cuda.mem_get_info()[0] < 125 << 30:
+        pytest.skip("needs 103 GB on the device")
+    per_code = []
+    for rows, cols in ((1 << 15, 32784), ((1 << 20) + 33, 32784)):
+        c = torch.full((rows, cols), 3, dtype=torch.int8, device="cuda")
+        s = (torch.arange(rows, device="cuda") % 251 + 1).to(torch.bfloat16)
+        y, ms = None, []
+        for _ in range(4):
+            y = None                                                # its memory serves the next call
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record()
+            y = ops.i8_dequant(c, row_scales=s)
+            b.record()
+            b.synchronize()
+            ms.append(a.elapsed_time(b))
+        per_code.append(min(ms) / c.numel())
+        for r in (0, 1, rows // 2, rows - 2, rows - 1):
+            assert torch.equal(y[r], c[r].to(torch.bfloat16) * s[r])
+        del c, y
+        torch.cuda.empty_cache()
+    assert per_code[1] < 3 * per_code[0], per_code
