@@ -167,3 +167,39 @@ def test_another_torch_makes_the_module_stale(monkeypatch):
     assert _lqhost.__file__ == build.HOST and not build._host_stale()
     monkeypatch.setattr(torch, "__version__", "2.0.0")
     assert build._host_stale()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M", [1, 17, 300])
+def test_plain_calls_are_served_by_the_native_functions(M, monkeypatch):
+    """Each plain call is answered by its native function, not by the Python behind it; what that refuses too raises."""
+    from latentq_llm_b200 import ops
+    N, K = 192, 256
+    x, dy = (torch.randn(M, c, device="cuda").to(torch.bfloat16) for c in (K, N))
+    w, s = torch.zeros(N * K // 2, dtype=torch.int8, device="cuda"), torch.ones(N * K // 128, 1, dtype=torch.bfloat16, device="cuda")
+    x8, w8, qs, one = torch.zeros(M, K, dtype=torch.int8, device="cuda"), torch.zeros(N, K, dtype=torch.int8, device="cuda"), s[:N], torch.ones(1, device="cuda")
+    bias = qs.view(-1)
+    served = []
+
+    class Recorder:
+        def __getattr__(self, name):
+            def f(*a, _native=getattr(native, name)):
+                r = _native(*a)
+                served.append((name, r is not None))
+                return r
+            return f
+    native = ops._host
+    monkeypatch.setattr(ops, "_host", Recorder())
+    for name, call in (("w4_gemm", lambda: ops.gemm_a16w4_fwd(x, w, s, s, bias, N, K)), ("w4_gemm", lambda: ops.gemm_a16w4_dgrad(dy, w, s, s, N, K)),
+                       ("a8w8_gemm", lambda: ops.gemm_a8w8(x8, w8, torch.ones(M, device="cuda"), None, 1.0, bias)), ("a8w8_module", lambda: ops.gemm_a8w8_module(x8, w8, one, 1.0, bias, qs)),
+                       ("act_quant_per_token", lambda: ops.act_quant_per_token(x)), ("act_quant_per_tensor", lambda: ops.act_quant_per_tensor(x)),
+                       ("i8_dequant", lambda: ops.i8_dequant(w8, row_scales=qs)), ("i8_dequant", lambda: ops.i8_dequant(x8, clampv=one))):
+        served.clear()
+        assert call() is not None and served == [(name, True)], (name, served)
+    for call in (lambda: ops.gemm_a16w4_fwd(x.float(), w, s, s, None, N, K), lambda: ops.gemm_a16w4_fwd(x, w, s, s, None, N, K, group=96),
+                 lambda: ops.gemm_a8w8(x8, w8[:, :128]), lambda: ops.gemm_a8w8_module(x8, w8, None, 1.0, bias[:-1], qs), lambda: ops.act_quant_per_token(x[:, :100]),
+                 lambda: ops.act_quant_per_tensor(x.half()), lambda: ops.i8_dequant(w8, row_scales=qs[:-1])):
+        served.clear()
+        with pytest.raises(Exception):
+            call()
+        assert not any(ok for _, ok in served)
