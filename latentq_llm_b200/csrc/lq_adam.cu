@@ -144,14 +144,14 @@ __global__ void __launch_bounds__(256) k_adam_quant(const AdamParams p) {
 //   states    encoded with a quotient from a two-term reciprocal and one residual correction (Markstein's theorem, see div_by), as is
 //             the division of the block's range by 255.
 //   fp32      two elements per instruction (fma / mul / add .f32x2) for int4 codes: 83 -> 74 instructions per weight, 157 -> 149 us for 4096 x
-//             11008.  The int8 kernel has no registers left for the pairs (64, two teams of 256 threads): 172 -> 178 us, so it keeps
+//             11008.  The int8 kernel has no registers left for the pairs (64, two teams of 256 threads): 11008 x 4096 172 -> 178 us, so it keeps
 //             one element per instruction.
 //   requantize  everything after Z = w/scale + zero from the table of the requantize fast path (int4: a byte per bf16 pattern,
 //             |Z| < 64; int8: two bytes, |Z| < 256); the kernel keeps the two runs of it that can be looked up and puts its other
 //             tables into the gap between them.
 // int4 codes: 50 KB and 256 threads per CTA, three CTAs per SM (four would fit, but at 64 registers the loop spills: 176 instead of
 // 157 us for 4096 x 11008); int8 codes: 100 KB, so two teams of 256 threads share the tables of a CTA and two CTAs fit.
-// Measured, a whole optimizer step of one 4096 x 11008 weight: int4 268 -> 149 us (2.4 TB/s), int8 586 -> 172 us.
+// Measured, a whole optimizer step of one 4096 x 11008 weight: int4 268 -> 149 us (2.4 TB/s), int8 586 -> 177 us.
 // A word whose Z leaves the table's range or is not finite, and every word of a block whose moments are not all finite, is
 // recomputed with IEEE operations (adam_word_generic).
 // ---------------------------------------------------------------------------------------------------------------

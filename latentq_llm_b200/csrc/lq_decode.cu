@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(ATT_THREADS) k_decode_attn(const __nv_bfloat16
 #pragma unroll
     for (int d = 0; d < D; ++d) acc[d] = 0.0f;
     // KPI keys per slot in flight: the K and V rows of all of them are requested before any arithmetic (the kernel is a
-    // chain of memory latencies otherwise; a split covers about 64 keys, i.e. one such round per slot).  A key beyond the
+    // chain of memory latencies otherwise; a ticket's split covers about 64 keys, one such round per slot, a cluster's up to a few hundred).  A key beyond the
     // range reads key j1-1 again and gets weight zero.
     for (int j = j0 + slot; j < j1; j += KPI * ATT_SLOTS) {
         uint4 kq[KPI][D / 8], vq[KPI][D / 8];

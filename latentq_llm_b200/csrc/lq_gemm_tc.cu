@@ -1159,7 +1159,7 @@ static int plan_splits(int tiles, int kb_total, int sms) {
 //   Where it errs: some grad-inputs of 45 .. 63 tokens take two tiles of 32, up to 0.7 us (6 %) slower than one of 64 (4352 x 1152 at 50 tokens
 // 12.5 / 11.7); a smaller price for the partial sums mends them and loses 4 to 11 % at 280 to 700 tokens.
 //   48, 80 and 112 tokens exist in the kernel of two k-blocks per stage, whose MMAs and token copies they shorten: 11008 rows at 40 / 72 / 100 tokens
-// 17.3 / 18.6 / 20.2 -> 16.4 / 17.9 / 19.3 us, 8192 x 2048 at 200 14.5 -> 13.5.  Taken where modelled at least 2 % shorter (below that the model's
+// 17.2 / 18.4 / 20.2 -> 16.3 / 17.8 / 19.3 us, 8192 x 2048 at 200 14.5 -> 13.4.  Taken where modelled at least 2 % shorter (below that the model's
 // choice between them and a split was up to 10 % wrong: 2048 x 2048 at 97 tokens 10.8 / 11.8).
 //   A forward whose group parameters are not staged has its own column: its loads of them bound the narrow tiles, so that
 // halving the width does not halve anything.  With the staged kernel's column 4096 -> 4096 with groups of 64 took 32-token tiles at 128
