@@ -565,13 +565,15 @@ static int attn_splits(int64_t B, int Hq, int64_t max_len) {
 // 15.6; 8 x 8 x 128 1000 15.1 / 16.0, 2048 20.1 / 23.3; 4 x 16 x 64 1000 14.5 / 12.5; clusters of four: 64 x 128 760 25.8 / 24.7, 1000 26.3 / 26.7.  Launched by itself the attention
 // would still gain from clusters up to about twice as many extra keys (32 x 128 3072 keys 15.0 / 14.0 us, from 16384 on 46.8 / 49.6; 8 x 128 8192 14.1 / 22.0), and so do
 // caches that are partly filled (70 %: 32 x 128 2048 keys 19.6 / 18.7, 16 x 128 16.0 / 14.8): the line is drawn a little beyond the crossing of full ones.
+// Above 60 rows of 128-wide heads eight splits leave no room beside the projection: they lose from 24 extra keys on (1700 keys), and up to there whole
+// decode steps differ by 2 % either way (2 x 32 heads 1500 keys 102.5 / 100.9 us, 4 x 16 82.1 / 84.0).
 static int attn_cluster(int64_t B, int Hq, int hd, int64_t max_len) {
     const int64_t rows = B * Hq, sms = sm_count();
-    const int c = max_len >= 512 && rows * 32 <= (hd == 64 ? 14 : 13) * sms ? 8 : max_len >= 192 && rows * 8 <= 7 * sms ? 4 : max_len > 64 && rows * 2 <= 4 * sms ? 2 : 0;
+    const int c = max_len >= 512 && rows * 16 <= 7 * sms ? 8 : max_len >= 192 && rows * 8 <= 7 * sms ? 4 : max_len > 64 && rows * 2 <= 4 * sms ? 2 : 0;
     const int tickets = attn_splits(B, Hq, max_len);
     if (!c || (rows > 64 && 10 * c < 7 * tickets)) return 0;
     const int64_t extra = (max_len + c - 1) / c - (max_len + tickets - 1) / tickets;
-    return extra <= (c == 8 ? 144 : 96) ? c : 0;
+    return extra <= (c < 8 ? 96 : hd == 64 || rows * 32 <= 13 * sms ? 144 : 24) ? c : 0;
 }
 
 size_t lq_decode_attention_workspace_bytes(int64_t B, int Hq, int hd, int64_t max_len) {

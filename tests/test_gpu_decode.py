@@ -169,7 +169,7 @@ def test_decode_attention_split_plans(ops, B, Hq, Hkv, hd, max_len):
 
 @pytest.mark.parametrize("B,Hq,Hkv,hd,max_len,cluster", [
     (1, 8, 8, 128, 1500, True), (1, 8, 8, 128, 2048, False), (1, 4, 4, 128, 8192, False), (1, 16, 16, 64, 4096, False), (1, 32, 8, 128, 3072, False),
-    (1, 32, 32, 128, 1500, True), (1, 32, 32, 128, 16384, False), (2, 32, 32, 128, 1500, False), (4, 16, 16, 64, 1000, True), (7, 8, 8, 128, 1800, True), (8, 8, 8, 128, 1000, False),
+    (1, 32, 32, 128, 1500, True), (1, 32, 32, 128, 16384, False), (2, 32, 32, 128, 1500, True), (4, 16, 16, 64, 4000, True), (7, 8, 8, 128, 1800, True), (8, 8, 8, 128, 2048, False),
     (2, 32, 32, 128, 600, True), (7, 16, 4, 128, 3072, False)])
 def test_decode_attention_long_contexts(ops, B, Hq, Hkv, hd, max_len, cluster):
     """Few rows and a long context keep the tickets, whose splits are finer (a cluster has eight at most).  The plan shows in the scratch:
