@@ -69,6 +69,25 @@ def test_rope_kv_store(ops, B, Hq, Hkv, hd, hf):
         assert not kcn[b][:, mask].any() and not vcn[b][:, mask].any()     # nothing else was written
 
 
+@pytest.mark.parametrize("hf", [True, False])
+@pytest.mark.parametrize("B,P,Hq,Hkv,hd", [(2, 200, 32, 32, 128), (16, 1, 64, 16, 64), (3, 67, 5, 5, 16), (1, 1100, 2, 1, 512), (7, 41, 6, 3, 40)])
+def test_rope_kv_store_of_many_tokens_equals_the_calls_of_single_tokens(ops, B, P, Hq, Hkv, hd, hf):
+    """From 1536 (token, head) pairs on a thread serves several heads; a token by itself takes the kernel of one rotation pair per thread.
+    The same bits: head sets that do not divide the heads, head sizes that leave threads idle, positions beyond the cache."""
+    g = torch.Generator(device="cuda").manual_seed(B + P)
+    qkv = torch.randn(B * P, (Hq + 2 * Hkv) * hd, device="cuda", generator=g).to(torch.bfloat16)
+    pos = torch.arange(P, device="cuda").repeat(B) + 3
+    pos[-1] = P + 40
+    inv_freq = 1.0 / (10000.0 ** (torch.arange(0, hd, 2, dtype=torch.float32, device="cuda") / hd))
+    caches = [torch.zeros(B, Hkv, P + 8, hd, dtype=torch.bfloat16, device="cuda") for _ in range(4)]
+    want = qkv.clone()
+    for m in range(B * P):
+        b = m // P
+        ops.rope_kv_store(want[m:m + 1], pos[m:m + 1], inv_freq, caches[0][b:b + 1], caches[1][b:b + 1], Hq, Hkv, hd, hf_rounding=hf)
+    ops.rope_kv_store(qkv, pos, inv_freq, caches[2], caches[3], Hq, Hkv, hd, tokens_per_seq=P, hf_rounding=hf)
+    assert torch.equal(qkv, want) and torch.equal(caches[2], caches[0]) and torch.equal(caches[3], caches[1])
+
+
 @pytest.mark.parametrize("B,Hq,Hkv,hd,max_len", [(1, 32, 32, 128, 1024), (16, 32, 32, 128, 640), (3, 8, 2, 64, 200), (64, 8, 8, 128, 96)])
 def test_decode_attention(ops, B, Hq, Hkv, hd, max_len):
     rng = np.random.default_rng(B * 3 + hd)
