@@ -94,8 +94,10 @@ class FusedLlamaGreedyDecoder:
     eight launches per layer at decode-sized batches, where silu(gate) * up is the epilogue of the gate|up launch, nine
     otherwise (the reference's fusion list: PTQ/quant/fused_attn.py:164-204 fused QKV, :8-58 RoPE,
     PTQ/quant/fused_mlp.py:84-168 gate/up with the silu epilogue, PTQ/quant/triton_norm.py:7-39 RMSNorm), captured
-    once as a CUDA graph and replayed per token.  The prompt is prefilled through the model's own modules into the
-    same static KV cache.  `hf_rounding=True` rounds intermediates like the eager modules' bf16 tensor ops."""
+    once as a CUDA graph and replayed per token.  The prompt goes through the same kernels at its own token count (fused
+    q|k|v and gate|up GEMMs, SDPA for its attention) into the same static KV cache, and only its last tokens through the
+    head; a model whose prompt differs from that in more than rounding goes through its own modules
+    (`_kernels_serve_prompts`).  `hf_rounding=True` rounds intermediates like the eager modules' bf16 tensor ops."""
 
     def __init__(self, model, batch: int, max_len: int, hf_rounding: bool = True):
         from transformers import StaticCache
@@ -140,6 +142,19 @@ class FusedLlamaGreedyDecoder:
         self.pos = torch.zeros((batch,), dtype=torch.long, device=dev)
         self.logits = None
         self.graph = None
+        self.prompt_kernels = self._kernels_serve_prompts()
+        if self.prompt_kernels:           # the modules would allocate the cache at their first call
+            self.cache.early_initialization(batch, self.Hkv, self.hd, torch.bfloat16, dev)
+
+    def _kernels_serve_prompts(self) -> bool:
+        """What the step's kernels compute is what the modules compute for a prompt, to rounding: frequencies that do not
+        depend on its length and need no scaling of the attention, keys kept for the whole length, silu, no further norms."""
+        cfg, rope = self.model.config, self.model.model.rotary_emb
+        attn = self.model.model.layers[0].self_attn
+        return (getattr(rope, "rope_type", "default") in ("default", "linear", "llama3") and getattr(rope, "attention_scaling", 1.0) == 1.0
+                and not any(getattr(l, "is_sliding", False) for l in self.cache.layers) and getattr(cfg, "hidden_act", "silu") == "silu"
+                and not hasattr(attn, "q_norm") and getattr(attn, "scaling", self.hd ** -0.5) == self.hd ** -0.5
+                and self.model.model.embed_tokens.weight.dtype == torch.bfloat16 and self.model.lm_head.bias is None)
 
     def _step(self):
         from . import ops
@@ -194,9 +209,33 @@ class FusedLlamaGreedyDecoder:
         self.tok.copy_(first); self.pos.fill_(p)
         self.h.copy_(torch.nn.functional.embedding(self.tok, self.model.model.embed_tokens.weight))
 
+    def _prompt_step(self, prompt):
+        """The layers over all tokens of the prompt; logits of the last token of every sequence."""
+        from . import ops
+        B, P = prompt.shape
+        D, I, Hq, Hkv, hd = self.D, self.I, self.Hq, self.Hkv, self.hd
+        pos = torch.arange(P, device=self.device).repeat(B)
+        h = torch.nn.functional.embedding(prompt.reshape(-1), self.model.model.embed_tokens.weight)
+        delta = None
+        for li, L in enumerate(self.layers):
+            kc, vc = self.cache.layers[li].keys, self.cache.layers[li].values
+            qkv = ops.gemm_a16w4_fwd(ops.add_rmsnorm(h, delta, L["ln1"], self.eps), *L["qkv"], None, (Hq + 2 * Hkv) * hd, D)
+            ops.rope_kv_store(qkv, pos, self.inv_freq, kc, vc, Hq, Hkv, hd, tokens_per_seq=P)
+            q = qkv.view(B, P, -1, hd)[:, :, :Hq].transpose(1, 2)
+            att = torch.nn.functional.scaled_dot_product_attention(q, kc[:, :, :P], vc[:, :, :P], is_causal=True, enable_gqa=Hq != Hkv)
+            o = ops.gemm_a16w4_fwd(att.transpose(1, 2).reshape(B * P, Hq * hd), *L["o"], None, D, Hq * hd)
+            act = ops.gemm_a16w4_fwd_silu(ops.add_rmsnorm(h, o, L["ln2"], self.eps), *L["gu"], I, D)
+            delta = ops.gemm_a16w4_fwd(act, *L["down"], None, D, I)
+        last = [t.view(B, P, D)[:, -1].contiguous() for t in (h, delta)]
+        xn = ops.add_rmsnorm(*last, self.model.model.norm.weight.detach(), self.eps)
+        return torch.nn.functional.linear(xn, self.model.lm_head.weight)
+
     @torch.no_grad()
     def _prefill(self, prompt):
         p = prompt.shape[1]
+        if self.prompt_kernels:
+            with sdpa_kernel(_SDPA):
+                return self._prompt_step(prompt).argmax(-1)
         self.cache.reset()
         with sdpa_kernel(_SDPA):
             out = self.model(input_ids=prompt, past_key_values=self.cache,
