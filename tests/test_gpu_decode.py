@@ -206,3 +206,20 @@ def test_decode_attention_long_contexts(ops, B, Hq, Hkv, hd, max_len, cluster):
     p = torch.softmax(q @ kc.double().transpose(-1, -2) * hd ** -0.5, -1)
     want = (p @ vc.double()).view(B, Hq * hd)
     assert float((out.double() - want).abs().max()) <= 2.0 ** -7 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("B,V,D", [(2, 16384, 64), (18, 16392, 8), (3, 100008, 4096), (40, 98304, 264)])
+def test_argmax_of_a_large_vocabulary_by_clusters(ops, B, V, D):
+    """Eight CTAs per row from 16384 logits on: maxima in the first and last place of a CTA's share, ties across shares, a NaN behind the maximum."""
+    logits = torch.randn(B, V, device="cuda", generator=torch.Generator(device="cuda").manual_seed(V)).to(torch.bfloat16)
+    share = (V // 8 + 7) // 8 * 8
+    logits[0, share - 1] = logits[0, share] = logits[0, V - 1] = 50.0
+    logits[1, 7 * share] = 50.0
+    if B > 2:
+        logits[2, 0], logits[2, V - 1] = 50.0, float("nan")
+    embed = torch.randn(V, D, device="cuda").to(torch.bfloat16)
+    tok, pos, h = torch.zeros(B, dtype=torch.long, device="cuda"), torch.arange(B, device="cuda"), torch.zeros(B, D, dtype=torch.bfloat16, device="cuda")
+    want = logits.float().argmax(-1)
+    assert want[:2].tolist() == [share - 1, 7 * share]
+    ops.argmax_embed(logits, tok, pos, embed, h)
+    assert torch.equal(tok, want) and torch.equal(pos, torch.arange(B, device="cuda") + 1) and torch.equal(h, embed[want])
