@@ -364,6 +364,9 @@ LQ_API int lq_gemm_a16w4_fwd_silu(const void* x, const int8_t* qweight, const vo
  * h[b, 0..D) = embed[tok[b], 0..D) when embed is not NULL (D a multiple of 8, both 16-byte aligned). */
 LQ_API int lq_argmax_embed(const void* logits, int64_t logits_stride, int64_t B, int64_t V, const void* embed, int64_t D,
                            int64_t* tok, int64_t* positions, void* h, lq_stream_t stream);
+/* y[M, N] = x[M, K] . w[N, K]^T, all bf16 row-major, fp32 sums: the head of a decode step (HF's lm_head in the loop that generate.py:150-190 drives).
+ * M <= 8, K = 2048 or 4096, x and w 16-byte aligned; other shapes return LQ_EUNSUPPORTED. */
+LQ_API int lq_linear_rows(const void* x, const void* w, void* y, int64_t M, int64_t N, int64_t K, lq_stream_t stream);
 /* act[M, I] = silu(gate_up[M, 0:I]) * gate_up[M, I:2I] (epilogue of PTQ/quant/fused_mlp.py:84-168; LlamaMLP). */
 LQ_API int lq_silu_mul(const void* gate_up, void* act, int64_t M, int64_t I, int hf_rounding, lq_stream_t stream);
 

@@ -602,6 +602,70 @@ k_argmax_embed_cluster(const __nv_bfloat16* __restrict__ logits, int64_t logits_
     att_cluster_sync();                               // the others' shared memory has been read
 }
 
+// ---------------------------------------------------------------------------------------------
+// y[M, N] = x[M, K] . W[N, K]^T in bf16 for up to 8 tokens: the head of a decode step, a stream of W.  One CTA of 16 warps per SM walks over blocks of 16 rows,
+// and the warps share K, so that a row is read in one piece.  (A warp with 16 rows of its own over the whole of K needs no sums between warps, but keeps
+// 32000 rows open at a time, 64 bytes each: 4.95 TB/s.)  A lane loads 16 bytes of its two rows per 32 k, a block of rows ahead of the arithmetic (128 KB in
+// flight per SM at K = 4096); they are the A fragments of two mma.sync as they lie, the tokens' 16 bytes at the same k the B fragments, because a contraction
+// does not care which k meet in which lane.  32000 x 4096 in a chain: 38.7 us for one or two tokens (6.78 TB/s), 39.9 for eight, against 45 .. 47 of the
+// library and a launch gap before it; 50272 x 2048 31.4 / 36.  (With two groups of tokens 16 tokens took 45.0 / 44.3: the library's.)
+// ---------------------------------------------------------------------------------------------
+constexpr int LR_WARPS = 16;
+__device__ __forceinline__ void lr_mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// NS: steps of 32 k per warp and block (K = 512 NS)
+template <int NS>
+__global__ void __launch_bounds__(LR_WARPS * 32, 1) k_linear_rows(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y, int M, int N) {
+    constexpr int VECS = 64 * NS, X_STRIDE = VECS + 4;  // 16-byte vectors of a row; token rows 64 bytes apart modulo 128, so that fragment loads are free of bank conflicts
+    extern __shared__ __align__(128) uint4 lr_x[];                                   // [M][X_STRIDE]
+    __shared__ float red[2][LR_WARPS][128];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const int n_blocks = (N + 15) / 16;
+    const uint4* base = reinterpret_cast<const uint4*>(w) + warp * (4 * NS) + t;
+    auto row = [&](int b, int r) { return base + (size_t)min(b * 16 + r, N - 1) * VECS; };    // clamped loads, guarded stores
+    uint4 qa[NS], qb[NS];
+    {
+        const uint4 *wa = row(blockIdx.x, g), *wb = row(blockIdx.x, g + 8);
+#pragma unroll
+        for (int u = 0; u < NS; ++u) { qa[u] = __ldg(wa + u * 4); qb[u] = __ldg(wb + u * 4); }
+    }
+    pdl_launch_dependents();
+    pdl_wait();                                       // the tokens are the predecessor's output
+    for (int m = 0; m < M; ++m)
+        for (int i = tid; i < VECS; i += LR_WARPS * 32) lr_x[m * X_STRIDE + i] = reinterpret_cast<const uint4*>(x)[(size_t)m * VECS + i];
+    __syncthreads();
+    const uint4* xr = lr_x + min(g, M - 1) * X_STRIDE + warp * (4 * NS) + t;          // a token that does not exist reads the last: its results are dropped
+    int buf = 0;
+    for (int blk = blockIdx.x; blk < n_blocks; blk += gridDim.x, buf ^= 1) {
+        const bool next = blk + (int)gridDim.x < n_blocks;
+        const uint4 *na = next ? row(blk + gridDim.x, g) : nullptr, *nb = next ? row(blk + gridDim.x, g + 8) : nullptr;
+        float acc[2][4] = {};
+#pragma unroll
+        for (int u = 0; u < NS; ++u) {
+            const uint4 a = qa[u], b = qb[u];
+            if (next) { qa[u] = __ldg(na + u * 4); qb[u] = __ldg(nb + u * 4); }
+            const uint4 f = xr[u * 4];
+            lr_mma(acc[0], a.x, b.x, a.y, b.y, f.x, f.y);
+            lr_mma(acc[1], a.z, b.z, a.w, b.w, f.z, f.w);
+        }
+        *reinterpret_cast<float4*>(&red[buf][warp][lane * 4]) = make_float4(acc[0][0] + acc[1][0], acc[0][1] + acc[1][1], acc[0][2] + acc[1][2], acc[0][3] + acc[1][3]);
+        __syncthreads();                              // one barrier per block: the other buffer is rewritten only after the next
+        if (tid < 128) {                              // d0,d1 = (row g, tokens 2t, 2t+1); d2,d3 = (row g+8, same tokens)
+            const int ln = tid >> 2, i = tid & 3, tok = 2 * (ln & 3) + (i & 1), r = blk * 16 + (ln >> 2) + (i >= 2 ? 8 : 0);
+            if (r < N && tok < M) {
+                float v[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) v[k] = red[buf][k][tid];
+#pragma unroll
+                for (int k = 4; k < LR_WARPS; ++k) v[k & 3] += red[buf][k][tid];
+                y[(size_t)tok * N + r] = __float2bfloat16_rn((v[0] + v[1]) + (v[2] + v[3]));
+            }
+        }
+    }
+}
+
 static inline bool al16p(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 }  // namespace lq
@@ -618,6 +682,24 @@ static void launch_attn_cluster(cudaLaunchConfig_t cfg, const __nv_bfloat16* q, 
     attr[1].val.clusterDim.x = 1; attr[1].val.clusterDim.y = cfg.gridDim.y; attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr; cfg.numAttrs = 2;
     cudaLaunchKernelEx(&cfg, k_decode_attn<HD, true>, q, q_row_stride, k, v, positions, out, Hq, Hkv, max_len, scale, (float*)nullptr, (unsigned int*)nullptr, prefetch);
+}
+
+template <int NS>
+static int launch_linear_rows(const void* x, const void* w, void* y, int64_t M, int64_t N, cudaStream_t st) {
+    static bool attr_done[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) return LQ_EUNSUPPORTED;
+    constexpr int row = (64 * NS + 4) * 16;                  // bytes of a staged token
+    if (!attr_done[dev]) {
+        cudaError_t e = cudaFuncSetAttribute(k_linear_rows<NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * row);
+        if (e != cudaSuccess) { set_cuda_error(e, "cudaFuncSetAttribute(k_linear_rows)"); return LQ_ECUDA; }
+        attr_done[dev] = true;
+    }
+    const int64_t blocks = (N + 15) / 16;
+    launch_pdl(k_linear_rows<NS>, dim3((unsigned)(blocks < sm_count() ? blocks : sm_count())), (unsigned)(LR_WARPS * 32), (size_t)M * row, st, (const __nv_bfloat16*)x,
+               (const __nv_bfloat16*)w, (__nv_bfloat16*)y, (int)M, (int)N);
+    return check_launch("k_linear_rows");
 }
 
 extern "C" {
@@ -768,6 +850,14 @@ int lq_argmax_embed(const void* logits, int64_t logits_stride, int64_t B, int64_
                logits_stride, (int)V, vec, (const __nv_bfloat16*)embed, (int)D, (long long*)tok, (long long*)positions,
                (__nv_bfloat16*)h);
     return check_launch("k_argmax_embed");
+}
+
+int lq_linear_rows(const void* x, const void* w, void* y, int64_t M, int64_t N, int64_t K, lq_stream_t stream) {
+    if (!x || !w || !y || !al16p(x) || !al16p(w)) return LQ_EINVAL;
+    if (M < 0 || M > 8 || N < 1 || N >= (1ll << 30) || (K != 2048 && K != 4096)) return LQ_EUNSUPPORTED;
+    if (M == 0) return LQ_OK;
+    { int rc = ensure_device_for(x); if (rc) return rc; }
+    return K == 2048 ? launch_linear_rows<4>(x, w, y, M, N, (cudaStream_t)stream) : launch_linear_rows<8>(x, w, y, M, N, (cudaStream_t)stream);
 }
 
 int lq_silu_mul(const void* gate_up, void* act, int64_t M, int64_t I, int hf_rounding, lq_stream_t stream) {

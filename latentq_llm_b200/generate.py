@@ -201,7 +201,7 @@ class FusedLlamaGreedyDecoder:
             ops.gemm_a16w4_fwd(self.act, *L["down"], None, D, I, out=self.tmp)
             delta = self.tmp
         ops.add_rmsnorm(h, delta, self.model.model.norm.weight.detach(), self.eps, out=self.xn, hf_rounding=self.hf)
-        self.logits = torch.nn.functional.linear(self.xn, self.model.lm_head.weight)
+        self.logits = ops.linear_rows(self.xn, self.model.lm_head.weight.detach())
         # argmax, position += 1 and the next step's embedding row in one launch
         ops.argmax_embed(self.logits, self.tok, self.pos, self.model.model.embed_tokens.weight.detach(), self.h)
 
@@ -228,7 +228,7 @@ class FusedLlamaGreedyDecoder:
             delta = ops.gemm_a16w4_fwd(act, *L["down"], None, D, I)
         last = [t.view(B, P, D)[:, -1].contiguous() for t in (h, delta)]
         xn = ops.add_rmsnorm(*last, self.model.model.norm.weight.detach(), self.eps)
-        return torch.nn.functional.linear(xn, self.model.lm_head.weight)
+        return ops.linear_rows(xn, self.model.lm_head.weight.detach())
 
     @torch.no_grad()
     def _prefill(self, prompt):

@@ -566,6 +566,22 @@ def gemm_a16w4_fwd_qkv_rope(x, qweight, scales, zeros, positions, inv_freq, k_ca
     return y
 
 
+def linear_rows(x, w, out=None):
+    """y [M, N] = x [M, K] @ w [N, K]^T in bf16, a stream of w for up to 8 tokens (the head of a decode step); more tokens and
+    widths that the kernel does not have go to torch's linear."""
+    _chk(x, "x", torch.bfloat16); _chk(w, "w", torch.bfloat16)
+    M, K = x.shape
+    assert w.dim() == 2 and w.shape[1] == K
+    if 1 <= M <= 8 and K in (2048, 4096) and _ptr(x) % 16 == 0 and _ptr(w) % 16 == 0:
+        y = out if out is not None else torch.empty((M, w.shape[0]), dtype=torch.bfloat16, device=x.device)
+        rc = L.lib.lq_linear_rows(_ptr(x), _ptr(w), _ptr(y), M, w.shape[0], K, _stream())
+        if rc != L.LQ_EUNSUPPORTED:
+            L.check("lq_linear_rows", rc)
+            return y
+    y = torch.nn.functional.linear(x, w)
+    return y if out is None else out.copy_(y)
+
+
 def argmax_embed(logits, tok, positions=None, embed=None, h=None):
     """Greedy step end in one launch: tok[b] = argmax(logits[b]) (first maximum, like torch.argmax); positions += 1 and
     h[b] = embed[tok[b]] when given (generate.py:150-190 drives HF's loop, which does these as separate ops)."""

@@ -223,3 +223,21 @@ def test_argmax_of_a_large_vocabulary_by_clusters(ops, B, V, D):
     assert want[:2].tolist() == [share - 1, 7 * share]
     ops.argmax_embed(logits, tok, pos, embed, h)
     assert torch.equal(tok, want) and torch.equal(pos, torch.arange(B, device="cuda") + 1) and torch.equal(h, embed[want])
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 32000, 4096), (8, 1003, 4096), (2, 16 * 149, 4096), (3, 50, 2048), (5, 50272, 2048), (1, 7, 2048), (9, 100, 4096), (2, 100, 512)])
+def test_linear_rows(ops, M, N, K):
+    """The head of a decode step against fp32 matmul: row counts that leave a block of 16 incomplete, fewer and more blocks than SMs, all token counts' edges; the
+    last two go to torch's linear.  One rounding to bf16, and fp32 sums of K products in any order."""
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    x = torch.randn(M, K, device="cuda", generator=g).to(torch.bfloat16)
+    w = (torch.randn(N, K, device="cuda", generator=g) * 0.02).to(torch.bfloat16)
+    ref = x.double() @ w.double().t()
+    bound = ref.abs() * 2.0 ** -8 + (x.double().abs() @ w.double().abs().t()) * (K * 2.0 ** -24)
+    out = torch.full((M, N), 7.0, device="cuda", dtype=torch.bfloat16)
+    for y in (ops.linear_rows(x, w), ops.linear_rows(x, w, out=out)):
+        if M > 8 or K == 512:                         # (the library may round its partial sums to bf16, which the bound does not hold for)
+            assert torch.equal(y, torch.nn.functional.linear(x, w))
+        else:
+            assert y.shape == (M, N) and bool(((y.double() - ref).abs() <= bound).all())
+    assert torch.equal(out, y)
