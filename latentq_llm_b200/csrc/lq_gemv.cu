@@ -820,10 +820,11 @@ __global__ void __launch_bounds__(RB_WARPS * 32, MT == 2 ? 1 : LQ_GEMV_MINB) k_s
                             const uint4 f = xs[(size_t)xrow[m] * x_stride + cg * 16 + w * 4 + t];
                             if (w == 0 && u % GC == 0) {            // first word of a group: no accumulator input
                                 mma_s_start(acc[m][0], a00, a01, a02, a03, f.x, f.y);
-                                mma_s_start(acc[m][1], a10, a11, a12, a13, f.z, f.w);
+                                if (MT == 1) mma_s_start(acc[m][1], a10, a11, a12, a13, f.z, f.w);
+                                else mma_s(acc[m][0], a10, a11, a12, a13, f.z, f.w);        // (one chain, as in k_skinny_wide)
                             } else {
                                 mma_s(acc[m][0], a00, a01, a02, a03, f.x, f.y);
-                                mma_s(acc[m][1], a10, a11, a12, a13, f.z, f.w);
+                                mma_s(acc[m][MT == 1], a10, a11, a12, a13, f.z, f.w);
                             }
                         }
                     }
@@ -834,10 +835,10 @@ __global__ void __launch_bounds__(RB_WARPS * 32, MT == 2 ? 1 : LQ_GEMV_MINB) k_s
 #pragma unroll
                         for (int m = 0; m < MT; ++m) {
                             const float2 sx = *reinterpret_cast<const float2*>(&sxs[(g_begin + grp) * (8 * MT) + m * 8 + 2 * t]);
-                            tot[m][0] = fmaf(s_a, (acc[m][0][0] + acc[m][1][0]) - z_a * sx.x, tot[m][0]);
-                            tot[m][1] = fmaf(s_a, (acc[m][0][1] + acc[m][1][1]) - z_a * sx.y, tot[m][1]);
-                            tot[m][2] = fmaf(s_b, (acc[m][0][2] + acc[m][1][2]) - z_b * sx.x, tot[m][2]);
-                            tot[m][3] = fmaf(s_b, (acc[m][0][3] + acc[m][1][3]) - z_b * sx.y, tot[m][3]);
+                            tot[m][0] = fmaf(s_a, (MT == 1 ? acc[m][0][0] + acc[m][1][0] : acc[m][0][0]) - z_a * sx.x, tot[m][0]);
+                            tot[m][1] = fmaf(s_a, (MT == 1 ? acc[m][0][1] + acc[m][1][1] : acc[m][0][1]) - z_a * sx.y, tot[m][1]);
+                            tot[m][2] = fmaf(s_b, (MT == 1 ? acc[m][0][2] + acc[m][1][2] : acc[m][0][2]) - z_b * sx.x, tot[m][2]);
+                            tot[m][3] = fmaf(s_b, (MT == 1 ? acc[m][0][3] + acc[m][1][3] : acc[m][0][3]) - z_b * sx.y, tot[m][3]);
                         }
                         ++grp;
                     }
@@ -873,6 +874,205 @@ __global__ void __launch_bounds__(RB_WARPS * 32, MT == 2 ? 1 : LQ_GEMV_MINB) k_s
         buf ^= 1;
         ra = na_row; rb = nb_row; wa = na; wb = nb;
     }
+}
+
+// ---------------------------------------------------------------------------------------------
+// The streaming kernel for K = 4096, groups of 128 and 9-16 tokens: persistent, one CTA per SM, two row blocks per step.
+// Twice the MMAs of eight tokens and four passes of the shared-memory path for each token fragment bound it, and the latencies of eight warps in between: a
+// fragment is therefore read once for two row blocks, and the MMAs of a group form one chain per row block and eight tokens, eight independent chains a
+// warp, with no sum of two chains behind them.  What it may not do is spill: a spilled weight that is still in flight is waited for, which undoes the
+// prefetch of a whole step (measured, gate|up at 16 tokens: 16 warps with 100 bytes of spills 29.5 us, without spills but one row block 19.1, this form 17.9).
+// 16 tokens, launches in a chain, one row block per step and two chains before: q|k|v (12288 rows) 14.9 -> 12.5 us, gate|up (22016 rows) 20.9 -> 17.9;
+// 9 tokens, q|k|v 13.6 -> 11.7.
+// ---------------------------------------------------------------------------------------------
+constexpr int SW_XS = 4096 / 8 + 4;           // vectors per staged token: 64 bytes apart modulo 128, two tokens by a quarter warp without conflicts
+__global__ void __launch_bounds__(RB_WARPS * 32, 1) k_skinny_wide(const SkinnyParams p) {
+    static_assert(RB_WARPS * 32 == 2 * 128, "one output of each row block per thread");
+    constexpr int MT = 2, K = 4096, GPR = K / 128, THREADS = RB_WARPS * 32, SXS = 8 * MT;
+    extern __shared__ __align__(128) uint8_t sw_smem[];
+    uint4* xs = reinterpret_cast<uint4*>(sw_smem);                                               // [M][SW_XS]
+    float* sxs = reinterpret_cast<float*>(xs + p.M * SW_XS);                                     // [GPR][SXS]
+    __shared__ __align__(128) float red[2][RB_WARPS][2][MT * 128];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const bool pair = p.pair_stride > 0;
+    const int rows_per_blk = pair ? 8 : 16, n_blocks = (p.N + rows_per_blk - 1) / rows_per_blk, n_steps = (n_blocks + 1) / 2;
+    int step = blockIdx.x;                                   // grid <= n_steps
+    // row r & 1 (fragment half) of row block r >> 1 of a step; loads are clamped, stores guarded
+    auto row_of = [&](int st, int r) {
+        const int b = min(2 * st + (r >> 1), n_blocks - 1), half = r & 1;
+        if (p.rope_hd) { const int bph = p.rope_hd >> 4; return (b / bph) * p.rope_hd + (b % bph) * 8 + g + half * p.pair_stride; }
+        return pair ? half * p.pair_stride + min(b * 8 + g, p.N - 1) : min(b * 16 + g + half * 8, p.N - 1);
+    };
+    auto wptr = [&](int row) { return reinterpret_cast<const uint4*>(p.qweight + (size_t)row * (K / 2) + warp * 256) + t; };
+    auto load_s4 = [&](int row) { return __ldg(reinterpret_cast<const uint2*>(p.scales) + (size_t)row * (GPR / 4) + warp); };
+    auto load_z4 = [&](int row) { return __ldg(reinterpret_cast<const uint2*>(p.zeros) + (size_t)row * (GPR / 4) + warp); };
+    uint4 q[4][4];                                           // [row][group of the warp's slice]
+    uint2 s4[4], z4[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const int row = row_of(step, r);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) q[r][u] = __ldg(wptr(row) + u * 4);
+        s4[r] = load_s4(row); z4[r] = load_z4(row);
+    }
+    pdl_launch_dependents();        // weight and group-parameter loads are issued: the next launch may start
+    pdl_wait();                     // the tokens may be the previous launch's output
+    // ---- tokens into shared memory in B-fragment order (see k_skinny_stream); a warp reads 512 contiguous bytes, each lane the vector that belongs in its place
+    {
+        constexpr int SB = 16;      // vectors per thread and round trip to L2
+        const int items = p.M * (K / 8);
+        for (int base = tid; base < items; base += SB * THREADS) {
+            uint4 v[SB];
+#pragma unroll
+            for (int h = 0; h < SB; ++h) {
+                const int i = base + h * THREADS;
+                v[h] = i < items ? reinterpret_cast<const uint4*>(p.x)[(i & ~15) | ((i & 3) << 2) | ((i >> 2) & 3)] : make_uint4(0, 0, 0, 0);
+            }
+#pragma unroll
+            for (int h = 0; h < SB; ++h) {
+                const int i = base + h * THREADS;
+                if (i >= items) break;
+                uint4 f;
+                f.x = __byte_perm(v[h].x, v[h].z, 0x5410); f.y = __byte_perm(v[h].x, v[h].z, 0x7632);
+                f.z = __byte_perm(v[h].y, v[h].w, 0x5410); f.w = __byte_perm(v[h].y, v[h].w, 0x7632);
+                xs[(i >> 9) * SW_XS + (i & 511)] = f;
+            }
+        }
+    }
+    __syncthreads();
+    const uint4* xbase[MT];                                  // a token that does not exist reads the last: its outputs are dropped
+#pragma unroll
+    for (int m = 0; m < MT; ++m) xbase[m] = xs + min(m * 8 + g, p.M - 1) * SW_XS + warp * 64 + t;
+    const float* sxbase = sxs + warp * 4 * SXS + 2 * t;
+    {   // token sums of the warp's four groups: the staged fragments against a tile of ones
+        const uint32_t ones = 0x3f803f80u;
+        float sacc[4][MT][4];
+#pragma unroll
+        for (int w = 0; w < 4; ++w)
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int m = 0; m < MT; ++m) {
+                    const uint4 f = xbase[m][u * 16 + w * 4];
+                    if (w == 0) mma_s_start(sacc[u][m], ones, ones, ones, ones, f.x, f.y);
+                    else mma_s(sacc[u][m], ones, ones, ones, ones, f.x, f.y);
+                    mma_s(sacc[u][m], ones, ones, ones, ones, f.z, f.w);
+                }
+        if (g == 0)                                          // every row of the D fragment holds the same sums
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int m = 0; m < MT; ++m) *reinterpret_cast<float2*>(&sxs[(warp * 4 + u) * SXS + m * 8 + 2 * t]) = make_float2(sacc[u][m][0], sacc[u][m][1]);
+        __syncwarp();                                        // a warp reads only the sums of its own groups
+    }
+    int buf = 0;
+    for (; step < n_steps; step += gridDim.x, buf ^= 1) {
+        const int nstep = step + (int)gridDim.x;
+        const bool has_next = nstep < n_steps;
+        const uint4* nw[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) nw[r] = wptr(row_of(has_next ? nstep : step, r));
+        float tot[2][MT][4];
+#pragma unroll
+        for (int b = 0; b < 2; ++b)
+#pragma unroll
+            for (int m = 0; m < MT; ++m)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) tot[b][m][i] = 0.0f;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            uint4 c[4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                c[r] = q[r][u];
+                if (has_next) q[r][u] = __ldg(nw[r] + u * 4);
+            }
+            float acc[2][MT][4];
+#pragma unroll
+            for (int w = 0; w < 4; ++w) {
+                uint4 f[MT];
+#pragma unroll
+                for (int m = 0; m < MT; ++m) f[m] = xbase[m][u * 16 + w * 4];
+#pragma unroll
+                for (int b = 0; b < 2; ++b) {
+                    const uint32_t va = w == 0 ? c[2 * b].x : (w == 1 ? c[2 * b].y : (w == 2 ? c[2 * b].z : c[2 * b].w));
+                    const uint32_t vb = w == 0 ? c[2 * b + 1].x : (w == 1 ? c[2 * b + 1].y : (w == 2 ? c[2 * b + 1].z : c[2 * b + 1].w));
+                    LQ_WORD_FRAGS(va, vb);
+#pragma unroll
+                    for (int m = 0; m < MT; ++m) {
+                        if (w == 0) mma_s_start(acc[b][m], a00, a01, a02, a03, f[m].x, f[m].y);
+                        else mma_s(acc[b][m], a00, a01, a02, a03, f[m].x, f[m].y);
+                        mma_s(acc[b][m], a10, a11, a12, a13, f[m].z, f[m].w);
+                    }
+                }
+            }
+            // group u of the slice: bf16 bits (u & 1 ? high : low) half of word (u >> 1) of the packed loads
+            float s[4], z[4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const uint32_t sw = u < 2 ? s4[r].x : s4[r].y, zw = u < 2 ? z4[r].x : z4[r].y;
+                s[r] = __uint_as_float((u & 1) ? (sw & 0xffff0000u) : (sw << 16));
+                z[r] = __uint_as_float((u & 1) ? (zw & 0xffff0000u) : (zw << 16)) + 128.0f;
+                if (u == 3 && has_next) { const int row = row_of(nstep, r); s4[r] = load_s4(row); z4[r] = load_z4(row); }
+            }
+#pragma unroll
+            for (int m = 0; m < MT; ++m) {
+                const float2 sx = *reinterpret_cast<const float2*>(sxbase + u * SXS + m * 8);
+#pragma unroll
+                for (int b = 0; b < 2; ++b) {
+                    tot[b][m][0] = fmaf(s[2 * b], acc[b][m][0] - z[2 * b] * sx.x, tot[b][m][0]);
+                    tot[b][m][1] = fmaf(s[2 * b], acc[b][m][1] - z[2 * b] * sx.y, tot[b][m][1]);
+                    tot[b][m][2] = fmaf(s[2 * b + 1], acc[b][m][2] - z[2 * b + 1] * sx.x, tot[b][m][2]);
+                    tot[b][m][3] = fmaf(s[2 * b + 1], acc[b][m][3] - z[2 * b + 1] * sx.y, tot[b][m][3]);
+                }
+            }
+        }
+#pragma unroll
+        for (int b = 0; b < 2; ++b)
+#pragma unroll
+            for (int m = 0; m < MT; ++m)
+                *reinterpret_cast<float4*>(&red[buf][warp][b][m * 128 + lane * 4]) = make_float4(tot[b][m][0], tot[b][m][1], tot[b][m][2], tot[b][m][3]);
+        __syncthreads();            // one barrier per step: the other buffer is rewritten only after the next barrier
+        // D fragment: d0,d1 = (row g, tokens 2t, 2t+1); d2,d3 = (row g+8, same tokens)
+        const int m = tid >> 7, ln = (tid & 127) >> 2, i = tid & 3, tok = m * 8 + 2 * (ln & 3) + (i & 1);
+        float o[2] = {0.0f, 0.0f};
+#pragma unroll
+        for (int b = 0; b < 2; ++b)
+#pragma unroll
+            for (int w = 0; w < RB_WARPS; ++w) o[b] = __fadd_rn(o[b], red[buf][w][b][tid]);
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+            const int blk = 2 * step + b;
+            const float v = bf16r(o[b]);
+            if (pair) {                                        // d0,d1 = gate[f], d2,d3 = up[f] of the same tokens
+                const float vu = __shfl_down_sync(0xffffffffu, v, 2);
+                const int f = blk * 8 + (ln >> 2);
+                if (i < 2 && f < p.N && tok < p.M) {
+                    if (p.rope_hd) rope_store(p, blk, ln >> 2, tok, v, vu);
+                    else p.out[(size_t)tok * p.N + f] = __float2bfloat16_rn(silu_mul_bf16(v, vu, p.hf_rounding));
+                }
+            } else {
+                const int row = blk * 16 + (ln >> 2) + ((i >= 2) ? 8 : 0);
+                if (row < p.N && tok < p.M) p.out[(size_t)tok * p.N + row] = __float2bfloat16_rn(p.bias ? __fadd_rn(v, __bfloat162float(p.bias[row])) : v);
+            }
+        }
+    }
+}
+
+static int launch_skinny_wide(const SkinnyParams& p, cudaStream_t st) {
+    static bool attr_done[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) return LQ_EUNSUPPORTED;
+    constexpr size_t sums = 32 * 16 * sizeof(float);
+    if (!attr_done[dev]) {
+        cudaError_t e = cudaFuncSetAttribute(k_skinny_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(16 * SW_XS * 16 + sums));
+        if (e != cudaSuccess) { set_cuda_error(e, "cudaFuncSetAttribute(k_skinny_wide)"); return LQ_ECUDA; }
+        attr_done[dev] = true;
+    }
+    const int rpb = p.pair_stride > 0 ? 8 : 16, n_blocks = (p.N + rpb - 1) / rpb;
+    launch_pdl(k_skinny_wide, dim3((unsigned)std::min((n_blocks + 1) / 2, sm_count())), RB_WARPS * 32, (size_t)p.M * SW_XS * 16 + sums, st, p);
+    return check_launch("k_skinny_wide");
 }
 
 bool skinny_norm_supported(int64_t M, int64_t K, int group) {
@@ -922,9 +1122,10 @@ static int launch_skinny_stream(const SkinnyParams& p, cudaStream_t st) {
         if (!nc4 || mt != 1) return LQ_EUNSUPPORTED;
         return launch_skinny_stream_v<1, 1, 4, true>(p, x_stride, smem, grid, st);
     }
-    if (nc4) return mt == 1 ? launch_skinny_stream_v<1, 1, 4>(p, x_stride, smem, grid, st) : launch_skinny_stream_v<2, 1, 4>(p, x_stride, smem, grid, st);
-    if (gc == 1 && p.K == 11008 && LQ_GEMV_PF == 4 && !getenv("LQ_SKINNY_NO_NC4"))      // eleven chunks per warp, written out
-        return mt == 1 ? launch_skinny_stream_v<1, 1, 11>(p, x_stride, smem, grid, st) : launch_skinny_stream_v<2, 1, 11>(p, x_stride, smem, grid, st);
+    // (k_skinny_wide also works for fewer tokens, but two CTAs per SM are the better half of eight: 8 tokens 14.8 / 14.9 us at 22016 rows, 5 tokens 13.9 / 14.6)
+    if (nc4) return mt == 1 ? launch_skinny_stream_v<1, 1, 4>(p, x_stride, smem, grid, st) : launch_skinny_wide(p, st);
+    if (mt == 1 && gc == 1 && p.K == 11008 && LQ_GEMV_PF == 4 && !getenv("LQ_SKINNY_NO_NC4"))      // eleven chunks per warp, written out
+        return launch_skinny_stream_v<1, 1, 11>(p, x_stride, smem, grid, st);
     if (mt == 1) return gc == 1 ? launch_skinny_stream_v<1, 1>(p, x_stride, smem, grid, st) : launch_skinny_stream_v<1, 2>(p, x_stride, smem, grid, st);
     return gc == 1 ? launch_skinny_stream_v<2, 1>(p, x_stride, smem, grid, st) : launch_skinny_stream_v<2, 2>(p, x_stride, smem, grid, st);
 }
@@ -932,7 +1133,7 @@ static int launch_skinny_stream(const SkinnyParams& p, cudaStream_t st) {
 int launch_skinny_rows(const SkinnyParams& p, cudaStream_t st) {
     if (!skinny_rows_supported(p.K, p.group)) return LQ_EUNSUPPORTED;
     // two CTAs per SM must fit: staged tokens + sums + 8-16 KB of static shared memory each
-    // 9-16 tokens at K = 4096: the same kernel with one CTA per SM (its 16 staged tokens take 130 KB); the row-block
+    // 9-16 tokens at K = 4096: k_skinny_wide, one CTA per SM (its 16 staged tokens take 130 KB); the row-block
     // kernel below re-reads every token from L2 in every CTA (128 KB per 32 KB of weights) and permutes it per use.
     // Staging the tokens is a fixed cost per CTA, so from three tokens on the kernel pays only for launches with many row
     // blocks per CTA (measured: the q|k|v and gate|up projections of the 7B shapes, not the 4096-row ones).

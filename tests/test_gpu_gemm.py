@@ -325,6 +325,30 @@ def test_mma_issue_rate_probe_runs_and_rejects_bad_arguments():
     assert lib.lq_mma_issue_rate(_lib.GEMM_A8W8, 1, 256, 1, 1024, 4, C.byref(cyc), None) == _lib.LQ_EINVAL          # int8 has no tensor-memory A here
 
 
+@pytest.mark.parametrize("M,N", [(9, 12288), (16, 12352), (13, 22016), (16, 12288 + 148 * 32)])
+def test_a16w4_nine_to_sixteen_tokens_of_a_large_projection(ops, M, N):
+    """9 to 16 tokens, K = 4096, from 768 row blocks on: two row blocks per step, as many steps as CTAs, one more, a remainder.  Against 64 bits: the sum
+    and the sum plus the bias are rounded to bf16 (8 significant bits: at most 2^-8 of a value, 2^-15 of it for the second order), and a group's sum of (128 + q) x, at most 143 sum |x|, is added up in 32 bits in at most 32 roundings or truncations
+    (2^-23 each).  The outputs of a token do not depend on the others, whatever those hold."""
+    K = 4096
+    codes, sb, zb = make_w4_layer(ops, N, K, seed=17)
+    g = torch.Generator(device="cuda").manual_seed(N + M)
+    x = torch.randn(M, K, device="cuda", generator=g).to(torch.bfloat16)
+    bias = (torch.randn(N, device="cuda", generator=g) * 0.1).to(torch.bfloat16)
+    b = codes.view(torch.uint8).view(N, -1)
+    q = torch.stack([b >> 4, b & 15], 2).view(N, K // 128, 128).double()
+    s, z = sb.double().view(N, K // 128, 1), zb.double().view(N, K // 128, 1)
+    v = x.double() @ ((q - z) * s).view(N, K).t()
+    acc = 143 * x.double().abs().view(M, K // 128, 128).sum(2) @ s.view(N, K // 128).abs().t()
+    y = ops.gemm_a16w4_fwd(x, codes, sb, zb, bias, N, K)
+    assert bool(((y.double() - v - bias.double()).abs() <= (2.0 ** -8 + 2.0 ** -15) * (2 * v.abs() + bias.double().abs()) + 2.0 ** -18 * acc).all())
+    act = ops.gemm_a16w4_fwd_silu(x, codes, sb, zb, N // 2, K)
+    assert torch.equal(act, ops.silu_mul(ops.gemm_a16w4_fwd(x, codes, sb, zb, None, N, K)))
+    x[3, 5], x[M - 1, 77], x[M - 2] = float("nan"), float("inf"), 3e38
+    y2, keep = ops.gemm_a16w4_fwd(x, codes, sb, zb, bias, N, K), [i for i in range(M) if i not in (3, M - 1, M - 2)]
+    assert torch.equal(y2[keep], y[keep]) and not bool(torch.isfinite(y2[[3, M - 1]].float()).any())
+
+
 @pytest.mark.parametrize("K", [4096, 11008])
 @pytest.mark.parametrize("M,N,force_stream", [(1, 4096, True), (2, 12288, True), (1, 1088, True), (12, 4160, True),
                                               (5, 4096, False), (16, 12288, False), (9, 1088, False), (3, 4160, False)])
