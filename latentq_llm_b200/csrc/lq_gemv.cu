@@ -1075,6 +1075,149 @@ static int launch_skinny_wide(const SkinnyParams& p, cudaStream_t st) {
     return check_launch("k_skinny_wide");
 }
 
+// ---------------------------------------------------------------------------------------------
+// The row-block kernel for 9-16 tokens and two row blocks per CTA (groups of 128): the twelve warps of a CTA split K in steps of two groups, and a token
+// fragment, read from L2 and put into order by the warp that needs it, serves both row blocks.  Those token loads bound the launch: 16 tokens of K = 11008 are
+// 352 KB, which every CTA reads through an L1 that delivers 64 bytes a cycle, so half as many CTAs halve them.  The rest is sized to what 168
+// registers per thread hold without a spill (a spilled weight in flight is waited for): one accumulator chain per row block and eight tokens, 32-bit offsets
+// in place of pointers, one step of weights and group parameters (a load of two groups each) ahead.
+// 11008 -> 4096 in a chain, 9 / 16 tokens: 12.5 / 13.4 -> 11.6 / 12.2 us, 5632 -> 4096 7.8 / 8.3 -> 7.0 / 7.35.  With 8, 11, 15 and 16 warps 12.8 / 13.3, 11.6 / 12.0 (5632: the
+// same; spills), 12.6 / 12.9, 12.7 / 13.0.
+// ---------------------------------------------------------------------------------------------
+constexpr int R2_WARPS = 12;
+__global__ void __launch_bounds__(R2_WARPS * 32, 1) k_skinny_rows2(const SkinnyParams p) {
+    constexpr int MT = 2, W = R2_WARPS;
+    __shared__ __align__(128) float red[W][2][MT * 128];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const bool pair = p.pair_stride > 0;
+    const int rows_per_blk = pair ? 8 : 16, n_blocks = (p.N + rows_per_blk - 1) / rows_per_blk;
+    const int pairs = p.K >> 8;                                                                 // 256-k steps per weight row
+    const int s_base = pairs / W, s_extra = pairs - s_base * W;
+    const int n = s_base + (warp < s_extra ? 1 : 0), begin = warp * s_base + min(warp, s_extra);
+    // row r & 1 (fragment half) of row block r >> 1; loads are clamped, stores guarded
+    auto row_of = [&](int r) {
+        const int b = min(2 * (int)blockIdx.x + (r >> 1), n_blocks - 1), half = r & 1;
+        if (p.rope_hd) { const int bph = p.rope_hd >> 4; return (b / bph) * p.rope_hd + (b % bph) * 8 + g + half * p.pair_stride; }
+        return pair ? half * p.pair_stride + min(b * 8 + g, p.N - 1) : min(b * 16 + g + half * 8, p.N - 1);
+    };
+    const uint4* const wbase = reinterpret_cast<const uint4*>(p.qweight) + begin * 8 + t;
+    const uint32_t *const sbase = reinterpret_cast<const uint32_t*>(p.scales) + begin, *const zbase = reinterpret_cast<const uint32_t*>(p.zeros) + begin;
+    uint32_t wo[4], so[4];                                   // a row's first load and its first pair of groups (16 GB of codes: the host's limit)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) { so[r] = (uint32_t)row_of(r) * (uint32_t)pairs; wo[r] = so[r] * 8; }
+    auto load_words = [&](int r, int c) { return __ldg(wbase + wo[r] + c * 4); };                // chunk c (64 bytes per row): this thread's four words
+    uint4 q[4][2];
+    uint32_t sw[4], zw[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        q[r][0] = q[r][1] = make_uint4(0, 0, 0, 0); sw[r] = zw[r] = 0;
+        if (n > 0) { q[r][0] = load_words(r, 0); q[r][1] = load_words(r, 1); sw[r] = __ldg(sbase + so[r]); zw[r] = __ldg(zbase + so[r]); }
+    }
+    pdl_launch_dependents();        // weight and group-parameter loads are issued: the next launch may start
+    pdl_wait();                     // the tokens may be the previous launch's output
+    const uint4* xp[MT];            // a token that does not exist reads the last: its outputs are dropped
+#pragma unroll
+    for (int m = 0; m < MT; ++m) xp[m] = reinterpret_cast<const uint4*>(p.x + (size_t)min(m * 8 + g, p.M - 1) * p.K + begin * 256) + t * 4;
+    float tot[2][MT][4];
+#pragma unroll
+    for (int b = 0; b < 2; ++b)
+#pragma unroll
+        for (int m = 0; m < MT; ++m)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) tot[b][m][i] = 0.0f;
+#pragma unroll 1
+    for (int st = 0; st < n; ++st) {
+        uint32_t nsw[4], nzw[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            nsw[r] = nzw[r] = 0;
+            if (st + 1 < n) { nsw[r] = __ldg(sbase + so[r] + st + 1); nzw[r] = __ldg(zbase + so[r] + st + 1); }
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int c = 2 * st + u;
+            uint4 xc[MT][4];
+#pragma unroll
+            for (int m = 0; m < MT; ++m)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) xc[m][j] = xp[m][c * 16 + j];
+            uint4 cw[4];
+            __nv_bfloat162 z2[4];
+            float s[4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                cw[r] = q[r][u];
+                if (st + 1 < n) q[r][u] = load_words(r, c + 2);
+                s[r] = __uint_as_float(u ? sw[r] & 0xffff0000u : sw[r] << 16);
+                z2[r] = __hadd2_rn(sk_u2(__byte_perm(zw[r], zw[r], u ? 0x3232 : 0x1010)), __float2bfloat162_rn(128.0f));
+            }
+            float acc[2][MT][4];
+#pragma unroll
+            for (int w = 0; w < 4; ++w) {
+                uint4 f[MT];
+#pragma unroll
+                for (int m = 0; m < MT; ++m) {
+                    const uint4 v = xc[m][w];
+                    f[m].x = __byte_perm(v.x, v.z, 0x5410); f[m].y = __byte_perm(v.x, v.z, 0x7632);
+                    f[m].z = __byte_perm(v.y, v.w, 0x5410); f[m].w = __byte_perm(v.y, v.w, 0x7632);
+                }
+#pragma unroll
+                for (int b = 0; b < 2; ++b) {
+                    const uint4 &ca = cw[2 * b], &cq = cw[2 * b + 1];
+                    const uint32_t va = w == 0 ? ca.x : (w == 1 ? ca.y : (w == 2 ? ca.z : ca.w)), vb = w == 0 ? cq.x : (w == 1 ? cq.y : (w == 2 ? cq.z : cq.w));
+                    LQ_WORD_FRAGS(va, vb);
+                    const __nv_bfloat162 za = z2[2 * b], zb = z2[2 * b + 1];
+                    const uint32_t d00 = sk_bf2(__hsub2_rn(sk_u2(a00), za)), d01 = sk_bf2(__hsub2_rn(sk_u2(a01), zb));
+                    const uint32_t d02 = sk_bf2(__hsub2_rn(sk_u2(a02), za)), d03 = sk_bf2(__hsub2_rn(sk_u2(a03), zb));
+                    const uint32_t d10 = sk_bf2(__hsub2_rn(sk_u2(a10), za)), d11 = sk_bf2(__hsub2_rn(sk_u2(a11), zb));
+                    const uint32_t d12 = sk_bf2(__hsub2_rn(sk_u2(a12), za)), d13 = sk_bf2(__hsub2_rn(sk_u2(a13), zb));
+#pragma unroll
+                    for (int m = 0; m < MT; ++m) {
+                        if (w == 0) mma_s_start(acc[b][m], d00, d01, d02, d03, f[m].x, f[m].y);
+                        else mma_s(acc[b][m], d00, d01, d02, d03, f[m].x, f[m].y);
+                        mma_s(acc[b][m], d10, d11, d12, d13, f[m].z, f[m].w);
+                    }
+                }
+            }
+            // fold the group: tot += s * sum x (q - z)
+#pragma unroll
+            for (int b = 0; b < 2; ++b)
+#pragma unroll
+                for (int m = 0; m < MT; ++m)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) tot[b][m][i] = fmaf(s[2 * b + (i >> 1)], acc[b][m][i], tot[b][m][i]);
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) { sw[r] = nsw[r]; zw[r] = nzw[r]; }
+    }
+#pragma unroll
+    for (int b = 0; b < 2; ++b)
+#pragma unroll
+        for (int m = 0; m < MT; ++m)
+            *reinterpret_cast<float4*>(&red[warp][b][m * 128 + lane * 4]) = make_float4(tot[b][m][0], tot[b][m][1], tot[b][m][2], tot[b][m][3]);
+    __syncthreads();
+    // D fragment: d0,d1 = (row g, tokens 2t, 2t+1); d2,d3 = (row g+8, same tokens)
+    for (int j = tid; j < 2 * MT * 128; j += W * 32) {
+        const int b = j / (MT * 128), idx = j % (MT * 128), m = idx >> 7, ln = (idx & 127) >> 2, i = idx & 3, tok = m * 8 + 2 * (ln & 3) + (i & 1), blk = 2 * blockIdx.x + b;
+        if (tok >= p.M || (pair && i >= 2)) continue;
+        float a = 0.0f, au = 0.0f;
+#pragma unroll
+        for (int w = 0; w < W; ++w) a = __fadd_rn(a, red[w][b][idx]);
+        const float v = bf16r(a);
+        if (pair) {                                            // d0,d1 = gate[f], d2,d3 = up[f] of the same tokens
+            const int f = blk * 8 + (ln >> 2);
+            if (f >= p.N) continue;
+#pragma unroll
+            for (int w = 0; w < W; ++w) au = __fadd_rn(au, red[w][b][idx + 2]);
+            if (p.rope_hd) rope_store(p, blk, ln >> 2, tok, v, bf16r(au));
+            else p.out[(size_t)tok * p.N + f] = __float2bfloat16_rn(silu_mul_bf16(v, bf16r(au), p.hf_rounding));
+            continue;
+        }
+        const int row = blk * 16 + (ln >> 2) + ((i >= 2) ? 8 : 0);
+        if (row < p.N) p.out[(size_t)tok * p.N + row] = __float2bfloat16_rn(p.bias ? __fadd_rn(v, __bfloat162float(p.bias[row])) : v);
+    }
+}
+
 bool skinny_norm_supported(int64_t M, int64_t K, int group) {
     return M >= 1 && M <= 2 && K == 4096 && group == 128 && LQ_GEMV_PF == 4 && !getenv("LQ_SKINNY_NO_NC4") && !getenv("LQ_SKINNY_NO_STREAM");
 }
@@ -1149,6 +1292,12 @@ int launch_skinny_rows(const SkinnyParams& p, cudaStream_t st) {
         skinny_stream_smem(p.M, p.K, p.group) <= (size_t)(p.M > 8 ? 144 : 96) * 1024)
         return launch_skinny_stream(p, st);
     if (p.norm_gamma) return LQ_EUNSUPPORTED;       // the fused-norm staging exists in the streaming kernel only
+    // 9-16 tokens: two row blocks per CTA where more than one falls to an SM anyway.  K = 4096 keeps its written-out loop (4096 -> 4096, 16 tokens 5.3 / 6.1 us).
+    if (p.M > 8 && p.group == 128 && p.K > 4096 && p.K % 256 == 0 && n_row_blocks > sm_count() && (int64_t)n_row_blocks * 16 * p.K < (int64_t)1 << 35 &&
+        ((reinterpret_cast<uintptr_t>(p.scales) | reinterpret_cast<uintptr_t>(p.zeros)) & 3) == 0) {
+        launch_pdl(k_skinny_rows2, dim3((n_row_blocks + 1) / 2), R2_WARPS * 32, 0, st, p);
+        return check_launch("k_skinny_rows2");
+    }
     const int rpb = p.pair_stride > 0 ? 8 : 16;
     const unsigned grid = (unsigned)((p.N + rpb - 1) / rpb);
     const bool g128 = p.group == 128;

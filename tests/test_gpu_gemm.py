@@ -349,6 +349,35 @@ def test_a16w4_nine_to_sixteen_tokens_of_a_large_projection(ops, M, N):
     assert torch.equal(y2[keep], y[keep]) and not bool(torch.isfinite(y2[[3, M - 1]].float()).any())
 
 
+@pytest.mark.parametrize("M,Hq,Hkv,K", [(9, 16, 4, 4352), (16, 32, 0, 11008), (12, 20, 5, 5632), (13, 19, 0, 4608)])
+def test_a16w4_nine_to_sixteen_tokens_over_a_long_contraction(ops, M, Hq, Hkv, K):
+    """9 to 16 tokens, K > 4096 in steps of 256 that the warps of a CTA share unevenly (17, 43, 22 and 18 steps), two row blocks of 16 per CTA.  Against 64 bits: two
+    roundings to bf16 (2^-8 each, as above), and group sums of (q - z) x, at most 15 sum |x|, in at most 32 roundings or truncations of 2^-23, K / 128
+    more where they are added up.  The fused epilogues give the bits of the separate launches."""
+    hd, N = 128, (Hq + 2 * Hkv) * 128
+    codes, sb, zb = make_w4_layer(ops, N, K, seed=19)
+    g = torch.Generator(device="cuda").manual_seed(N + M)
+    x = torch.randn(M, K, device="cuda", generator=g).to(torch.bfloat16)
+    bias = (torch.randn(N, device="cuda", generator=g) * 0.1).to(torch.bfloat16)
+    b = codes.view(torch.uint8).view(N, -1)
+    q = torch.stack([b >> 4, b & 15], 2).view(N, K // 128, 128).double()
+    s, z = sb.double().view(N, K // 128, 1), zb.double().view(N, K // 128, 1)
+    v = x.double() @ ((q - z) * s).view(N, K).t()
+    acc = 15 * x.double().abs().view(M, K // 128, 128).sum(2) @ s.view(N, K // 128).abs().t()
+    y = ops.gemm_a16w4_fwd(x, codes, sb, zb, bias, N, K)
+    assert bool(((y.double() - v - bias.double()).abs() <= (2.0 ** -8 + 2.0 ** -15) * (2 * v.abs() + bias.double().abs()) + (32 + K // 128) * 2.0 ** -23 * acc).all())
+    plain = ops.gemm_a16w4_fwd(x, codes, sb, zb, None, N, K)
+    assert torch.equal(ops.gemm_a16w4_fwd_silu(x, codes, sb, zb, N // 2, K), ops.silu_mul(plain))
+    if Hkv:
+        pos = torch.randint(0, 60, (M,), device="cuda", generator=g)
+        inv_freq = (1.0 / (10000.0 ** (torch.arange(0, hd, 2, dtype=torch.float32) / hd))).cuda()
+        kc, vc = (torch.zeros(M, Hkv, 64, hd, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+        kw, vw = kc.clone(), vc.clone()
+        got = ops.gemm_a16w4_fwd_qkv_rope(x, codes, sb, zb, pos, inv_freq, kc, vc, Hq, Hkv, hd, K)
+        ops.rope_kv_store(plain, pos, inv_freq, kw, vw, Hq, Hkv, hd)
+        assert torch.equal(got, plain) and torch.equal(kc, kw) and torch.equal(vc, vw)
+
+
 @pytest.mark.parametrize("K", [4096, 11008])
 @pytest.mark.parametrize("M,N,force_stream", [(1, 4096, True), (2, 12288, True), (1, 1088, True), (12, 4160, True),
                                               (5, 4096, False), (16, 12288, False), (9, 1088, False), (3, 4160, False)])
