@@ -1076,7 +1076,7 @@ static int launch_skinny_wide(const SkinnyParams& p, cudaStream_t st) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// The row-block kernel for 9-16 tokens and two row blocks per CTA (groups of 128): the twelve warps of a CTA split K in steps of two groups, and a token
+// The row-block kernel for two row blocks per CTA (groups of 128): the twelve warps of a CTA split K in steps of two groups, and a token
 // fragment, read from L2 and put into order by the warp that needs it, serves both row blocks.  Those token loads bound the launch: 16 tokens of K = 11008 are
 // 352 KB, which every CTA reads through an L1 that delivers 64 bytes a cycle, so half as many CTAs halve them.  The rest is sized to what 168
 // registers per thread hold without a spill (a spilled weight in flight is waited for): one accumulator chain per row block and eight tokens, 32-bit offsets
@@ -1085,8 +1085,9 @@ static int launch_skinny_wide(const SkinnyParams& p, cudaStream_t st) {
 // same; spills), 12.6 / 12.9, 12.7 / 13.0.
 // ---------------------------------------------------------------------------------------------
 constexpr int R2_WARPS = 12;
+template <int MT>
 __global__ void __launch_bounds__(R2_WARPS * 32, 1) k_skinny_rows2(const SkinnyParams p) {
-    constexpr int MT = 2, W = R2_WARPS;
+    constexpr int W = R2_WARPS;
     __shared__ __align__(128) float red[W][2][MT * 128];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     const bool pair = p.pair_stride > 0;
@@ -1292,10 +1293,14 @@ int launch_skinny_rows(const SkinnyParams& p, cudaStream_t st) {
         skinny_stream_smem(p.M, p.K, p.group) <= (size_t)(p.M > 8 ? 144 : 96) * 1024)
         return launch_skinny_stream(p, st);
     if (p.norm_gamma) return LQ_EUNSUPPORTED;       // the fused-norm staging exists in the streaming kernel only
-    // 9-16 tokens: two row blocks per CTA where more than one falls to an SM anyway.  K = 4096 keeps its written-out loop (4096 -> 4096, 16 tokens 5.3 / 6.1 us).
-    if (p.M > 8 && p.group == 128 && p.K > 4096 && p.K % 256 == 0 && n_row_blocks > sm_count() && (int64_t)n_row_blocks * 16 * p.K < (int64_t)1 << 35 &&
+    // Two row blocks per CTA where more than one falls to an SM anyway.  K = 4096 keeps its written-out loop (4096 -> 4096, 16 tokens 5.3 / 6.1 us), and so does
+    // K = 11008 up to 8 tokens (8.7 .. 9.6 / 9.0 .. 9.6 us).  Up to 8 tokens, old and new (us at 1 / 8 tokens): 4352 -> 2432 4.5 / 4.65, 4.4 / 4.75; 4608 -> 4096 5.0 / 5.5,
+    // 4.9 / 5.35; 5632 -> 4096 6.0 / 6.35, 5.5 / 5.9; 14336 -> 4096 12.3 / 13.0, 10.8 / 11.45; where a CTA per SM is not enough, at 3 tokens: 5632 -> 11264 15.4, 15.7; 14336 -> 8192 23.9, 21.9.
+    const bool few_ok = p.K >= 4608 && p.K != 11008 && (n_row_blocks <= 2 * sm_count() || p.K >= 8192);
+    if ((p.M > 8 ? p.K > 4096 : few_ok) && p.group == 128 && p.K % 256 == 0 && n_row_blocks > sm_count() && (int64_t)n_row_blocks * 16 * p.K < (int64_t)1 << 35 &&
         ((reinterpret_cast<uintptr_t>(p.scales) | reinterpret_cast<uintptr_t>(p.zeros)) & 3) == 0) {
-        launch_pdl(k_skinny_rows2, dim3((n_row_blocks + 1) / 2), R2_WARPS * 32, 0, st, p);
+        if (p.M > 8) launch_pdl(k_skinny_rows2<2>, dim3((n_row_blocks + 1) / 2), R2_WARPS * 32, 0, st, p);
+        else launch_pdl(k_skinny_rows2<1>, dim3((n_row_blocks + 1) / 2), R2_WARPS * 32, 0, st, p);
         return check_launch("k_skinny_rows2");
     }
     const int rpb = p.pair_stride > 0 ? 8 : 16;

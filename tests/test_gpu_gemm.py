@@ -349,9 +349,9 @@ def test_a16w4_nine_to_sixteen_tokens_of_a_large_projection(ops, M, N):
     assert torch.equal(y2[keep], y[keep]) and not bool(torch.isfinite(y2[[3, M - 1]].float()).any())
 
 
-@pytest.mark.parametrize("M,Hq,Hkv,K", [(9, 16, 4, 4352), (16, 32, 0, 11008), (12, 20, 5, 5632), (13, 19, 0, 4608)])
-def test_a16w4_nine_to_sixteen_tokens_over_a_long_contraction(ops, M, Hq, Hkv, K):
-    """9 to 16 tokens, K > 4096 in steps of 256 that the warps of a CTA share unevenly (17, 43, 22 and 18 steps), two row blocks of 16 per CTA.  Against 64 bits: two
+@pytest.mark.parametrize("M,Hq,Hkv,K", [(9, 16, 4, 4352), (16, 32, 0, 11008), (12, 20, 5, 5632), (13, 19, 0, 4608), (1, 16, 4, 4608), (8, 20, 5, 5632), (3, 64, 0, 8192)])
+def test_a16w4_decode_projection_over_a_long_contraction(ops, M, Hq, Hkv, K):
+    """Up to 16 tokens, K > 4096 in steps of 256 that the warps of a CTA share unevenly (17, 43, 22, 18 and 32 steps), two row blocks of 16 per CTA.  Against 64 bits: two
     roundings to bf16 (2^-8 each, as above), and group sums of (q - z) x, at most 15 sum |x|, in at most 32 roundings or truncations of 2^-23, K / 128
     more where they are added up.  The fused epilogues give the bits of the separate launches."""
     hd, N = 128, (Hq + 2 * Hkv) * 128
