@@ -567,12 +567,11 @@ def gemm_a16w4_fwd_qkv_rope(x, qweight, scales, zeros, positions, inv_freq, k_ca
 
 
 def linear_rows(x, w, out=None):
-    """y [M, N] = x [M, K] @ w [N, K]^T in bf16, a stream of w for up to 8 tokens (the head of a decode step); more tokens and
-    widths that the kernel does not have go to torch's linear."""
-    _chk(x, "x", torch.bfloat16); _chk(w, "w", torch.bfloat16)
+    """y [M, N] = x [M, K] @ w [N, K]^T in bf16, a stream of w for up to 8 tokens (the head of a decode step); more tokens, and
+    widths, types and strides that the kernel does not have, go to torch's linear."""
     M, K = x.shape
-    assert w.dim() == 2 and w.shape[1] == K
-    if 1 <= M <= 8 and K in (2048, 4096) and _ptr(x) % 16 == 0 and _ptr(w) % 16 == 0:
+    served = all(t.is_cuda and t.dtype == torch.bfloat16 and t.is_contiguous() and _ptr(t) % 16 == 0 for t in (x, w)) and w.shape[1:] == (K,)
+    if served and 1 <= M <= 8 and K in (2048, 4096) and (out is None or (out.is_contiguous() and out.dtype == x.dtype and out.shape == (M, w.shape[0]))):
         y = out if out is not None else torch.empty((M, w.shape[0]), dtype=torch.bfloat16, device=x.device)
         rc = L.lib.lq_linear_rows(_ptr(x), _ptr(w), _ptr(y), M, w.shape[0], K, _stream())
         if rc != L.LQ_EUNSUPPORTED:

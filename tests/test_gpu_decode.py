@@ -241,3 +241,5 @@ def test_linear_rows(ops, M, N, K):
         else:
             assert y.shape == (M, N) and bool(((y.double() - ref).abs() <= bound).all())
     assert torch.equal(out, y)
+    wt = w.t().contiguous().t()                           # strides that the kernel does not have
+    assert torch.equal(ops.linear_rows(x, wt), torch.nn.functional.linear(x, wt))
