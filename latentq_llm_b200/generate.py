@@ -16,6 +16,14 @@ from torch.nn.attention import SDPBackend, sdpa_kernel
 # the cuDNN attention backend rebuilds its plan for every new KV length (milliseconds of host time per layer and token)
 _SDPA = [SDPBackend.FLASH_ATTENTION, SDPBackend.EFFICIENT_ATTENTION, SDPBackend.MATH]
 
+_PROJECTIONS = (("self_attn", ("q_proj", "k_proj", "v_proj")), ("mlp", ("gate_proj", "up_proj")), ("self_attn", ("o_proj",)), ("mlp", ("down_proj",)))
+
+
+def _words(t):
+    """A flat tensor in 8-byte words where it consists of them (copies of many tensors in one launch move one element per thread at a time)."""
+    whole = t.numel() * t.element_size() % 8 == 0 and t.storage_offset() * t.element_size() % 8 == 0 and t.data_ptr() % 8 == 0
+    return t.view(torch.int64) if whole else t
+
 
 class GraphedGreedyDecoder:
     """`decoder = GraphedGreedyDecoder(model, batch, max_len)`; `tokens = decoder.generate(prompt, max_new_tokens)`.
@@ -97,36 +105,37 @@ class FusedLlamaGreedyDecoder:
     once as a CUDA graph and replayed per token.  The prompt goes through the same kernels at its own token count (fused
     q|k|v and gate|up GEMMs, SDPA for its attention) into the same static KV cache, and only its last tokens through the
     head; a model whose prompt differs from that in more than rounding goes through its own modules
-    (`_kernels_serve_prompts`).  `hf_rounding=True` rounds intermediates like the eager modules' bf16 tensor ops."""
+    (`_kernels_serve_prompts`).  `hf_rounding=True` rounds the steps' intermediates like the eager modules' bf16 tensor ops; a prompt
+    is always rounded so, whichever way it goes.
+
+    The weights are the model's at the start of each `generate` call: the fused projections are copies, which every call brings
+    up to date (75 MB read and written for a layer of 4096 x 11008)."""
 
     def __init__(self, model, batch: int, max_len: int, hf_rounding: bool = True):
         from transformers import StaticCache
-        from .quant import QLinearA16W4
         cfg = model.config
         self.model, self.batch, self.max_len, self.hf = model, batch, max_len, hf_rounding
         self.device = dev = next(model.parameters()).device
         self.Hq, self.Hkv = cfg.num_attention_heads, getattr(cfg, "num_key_value_heads", None) or cfg.num_attention_heads
         self.hd = getattr(cfg, "head_dim", None) or cfg.hidden_size // cfg.num_attention_heads
         self.D, self.I, self.eps = cfg.hidden_size, cfg.intermediate_size, cfg.rms_norm_eps
-        self.inv_freq = model.model.rotary_emb.inv_freq.detach().to(dev, torch.float32).contiguous()
+        self.inv_freq = model.model.rotary_emb.inv_freq.detach().to(dev, torch.float32, copy=True).contiguous()
         self.cache = StaticCache(config=cfg, max_cache_len=max_len)
-
-        def flat(lin):
-            if not isinstance(lin, QLinearA16W4) or lin.bias is not None:
-                raise TypeError("FusedLlamaGreedyDecoder needs bias-free QLinearA16W4 projections")
-            sc, zr, _ = lin.weight.qparam
-            return lin.weight.data.reshape(-1), sc.reshape(-1), zr.reshape(-1)
-
-        def fuse(*lins):
-            parts = [flat(l) for l in lins]
-            return tuple(torch.cat([p[i] for p in parts]).contiguous() for i in range(3))
 
         self.layers = []
         for layer in model.model.layers:
-            a, m = layer.self_attn, layer.mlp
-            self.layers.append(dict(ln1=layer.input_layernorm.weight.detach(), ln2=layer.post_attention_layernorm.weight.detach(),
-                                    qkv=fuse(a.q_proj, a.k_proj, a.v_proj), o=flat(a.o_proj),
-                                    gu=fuse(m.gate_proj, m.up_proj), down=flat(m.down_proj)))
+            now = self._tensors(layer)
+            if now is None:
+                raise TypeError("FusedLlamaGreedyDecoder needs bias-free QLinearA16W4 projections")
+            L = self._flat(now)
+            rows = []
+            for name, i, j in (("qkv", 0, 9), ("gu", 9, 15)):
+                parts = [L["src"][n:j:3] for n in range(i, i + 3)]                # codes, scales, zeros of the projections
+                L[name] = tuple(torch.cat(p) for p in parts)
+                rows += [r for of in zip(*(t.split([x.numel() for x in p]) for t, p in zip(L[name], parts))) for r in of]
+            L["rows"] = [_words(r) for r in rows]
+            self.layers.append(L)
+        self.ends = self._live_ends()
         bf = dict(dtype=torch.bfloat16, device=dev)
         self.h = torch.zeros((batch, self.D), **bf)
         self.xn = torch.zeros((batch, self.D), **bf)
@@ -143,8 +152,65 @@ class FusedLlamaGreedyDecoder:
         self.logits = None
         self.graph = None
         self.prompt_kernels = self._kernels_serve_prompts()
-        if self.prompt_kernels:           # the modules would allocate the cache at their first call
-            self.cache.early_initialization(batch, self.Hkv, self.hd, torch.bfloat16, dev)
+
+    @staticmethod
+    def _tensors(layer):
+        """Codes, scales and zeros of q, k, v, gate, up, o, down and the weights of the two norms, where the model has them now; None unless
+        all seven projections are bias-free int4 linears."""
+        from .quant import QLinearA16W4
+        sub, out = layer._modules, []                     # (a module's __getattr__ costs several times as much, in every call)
+        for part, names in _PROJECTIONS:
+            own = sub[part]._modules
+            for name in names:
+                lin = own[name]
+                if not isinstance(lin, QLinearA16W4) or lin.bias is not None:
+                    return None
+                w = lin.weight
+                scales, zeros, _ = w.qparam
+                out += (w.data, scales, zeros)
+        return out + [sub["input_layernorm"].weight, sub["post_attention_layernorm"].weight]
+
+    @staticmethod
+    def _flat(now):
+        src = [t.detach().reshape(-1) for t in now]
+        return dict(src=src, words=[_words(t) for t in src[:15]], at=[(t.data_ptr(), t.numel()) for t in src], o=tuple(src[15:18]), down=tuple(src[18:21]), ln1=src[21], ln2=src[22])
+
+    def _live_ends(self):
+        m = self.model
+        return m.model.norm.weight.detach(), m.lm_head.weight.detach(), m.model.embed_tokens.weight.detach()
+
+    @torch.no_grad()
+    def _take_weights(self):
+        """The weights as they are now, for the steps and for a prompt through the kernels: the rows of the fused projections are copied
+        anew, in place, where the captured step reads them; a weight that it reads in the model and that has moved since drops it.  (No version or
+        address shows that the library's optimizer wrote a weight in place.)  Layers whose projections were replaced by something else stay."""
+        to, frm, moved = [], [], False
+
+        def same(now, at):                                # (what lay there is held: no other tensor has its address)
+            return all(t.data_ptr() == p and t.numel() == n and t.is_contiguous() for t, (p, n) in zip(now, at))
+
+        for L, layer in zip(self.layers, self.model.model.layers):
+            now = self._tensors(layer)
+            if now is None:
+                continue
+            if not same(now, L["at"]):
+                if any(t.numel() != h.numel() or t.dtype != h.dtype for t, h in zip(now, L["src"])):
+                    continue
+                moved |= not same(now[15:], L["at"][15:])
+                L.update(self._flat(now))
+            to += L["rows"]; frm += L["words"]
+        ends = self._live_ends()
+        if any(t.data_ptr() != h.data_ptr() or t.stride() != h.stride() for t, h in zip(ends, self.ends)):
+            moved, self.ends = True, ends
+        if to and all(t.dtype == torch.int64 for t in to + frm):
+            torch._foreach_copy_(to, frm)                 # two layers of 4096 x 11008: 53 us, 168 in bytes and bf16, 149 as copies one by one
+        else:
+            for d, t in zip(to, frm):
+                d.view(torch.uint8).copy_(t.view(torch.uint8))
+        if self.prompt_kernels:                           # (else they may belong to the length of the last prompt)
+            self.inv_freq.copy_(self.model.model.rotary_emb.inv_freq)
+        if moved:
+            self.graph = None
 
     def _kernels_serve_prompts(self) -> bool:
         """What the step's kernels compute is what the modules compute for a prompt, to rounding: frequencies that do not
@@ -200,22 +266,26 @@ class FusedLlamaGreedyDecoder:
                 h, h_alt = h_alt, h
             ops.gemm_a16w4_fwd(self.act, *L["down"], None, D, I, out=self.tmp)
             delta = self.tmp
-        ops.add_rmsnorm(h, delta, self.model.model.norm.weight.detach(), self.eps, out=self.xn, hf_rounding=self.hf)
-        self.logits = ops.linear_rows(self.xn, self.model.lm_head.weight.detach())
+        norm, head, embed = self.ends
+        ops.add_rmsnorm(h, delta, norm, self.eps, out=self.xn, hf_rounding=self.hf)
+        self.logits = ops.linear_rows(self.xn, head)
         # argmax, position += 1 and the next step's embedding row in one launch
-        ops.argmax_embed(self.logits, self.tok, self.pos, self.model.model.embed_tokens.weight.detach(), self.h)
+        ops.argmax_embed(self.logits, self.tok, self.pos, embed, self.h)
 
     def _seed(self, first, p):
         self.tok.copy_(first); self.pos.fill_(p)
-        self.h.copy_(torch.nn.functional.embedding(self.tok, self.model.model.embed_tokens.weight))
+        self.h.copy_(torch.nn.functional.embedding(self.tok, self.ends[2]))
 
     def _prompt_step(self, prompt):
         """The layers over all tokens of the prompt; logits of the last token of every sequence."""
         from . import ops
         B, P = prompt.shape
         D, I, Hq, Hkv, hd = self.D, self.I, self.Hq, self.Hkv, self.hd
+        norm, head, embed = self.ends
+        if not self.cache.layers[0].is_initialized:       # the modules would allocate the cache at their first call
+            self.cache.early_initialization(B, Hkv, hd, torch.bfloat16, self.device)
         pos = torch.arange(P, device=self.device).repeat(B)
-        h = torch.nn.functional.embedding(prompt.reshape(-1), self.model.model.embed_tokens.weight)
+        h = torch.nn.functional.embedding(prompt.reshape(-1), embed)
         delta = None
         for li, L in enumerate(self.layers):
             kc, vc = self.cache.layers[li].keys, self.cache.layers[li].values
@@ -227,8 +297,7 @@ class FusedLlamaGreedyDecoder:
             act = ops.gemm_a16w4_fwd_silu(ops.add_rmsnorm(h, o, L["ln2"], self.eps), *L["gu"], I, D)
             delta = ops.gemm_a16w4_fwd(act, *L["down"], None, D, I)
         last = [t.view(B, P, D)[:, -1].contiguous() for t in (h, delta)]
-        xn = ops.add_rmsnorm(*last, self.model.model.norm.weight.detach(), self.eps)
-        return ops.linear_rows(xn, self.model.lm_head.weight.detach())
+        return ops.linear_rows(ops.add_rmsnorm(*last, norm, self.eps), head)
 
     @torch.no_grad()
     def _prefill(self, prompt):
@@ -261,8 +330,9 @@ class FusedLlamaGreedyDecoder:
         if b != self.batch or p + max_new_tokens > self.max_len:
             raise ValueError("prompt does not fit the decoder's batch size / cache length")
         self.model.eval()
+        self._take_weights()
         if use_graph and self.graph is None:
-            self._capture(self._prefill(prompt), p)         # throw-away prefill: capture needs an initialised cache
+            self._capture(self._prefill(prompt), p)         # throw-away prefill: capture needs an allocated cache and tokens to start from
         first = self._prefill(prompt)
         self._seed(first, p)
         toks = [first.clone()]

@@ -95,3 +95,39 @@ def test_fused_decoder_with_the_norm_inside_the_projections_decodes_the_same_tok
     assert calls and torch.equal(got, want) and torch.equal(fused.logits, want_logits)
     assert torch.equal(fused.generate(prompt, T, use_graph=True), want)
     assert torch.equal(fused.logits, want_logits)
+
+
+@pytest.mark.parametrize("arch,use_graph", [("llama-gqa-tiny", False), ("llama-gqa-tiny", True), ("llama-wide-tiny", True)])
+def test_fused_decoder_after_the_weights_changed_equals_a_new_decoder(arch, use_graph):
+    """Codes and scales written in place (as an optimizer step does), codes set anew, a norm and the head elsewhere: prompt and steps of the next call
+    have the new weights, whether the step was captured before or not."""
+    from latentq_llm_b200 import finetune as ft
+    from latentq_llm_b200.generate import FusedLlamaGreedyDecoder
+    model = ft.build_model(arch, "cuda", seed=3)
+    ft.quantize_decoder(model, lbit=0, gbit=16)
+    model.eval()
+    B, P, T = 2, 40, 6
+    g = torch.Generator(device="cuda").manual_seed(1)
+    prompt = torch.randint(0, 1024, (B, P), device="cuda", generator=g)
+    dec = FusedLlamaGreedyDecoder(model, batch=B, max_len=64)
+    dec.generate(prompt, T, use_graph=use_graph)
+    before = dec.logits.clone()
+    for change in range(3):
+        layer = model.model.layers[change % 2]
+        if change == 0:
+            layer.self_attn.k_proj.weight.data.copy_(layer.self_attn.k_proj.weight.data.flip(0))
+            layer.mlp.up_proj.scales.data.mul_(0.5)
+        elif change == 1:
+            w = layer.self_attn.q_proj.weight
+            w.set_value(w.data.flip(0), w.qparam)
+        else:
+            layer.input_layernorm.weight.data = layer.input_layernorm.weight.data * 1.5
+            model.lm_head.weight.data = model.lm_head.weight.data.flip(0)
+            w = layer.mlp.down_proj.weight
+            w.set_value(w.data.flip(0), w.qparam)
+        got = dec.generate(prompt, T, use_graph=use_graph)
+        new = FusedLlamaGreedyDecoder(model, batch=B, max_len=64)
+        want = new.generate(prompt, T, use_graph=use_graph)
+        assert torch.equal(got, want) and torch.equal(dec.logits, new.logits) and not torch.equal(dec.logits, before), change
+        assert torch.equal(dec.generate(prompt, 1, use_graph=use_graph)[:, 0], want[:, 0])
+        before = dec.logits.clone()
