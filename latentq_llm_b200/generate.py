@@ -104,7 +104,7 @@ class FusedLlamaGreedyDecoder:
     PTQ/quant/fused_mlp.py:84-168 gate/up with the silu epilogue, PTQ/quant/triton_norm.py:7-39 RMSNorm), captured
     once as a CUDA graph and replayed per token.  The prompt goes through the same kernels at its own token count (fused
     q|k|v and gate|up GEMMs, SDPA for its attention) into the same static KV cache, and only its last tokens through the
-    head; a model whose prompt differs from that in more than rounding goes through its own modules
+    head; a model whose modules do anything else, or are watched by hooks, runs its prompt through them
     (`_kernels_serve_prompts`).  `hf_rounding=True` rounds the steps' intermediates like the eager modules' bf16 tensor ops; a prompt
     is always rounded so, whichever way it goes.
 
@@ -213,14 +213,41 @@ class FusedLlamaGreedyDecoder:
             self.graph = None
 
     def _kernels_serve_prompts(self) -> bool:
-        """What the step's kernels compute is what the modules compute for a prompt, to rounding: frequencies that do not
-        depend on its length and need no scaling of the attention, keys kept for the whole length, silu, no further norms."""
-        cfg, rope = self.model.config, self.model.model.rotary_emb
-        attn = self.model.model.layers[0].self_attn
-        return (getattr(rope, "rope_type", "default") in ("default", "linear", "llama3") and getattr(rope, "attention_scaling", 1.0) == 1.0
-                and not any(getattr(l, "is_sliding", False) for l in self.cache.layers) and getattr(cfg, "hidden_act", "silu") == "silu"
-                and not hasattr(attn, "q_norm") and getattr(attn, "scaling", self.hd ** -0.5) == self.hd ** -0.5
-                and self.model.model.embed_tokens.weight.dtype == torch.bfloat16 and self.model.lm_head.bias is None)
+        """What the step's kernels compute is what the modules compute for a prompt, to rounding, and nothing watches the modules: the
+        Llama classes themselves with their forwards untouched, torch's attention, silu, bf16, no autocast, frequencies that do not depend
+        on the length of a prompt and need no scaling of the attention, keys kept for the whole length."""
+        from torch.nn.modules import module as nn_module
+        from transformers.activations import ACT2FN
+        from transformers.models.llama import modeling_llama as hf
+        from .quant import QLinearA16W4
+
+        def own(mod, cls):                                # of the class itself, its forward neither replaced nor watched
+            d = mod.__dict__
+            return type(mod) is cls and not (d["_forward_hooks"] or d["_forward_pre_hooks"] or "forward" in d)
+
+        def norm(mod):
+            return own(mod, hf.LlamaRMSNorm) and mod.variance_epsilon == self.eps and mod.weight.dtype == bf
+
+        bf, silu, scaling = torch.bfloat16, type(ACT2FN["silu"]), self.hd ** -0.5
+        model = self.model
+        if not own(model, hf.LlamaForCausalLM) or not own(model.model, hf.LlamaModel):
+            return False
+        cfg, inner = model.config, model.model
+        rope, emb, head = inner.rotary_emb, inner.embed_tokens, model.lm_head
+        for layer in inner.layers:
+            sub = layer._modules
+            if not (own(layer, hf.LlamaDecoderLayer) and own(sub["self_attn"], hf.LlamaAttention) and own(sub["mlp"], hf.LlamaMLP) and sub["self_attn"].scaling == scaling
+                    and own(sub["mlp"]._modules["act_fn"], silu) and norm(sub["input_layernorm"]) and norm(sub["post_attention_layernorm"])
+                    and all(own(sub[part]._modules[name], QLinearA16W4) for part, names in _PROJECTIONS for name in names)):
+                return False
+        if nn_module._global_forward_hooks or nn_module._global_forward_pre_hooks or torch.is_autocast_enabled(self.device.type):
+            return False
+        return (own(emb, torch.nn.Embedding) and own(rope, hf.LlamaRotaryEmbedding) and own(head, torch.nn.Linear) and norm(inner.norm)
+                and len(inner.layers) == cfg.num_hidden_layers == len(self.layers) and cfg._attn_implementation == "sdpa"
+                and rope.rope_type in ("default", "linear", "llama3") and rope.attention_scaling == 1.0
+                and rope.inv_freq.shape == self.inv_freq.shape and not any(l.is_sliding for l in self.cache.layers)
+                and self.hd % 4 == 0 and 8 <= self.hd <= 512
+                and emb.weight.dtype == bf and emb.max_norm is None and head.weight.dtype == bf and head.bias is None)
 
     def _step(self):
         from . import ops
@@ -330,6 +357,7 @@ class FusedLlamaGreedyDecoder:
         if b != self.batch or p + max_new_tokens > self.max_len:
             raise ValueError("prompt does not fit the decoder's batch size / cache length")
         self.model.eval()
+        self.prompt_kernels = self._kernels_serve_prompts()
         self._take_weights()
         if use_graph and self.graph is None:
             self._capture(self._prefill(prompt), p)         # throw-away prefill: capture needs an allocated cache and tokens to start from

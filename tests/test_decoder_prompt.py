@@ -1,4 +1,5 @@
-"""FusedLlamaGreedyDecoder, what needs no kernel: a call works with the model's weights as they are then."""
+"""FusedLlamaGreedyDecoder, what needs no kernel: which route a prompt takes, and that a call works with the model's weights as they are then."""
+import pytest
 import torch
 from transformers import LlamaConfig, LlamaForCausalLM
 
@@ -30,6 +31,78 @@ def _model(**cfg):
 
 def _decoder(model):
     return FusedLlamaGreedyDecoder(model, batch=2, max_len=64)
+
+
+def test_llama_prompts_go_through_the_kernels():
+    for rope in (None, {"rope_type": "linear", "factor": 2.0, "rope_theta": 10000.0},
+                 {"rope_type": "llama3", "factor": 8.0, "low_freq_factor": 1.0, "high_freq_factor": 4.0, "original_max_position_embeddings": 32, "rope_theta": 10000.0}):
+        assert _decoder(_model(**({"rope_parameters": rope} if rope else {})))._kernels_serve_prompts(), rope
+
+
+class _OtherLinear(QLinearA16W4):
+    def forward(self, x):
+        return super().forward(x) * 2
+
+
+def _replace(path, make):
+    def change(model):
+        owner = model.model.layers[1]                      # the last layer: every layer is looked at
+        *parents, leaf = path.split(".")
+        for name in parents:
+            owner = getattr(owner, name)
+        setattr(owner, leaf, make(getattr(owner, leaf)))
+    return change
+
+
+def _forward_of_its_own(module):
+    old = module.forward
+    module.forward = lambda *a, **k: old(*a, **k)
+
+
+CHANGES = {
+    "hook of a projection": lambda m: m.model.layers[1].mlp.up_proj.register_forward_hook(lambda *a: None),
+    "hook before a layer": lambda m: m.model.layers[1].register_forward_pre_hook(lambda *a: None),
+    "hook of the head": lambda m: m.lm_head.register_forward_hook(lambda *a: None),
+    "hook of the model": lambda m: m.register_forward_hook(lambda *a: None),
+    "forward of one object": lambda m: _forward_of_its_own(m.model.layers[1].self_attn),
+    "linear of a subclass": _replace("self_attn.v_proj", lambda old: _int4_linear(*old.wshape, torch.Generator(), _OtherLinear)),
+    "norm of another class": _replace("input_layernorm", lambda old: torch.nn.RMSNorm(256, dtype=torch.bfloat16)),
+    "norm with another epsilon": lambda m: setattr(m.model.layers[1].post_attention_layernorm, "variance_epsilon", 1e-3),
+    "other activation": _replace("mlp.act_fn", lambda old: torch.nn.GELU()),
+    "scaled attention": lambda m: setattr(m.model.layers[1].self_attn, "scaling", 0.5),
+    "embedding in fp32": lambda m: m.model.embed_tokens.float(),
+    "head of another class": lambda m: setattr(m, "lm_head", torch.nn.Sequential(torch.nn.Linear(256, 64, bias=False))),
+}
+
+
+@pytest.mark.parametrize("change", CHANGES)
+def test_models_that_do_something_else_run_their_prompt_themselves(change):
+    model = _model()
+    dec = _decoder(model)
+    assert dec._kernels_serve_prompts()
+    CHANGES[change](model)
+    assert not dec._kernels_serve_prompts()
+    if change not in ("head of another class", "linear of a subclass"):
+        assert not _decoder(model)._kernels_serve_prompts()
+
+
+@pytest.mark.parametrize("cfg", [{"rope_parameters": {"rope_type": "yarn", "factor": 4.0, "rope_theta": 10000.0}},
+                                 {"rope_parameters": {"rope_type": "dynamic", "factor": 2.0, "rope_theta": 10000.0}},
+                                 {"hidden_act": "gelu"}, {"sliding_window": 16}, {"attn_implementation": "eager"}], ids=str)
+def test_configurations_that_the_kernels_do_not_compute(cfg):
+    assert not _decoder(_model(**cfg))._kernels_serve_prompts()
+
+
+def test_autocast_and_global_hooks_are_the_modules_business():
+    dec = _decoder(_model())
+    with torch.autocast("cpu", dtype=torch.bfloat16):
+        assert not dec._kernels_serve_prompts()
+    handle = torch.nn.modules.module.register_module_forward_hook(lambda *a: None)
+    try:
+        assert not dec._kernels_serve_prompts()
+    finally:
+        handle.remove()
+    assert dec._kernels_serve_prompts()
 
 
 def _fresh_equals(dec, model):
@@ -88,8 +161,8 @@ def test_rows_that_are_not_whole_words_are_copied_too():
     _fresh_equals(dec, model)
 
 
-def test_a_prompt_sees_the_present_weights(monkeypatch):
-    """The order inside `generate`: the weights of the call before its prompt."""
+def test_a_prompt_sees_the_present_weights_and_route(monkeypatch):
+    """The order inside `generate`: the route and the weights of the call before its prompt."""
     model = _model()
     dec = _decoder(model)
     seen = []
@@ -99,3 +172,8 @@ def test_a_prompt_sees_the_present_weights(monkeypatch):
         model.model.layers[0].self_attn.q_proj.weight.data.fill_(value)
         dec.generate(prompt, 1, use_graph=False)
     assert seen == [("kernels", 3), ("kernels", 4)]
+    fired = []
+    model.model.embed_tokens.register_forward_hook(lambda *a: (fired.append(1), 1 / 0))
+    with pytest.raises(ZeroDivisionError):                 # through the modules, whose kernels need a GPU: as far as the first hook
+        dec.generate(prompt, 1, use_graph=False)
+    assert fired and len(seen) == 2

@@ -131,3 +131,90 @@ def test_fused_decoder_after_the_weights_changed_equals_a_new_decoder(arch, use_
         assert torch.equal(got, want) and torch.equal(dec.logits, new.logits) and not torch.equal(dec.logits, before), change
         assert torch.equal(dec.generate(prompt, 1, use_graph=use_graph)[:, 0], want[:, 0])
         before = dec.logits.clone()
+
+
+def _in_64_bits(model):
+    """The model with its weights as the codes say, in 64 bits (norms and angles stay in 32, as the classes compute them)."""
+    from transformers import LlamaForCausalLM
+    from latentq_llm_b200.quant import QLinearA16W4
+    with torch.device("cuda"):
+        ref = LlamaForCausalLM(model.config).double().eval()
+    ref.model.rotary_emb.inv_freq = model.model.rotary_emb.inv_freq.float()
+    own = dict(model.named_modules())
+    with torch.no_grad():
+        for name, mod in ref.named_modules():
+            src = own[name]
+            if isinstance(src, QLinearA16W4):
+                n, k = src.wshape
+                b = src.weight.data.view(torch.uint8).view(n, -1)
+                q = torch.stack([b >> 4, b & 15], 2).view(n, k // 128, 128).double()
+                s, z = (t.double().view(n, k // 128, 1) for t in src.weight.qparam[:2])
+                mod.weight.copy_(((q - z) * s).view(n, k))
+            elif isinstance(getattr(mod, "weight", None), torch.nn.Parameter):
+                mod.weight.copy_(src.weight)
+    return ref
+
+
+LLAMA3 = {"rope_type": "llama3", "factor": 8.0, "low_freq_factor": 1.0, "high_freq_factor": 4.0, "original_max_position_embeddings": 32, "rope_theta": 10000.0}
+
+
+@pytest.mark.parametrize("arch,P,rope", [("llama-tiny", 1, None), ("llama-tiny", 67, {"rope_type": "linear", "factor": 2.0, "rope_theta": 10000.0}),
+                                         ("llama-gqa-tiny", 9, None), ("llama-gqa-tiny", 131, LLAMA3), ("llama-wide-tiny", 40, None)])
+def test_prompt_through_the_kernels_and_through_the_modules(monkeypatch, arch, P, rope):
+    """Logits of the last prompt token and the cache rows of every layer, against 64 bits: the kernels' route is no further off than the modules' (both round
+    to bf16 in the same places, so their errors are samples of one distribution: half more is allowed).  One token, token counts of the decode kernels and of
+    the GEMM, the RoPE kernels of few and of many heads, grouped key heads, frequencies of other rope types."""
+    from latentq_llm_b200 import finetune as ft
+    from latentq_llm_b200.generate import FusedLlamaGreedyDecoder
+    monkeypatch.setitem(ft.ARCHS, "under test", dict(ft.ARCHS[arch], **({"rope_parameters": rope} if rope else {})))
+    model = ft.build_model("under test", "cuda", seed=3)
+    ft.quantize_decoder(model, lbit=0, gbit=16)
+    model.eval()
+    B = 2
+    prompt = torch.randint(0, 1024, (B, P), device="cuda", generator=torch.Generator(device="cuda").manual_seed(P))
+    with torch.no_grad():
+        out = _in_64_bits(model)(input_ids=prompt, use_cache=True)
+    want = [out.logits[:, -1]] + [t for l in out.past_key_values.layers for t in (l.keys, l.values)]
+
+    def of(dec, logits):
+        return [logits] + [t[:, :, :P] for l in dec.cache.layers for t in (l.keys, l.values)]
+
+    dec, logits = FusedLlamaGreedyDecoder(model, batch=B, max_len=160), []
+    real = dec._prompt_step
+    monkeypatch.setattr(dec, "_prompt_step", lambda p: (logits.append(real(p)), logits[-1])[1])
+    first = dec.generate(prompt, 1, use_graph=False)[:, 0]
+    assert dec.prompt_kernels and len(logits) == 1 and torch.equal(first, logits[0].argmax(-1))
+    assert not any(t[:, :, P:].any() for l in dec.cache.layers for t in (l.keys, l.values))
+    kernels = of(dec, logits[0])
+
+    seen = []
+    hook = model.lm_head.register_forward_hook(lambda mod, args, output: seen.append(output[:, -1]))
+    watched = FusedLlamaGreedyDecoder(model, batch=B, max_len=160)
+    first = watched.generate(prompt, 1, use_graph=False)[:, 0]
+    assert not watched.prompt_kernels and len(seen) == 1 and torch.equal(first, seen[0].argmax(-1))
+    modules = of(watched, seen[0])
+    hook.remove()
+
+    for i, (k, m, w) in enumerate(zip(kernels, modules, want)):
+        ek, em = (float((t.double() - w).norm() / w.norm()) for t in (k, m))
+        assert ek <= 1.5 * em and em < 0.05, (i, ek, em)
+
+
+@pytest.mark.parametrize("cfg", [{"rope_parameters": {"rope_type": "yarn", "factor": 4.0, "rope_theta": 10000.0}},
+                                 {"rope_parameters": {"rope_type": "dynamic", "factor": 2.0, "rope_theta": 10000.0}}, {"attn_implementation": "eager"}], ids=str)
+def test_prompts_that_stay_with_the_modules(monkeypatch, cfg):
+    """The first token is the modules' own; graph replay equals the eager chain behind such a prompt too."""
+    from latentq_llm_b200 import finetune as ft
+    from latentq_llm_b200.generate import FusedLlamaGreedyDecoder
+    monkeypatch.setitem(ft.ARCHS, "under test", dict(ft.ARCHS["llama-gqa-tiny"], **cfg))
+    model = ft.build_model("under test", "cuda", seed=3)
+    ft.quantize_decoder(model, lbit=0, gbit=16)
+    model.eval()
+    prompt = torch.randint(0, 1024, (2, 40), device="cuda", generator=torch.Generator(device="cuda").manual_seed(1))
+    with torch.no_grad():
+        logits = model(input_ids=prompt).logits[:, -1].float()
+    dec = FusedLlamaGreedyDecoder(model, batch=2, max_len=64)
+    got = dec.generate(prompt, 6)
+    assert not dec.prompt_kernels and torch.equal(got, dec.generate(prompt, 6, use_graph=False))
+    chosen = logits.gather(1, got[:, :1])[:, 0]
+    assert bool((chosen >= logits.max(1).values - 0.01 * (logits.max() - logits.min())).all())        # (near-ties: another attention backend without a cache)
