@@ -566,14 +566,30 @@ def gemm_a16w4_fwd_qkv_rope(x, qweight, scales, zeros, positions, inv_freq, k_ca
     return y
 
 
+def _linear_rows_serves(x, w, out):
+    """Whether `lq_linear_rows` may have these operands: plain bf16 matrices of the current device, as the kernel reads and writes them, `out` apart
+    from both (CTAs still read x and w when others write), and nothing that autograd, a transform or a trace would have to see."""
+    if (torch._C._are_functorch_transforms_active() or torch.autograd.forward_ad._current_level >= 0 or torch._C._is_tracing() or torch.compiler.is_compiling()):
+        return False
+    operands = (x, w) if out is None else (x, w, out)
+    if not all(type(t) in (torch.Tensor, torch.nn.Parameter) and t.is_cuda and t.device.index == _current_device() and t.dtype == torch.bfloat16 and t.dim() == 2
+               and t.is_contiguous() for t in operands):
+        return False
+    if torch.is_grad_enabled() and any(t.requires_grad for t in operands):
+        return False
+    (M, K), N = x.shape, w.shape[0]
+    if not (1 <= M <= 8 and N >= 1 and K in (2048, 4096) and w.shape[1] == K and _ptr(x) % 16 == 0 and _ptr(w) % 16 == 0):
+        return False
+    return out is None or (out.shape == (M, N) and all(_ptr(out) + 2 * M * N <= _ptr(t) or _ptr(t) + 2 * t.numel() <= _ptr(out) for t in (x, w)))
+
+
 def linear_rows(x, w, out=None):
-    """y [M, N] = x [M, K] @ w [N, K]^T in bf16, a stream of w for up to 8 tokens (the head of a decode step); more tokens, and
-    widths, types and strides that the kernel does not have, go to torch's linear."""
-    M, K = x.shape
-    served = all(t.is_cuda and t.dtype == torch.bfloat16 and t.is_contiguous() and _ptr(t) % 16 == 0 for t in (x, w)) and w.shape[1:] == (K,)
-    if served and 1 <= M <= 8 and K in (2048, 4096) and (out is None or (out.is_contiguous() and out.dtype == x.dtype and out.shape == (M, w.shape[0]))):
-        y = out if out is not None else torch.empty((M, w.shape[0]), dtype=torch.bfloat16, device=x.device)
-        rc = L.lib.lq_linear_rows(_ptr(x), _ptr(w), _ptr(y), M, w.shape[0], K, _stream())
+    """y [M, N] = x [M, K] @ w [N, K]^T in bf16, a stream of w for up to 8 tokens (the head of a decode step).  Everything that the kernel does
+    not have (more tokens, other widths, types, strides and devices, an `out` that overlaps an operand, gradients) goes to torch's linear."""
+    if _linear_rows_serves(x, w, out):
+        (M, K), N = x.shape, w.shape[0]
+        y = out if out is not None else torch.empty((M, N), dtype=torch.bfloat16, device=x.device)
+        rc = L.lib.lq_linear_rows(_ptr(x), _ptr(w), _ptr(y), M, N, K, _stream())
         if rc != L.LQ_EUNSUPPORTED:
             L.check("lq_linear_rows", rc)
             return y

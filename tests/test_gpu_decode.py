@@ -243,3 +243,14 @@ def test_linear_rows(ops, M, N, K):
     assert torch.equal(out, y)
     wt = w.t().contiguous().t()                           # strides that the kernel does not have
     assert torch.equal(ops.linear_rows(x, wt), torch.nn.functional.linear(x, wt))
+    x8, w8 = x[:1].clone().requires_grad_(True), w.clone()                # gradients at every token count
+    ops.linear_rows(x8, w8).sum().backward()
+    assert torch.equal(x8.grad, torch.autograd.grad(torch.nn.functional.linear(x8, w8).sum(), x8)[0])
+    host = torch.empty(M, N, dtype=torch.bfloat16)
+    assert torch.equal(ops.linear_rows(x, w, out=host), torch.nn.functional.linear(x, w).cpu())
+    if N >= K:                                            # the result over the tokens
+        both = torch.cat([x.reshape(-1), torch.zeros(M * (N - K), dtype=x.dtype, device="cuda")])
+        ops.linear_rows(both[:M * K].view(M, K), w, out=both.view(M, N))
+        assert torch.equal(both.view(M, N), torch.nn.functional.linear(x, w))
+    with pytest.raises(RuntimeError):
+        ops.linear_rows(x, w.cpu())

@@ -203,3 +203,61 @@ def test_plain_calls_are_served_by_the_native_functions(M, monkeypatch):
         with pytest.raises(Exception):
             call()
         assert not any(ok for _, ok in served)
+
+
+class _OnGpu:
+    """What `linear_rows` may ask of a CUDA tensor, without one."""
+
+    def __init__(self, *shape, at=0, index=0, dtype=torch.bfloat16, cuda=True, contiguous=True, grad=False):
+        self.shape, self.at, self.dtype, self.is_cuda, self.requires_grad, self._contiguous = torch.Size(shape), at, dtype, cuda, grad, contiguous
+        self.device = torch.device("cuda", index) if cuda else torch.device("cpu")
+
+    def is_contiguous(self):
+        return self._contiguous
+
+    def data_ptr(self):
+        return self.at
+
+    def dim(self):
+        return len(self.shape)
+
+    def numel(self):
+        return self.shape.numel()
+
+    def copy_(self, y):
+        return self
+
+
+def test_linear_rows_gives_the_kernel_nothing_that_it_may_not_touch(monkeypatch):
+    """Which calls reach the library's entry (a stub here) and which torch's linear, which moves, records or refuses as it always does."""
+    from types import SimpleNamespace
+
+    from latentq_llm_b200 import ops
+    monkeypatch.setattr(torch, "Tensor", _OnGpu)                     # (the stand-ins count as plain tensors)
+    went = []
+    monkeypatch.setattr(ops.L, "lib", SimpleNamespace(lq_linear_rows=lambda *a: (went.append("kernel"), 0)[1]))
+    monkeypatch.setattr(torch.nn.functional, "linear", lambda x, w: (went.append("torch"), _OnGpu(1))[1])
+    monkeypatch.setattr(torch, "empty", lambda shape, dtype=None, device=None: _OnGpu(*shape, at=1 << 40))
+    monkeypatch.setattr(ops, "_current_device", lambda: 0)
+    monkeypatch.setattr(ops, "_stream", lambda: 0)
+    M, N, K, mib = 4, 100, 4096, 1 << 20
+
+    def route(x=None, w=None, out=None, **ctx):
+        went.clear()
+        ops.linear_rows(x or _OnGpu(M, K, at=mib), w or _OnGpu(N, K, at=2 * mib), out)
+        return went
+
+    assert route() == ["kernel"] and route(out=_OnGpu(M, N, at=16 * mib)) == ["kernel"]
+    assert route(out=_OnGpu(M, N, at=mib + 2 * M * K)) == ["kernel"] and route(out=_OnGpu(M, N, at=mib - 2 * M * N)) == ["kernel"]     # side by side
+    for case in (dict(out=_OnGpu(M, N, at=16 * mib, cuda=False)), dict(out=_OnGpu(M, N, at=16 * mib, index=1)), dict(w=_OnGpu(N, K, at=2 * mib, index=1)),
+                 dict(w=_OnGpu(N, K, at=2 * mib, cuda=False)), dict(x=_OnGpu(M, K, at=mib, index=1), w=_OnGpu(N, K, at=2 * mib, index=1)),     # not the current device
+                 dict(out=_OnGpu(M, N, at=mib)), dict(out=_OnGpu(M, N, at=mib + 2 * M * K - 2)), dict(out=_OnGpu(M, N, at=mib - 2 * M * N + 2)),
+                 dict(out=_OnGpu(M, N, at=2 * mib + 64)), dict(out=_OnGpu(N, M, at=16 * mib)), dict(out=_OnGpu(M, N, at=16 * mib, dtype=torch.float32)),
+                 dict(x=_OnGpu(9, K, at=mib)), dict(x=_OnGpu(0, K, at=mib)), dict(x=_OnGpu(M, K, at=mib + 2)), dict(w=_OnGpu(N, K, at=2 * mib, contiguous=False)),
+                 dict(w=_OnGpu(N, 2048, at=2 * mib)), dict(x=_OnGpu(M, K, at=mib, grad=True)), dict(w=_OnGpu(N, K, at=2 * mib, grad=True)),
+                 dict(x=_OnGpu(2, 2, K, at=mib))):
+        assert route(**case) == ["torch"], vars(next(iter(case.values())))
+    with torch.no_grad():
+        assert route(w=_OnGpu(N, K, at=2 * mib, grad=True)) == ["kernel"]
+        with torch.autograd.forward_ad.dual_level():
+            assert route() == ["torch"]
