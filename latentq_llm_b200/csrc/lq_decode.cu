@@ -730,10 +730,14 @@ int lq_rope_kv_store(void* qkv, const int64_t* positions, const float* inv_freq,
         return LQ_EUNSUPPORTED;
     if (M == 0) return LQ_OK;
     { int rc = ensure_device_for(qkv); if (rc) return rc; }
-    // Several heads per thread where all of the work does not fit the chip at once, in vectors of four pairs (8 bytes).  Kernel of one pair per thread / this
-    // one, us, heads of 128: 20 tokens of 48 heads 1.63 / 2.09 (its four angles one after the other), 40 of 48 2.47 / 2.25, 30 of 96 3.46 / 2.27,
-    // 64 of 96 6.9 / 3.2, 400 of 96 40 / 5.7, 3000 of 96 297 / 33.
-    if ((int64_t)M * (Hq + 2 * Hkv) >= 1536 && (hd % 8) == 0 && ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 7) == 0) {
+    // Several heads per thread where all of the work does not fit the chip at once, in vectors of four pairs (8 bytes): 64 tokens of 96 heads of 128 6.9 -> 3.2 us,
+    // 400 40 -> 5.7, 3000 297 -> 33.  A thread's four angles come one after the other, and with few heads or heads above 128 a CTA has few to share them, so small
+    // calls keep the kernel of one pair per thread: time against it at 1536 / 1792 / 2048 / 2560 / 3072 / 4096 / 6144 (token, head) pairs 1.04 / 0.96 / 0.85 / 0.81 / 0.74 /
+    // 0.64 / 0.48 with 48 heads of 128, 1.33 / 1.16 / 1.20 / 1.06 / 0.88 / 0.78 / 0.58 with 48 of 256, 1.16 / 1.04 / 1.06 / 0.94 / 0.81 / 0.69 / 0.48 with 8 of 128,
+    // 1.49 / 1.32 / 1.16 / 1.00 / 1.12 / 0.98 / 0.90 with 3 of 128 (heads of 16, 64 and 512, and 4, 6, 12, 24 and 96 of them, lie in between).
+    const int heads_all = Hq + 2 * Hkv;
+    const int64_t pairs_min = heads_all < 4 ? 6144 : (heads_all < 12 || hd > 128 ? 3072 : 1792);
+    if (M * heads_all >= pairs_min && (hd % 8) == 0 && ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 7) == 0) {
         const int per = 256 / (hd / 8), sets = (Hq + 2 * Hkv + per - 1) / per;
         const int64_t want = (4 * (int64_t)sm_count() + M - 1) / M;
         const dim3 grid4((unsigned)M, (unsigned)(want < sets ? want : sets));

@@ -12,6 +12,20 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA device (run on the B200 box)")
 
 
+@pytest.fixture
+def kernels_of():
+    """Names of the kernels that a call launches, as one text (which of several kernels a size went to)."""
+    def names(call):
+        import torch
+        from torch.profiler import ProfilerActivity, profile
+        torch.cuda.synchronize()
+        with profile(activities=[ProfilerActivity.CUDA], acc_events=True) as p:
+            call()
+            torch.cuda.synchronize()
+        return " ".join(e.name for e in p.events())
+    return names
+
+
 @pytest.fixture(scope="session")
 def golden():
     import numpy as np

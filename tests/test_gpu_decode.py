@@ -70,9 +70,9 @@ def test_rope_kv_store(ops, B, Hq, Hkv, hd, hf):
 
 
 @pytest.mark.parametrize("hf", [True, False])
-@pytest.mark.parametrize("B,P,Hq,Hkv,hd", [(2, 200, 32, 32, 128), (16, 1, 64, 16, 64), (3, 67, 5, 5, 16), (1, 1100, 2, 1, 512), (7, 41, 6, 3, 40)])
+@pytest.mark.parametrize("B,P,Hq,Hkv,hd", [(2, 200, 32, 32, 128), (16, 1, 64, 16, 64), (19, 1, 64, 16, 64), (3, 67, 5, 5, 16), (1, 1100, 2, 1, 512), (7, 41, 6, 3, 40)])
 def test_rope_kv_store_of_many_tokens_equals_the_calls_of_single_tokens(ops, B, P, Hq, Hkv, hd, hf):
-    """From 1536 (token, head) pairs on a thread serves several heads; a token by itself takes the kernel of one rotation pair per thread.
+    """In large calls a thread serves several heads; a token by itself takes the kernel of one rotation pair per thread.
     The same bits: head sets that do not divide the heads, head sizes that leave threads idle, positions beyond the cache."""
     g = torch.Generator(device="cuda").manual_seed(B + P)
     qkv = torch.randn(B * P, (Hq + 2 * Hkv) * hd, device="cuda", generator=g).to(torch.bfloat16)
@@ -86,6 +86,18 @@ def test_rope_kv_store_of_many_tokens_equals_the_calls_of_single_tokens(ops, B, 
         ops.rope_kv_store(want[m:m + 1], pos[m:m + 1], inv_freq, caches[0][b:b + 1], caches[1][b:b + 1], Hq, Hkv, hd, hf_rounding=hf)
     ops.rope_kv_store(qkv, pos, inv_freq, caches[2], caches[3], Hq, Hkv, hd, tokens_per_seq=P, hf_rounding=hf)
     assert torch.equal(qkv, want) and torch.equal(caches[2], caches[0]) and torch.equal(caches[3], caches[1])
+
+
+@pytest.mark.parametrize("P,Hq,Hkv,hd,several", [(18, 32, 32, 128, False), (19, 32, 32, 128, True), (383, 4, 2, 64, False), (384, 4, 2, 64, True),
+                                                 (63, 32, 8, 256, False), (64, 32, 8, 256, True), (2047, 1, 1, 128, False), (2048, 1, 1, 128, True),
+                                                 (400, 6, 3, 12, False)])
+def test_rope_kernel_of_small_and_of_large_calls(ops, kernels_of, P, Hq, Hkv, hd, several):
+    """Both sides of each line of the rule: many heads, few, large ones, three; a head size that is not a multiple of eight keeps the general kernel."""
+    qkv = torch.zeros(P, (Hq + 2 * Hkv) * hd, device="cuda", dtype=torch.bfloat16)
+    cache = [torch.zeros(1, Hkv, P, hd, dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+    pos, inv_freq = torch.arange(P, device="cuda"), torch.ones(hd // 2, device="cuda")
+    names = kernels_of(lambda: ops.rope_kv_store(qkv, pos, inv_freq, *cache, Hq, Hkv, hd, tokens_per_seq=P))
+    assert "k_rope_kv_store" in names and ("k_rope_kv_store4" in names) == several
 
 
 @pytest.mark.parametrize("B,Hq,Hkv,hd,max_len", [(1, 32, 32, 128, 1024), (16, 32, 32, 128, 640), (3, 8, 2, 64, 200), (64, 8, 8, 128, 96)])
