@@ -844,8 +844,13 @@ int lq_argmax_embed(const void* logits, int64_t logits_stride, int64_t B, int64_
     { int rc = ensure_device_for(logits); if (rc) return rc; }
     const int vec = al16p(logits) && (logits_stride % 8) == 0 && (V % 8) == 0;
     // One CTA / a cluster per row, us in a chain: 32000 logits 1 or 2 rows 5.2 / 3.9, 16 rows 5.4 / 4.6, 64 rows 5.5 / 7.4 (four waves of barriers); 8192 logits 3.2 / 3.5;
-    // 50272 logits 2 rows 7.0 / 4.5; 128256 logits 2 rows 13.1 / 6.0, 64 rows 13.6 / 12.3.
-    if (vec && V >= 16384 && (B * AMC <= sm_count() || (V >= 98304 && B <= (1 << 27)))) {
+    // 16384 logits 12 rows 0.96 of the time, 18 rows 1.05, 24576 logits 18 rows 0.98; 50272 logits 2 rows 7.0 / 4.5.  Rows beyond the SMs' number of clusters pay
+    // for large vocabularies, except where single CTAs fill the chip just once: 98304 logits 64 rows 11.0 / 10.9, 128 rows 11.3 / 14.4, 256 rows 20.9 / 23.6;
+    // 150000 logits 48 / 96 / 128 / 192 / 256 / 1000 rows 0.77 / 0.93 / 1.15 / 0.86 / 0.96 / 0.84 of the time, 256000 logits 0.69 / 0.85 / 1.00 / 0.68 / 0.81 / 0.79.
+    const int64_t sms = sm_count();
+    const bool few_rows = B * AMC <= sms && (V >= 24576 || 3 * B * AMC <= 2 * sms);
+    const bool long_rows = (V >= 98304 && B <= 64) || (V >= 131072 && (3 * B <= 2 * sms || B > sms) && B <= (1 << 27));
+    if (vec && V >= 16384 && (few_rows || long_rows)) {
         launch_pdl(k_argmax_embed_cluster, dim3((unsigned)(B * AMC)), (unsigned)AMC_THREADS, 0, (cudaStream_t)stream, (const __nv_bfloat16*)logits, logits_stride, (int)V,
                    (const __nv_bfloat16*)embed, (int)D, (long long*)tok, (long long*)positions, (__nv_bfloat16*)h);
         return check_launch("k_argmax_embed_cluster");

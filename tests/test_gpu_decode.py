@@ -220,7 +220,7 @@ def test_decode_attention_long_contexts(ops, B, Hq, Hkv, hd, max_len, cluster):
     assert float((out.double() - want).abs().max()) <= 2.0 ** -7 * float(want.abs().max())
 
 
-@pytest.mark.parametrize("B,V,D", [(2, 16384, 64), (18, 16392, 8), (3, 100008, 4096), (40, 98304, 264)])
+@pytest.mark.parametrize("B,V,D", [(2, 16384, 64), (18, 16392, 8), (18, 24584, 8), (3, 100008, 4096), (40, 98304, 264)])
 def test_argmax_of_a_large_vocabulary_by_clusters(ops, B, V, D):
     """Eight CTAs per row from 16384 logits on: maxima in the first and last place of a CTA's share, ties across shares, a NaN behind the maximum."""
     logits = torch.randn(B, V, device="cuda", generator=torch.Generator(device="cuda").manual_seed(V)).to(torch.bfloat16)
@@ -235,6 +235,19 @@ def test_argmax_of_a_large_vocabulary_by_clusters(ops, B, V, D):
     assert want[:2].tolist() == [share - 1, 7 * share]
     ops.argmax_embed(logits, tok, pos, embed, h)
     assert torch.equal(tok, want) and torch.equal(pos, torch.arange(B, device="cuda") + 1) and torch.equal(h, embed[want])
+
+
+@pytest.mark.parametrize("B,V,cluster", [(2, 16376, False), (12, 16384, True), (13, 16384, False), (18, 24576, True), (19, 24576, False), (64, 98304, True),
+                                         (65, 98304, False), (98, 131072, True), (99, 131072, False), (148, 131072, False), (149, 131072, True), (2, 16390, False)])
+def test_argmax_by_clusters_where_they_are_faster(ops, kernels_of, B, V, cluster):
+    """Both sides of each line of the rule, on 148 SMs; rows that are not whole vectors keep the single CTA."""
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the numbers of rows are those of 148 SMs")
+    logits = torch.randn(B, V, device="cuda", generator=torch.Generator(device="cuda").manual_seed(V)).to(torch.bfloat16)
+    tok = torch.zeros(B, dtype=torch.long, device="cuda")
+    names = kernels_of(lambda: ops.argmax_embed(logits, tok))
+    assert "k_argmax_embed" in names and ("k_argmax_embed_cluster" in names) == cluster
+    assert torch.equal(tok, logits.float().argmax(-1))
 
 
 @pytest.mark.parametrize("M,N,K", [(1, 32000, 4096), (8, 1003, 4096), (2, 16 * 149, 4096), (3, 50, 2048), (5, 50272, 2048), (1, 7, 2048), (9, 100, 4096), (2, 100, 512)])
