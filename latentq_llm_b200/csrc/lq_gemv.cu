@@ -1219,6 +1219,7 @@ __global__ void __launch_bounds__(R2_WARPS * 32, 1) k_skinny_rows2(const SkinnyP
     }
 }
 
+constexpr int SK_UNROLLED_K = 11008;      // the contraction, besides 4096, that the kernels of one row block per CTA have a written-out loop for (eleven chunks a warp)
 bool skinny_norm_supported(int64_t M, int64_t K, int group) {
     return M >= 1 && M <= 2 && K == 4096 && group == 128 && LQ_GEMV_PF == 4 && !getenv("LQ_SKINNY_NO_NC4") && !getenv("LQ_SKINNY_NO_STREAM");
 }
@@ -1268,7 +1269,7 @@ static int launch_skinny_stream(const SkinnyParams& p, cudaStream_t st) {
     }
     // (k_skinny_wide also works for fewer tokens, but two CTAs per SM are the better half of eight: 8 tokens 14.8 / 14.9 us at 22016 rows, 5 tokens 13.9 / 14.6)
     if (nc4) return mt == 1 ? launch_skinny_stream_v<1, 1, 4>(p, x_stride, smem, grid, st) : launch_skinny_wide(p, st);
-    if (mt == 1 && gc == 1 && p.K == 11008 && LQ_GEMV_PF == 4 && !getenv("LQ_SKINNY_NO_NC4"))      // eleven chunks per warp, written out
+    if (mt == 1 && gc == 1 && p.K == SK_UNROLLED_K && LQ_GEMV_PF == 4 && !getenv("LQ_SKINNY_NO_NC4"))      // eleven chunks per warp, written out
         return launch_skinny_stream_v<1, 1, 11>(p, x_stride, smem, grid, st);
     if (mt == 1) return gc == 1 ? launch_skinny_stream_v<1, 1>(p, x_stride, smem, grid, st) : launch_skinny_stream_v<1, 2>(p, x_stride, smem, grid, st);
     return gc == 1 ? launch_skinny_stream_v<2, 1>(p, x_stride, smem, grid, st) : launch_skinny_stream_v<2, 2>(p, x_stride, smem, grid, st);
@@ -1293,11 +1294,21 @@ int launch_skinny_rows(const SkinnyParams& p, cudaStream_t st) {
         skinny_stream_smem(p.M, p.K, p.group) <= (size_t)(p.M > 8 ? 144 : 96) * 1024)
         return launch_skinny_stream(p, st);
     if (p.norm_gamma) return LQ_EUNSUPPORTED;       // the fused-norm staging exists in the streaming kernel only
-    // Two row blocks per CTA where more than one falls to an SM anyway.  K = 4096 keeps its written-out loop (4096 -> 4096, 16 tokens 5.3 / 6.1 us), and so does
-    // K = 11008 up to 8 tokens (8.7 .. 9.6 / 9.0 .. 9.6 us).  Up to 8 tokens, old and new (us at 1 / 8 tokens): 4352 -> 2432 4.5 / 4.65, 4.4 / 4.75; 4608 -> 4096 5.0 / 5.5,
-    // 4.9 / 5.35; 5632 -> 4096 6.0 / 6.35, 5.5 / 5.9; 14336 -> 4096 12.3 / 13.0, 10.8 / 11.45; where a CTA per SM is not enough, at 3 tokens: 5632 -> 11264 15.4, 15.7; 14336 -> 8192 23.9, 21.9.
-    const bool few_ok = p.K >= 4608 && p.K != 11008 && (n_row_blocks <= 2 * sm_count() || p.K >= 8192);
-    if ((p.M > 8 ? p.K > 4096 : few_ok) && p.group == 128 && p.K % 256 == 0 && n_row_blocks > sm_count() && (int64_t)n_row_blocks * 16 * p.K < (int64_t)1 << 35 &&
+    // Two row blocks per CTA where more than one falls to an SM anyway.  A CTA has twelve warps to share K / 256 steps and an SM has one CTA, so what counts is how
+    // evenly the steps fall to the warps (K = 5376, 5632, 6144, 9216 or 12288: 7/8 or more of them busy throughout; 4608, 5120, 6912, 7168: 3/4 to 5/6) and whether the last
+    // round of CTAs fills the SMs.  K = 4096 keeps its written-out loop (4096 -> 4096, 16 tokens 5.3 / 6.1 us), and so does K = 11008 but for one round of 9-16 tokens.
+    // Time against the kernel of one row block per CTA, 152 / 256 / 296 / 300 / 352 / 444 / 512 / 592 / 600 / 900 / 1376 row blocks:
+    //   9 tokens   K = 5120  0.95 / 0.98 / 0.98 / 1.05 / 1.04 / 1.01 / 0.96 / 0.97 / 1.00 / 1.00 / 0.97     6912  0.95 / 0.98 / 0.99 / 1.07 / 1.09 / 1.03 / 0.99 / 0.99 / 1.05 / 1.04 / 1.00
+    //              K = 9216  0.84 / 0.89 / 0.90 / 0.97 / 0.98 / 0.93 / 0.90 / 0.91 / 0.97 / 0.96 / 0.91    11008  0.89 / 0.93 / 0.95 / 1.04 / 1.05 / 0.99 / 0.95 / 0.95 / 1.04 / 1.02 / 0.95
+    //   8 tokens   K = 5120  1.04 / 0.96 / 0.92     5376  0.92 / 0.91 / 0.93     6912  1.02 / 0.97 / 0.96     8192  0.87 / 0.84 / 0.83
+    //              K = 9216  0.92 / 0.91 / 0.91 / 1.02 / 1.02 / 0.95 / 0.91 / 0.92 / 0.98 / 0.96 / 0.92    12288  0.82 / 0.84 / 0.87 / 0.94 / 0.97 / 0.86 / 0.85 / 0.86 / 0.93 / 0.91 / 0.87
+    // and at 3 tokens 5632 -> 11264 15.4 / 15.7 us, so that up to 8 tokens more than one round needs K >= 8192.
+    const int64_t sms = sm_count(), ctas = (n_row_blocks + 1) / 2, slots = (ctas + sms - 1) / sms * sms, idle = slots - ctas;
+    const int steps = p.K / 256, turns = (steps + R2_WARPS - 1) / R2_WARPS;
+    const bool even = 8 * steps >= 7 * R2_WARPS * turns, unrolled = p.K == 4096 || p.K == SK_UNROLLED_K;
+    const bool rows2 = p.M > 8 ? p.K > 4096 && (ctas <= sms || 20 * idle <= 3 * slots || (p.K >= 8192 && even && !unrolled))
+                               : p.K > 4096 && !unrolled && (ctas <= sms ? even || p.K >= 8192 : p.K >= 8192 && (4 * idle <= slots || p.K >= 12288));
+    if (rows2 && p.group == 128 && p.K % 256 == 0 && n_row_blocks > sms && (int64_t)n_row_blocks * 16 * p.K < (int64_t)1 << 35 &&
         ((reinterpret_cast<uintptr_t>(p.scales) | reinterpret_cast<uintptr_t>(p.zeros)) & 3) == 0) {
         if (p.M > 8) launch_pdl(k_skinny_rows2<2>, dim3((n_row_blocks + 1) / 2), R2_WARPS * 32, 0, st, p);
         else launch_pdl(k_skinny_rows2<1>, dim3((n_row_blocks + 1) / 2), R2_WARPS * 32, 0, st, p);
@@ -1316,7 +1327,7 @@ int launch_skinny_rows(const SkinnyParams& p, cudaStream_t st) {
         if (p.M > 8) launch_pdl(k_skinny_rows<2, 1, 4, true>, g, th, 0, st, p);
         else if (w64) launch_pdl(k_skinny_rows<1, 1, 4, true>, g, th, 0, st, p);
         else launch_pdl(k_skinny_rows<1, 1, 4>, g, th, 0, st, p);
-    } else if (g128 && p.K == 11008 && !getenv("LQ_SKINNY_NO_NC4")) {          // eleven chunks per warp, written out
+    } else if (g128 && p.K == SK_UNROLLED_K && !getenv("LQ_SKINNY_NO_NC4")) {          // eleven chunks per warp, written out
         if (p.M > 8) launch_pdl(k_skinny_rows<2, 1, 11, true>, g, th, 0, st, p);
         else if (w64) launch_pdl(k_skinny_rows<1, 1, 11, true>, g, th, 0, st, p);
         else launch_pdl(k_skinny_rows<1, 1, 11>, g, th, 0, st, p);

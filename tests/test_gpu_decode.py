@@ -251,7 +251,7 @@ def test_argmax_by_clusters_where_they_are_faster(ops, kernels_of, B, V, cluster
 
 
 @pytest.mark.parametrize("M,N,K", [(1, 32000, 4096), (8, 1003, 4096), (2, 16 * 149, 4096), (3, 50, 2048), (5, 50272, 2048), (1, 7, 2048), (9, 100, 4096), (2, 100, 512)])
-def test_linear_rows(ops, M, N, K):
+def test_linear_rows(ops, kernels_of, M, N, K):
     """The head of a decode step against fp32 matmul: row counts that leave a block of 16 incomplete, fewer and more blocks than SMs, all token counts' edges; the
     last two go to torch's linear.  One rounding to bf16, and fp32 sums of K products in any order."""
     g = torch.Generator(device="cuda").manual_seed(M + N)
@@ -265,7 +265,7 @@ def test_linear_rows(ops, M, N, K):
             assert torch.equal(y, torch.nn.functional.linear(x, w))
         else:
             assert y.shape == (M, N) and bool(((y.double() - ref).abs() <= bound).all())
-    assert torch.equal(out, y)
+    assert torch.equal(out, y) and ("k_linear_rows" in kernels_of(lambda: ops.linear_rows(x, w))) == (M <= 8 and K != 512)
     wt = w.t().contiguous().t()                           # strides that the kernel does not have
     assert torch.equal(ops.linear_rows(x, wt), torch.nn.functional.linear(x, wt))
     x8, w8 = x[:1].clone().requires_grad_(True), w.clone()                # gradients at every token count

@@ -326,7 +326,7 @@ def test_mma_issue_rate_probe_runs_and_rejects_bad_arguments():
 
 
 @pytest.mark.parametrize("M,N", [(9, 12288), (16, 12352), (13, 22016), (16, 12288 + 148 * 32)])
-def test_a16w4_nine_to_sixteen_tokens_of_a_large_projection(ops, M, N):
+def test_a16w4_nine_to_sixteen_tokens_of_a_large_projection(ops, kernels_of, M, N):
     """9 to 16 tokens, K = 4096, from 768 row blocks on: two row blocks per step, as many steps as CTAs, one more, a remainder.  Against 64 bits: the sum
     and the sum plus the bias are rounded to bf16 (8 significant bits: at most 2^-8 of a value, 2^-15 of it for the second order), and a group's sum of (128 + q) x, at most 143 sum |x|, is added up in 32 bits in at most 32 roundings or truncations
     (2^-23 each).  The outputs of a token do not depend on the others, whatever those hold."""
@@ -341,6 +341,7 @@ def test_a16w4_nine_to_sixteen_tokens_of_a_large_projection(ops, M, N):
     v = x.double() @ ((q - z) * s).view(N, K).t()
     acc = 143 * x.double().abs().view(M, K // 128, 128).sum(2) @ s.view(N, K // 128).abs().t()
     y = ops.gemm_a16w4_fwd(x, codes, sb, zb, bias, N, K)
+    assert "k_skinny_wide" in kernels_of(lambda: ops.gemm_a16w4_fwd(x, codes, sb, zb, bias, N, K))
     assert bool(((y.double() - v - bias.double()).abs() <= (2.0 ** -8 + 2.0 ** -15) * (2 * v.abs() + bias.double().abs()) + 2.0 ** -18 * acc).all())
     act = ops.gemm_a16w4_fwd_silu(x, codes, sb, zb, N // 2, K)
     assert torch.equal(act, ops.silu_mul(ops.gemm_a16w4_fwd(x, codes, sb, zb, None, N, K)))
@@ -349,9 +350,10 @@ def test_a16w4_nine_to_sixteen_tokens_of_a_large_projection(ops, M, N):
     assert torch.equal(y2[keep], y[keep]) and not bool(torch.isfinite(y2[[3, M - 1]].float()).any())
 
 
-@pytest.mark.parametrize("M,Hq,Hkv,K", [(9, 16, 4, 4352), (16, 32, 0, 11008), (12, 20, 5, 5632), (13, 19, 0, 4608), (1, 16, 4, 4608), (8, 20, 5, 5632), (3, 64, 0, 8192)])
-def test_a16w4_decode_projection_over_a_long_contraction(ops, M, Hq, Hkv, K):
-    """Up to 16 tokens, K > 4096 in steps of 256 that the warps of a CTA share unevenly (17, 43, 22, 18 and 32 steps), two row blocks of 16 per CTA.  Against 64 bits: two
+@pytest.mark.parametrize("M,Hq,Hkv,K", [(9, 16, 4, 4352), (16, 32, 0, 11008), (12, 20, 5, 5632), (13, 19, 0, 4608), (1, 16, 4, 4608), (8, 20, 5, 5632), (3, 64, 0, 8192),
+                                        (1, 16, 4, 5632), (10, 64, 0, 6144), (5, 40, 0, 12288)])
+def test_a16w4_decode_projection_over_a_long_contraction(ops, kernels_of, M, Hq, Hkv, K):
+    """Up to 16 tokens, K > 4096 in steps of 256 that the warps of a CTA share unevenly (17, 43, 22, 18, 32, 24 and 48 steps), two row blocks of 16 per CTA.  Against 64 bits: two
     roundings to bf16 (2^-8 each, as above), and group sums of (q - z) x, at most 15 sum |x|, in at most 32 roundings or truncations of 2^-23, K / 128
     more where they are added up.  The fused epilogues give the bits of the separate launches."""
     hd, N = 128, (Hq + 2 * Hkv) * 128
@@ -366,6 +368,7 @@ def test_a16w4_decode_projection_over_a_long_contraction(ops, M, Hq, Hkv, K):
     acc = 15 * x.double().abs().view(M, K // 128, 128).sum(2) @ s.view(N, K // 128).abs().t()
     y = ops.gemm_a16w4_fwd(x, codes, sb, zb, bias, N, K)
     assert bool(((y.double() - v - bias.double()).abs() <= (2.0 ** -8 + 2.0 ** -15) * (2 * v.abs() + bias.double().abs()) + (32 + K // 128) * 2.0 ** -23 * acc).all())
+    assert ("k_skinny_rows2" in kernels_of(lambda: ops.gemm_a16w4_fwd(x, codes, sb, zb, bias, N, K))) == ((M, K) != (1, 4608))      # (18 steps for 12 warps)
     plain = ops.gemm_a16w4_fwd(x, codes, sb, zb, None, N, K)
     assert torch.equal(ops.gemm_a16w4_fwd_silu(x, codes, sb, zb, N // 2, K), ops.silu_mul(plain))
     if Hkv:
@@ -376,6 +379,25 @@ def test_a16w4_decode_projection_over_a_long_contraction(ops, M, Hq, Hkv, K):
         got = ops.gemm_a16w4_fwd_qkv_rope(x, codes, sb, zb, pos, inv_freq, kc, vc, Hq, Hkv, hd, K)
         ops.rope_kv_store(plain, pos, inv_freq, kw, vw, Hq, Hkv, hd)
         assert torch.equal(got, plain) and torch.equal(kc, kw) and torch.equal(vc, vw)
+
+
+@pytest.mark.parametrize("M,blocks,K,two", [(9, 148, 4352, False), (9, 152, 4352, True), (16, 296, 11008, True), (12, 300, 11008, False), (9, 300, 5120, False),
+                                            (16, 512, 5120, True), (9, 300, 8192, True), (9, 300, 10240, False), (8, 256, 4608, False), (1, 256, 5376, True),
+                                            (8, 256, 6912, False), (8, 256, 10240, True), (8, 256, 11008, False), (3, 300, 8192, False), (3, 444, 8192, True),
+                                            (8, 300, 12288, True), (3, 512, 5632, False), (16, 296, 4096, False)])
+def test_a16w4_two_row_blocks_per_cta_where_they_are_faster(ops, kernels_of, M, blocks, K, two):
+    """Both sides of each line of the rule, on 148 SMs: more row blocks than SMs, rounds of CTAs that leave SMs idle, steps that leave warps idle, contractions with
+    a written-out loop.  Either kernel's result against the dequantized weight."""
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the numbers of row blocks are those of 148 SMs")
+    N = 16 * blocks
+    codes, sb, zb = make_w4_layer(ops, N, K, seed=23)
+    x = torch.randn(M, K, device="cuda", generator=torch.Generator(device="cuda").manual_seed(M)).to(torch.bfloat16)
+    out = []
+    names = kernels_of(lambda: out.append(ops.gemm_a16w4_fwd(x, codes, sb, zb, None, N, K)))
+    assert "k_skinny_" in names and ("k_skinny_rows2" in names) == two
+    e_max, e_fro = rel_err(out[0], x.float() @ ops.a16w4_dequant(codes, sb, zb, (N, K), torch.bfloat16).float().t())
+    assert e_max < RTOL and e_fro < RTOL
 
 
 @pytest.mark.parametrize("K", [4096, 11008])
