@@ -402,20 +402,22 @@ def test_a16w4_two_row_blocks_per_cta_where_they_are_faster(ops, kernels_of, M, 
 
 @pytest.mark.parametrize("K", [4096, 11008])
 @pytest.mark.parametrize("M,N,force_stream", [(1, 4096, True), (2, 12288, True), (1, 1088, True), (12, 4160, True),
-                                              (5, 4096, False), (16, 12288, False), (9, 1088, False), (3, 4160, False)])
-def test_a16w4_decode_kernels_written_out_loop_equals_general_loop(ops, monkeypatch, M, N, force_stream, K):
+                                              (5, 4096, False), (16, 12288, False), (9, 1088, False), (3, 4160, False),
+                                              (12, 2304, True), (16, 2368, False)])
+def test_a16w4_decode_kernels_written_out_loop_equals_general_loop(ops, monkeypatch, kernels_of, M, N, force_stream, K):
     """K = 4096 with groups of 128 runs the decode kernels' written-out loops (four chunks per warp, group parameters
     as 8-byte loads, constant offsets): the streaming kernel (one or two tokens, or forced) and the row-block kernel.
     Same operations in the same order as the general loops: identical bits, with bias, for more and for fewer row
     blocks than persistent CTAs, one and two token groups; the fused gate|up + silu epilogue included.  K = 11008 (eleven
-    chunks per warp, nine in the last one) has written-out loops of its own."""
+    chunks per warp, nine in the last one) has written-out loops of its own; 9 to 16 tokens of it take them up to 148 row blocks (N = 2368), beyond that
+    the kernel of two row blocks per CTA, which has one loop."""
     codes, sb, zb = make_w4_layer(ops, N, K, seed=11)
     g = torch.Generator(device="cuda").manual_seed(N + M)
     x = torch.randn(M, K, device="cuda", generator=g).to(torch.bfloat16)
     bias = (torch.randn(N, device="cuda", generator=g) * 0.1).to(torch.bfloat16)
     if force_stream:
         monkeypatch.setenv("LQ_SKINNY_STREAM_ALL", "1")         # (M = 12 takes the streaming kernel only when forced)
-    out = {}
+    out, ran = {}, {}
     for mode in ("written_out", "general"):
         if mode == "general":
             monkeypatch.setenv("LQ_SKINNY_NO_NC4", "1")
@@ -425,6 +427,8 @@ def test_a16w4_decode_kernels_written_out_loop_equals_general_loop(ops, monkeypa
         y = ops.gemm_a16w4_fwd(x, codes, sb, zb, bias, N, K)
         act = ops.gemm_a16w4_fwd_silu(x, codes, sb, zb, N // 2, K, hf_rounding=1) if N % 16 == 0 else None
         out[mode] = (y, act)
+        ran[mode] = kernels_of(lambda: ops.gemm_a16w4_fwd(x, codes, sb, zb, bias, N, K))
+    assert "k_skinny_" in ran["general"] and (ran["general"] != ran["written_out"]) == (K == 4096 or M <= 8 or N <= 2368)
     assert torch.equal(out["written_out"][0], out["general"][0])
     if out["general"][1] is not None:
         assert torch.equal(out["written_out"][1], out["general"][1])
