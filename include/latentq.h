@@ -38,6 +38,8 @@ LQ_API int lq_version(void);
 LQ_API const char* lq_status_string(int status);
 /* cudaGetLastError-style text of the most recent LQ_ECUDA on this thread. */
 LQ_API const char* lq_last_cuda_error(void);
+/* Name of the kernel, or of the family of kernels, that this thread launched last ("" before the first): which of several a size went to. */
+LQ_API const char* lq_last_launch(void);
 
 /* ------------------------------------------------------------------------
  * Residual codecs: the five functions of the pybind module `MyQuantDequant`

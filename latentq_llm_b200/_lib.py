@@ -60,7 +60,7 @@ SIGNATURES = {
     "lq_version": [],
     "lq_decode_chain": [_i],
     "lq_status_string": [_i],
-    "lq_last_cuda_error": [],
+    "lq_last_cuda_error": [], "lq_last_launch": [],
     "lq_res3_quant": [_p, _i, _p, _i64, _i, _f, _i, _f, _i, _f, _p],
     "lq_res3_dequant": [_p, _p, _i, _i64, _i, _f, _i, _f, _i, _p],
     "lq_resu_quant": [_p, _i, _p, _i64, _f, _p],
@@ -114,7 +114,7 @@ SIGNATURES = {
     "lq_silu_mul": [_p, _p, _i64, _i64, _i, _p],
     "lq_gemm_a16w4_fwd_silu": [_p, _p, _p, _p, _p, _i64, _i64, _i64, _i, _i, _p],
 }
-_RESTYPE = {"lq_status_string": C.c_char_p, "lq_last_cuda_error": C.c_char_p, "lq_gemm_workspace_bytes": C.c_size_t,
+_RESTYPE = {"lq_status_string": C.c_char_p, "lq_last_cuda_error": C.c_char_p, "lq_last_launch": C.c_char_p, "lq_gemm_workspace_bytes": C.c_size_t,
             "lq_gemm_a16w4_fwd_static_max_bytes": C.c_size_t, "lq_decode_attention_workspace_bytes": C.c_size_t}
 
 for _name, _args in SIGNATURES.items():

@@ -494,7 +494,7 @@ template <int MT, int GC, int NCH, bool NORM = false>
 __global__ void __launch_bounds__(RB_WARPS * 32, MT == 2 ? 1 : LQ_GEMV_MINB) k_skinny_stream(const SkinnyParams p, const int x_stride) {
     constexpr int PF = LQ_GEMV_PF;
     constexpr bool NC4 = NCH == 4;
-    static_assert(NCH == 0 || (GC == 1 && PF == 4), "the written-out loops are for group 128 and a ring of four chunks");
+    static_assert(NCH == 0 || (MT == 1 && GC == 1 && PF == 4), "the written-out loops are for up to 8 tokens, group 128 and a ring of four chunks");
     extern __shared__ __align__(16) uint8_t ss_smem[];
     uint4* xs = reinterpret_cast<uint4*>(ss_smem);                                               // [M][x_stride]
     float* sxs = reinterpret_cast<float*>(ss_smem + (size_t)p.M * x_stride * 16);               // [groups][8 * MT]
@@ -689,11 +689,9 @@ __global__ void __launch_bounds__(RB_WARPS * 32, MT == 2 ? 1 : LQ_GEMV_MINB) k_s
     }
 
     int buf = 0;
-    // NC4: per-warp bases of the staged tokens and token sums (everything else is a compile-time offset)
-    const uint4* xbase[MT];
-#pragma unroll
-    for (int m = 0; m < MT; ++m) xbase[m] = xs + (size_t)xrow[m] * x_stride + g_begin * 16 + t;
-    const float* sxbase = sxs + g_begin * (8 * MT) + 2 * t;
+    // written-out loops: per-warp bases of the staged tokens and token sums (everything else is a compile-time offset)
+    const uint4* xbase = xs + (size_t)xrow[0] * x_stride + g_begin * 16 + t;
+    const float* sxbase = sxs + g_begin * 8 + 2 * t;
     for (; blk < n_blocks; blk += gridDim.x) {
         const int nblk = blk + (int)gridDim.x;
         const bool has_next = nblk < n_blocks;
@@ -715,16 +713,13 @@ __global__ void __launch_bounds__(RB_WARPS * 32, MT == 2 ? 1 : LQ_GEMV_MINB) k_s
 #pragma unroll
                 for (int w = 0; w < 4; ++w) {
                     LQ_WORD_FRAGS(wsa[w], wsb[w]);
-#pragma unroll
-                    for (int m = 0; m < MT; ++m) {
-                        const uint4 f = xbase[m][u * 16 + w * 4];
-                        if (w == 0) {
-                            mma_s_start(acc[m][0], a00, a01, a02, a03, f.x, f.y);
-                            mma_s_start(acc[m][1], a10, a11, a12, a13, f.z, f.w);
-                        } else {
-                            mma_s(acc[m][0], a00, a01, a02, a03, f.x, f.y);
-                            mma_s(acc[m][1], a10, a11, a12, a13, f.z, f.w);
-                        }
+                    const uint4 f = xbase[u * 16 + w * 4];
+                    if (w == 0) {
+                        mma_s_start(acc[0][0], a00, a01, a02, a03, f.x, f.y);
+                        mma_s_start(acc[0][1], a10, a11, a12, a13, f.z, f.w);
+                    } else {
+                        mma_s(acc[0][0], a00, a01, a02, a03, f.x, f.y);
+                        mma_s(acc[0][1], a10, a11, a12, a13, f.z, f.w);
                     }
                 }
                 // group u of the slice: bf16 bits (u & 1 ? high : low) half of word (u >> 1) of the packed loads
@@ -734,14 +729,11 @@ __global__ void __launch_bounds__(RB_WARPS * 32, MT == 2 ? 1 : LQ_GEMV_MINB) k_s
                 const float z_a = __uint_as_float((u & 1) ? (zw_a & 0xffff0000u) : (zw_a << 16)) + 128.0f;
                 const float s_b = __uint_as_float((u & 1) ? (sw_b & 0xffff0000u) : (sw_b << 16));
                 const float z_b = __uint_as_float((u & 1) ? (zw_b & 0xffff0000u) : (zw_b << 16)) + 128.0f;
-#pragma unroll
-                for (int m = 0; m < MT; ++m) {
-                    const float2 sx = *reinterpret_cast<const float2*>(sxbase + u * (8 * MT) + m * 8);
-                    tot[m][0] = fmaf(s_a, (acc[m][0][0] + acc[m][1][0]) - z_a * sx.x, tot[m][0]);
-                    tot[m][1] = fmaf(s_a, (acc[m][0][1] + acc[m][1][1]) - z_a * sx.y, tot[m][1]);
-                    tot[m][2] = fmaf(s_b, (acc[m][0][2] + acc[m][1][2]) - z_b * sx.x, tot[m][2]);
-                    tot[m][3] = fmaf(s_b, (acc[m][0][3] + acc[m][1][3]) - z_b * sx.y, tot[m][3]);
-                }
+                const float2 sx = *reinterpret_cast<const float2*>(sxbase + u * 8);
+                tot[0][0] = fmaf(s_a, (acc[0][0][0] + acc[0][1][0]) - z_a * sx.x, tot[0][0]);
+                tot[0][1] = fmaf(s_a, (acc[0][0][1] + acc[0][1][1]) - z_a * sx.y, tot[0][1]);
+                tot[0][2] = fmaf(s_b, (acc[0][0][2] + acc[0][1][2]) - z_b * sx.x, tot[0][2]);
+                tot[0][3] = fmaf(s_b, (acc[0][0][3] + acc[0][1][3]) - z_b * sx.y, tot[0][3]);
             }
             s4a = ns4a; z4a = nz4a; s4b = ns4b; z4b = nz4b;
         }
@@ -770,28 +762,22 @@ __global__ void __launch_bounds__(RB_WARPS * 32, MT == 2 ? 1 : LQ_GEMV_MINB) k_s
 #pragma unroll
                     for (int w = 0; w < 4; ++w) {
                         LQ_WORD_FRAGS(wsa[w], wsb[w]);
-#pragma unroll
-                        for (int m = 0; m < MT; ++m) {
-                            const uint4 f = xbase[m][c * 16 + w * 4];
-                            if (w == 0) {
-                                mma_s_start(acc[m][0], a00, a01, a02, a03, f.x, f.y);
-                                mma_s_start(acc[m][1], a10, a11, a12, a13, f.z, f.w);
-                            } else {
-                                mma_s(acc[m][0], a00, a01, a02, a03, f.x, f.y);
-                                mma_s(acc[m][1], a10, a11, a12, a13, f.z, f.w);
-                            }
+                        const uint4 f = xbase[c * 16 + w * 4];
+                        if (w == 0) {
+                            mma_s_start(acc[0][0], a00, a01, a02, a03, f.x, f.y);
+                            mma_s_start(acc[0][1], a10, a11, a12, a13, f.z, f.w);
+                        } else {
+                            mma_s(acc[0][0], a00, a01, a02, a03, f.x, f.y);
+                            mma_s(acc[0][1], a10, a11, a12, a13, f.z, f.w);
                         }
                     }
                     const float s_a = __uint_as_float(sz_a << 16), z_a = __uint_as_float(sz_a & 0xffff0000u) + 128.0f;
                     const float s_b = __uint_as_float(sz_b << 16), z_b = __uint_as_float(sz_b & 0xffff0000u) + 128.0f;
-#pragma unroll
-                    for (int m = 0; m < MT; ++m) {
-                        const float2 sx = *reinterpret_cast<const float2*>(sxbase + c * (8 * MT) + m * 8);
-                        tot[m][0] = fmaf(s_a, (acc[m][0][0] + acc[m][1][0]) - z_a * sx.x, tot[m][0]);
-                        tot[m][1] = fmaf(s_a, (acc[m][0][1] + acc[m][1][1]) - z_a * sx.y, tot[m][1]);
-                        tot[m][2] = fmaf(s_b, (acc[m][0][2] + acc[m][1][2]) - z_b * sx.x, tot[m][2]);
-                        tot[m][3] = fmaf(s_b, (acc[m][0][3] + acc[m][1][3]) - z_b * sx.y, tot[m][3]);
-                    }
+                    const float2 sx = *reinterpret_cast<const float2*>(sxbase + c * 8);
+                    tot[0][0] = fmaf(s_a, (acc[0][0][0] + acc[0][1][0]) - z_a * sx.x, tot[0][0]);
+                    tot[0][1] = fmaf(s_a, (acc[0][0][1] + acc[0][1][1]) - z_a * sx.y, tot[0][1]);
+                    tot[0][2] = fmaf(s_b, (acc[0][0][2] + acc[0][1][2]) - z_b * sx.x, tot[0][2]);
+                    tot[0][3] = fmaf(s_b, (acc[0][0][3] + acc[0][1][3]) - z_b * sx.y, tot[0][3]);
                 }
             }
         }

@@ -19,7 +19,9 @@ static thread_local std::string g_last_error;
 void set_cuda_error(cudaError_t e, const char* where) {
     g_last_error = std::string(where) + ": " + cudaGetErrorString(e);
 }
+static thread_local const char* g_last_launch = "";
 int check_launch(const char* where) {
+    g_last_launch = where;
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) { set_cuda_error(e, where); return LQ_ECUDA; }
     return LQ_OK;
@@ -1191,6 +1193,7 @@ const char* lq_status_string(int s) {
     return "unknown status";
 }
 const char* lq_last_cuda_error(void) { return g_last_error.c_str(); }
+const char* lq_last_launch(void) { return lq::g_last_launch; }
 
 int lq_res3_quant(void* x, int dtype, int32_t* words, int64_t n_words, int k1, float b1, int k2, float b2, int k3,
                   float v0, lq_stream_t stream) {

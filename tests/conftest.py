@@ -13,17 +13,13 @@ def pytest_configure(config):
 
 
 @pytest.fixture
-def kernels_of():
-    """Names of the kernels that a call launches, as one text (which of several kernels a size went to)."""
-    def names(call):
-        import torch
-        from torch.profiler import ProfilerActivity, profile
-        torch.cuda.synchronize()
-        with profile(activities=[ProfilerActivity.CUDA], acc_events=True) as p:
-            call()
-            torch.cuda.synchronize()
-        return " ".join(e.name for e in p.events())
-    return names
+def kernel_of():
+    """Name of the kernel that a call launched last (which of several a size went to)."""
+    def name(call):
+        from latentq_llm_b200 import _lib
+        call()
+        return _lib.lib.lq_last_launch().decode()
+    return name
 
 
 @pytest.fixture(scope="session")

@@ -326,7 +326,7 @@ def test_mma_issue_rate_probe_runs_and_rejects_bad_arguments():
 
 
 @pytest.mark.parametrize("M,N", [(9, 12288), (16, 12352), (13, 22016), (16, 12288 + 148 * 32)])
-def test_a16w4_nine_to_sixteen_tokens_of_a_large_projection(ops, kernels_of, M, N):
+def test_a16w4_nine_to_sixteen_tokens_of_a_large_projection(ops, kernel_of, M, N):
     """9 to 16 tokens, K = 4096, from 768 row blocks on: two row blocks per step, as many steps as CTAs, one more, a remainder.  Against 64 bits: the sum
     and the sum plus the bias are rounded to bf16 (8 significant bits: at most 2^-8 of a value, 2^-15 of it for the second order), and a group's sum of (128 + q) x, at most 143 sum |x|, is added up in 32 bits in at most 32 roundings or truncations
     (2^-23 each).  The outputs of a token do not depend on the others, whatever those hold."""
@@ -341,7 +341,7 @@ def test_a16w4_nine_to_sixteen_tokens_of_a_large_projection(ops, kernels_of, M, 
     v = x.double() @ ((q - z) * s).view(N, K).t()
     acc = 143 * x.double().abs().view(M, K // 128, 128).sum(2) @ s.view(N, K // 128).abs().t()
     y = ops.gemm_a16w4_fwd(x, codes, sb, zb, bias, N, K)
-    assert "k_skinny_wide" in kernels_of(lambda: ops.gemm_a16w4_fwd(x, codes, sb, zb, bias, N, K))
+    assert kernel_of(lambda: ops.gemm_a16w4_fwd(x, codes, sb, zb, bias, N, K)) == "k_skinny_wide"
     assert bool(((y.double() - v - bias.double()).abs() <= (2.0 ** -8 + 2.0 ** -15) * (2 * v.abs() + bias.double().abs()) + 2.0 ** -18 * acc).all())
     act = ops.gemm_a16w4_fwd_silu(x, codes, sb, zb, N // 2, K)
     assert torch.equal(act, ops.silu_mul(ops.gemm_a16w4_fwd(x, codes, sb, zb, None, N, K)))
@@ -352,7 +352,7 @@ def test_a16w4_nine_to_sixteen_tokens_of_a_large_projection(ops, kernels_of, M, 
 
 @pytest.mark.parametrize("M,Hq,Hkv,K", [(9, 16, 4, 4352), (16, 32, 0, 11008), (12, 20, 5, 5632), (13, 19, 0, 4608), (1, 16, 4, 4608), (8, 20, 5, 5632), (3, 64, 0, 8192),
                                         (1, 16, 4, 5632), (10, 64, 0, 6144), (5, 40, 0, 12288)])
-def test_a16w4_decode_projection_over_a_long_contraction(ops, kernels_of, M, Hq, Hkv, K):
+def test_a16w4_decode_projection_over_a_long_contraction(ops, kernel_of, M, Hq, Hkv, K):
     """Up to 16 tokens, K > 4096 in steps of 256 that the warps of a CTA share unevenly (17, 43, 22, 18, 32, 24 and 48 steps), two row blocks of 16 per CTA.  Against 64 bits: two
     roundings to bf16 (2^-8 each, as above), and group sums of (q - z) x, at most 15 sum |x|, in at most 32 roundings or truncations of 2^-23, K / 128
     more where they are added up.  The fused epilogues give the bits of the separate launches."""
@@ -368,7 +368,8 @@ def test_a16w4_decode_projection_over_a_long_contraction(ops, kernels_of, M, Hq,
     acc = 15 * x.double().abs().view(M, K // 128, 128).sum(2) @ s.view(N, K // 128).abs().t()
     y = ops.gemm_a16w4_fwd(x, codes, sb, zb, bias, N, K)
     assert bool(((y.double() - v - bias.double()).abs() <= (2.0 ** -8 + 2.0 ** -15) * (2 * v.abs() + bias.double().abs()) + (32 + K // 128) * 2.0 ** -23 * acc).all())
-    assert ("k_skinny_rows2" in kernels_of(lambda: ops.gemm_a16w4_fwd(x, codes, sb, zb, bias, N, K))) == ((M, K) != (1, 4608))      # (18 steps for 12 warps)
+    ran = kernel_of(lambda: ops.gemm_a16w4_fwd(x, codes, sb, zb, bias, N, K))
+    assert ran == ("k_skinny_rows2" if (M, K) != (1, 4608) else "k_skinny_rows")                       # (18 steps for 12 warps)
     plain = ops.gemm_a16w4_fwd(x, codes, sb, zb, None, N, K)
     assert torch.equal(ops.gemm_a16w4_fwd_silu(x, codes, sb, zb, N // 2, K), ops.silu_mul(plain))
     if Hkv:
@@ -385,7 +386,7 @@ def test_a16w4_decode_projection_over_a_long_contraction(ops, kernels_of, M, Hq,
                                             (16, 512, 5120, True), (9, 300, 8192, True), (9, 300, 10240, False), (8, 256, 4608, False), (1, 256, 5376, True),
                                             (8, 256, 6912, False), (8, 256, 10240, True), (8, 256, 11008, False), (3, 300, 8192, False), (3, 444, 8192, True),
                                             (8, 300, 12288, True), (3, 512, 5632, False), (16, 296, 4096, False)])
-def test_a16w4_two_row_blocks_per_cta_where_they_are_faster(ops, kernels_of, M, blocks, K, two):
+def test_a16w4_two_row_blocks_per_cta_where_they_are_faster(ops, kernel_of, M, blocks, K, two):
     """Both sides of each line of the rule, on 148 SMs: more row blocks than SMs, rounds of CTAs that leave SMs idle, steps that leave warps idle, contractions with
     a written-out loop.  Either kernel's result against the dequantized weight."""
     if torch.cuda.get_device_properties(0).multi_processor_count != 148:
@@ -394,8 +395,8 @@ def test_a16w4_two_row_blocks_per_cta_where_they_are_faster(ops, kernels_of, M, 
     codes, sb, zb = make_w4_layer(ops, N, K, seed=23)
     x = torch.randn(M, K, device="cuda", generator=torch.Generator(device="cuda").manual_seed(M)).to(torch.bfloat16)
     out = []
-    names = kernels_of(lambda: out.append(ops.gemm_a16w4_fwd(x, codes, sb, zb, None, N, K)))
-    assert "k_skinny_" in names and ("k_skinny_rows2" in names) == two
+    ran = kernel_of(lambda: out.append(ops.gemm_a16w4_fwd(x, codes, sb, zb, None, N, K)))
+    assert ran == ("k_skinny_rows2" if two else "k_skinny_rows")
     e_max, e_fro = rel_err(out[0], x.float() @ ops.a16w4_dequant(codes, sb, zb, (N, K), torch.bfloat16).float().t())
     assert e_max < RTOL and e_fro < RTOL
 
@@ -404,7 +405,7 @@ def test_a16w4_two_row_blocks_per_cta_where_they_are_faster(ops, kernels_of, M, 
 @pytest.mark.parametrize("M,N,force_stream", [(1, 4096, True), (2, 12288, True), (1, 1088, True), (12, 4160, True),
                                               (5, 4096, False), (16, 12288, False), (9, 1088, False), (3, 4160, False),
                                               (12, 2304, True), (16, 2368, False)])
-def test_a16w4_decode_kernels_written_out_loop_equals_general_loop(ops, monkeypatch, kernels_of, M, N, force_stream, K):
+def test_a16w4_decode_kernels_written_out_loop_equals_general_loop(ops, monkeypatch, kernel_of, M, N, force_stream, K):
     """K = 4096 with groups of 128 runs the decode kernels' written-out loops (four chunks per warp, group parameters
     as 8-byte loads, constant offsets): the streaming kernel (one or two tokens, or forced) and the row-block kernel.
     Same operations in the same order as the general loops: identical bits, with bias, for more and for fewer row
@@ -417,7 +418,7 @@ def test_a16w4_decode_kernels_written_out_loop_equals_general_loop(ops, monkeypa
     bias = (torch.randn(N, device="cuda", generator=g) * 0.1).to(torch.bfloat16)
     if force_stream:
         monkeypatch.setenv("LQ_SKINNY_STREAM_ALL", "1")         # (M = 12 takes the streaming kernel only when forced)
-    out, ran = {}, {}
+    out = {}
     for mode in ("written_out", "general"):
         if mode == "general":
             monkeypatch.setenv("LQ_SKINNY_NO_NC4", "1")
@@ -427,8 +428,8 @@ def test_a16w4_decode_kernels_written_out_loop_equals_general_loop(ops, monkeypa
         y = ops.gemm_a16w4_fwd(x, codes, sb, zb, bias, N, K)
         act = ops.gemm_a16w4_fwd_silu(x, codes, sb, zb, N // 2, K, hf_rounding=1) if N % 16 == 0 else None
         out[mode] = (y, act)
-        ran[mode] = kernels_of(lambda: ops.gemm_a16w4_fwd(x, codes, sb, zb, bias, N, K))
-    assert "k_skinny_" in ran["general"] and (ran["general"] != ran["written_out"]) == (K == 4096 or M <= 8 or N <= 2368)
+        ran = kernel_of(lambda: ops.gemm_a16w4_fwd(x, codes, sb, zb, bias, N, K))
+        assert (ran == "k_skinny_rows2") == (K == 11008 and M > 8 and N > 2368)
     assert torch.equal(out["written_out"][0], out["general"][0])
     if out["general"][1] is not None:
         assert torch.equal(out["written_out"][1], out["general"][1])
