@@ -8,6 +8,7 @@ device buffers that the captured step itself advances, so a replay needs no host
 """
 from __future__ import annotations
 
+import functools
 import os
 
 import torch
@@ -17,6 +18,16 @@ from torch.nn.attention import SDPBackend, sdpa_kernel
 _SDPA = [SDPBackend.FLASH_ATTENTION, SDPBackend.EFFICIENT_ATTENTION, SDPBackend.MATH]
 
 _PROJECTIONS = (("self_attn", ("q_proj", "k_proj", "v_proj")), ("mlp", ("gate_proj", "up_proj")), ("self_attn", ("o_proj",)), ("mlp", ("down_proj",)))
+
+
+@functools.cache
+def _classes():
+    """What a prompt's route is decided by (looked up once: an import statement in a function costs microseconds in every call)."""
+    from torch.nn.modules import module as nn_module
+    from transformers.activations import ACT2FN
+    from transformers.models.llama import modeling_llama as hf
+    from .quant import QLinearA16W4
+    return hf, type(ACT2FN["silu"]), QLinearA16W4, (nn_module._global_forward_hooks, nn_module._global_forward_pre_hooks)
 
 
 def _words(t):
@@ -157,13 +168,13 @@ class FusedLlamaGreedyDecoder:
     def _tensors(layer):
         """Codes, scales and zeros of q, k, v, gate, up, o, down and the weights of the two norms, where the model has them now; None unless
         all seven projections are bias-free int4 linears."""
-        from .quant import QLinearA16W4
+        QLinearA16W4 = _classes()[2]
         sub, out = layer._modules, []                     # (a module's __getattr__ costs several times as much, in every call)
         for part, names in _PROJECTIONS:
             own = sub[part]._modules
             for name in names:
                 lin = own[name]
-                if not isinstance(lin, QLinearA16W4) or lin.bias is not None:
+                if not isinstance(lin, QLinearA16W4) or lin._parameters.get("bias") is not None:
                     return None
                 w = lin.weight
                 scales, zeros, _ = w.qparam
@@ -173,7 +184,8 @@ class FusedLlamaGreedyDecoder:
     @staticmethod
     def _flat(now):
         src = [t.detach().reshape(-1) for t in now]
-        return dict(src=src, words=[_words(t) for t in src[:15]], at=[(t.data_ptr(), t.numel()) for t in src], o=tuple(src[15:18]), down=tuple(src[18:21]), ln1=src[21], ln2=src[22])
+        return dict(src=src, words=[_words(t) for t in src[:15]], at=[t.data_ptr() for t in src], sizes=[t.numel() for t in src],
+                    o=tuple(src[15:18]), down=tuple(src[18:21]), ln1=src[21], ln2=src[22])
 
     def _live_ends(self):
         m = self.model
@@ -184,31 +196,29 @@ class FusedLlamaGreedyDecoder:
         """The weights as they are now, for the steps and for a prompt through the kernels: the rows of the fused projections are copied
         anew, in place, where the captured step reads them; a weight that it reads in the model and that has moved since drops it.  (No version or
         address shows that the library's optimizer wrote a weight in place.)  Layers whose projections were replaced by something else stay."""
-        to, frm, moved = [], [], False
+        to, frm, moved, T = [], [], False, torch.Tensor
 
-        def same(now, at):                                # (what lay there is held: no other tensor has its address)
-            return all(t.data_ptr() == p and t.numel() == n and t.is_contiguous() for t, (p, n) in zip(now, at))
+        def same(now, at, sizes):                         # (what lay there is held: no other tensor has its address)
+            return list(map(T.data_ptr, now)) == at and list(map(T.numel, now)) == sizes and all(map(T.is_contiguous, now))
 
         for L, layer in zip(self.layers, self.model.model.layers):
             now = self._tensors(layer)
             if now is None:
                 continue
-            if not same(now, L["at"]):
+            if not same(now, L["at"], L["sizes"]):
                 if any(t.numel() != h.numel() or t.dtype != h.dtype for t, h in zip(now, L["src"])):
                     continue
-                moved |= not same(now[15:], L["at"][15:])
+                moved |= not same(now[15:], L["at"][15:], L["sizes"][15:])
                 L.update(self._flat(now))
             to += L["rows"]; frm += L["words"]
         ends = self._live_ends()
-        if any(t.data_ptr() != h.data_ptr() or t.stride() != h.stride() for t, h in zip(ends, self.ends)):
+        if any(t.data_ptr() != h.data_ptr() or t.shape != h.shape or t.stride() != h.stride() for t, h in zip(ends, self.ends)):
             moved, self.ends = True, ends
-        if to and all(t.dtype == torch.int64 for t in to + frm):
+        if to and {t.dtype for t in to + frm} == {torch.int64}:
             torch._foreach_copy_(to, frm)                 # two layers of 4096 x 11008: 53 us, 168 in bytes and bf16, 149 as copies one by one
         else:
             for d, t in zip(to, frm):
                 d.view(torch.uint8).copy_(t.view(torch.uint8))
-        if self.prompt_kernels:                           # (else they may belong to the length of the last prompt)
-            self.inv_freq.copy_(self.model.model.rotary_emb.inv_freq)
         if moved:
             self.graph = None
 
@@ -216,10 +226,7 @@ class FusedLlamaGreedyDecoder:
         """What the step's kernels compute is what the modules compute for a prompt, to rounding, and nothing watches the modules: the
         Llama classes themselves with their forwards untouched, torch's attention, silu, bf16, no autocast, frequencies that do not depend
         on the length of a prompt and need no scaling of the attention, keys kept for the whole length."""
-        from torch.nn.modules import module as nn_module
-        from transformers.activations import ACT2FN
-        from transformers.models.llama import modeling_llama as hf
-        from .quant import QLinearA16W4
+        hf, silu, QLinearA16W4, global_hooks = _classes()
 
         def own(mod, cls):                                # of the class itself, its forward neither replaced nor watched
             d = mod.__dict__
@@ -228,7 +235,7 @@ class FusedLlamaGreedyDecoder:
         def norm(mod):
             return own(mod, hf.LlamaRMSNorm) and mod.variance_epsilon == self.eps and mod.weight.dtype == bf
 
-        bf, silu, scaling = torch.bfloat16, type(ACT2FN["silu"]), self.hd ** -0.5
+        bf, scaling = torch.bfloat16, self.hd ** -0.5
         model = self.model
         if not own(model, hf.LlamaForCausalLM) or not own(model.model, hf.LlamaModel):
             return False
@@ -240,7 +247,7 @@ class FusedLlamaGreedyDecoder:
                     and own(sub["mlp"]._modules["act_fn"], silu) and norm(sub["input_layernorm"]) and norm(sub["post_attention_layernorm"])
                     and all(own(sub[part]._modules[name], QLinearA16W4) for part, names in _PROJECTIONS for name in names)):
                 return False
-        if nn_module._global_forward_hooks or nn_module._global_forward_pre_hooks or torch.is_autocast_enabled(self.device.type):
+        if any(global_hooks) or torch.is_autocast_enabled(self.device.type):
             return False
         return (own(emb, torch.nn.Embedding) and own(rope, hf.LlamaRotaryEmbedding) and own(head, torch.nn.Linear) and norm(inner.norm)
                 and len(inner.layers) == cfg.num_hidden_layers == len(self.layers) and cfg._attn_implementation == "sdpa"
@@ -357,8 +364,10 @@ class FusedLlamaGreedyDecoder:
         if b != self.batch or p + max_new_tokens > self.max_len:
             raise ValueError("prompt does not fit the decoder's batch size / cache length")
         self.model.eval()
+        self._take_weights()                                # (its copies run while the host looks at the modules)
         self.prompt_kernels = self._kernels_serve_prompts()
-        self._take_weights()
+        if self.prompt_kernels:                             # (else they may belong to the length of the last prompt)
+            self.inv_freq.copy_(self.model.model.rotary_emb.inv_freq)
         if use_graph and self.graph is None:
             self._capture(self._prefill(prompt), p)         # throw-away prefill: capture needs an allocated cache and tokens to start from
         first = self._prefill(prompt)

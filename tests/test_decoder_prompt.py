@@ -111,7 +111,7 @@ def _fresh_equals(dec, model):
         for name in ("qkv", "gu", "o", "down"):
             assert all(torch.equal(a, b) for a, b in zip(L[name], N[name])), name
         assert torch.equal(L["ln1"], N["ln1"]) and torch.equal(L["ln2"], N["ln2"])
-    assert all(torch.equal(a, b) for a, b in zip(dec.ends, new.ends)) and torch.equal(dec.inv_freq, new.inv_freq)
+    assert all(torch.equal(a, b) for a, b in zip(dec.ends, new.ends))
 
 
 def test_a_call_takes_the_weights_as_they_are():
@@ -125,7 +125,6 @@ def test_a_call_takes_the_weights_as_they_are():
             lin.weight.data.copy_(torch.randint(-128, 128, lin.weight.data.shape, generator=g, dtype=torch.int64))
             lin.scales.data.add_(1)
         layer.input_layernorm.weight.data.mul_(0.5)
-    model.model.rotary_emb.inv_freq.mul_(0.5)
     dec._take_weights()
     _fresh_equals(dec, model)
     assert dec.graph is captured and held == [L[name][i].data_ptr() for L in dec.layers for name in ("qkv", "gu") for i in range(3)]
@@ -172,8 +171,11 @@ def test_a_prompt_sees_the_present_weights_and_route(monkeypatch):
         model.model.layers[0].self_attn.q_proj.weight.data.fill_(value)
         dec.generate(prompt, 1, use_graph=False)
     assert seen == [("kernels", 3), ("kernels", 4)]
+    model.model.rotary_emb.inv_freq.mul_(0.5)
+    dec.generate(prompt, 1, use_graph=False)
+    assert torch.equal(dec.inv_freq, model.model.rotary_emb.inv_freq.float())
     fired = []
     model.model.embed_tokens.register_forward_hook(lambda *a: (fired.append(1), 1 / 0))
     with pytest.raises(ZeroDivisionError):                 # through the modules, whose kernels need a GPU: as far as the first hook
         dec.generate(prompt, 1, use_graph=False)
-    assert fired and len(seen) == 2
+    assert fired and len(seen) == 3
