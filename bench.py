@@ -595,7 +595,7 @@ def finetune_measurement(torch, arch="opt-1.3b", steps=10, warmup=2, micro_batch
         res["greedy_decode"] = dec
         res["greedy_decode_note"] = ("512-token random prompts; hf_generate = the reference's route (eager loop, host-bound); "
                                      "graphed = decode step of the eager modules captured as one CUDA graph on a static KV cache; "
-                                     "fused = decode step as nine library kernels per layer, one CUDA graph")
+                                     "fused = decode step as five (one or two sequences), seven (up to 16) or nine library kernels per layer, one CUDA graph")
     del tuner, opt, model
     torch.cuda.empty_cache()
     return res

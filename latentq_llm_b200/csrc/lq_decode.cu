@@ -608,7 +608,8 @@ k_argmax_embed_cluster(const __nv_bfloat16* __restrict__ logits, int64_t logits_
 // 32000 rows open at a time, 64 bytes each: 4.95 TB/s.)  A lane loads 16 bytes of its two rows per 32 k, a block of rows ahead of the arithmetic (128 KB in
 // flight per SM at K = 4096); they are the A fragments of two mma.sync as they lie, the tokens' 16 bytes at the same k the B fragments, because a contraction
 // does not care which k meet in which lane.  32000 x 4096 in a chain: 38.7 us for one or two tokens (6.78 TB/s), 39.9 for eight, against 45 .. 47 of the
-// library and a launch gap before it; 50272 x 2048 31.4 / 36.  (With two groups of tokens 16 tokens took 45.0 / 44.3: the library's.)
+// library and a launch gap before it; K = 2048, 1 / 3 / 8 tokens: 32000 rows 20.7 / 21.3 / 21.3 against 23.0 / 23.2 / 24.0, 50272 rows 31.2 / 32.0 / 32.2 against 36.2 / 36.7 / 37.0.  (With two
+// groups of tokens 16 tokens took 45.0 / 44.3: the library's.)
 // ---------------------------------------------------------------------------------------------
 constexpr int LR_WARPS = 16;
 __device__ __forceinline__ void lr_mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {

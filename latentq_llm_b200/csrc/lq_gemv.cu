@@ -867,9 +867,9 @@ __global__ void __launch_bounds__(RB_WARPS * 32, MT == 2 ? 1 : LQ_GEMV_MINB) k_s
 // Twice the MMAs of eight tokens and four passes of the shared-memory path for each token fragment bound it, and the latencies of eight warps in between: a
 // fragment is therefore read once for two row blocks, and the MMAs of a group form one chain per row block and eight tokens, eight independent chains a
 // warp, with no sum of two chains behind them.  What it may not do is spill: a spilled weight that is still in flight is waited for, which undoes the
-// prefetch of a whole step (measured, gate|up at 16 tokens: 16 warps with 100 bytes of spills 29.5 us, without spills but one row block 19.1, this form 17.9).
-// 16 tokens, launches in a chain, one row block per step and two chains before: q|k|v (12288 rows) 14.9 -> 12.5 us, gate|up (22016 rows) 20.9 -> 17.9;
-// 9 tokens, q|k|v 13.6 -> 11.7.
+// prefetch of a whole step (measured, gate|up at 16 tokens: 16 warps with 100 bytes of spills 29.5 us, without spills but one row block 19.1).
+// Launches in a chain, weights from HBM, one row block per step and two chains before: 16 tokens q|k|v (12288 rows) 15.4 -> 13.3 us, gate|up (22016 rows)
+// 22.5 -> 19.2; 9 tokens 14.3 -> 12.5 and 21.2 -> 18.7.
 // ---------------------------------------------------------------------------------------------
 constexpr int SW_XS = 4096 / 8 + 4;           // vectors per staged token: 64 bytes apart modulo 128, two tokens by a quarter warp without conflicts
 __global__ void __launch_bounds__(RB_WARPS * 32, 1) k_skinny_wide(const SkinnyParams p) {
@@ -1067,8 +1067,8 @@ static int launch_skinny_wide(const SkinnyParams& p, cudaStream_t st) {
 // 352 KB, which every CTA reads through an L1 that delivers 64 bytes a cycle, so half as many CTAs halve them.  The rest is sized to what 168
 // registers per thread hold without a spill (a spilled weight in flight is waited for): one accumulator chain per row block and eight tokens, 32-bit offsets
 // in place of pointers, one step of weights and group parameters (a load of two groups each) ahead.
-// 11008 -> 4096 in a chain, 9 / 16 tokens: 12.5 / 13.4 -> 11.6 / 12.2 us, 5632 -> 4096 7.8 / 8.3 -> 7.0 / 7.35.  With 8, 11, 15 and 16 warps 12.8 / 13.3, 11.6 / 12.0 (5632: the
-// same; spills), 12.6 / 12.9, 12.7 / 13.0.
+// 11008 -> 4096 in a chain, weights from HBM, 9 / 16 tokens: 13.0 / 13.9 -> 12.1 / 12.7 us, 5632 -> 4096 8.0 / 8.5 -> 7.3 / 7.6, 14336 -> 3840 17.4 / 18.6 -> 14.6 / 15.4.  With 8, 11, 15 and 16
+// warps instead of twelve 11008 -> 4096 takes 8 % more, 1 % less (but spills, and 5632 gains nothing), 7 % and 8 % more.
 // ---------------------------------------------------------------------------------------------
 constexpr int R2_WARPS = 12;
 template <int MT>

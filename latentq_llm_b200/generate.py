@@ -110,8 +110,8 @@ class FusedLlamaGreedyDecoder:
                     residual add + RMSNorm -> fused gate|up projection (N = 2 I) -> silu(gate) * up -> down projection
         then        residual add + final RMSNorm -> lm_head -> argmax -> embedding of the new token
 
-    eight launches per layer at decode-sized batches, where silu(gate) * up is the epilogue of the gate|up launch, nine
-    otherwise (the reference's fusion list: PTQ/quant/fused_attn.py:164-204 fused QKV, :8-58 RoPE,
+    five launches per layer for one or two sequences at hidden size 4096 (both norms, RoPE with the cache write and silu * up inside the
+    projections' launches), seven up to 16 sequences, nine otherwise (the reference's fusion list: PTQ/quant/fused_attn.py:164-204 fused QKV, :8-58 RoPE,
     PTQ/quant/fused_mlp.py:84-168 gate/up with the silu epilogue, PTQ/quant/triton_norm.py:7-39 RMSNorm), captured
     once as a CUDA graph and replayed per token.  The prompt goes through the same kernels at its own token count (fused
     q|k|v and gate|up GEMMs, SDPA for its attention) into the same static KV cache, and only its last tokens through the
